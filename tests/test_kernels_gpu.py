@@ -94,6 +94,34 @@ def test_gemm_simt_float32_is_true_32bit(ops, M, N, K):
     assert err / scale < 2e-6 * math.sqrt(K) + 1e-6, (err, scale)
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 8, 9, 16, 17, 33, 64, 65, 129, 300])
+@pytest.mark.parametrize("N,K", [(1, 4), (127, 60), (130, 132), (260, 1028), (1024, 2048), (20000, 256)])
+def test_gemm_f32_at_the_edges_of_its_tiles(ops, M, N, K):
+    x, w = rand((M, K), torch.float32, 21), rand((N, K), torch.float32, 22)
+    x[:, ::3] *= 1e-3                                   # products of very different sizes
+    got = ops.gemm_simt(x, w, torch.float32)
+    want = x.double() @ w.double().t()
+    # any order of K rounded 32-bit additions stays below K 2^-24 of the sum of the products' sizes; parts of products that
+    # are left out (three, below 2^-23 each) and the last additions add a few units
+    bound = (K + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert ((got.double() - want).abs() <= bound).all()
+    # and rounding errors do not line up: one multiply-add after the other measures 8.1e-7 at K = 2,048
+    assert ((got.double() - want).norm() / want.norm()).item() < 8e-7
+    ops.check_status()
+
+
+@pytest.mark.parametrize("M", [4, 12, 70])
+def test_gemm_f32_with_numbers_that_are_not_finite(ops, M):
+    x, w = rand((M, 512), torch.float32, 23), rand((300, 512), torch.float32, 24)
+    x[1, 5], x[2, 7], w[17, 9], x[3, 11], w[:, 13] = float("inf"), float("nan"), -float("inf"), 1e-42, 0.0
+    x[0, 13] = 3.4028234e38                             # the largest number, against zeros
+    got = ops.gemm_simt(x, w, torch.float32).double()
+    want = x.double() @ w.double().t()
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+    fine = torch.isfinite(want)
+    assert torch.isfinite(got[fine]).all() and ((got - want)[fine].norm() / want[fine].norm()).item() < 8e-7
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1000, 96), (7, 65, 17), (33, 130, 200)])
 @pytest.mark.parametrize("out_dtype", DTYPES)
 def test_gemm_simt_bfloat16_operands(ops, M, N, K, out_dtype):

@@ -1,0 +1,528 @@
+// C[M, N] = A[M, K] . W[N, K]^T, everything float32: the projections of the true 32-bit path.  Both operands are K-major as
+// stored and 16-byte aligned with K % 4 == 0 (gemm_simt.cu takes the rest).  Two kernels; relative errors (2-norm, against
+// 64 bits, K = 2,048 / 8,192) beside those of plain multiply-adds one after the other along K (gemm_simt.cu: 8.1e-7 / 1.6e-6).
+//
+// few rows (M <= 8, decode steps): bound by reading W once from HBM.  A warp owns four rows of W and a part of K; its lanes
+//   lie along K, 16 bytes each, with four 2 KB pieces of W in flight per warp (16 warps an SM: 128 KB, about twice what
+//   6.5 TB/s times the latency needs).  The sums over a warp's lanes are taken at the end by a transposing butterfly, those
+//   over the warps that share rows through shared memory, in a fixed order.  Error 1.0e-7 to 1.6e-7.
+//   4 rows against [16384, 2048] 29.5 us (4.6 TB/s), [2048, 8192] 16.5, [128256, 2048] 192 (5.5 TB/s); 210, 557 and 1,161 us
+//   before, when a 64 x 64 tile per CTA walked K alone.  (At 8 rows it is still ahead of the other kernel: 9.1 against 12.6 us
+//   for [2048, 2048], even for the head.)
+//
+// more rows: bound by arithmetic, and the CUDA cores' multiply-adds give 75 TFLOP/s at most (64 x 128 register tiles: 28 to 45
+//   measured).  So each number is cut into three bfloat16 whose sum it is exactly (8 + 8 + 8 bits), and the tensor cores
+//   multiply the parts: six of the nine products, the three that are left out being below 2^-23 of the whole each.  The leading
+//   products are added up in tensor memory over 128 positions of K only and then in registers, rounded to nearest; the small
+//   ones have an accumulator of their own.  Error 1.8e-7 to 4.6e-7.  Eight warps fetch both operands, cut them and
+//   store the parts as tiles of 128-byte-swizzled shared memory, while one warp issues the products of the stage before; the
+//   same eight drain the accumulators.  Tiles that are too few for 148 SMs are cut along K over a cluster of up to eight CTAs
+//   that add up through distributed shared memory.  Numbers that are not finite have no such parts: a CTA that meets one takes
+//   its sums again with plain multiply-adds.
+//   300 rows against [16384, 2048] 201 us (100 TFLOP/s), [2048, 8192] 128, [128256, 2048] 1,390; 866, 828 and 6,397 us before.
+//
+// In both, the order in which a row's products are added depends on the shapes, never on the other rows' contents.
+#include "common.cuh"
+
+namespace {
+
+constexpr int kSMs = 148;
+
+// ---------------------------------------------------------------------------------------------- few rows
+constexpr int RV = 4;            // rows of W per warp
+constexpr int WARPS = 8;
+
+__device__ __forceinline__ float4 load_stream(const float* p) {
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
+// lane i of the warp gets the sum over all lanes of v[i % N] (N a power of two up to 32): halves of the values change
+// lanes at every step, so N values cost about N shuffles
+template <int N>
+__device__ __forceinline__ float transposed_sum(float (&v)[N]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = N / 2; o >= 1; o >>= 1) {
+        const bool upper = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            if (i < o) {
+                const float give = upper ? v[i] : v[i + o], keep = upper ? v[i + o] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+    }
+    float s = v[0];
+#pragma unroll
+    for (int o = N; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// DEPTH: pieces of 128 K positions in flight per warp
+template <int MT, int DEPTH>
+__global__ void __launch_bounds__(WARPS * 32, 2) gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
+                                                                      int M, int N, int K, int ksplit) {
+    __shared__ float part[WARPS][MT * RV];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int group = blockIdx.x * (WARPS / ksplit) + warp / ksplit, ks = warp % ksplit;
+    const int n0 = group * RV;
+    const int pieces = (K + 127) >> 7;
+    const float* w[RV];
+#pragma unroll
+    for (int r = 0; r < RV; ++r) w[r] = W + (size_t)min(n0 + r, N - 1) * K + lane * 4;
+    const bool live = n0 < N;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 buf[DEPTH][RV];
+    auto fetch = [&](int d, int piece) {
+        const bool in = live && piece < pieces && piece * 128 + lane * 4 < K;
+#pragma unroll
+        for (int r = 0; r < RV; ++r) buf[d][r] = in ? load_stream(w[r] + (size_t)piece * 128) : zero;
+    };
+    // (W is nobody's output: its first pieces travel while the kernel before this one ends)
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) fetch(d, ks + d * ksplit);
+    grid_dependency_wait();
+    grid_launch_dependents();
+    float acc[MT * RV];
+#pragma unroll
+    for (int i = 0; i < MT * RV; ++i) acc[i] = 0.f;
+    const float* a = A + lane * 4;
+    for (int p0 = ks; p0 < pieces; p0 += DEPTH * ksplit) {
+#pragma unroll
+        for (int d = 0; d < DEPTH; ++d) {
+            const int piece = p0 + d * ksplit;
+            if (piece < pieces) {
+                const bool in = piece * 128 + lane * 4 < K;
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const float4 x = in ? *reinterpret_cast<const float4*>(a + (size_t)min(m, M - 1) * K + (size_t)piece * 128) : zero;
+#pragma unroll
+                    for (int r = 0; r < RV; ++r) {
+                        float& s = acc[m * RV + r];
+                        s = fmaf(x.x, buf[d][r].x, s);
+                        s = fmaf(x.y, buf[d][r].y, s);
+                        s = fmaf(x.z, buf[d][r].z, s);
+                        s = fmaf(x.w, buf[d][r].w, s);
+                    }
+                }
+                fetch(d, piece + DEPTH * ksplit);
+            }
+        }
+    }
+    const float sum = transposed_sum<MT * RV>(acc);
+    if (lane < MT * RV) part[warp][lane] = sum;
+    __syncthreads();
+    if (ks == 0 && live && lane < MT * RV) {
+        float s = part[warp][lane];
+        for (int q = 1; q < ksplit; ++q) s += part[warp + q][lane];
+        const int m = lane / RV, n = n0 + lane % RV;
+        if (m < M && n < N) C[(size_t)m * N + n] = s;
+    }
+}
+
+template <int MT>
+int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, cudaStream_t s) {
+    // as many warps as keep every SM's memory pipeline full, but at least two pieces of K each
+    const int groups = (N + RV - 1) / RV, pieces = (K + 127) / 128;
+    int ksplit = 1;
+    while (ksplit < WARPS && groups * ksplit < kSMs * 16 && pieces >= 4 * ksplit) ksplit *= 2;
+    const int per = WARPS / ksplit;
+    const cudaError_t e = tl_launch(gemm_f32_rows_kernel<MT, MT <= 4 ? 4 : 3>, dim3((groups + per - 1) / per), dim3(WARPS * 32), 0, s, A, W, C, M, N, K, ksplit);
+    return e == cudaSuccess ? TL_OK : (int)e;
+}
+
+// ---------------------------------------------------------------------------------------------- more rows
+constexpr int BP = 128;                    // rows of W per CTA: the 128 rows of a tcgen05.mma
+constexpr int BK = 64;                     // K per stage: 64 bfloat16, one 128-byte swizzle row
+constexpr int CHUNK = 2;                   // stages whose leading products are added up in tensor memory
+constexpr int CONVERTERS = 8;              // warps
+constexpr int THREADS = (CONVERTERS + 1) * 32;
+constexpr unsigned long long WAIT_LIMIT_NS = 2000ull * 1000ull * 1000ull;
+enum : int { ERR_STAGE_WAIT = 121, ERR_MMA_WAIT = 122, ERR_SUM_WAIT = 123 };
+
+__device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// by a whole warp: false (for all its lanes) once the limit has passed or another role has given up
+__device__ __forceinline__ bool warp_wait(unsigned long long* bar, unsigned parity, volatile int* abort_flag) {
+    bool ok = mbar_try_wait(bar, parity);
+    if (!ok) {
+        const unsigned long long t0 = global_ns();
+        for (unsigned i = 1; !ok; ++i) {
+            ok = mbar_try_wait(bar, parity);
+            if (!ok && (i & 255u) == 0u && (*abort_flag || global_ns() - t0 > WAIT_LIMIT_NS)) break;
+        }
+    }
+    return __all_sync(0xffffffffu, ok);
+}
+
+// shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024 bytes apart
+__device__ __forceinline__ unsigned long long umma_desc(unsigned addr) {
+    return (unsigned long long)((addr & 0x3FFFFu) >> 4) | (unsigned long long)(1024u >> 4) << 32 | (unsigned long long)1u << 46 | (unsigned long long)2u << 61;
+}
+// both for a whole warp in step, of which one elected lane issues
+__device__ __forceinline__ void umma_bf16(unsigned tmem_d, unsigned long long a_desc, unsigned long long b_desc, unsigned idesc, bool accumulate) {
+    asm volatile("{\n\t.reg .pred p, e;\n\telect.sync _|e, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((unsigned)accumulate) : "memory");
+}
+__device__ __forceinline__ void umma_commit(unsigned long long* bar) {
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+                 "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)) : "memory");
+}
+// eight columns of this thread's lane of tensor memory
+__device__ __forceinline__ void tmem_load8(unsigned addr, unsigned (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(addr));
+}
+
+// Four numbers as three bfloat16 each, by truncation: v == hi + mid + lo exactly (8 + 8 + 8 bits of significand).  `sick`
+// becomes NaN where a number is not finite (its remainder is then NaN).
+struct Parts { uint2 hi, mid, lo; };
+__device__ __forceinline__ Parts split4(const float4& v, float& sick) {
+    unsigned h[4], m[4], l[4];
+    const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        h[e] = __float_as_uint(x[e]) & 0xffff0000u;
+        const float r = x[e] - __uint_as_float(h[e]);
+        m[e] = __float_as_uint(r) & 0xffff0000u;
+        const float t = r - __uint_as_float(m[e]);
+        l[e] = __float_as_uint(t);
+        sick = fmaf(t, 0.f, sick);
+    }
+    Parts p;
+    p.hi = make_uint2(__byte_perm(h[0], h[1], 0x7632), __byte_perm(h[2], h[3], 0x7632));
+    p.mid = make_uint2(__byte_perm(m[0], m[1], 0x7632), __byte_perm(m[2], m[3], 0x7632));
+    p.lo = make_uint2(__byte_perm(l[0], l[1], 0x7632), __byte_perm(l[2], l[3], 0x7632));
+    return p;
+}
+
+// BQ: tokens per CTA at most (the launch says how many, a multiple of 16); AHEAD: stages of both operands in registers
+template <int BQ, int AHEAD>
+struct Shape {
+    static constexpr unsigned W_PART = BP * BK * 2, A_PART = BQ * BK * 2, STAGE = 3 * (W_PART + A_PART);
+    static constexpr unsigned SUMS = BQ * BP * 4;
+    static constexpr unsigned SMEM = (2 * STAGE > SUMS ? 2 * STAGE : SUMS) + 1024;
+    static constexpr unsigned COLS = BQ == 128 ? 512 : BQ == 64 ? 256 : BQ == 32 ? 128 : 64;      // three accumulators, a power of two
+};
+
+template <int BQ, int AHEAD>
+__global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
+                                                                    int* status, int M, int N, int K, int bq, int token_tiles, int ksplit) {
+    using S = Shape<BQ, AHEAD>;
+    constexpr int WL = BP / 16, AL = BQ / 16, HALF = BQ / 2;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
+    __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2], sum_full[2], sum_empty[2];
+    __shared__ unsigned tmem_slot;
+    __shared__ int abort_flag, sick_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = blockIdx.x % ksplit, tile = blockIdx.x / ksplit;
+    const int m0 = (tile % token_tiles) * bq, n0 = (tile / token_tiles) * BP;      // the tiles that read a slab of W follow one another
+    const int blocks_all = (K + BK - 1) / BK;
+    const int first = (int)((long long)blocks_all * rank / ksplit), blocks = (int)((long long)blocks_all * (rank + 1) / ksplit) - first;
+    const int chunks = (blocks + CHUNK - 1) / CHUNK;
+    volatile int* aborted = &abort_flag;
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        sick_flag = 0;
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&full_bar[s], CONVERTERS);
+            mbar_init(&empty_bar[s], 1);
+            mbar_init(&sum_full[s], 1);
+            mbar_init(&sum_empty[s], CONVERTERS);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == CONVERTERS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(S::COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const unsigned tmem = tmem_slot;
+    float acc[HALF];
+#pragma unroll
+    for (int j = 0; j < HALF; ++j) acc[j] = 0.f;
+    bool ok = true;
+    const int quarter = warp & 3, half = warp >> 2;                        // a converter's share of the accumulators
+    const unsigned lanes = (unsigned)(quarter * 32) << 16;
+
+    if (warp < CONVERTERS) {
+        // rows warp * 2 + lane / 16 + 16 i of both tiles, 16 bytes at lane % 16 along K
+        const int r0 = warp * 2 + (lane >> 4), kl = (lane & 15) * 4;
+        const float *wp = W + (size_t)(n0 + r0) * K + kl, *ap = A + (size_t)(m0 + r0) * K + kl;
+        const int w_rows = N - n0 - r0, a_rows = min(M - m0, bq) - r0;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 wb[AHEAD][WL], ab[AHEAD][AL];
+        auto w_at = [&](int i, int b) {
+            const int k = (first + b) * BK;
+            return (b < blocks && 16 * i < w_rows && k + kl < K) ? load_stream(wp + (size_t)(16 * i) * K + k) : zero;
+        };
+        auto a_at = [&](int i, int b) {
+            const int k = (first + b) * BK;
+            return (b < blocks && 16 * i < a_rows && k + kl < K) ? *reinterpret_cast<const float4*>(ap + (size_t)(16 * i) * K + k) : zero;
+        };
+#pragma unroll
+        for (int d = 0; d < AHEAD; ++d)
+#pragma unroll
+            for (int i = 0; i < WL; ++i) wb[d][i] = w_at(i, d);
+        grid_dependency_wait();
+        grid_launch_dependents();
+#pragma unroll
+        for (int d = 0; d < AHEAD; ++d)
+#pragma unroll
+            for (int i = 0; i < AL; ++i) ab[d][i] = a_at(i, d);
+        unsigned char* put = tiles + r0 * 128 + ((((lane & 15) >> 1) ^ (r0 & 7)) << 4) + (lane & 1) * 8;
+        float sick = 0.f;
+        int drained = 0;
+        auto drain = [&]() {
+            const int c = drained++;
+            ok = ok && warp_wait(&sum_full[c & 1], (c >> 1) & 1, aborted);
+            if (!ok) return;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < HALF; j += 8) {
+                unsigned r[8];
+                tmem_load8(tmem + lanes + (unsigned)((c & 1) * BQ + half * HALF + j), r);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(r[e]);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sum_empty[c & 1]);
+        };
+        for (int b0 = 0; b0 < blocks && ok; b0 += AHEAD) {
+#pragma unroll
+            for (int d = 0; d < AHEAD; ++d) {
+                const int b = b0 + d;
+                if (b >= blocks || !ok) break;
+                const int s = b & 1;
+                if (b >= 2) ok = warp_wait(&empty_bar[s], ((b >> 1) - 1) & 1, aborted);
+                if (!ok) break;
+                unsigned char* to = put + s * S::STAGE;
+#pragma unroll
+                for (int i = 0; i < WL; ++i) {
+                    const Parts q = split4(wb[d][i], sick);
+                    *reinterpret_cast<uint2*>(to + i * 2048) = q.hi;
+                    *reinterpret_cast<uint2*>(to + i * 2048 + S::W_PART) = q.mid;
+                    *reinterpret_cast<uint2*>(to + i * 2048 + 2 * S::W_PART) = q.lo;
+                    wb[d][i] = w_at(i, b + AHEAD);
+                }
+#pragma unroll
+                for (int i = 0; i < AL; ++i) {
+                    const Parts q = split4(ab[d][i], sick);
+                    *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART) = q.hi;
+                    *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + S::A_PART) = q.mid;
+                    *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + 2 * S::A_PART) = q.lo;
+                    ab[d][i] = a_at(i, b + AHEAD);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full_bar[s]);
+                if ((b % CHUNK) == CHUNK - 1 && b >= 2 * CHUNK - 1) drain();
+            }
+        }
+        while (ok && drained < chunks) drain();
+        if (ok && blocks > 0) {
+            // the small products, added up over the whole range; the last chunk's signal covers them
+#pragma unroll
+            for (int j = 0; j < HALF; j += 8) {
+                unsigned r[8];
+                tmem_load8(tmem + lanes + (unsigned)(2 * BQ + half * HALF + j), r);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(r[e]);
+            }
+        }
+        if (sick != sick) sick_flag = 1;
+        if (!ok && lane == 0) {
+            abort_flag = 1;
+            atomicExch(status, ERR_SUM_WAIT);
+        }
+    } else {
+        // ---- tensor-core issuer: the whole warp in step, one elected lane issuing
+        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bq >> 3) << 17) | ((unsigned)(BP >> 4) << 24);
+        for (int b = 0; b < blocks; ++b) {
+            const int s = b & 1, c = b / CHUNK;
+            ok = warp_wait(&full_bar[s], (b >> 1) & 1, aborted);
+            if (ok && b % CHUNK == 0 && c >= 2) ok = warp_wait(&sum_empty[c & 1], ((c >> 1) - 1) & 1, aborted);
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const unsigned wt = smem_u32(tiles) + s * S::STAGE, at = wt + 3 * S::W_PART;
+            const unsigned lead = tmem + (unsigned)((c & 1) * BQ), small = tmem + 2 * BQ;
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k) {
+                unsigned long long w[3], a[3];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    w[q] = umma_desc(wt + q * S::W_PART + k * 32);
+                    a[q] = umma_desc(at + q * S::A_PART + k * 32);
+                }
+                umma_bf16(small, w[2], a[0], idesc, b > 0 || k > 0);
+                umma_bf16(small, w[0], a[2], idesc, true);
+                umma_bf16(small, w[1], a[1], idesc, true);
+                umma_bf16(small, w[1], a[0], idesc, true);
+                umma_bf16(small, w[0], a[1], idesc, true);
+                umma_bf16(lead, w[0], a[0], idesc, b % CHUNK > 0 || k > 0);
+            }
+            umma_commit(&empty_bar[s]);
+            if (b % CHUNK == CHUNK - 1 || b == blocks - 1) umma_commit(&sum_full[c & 1]);
+        }
+        if (!ok && lane == 0) {
+            abort_flag = 1;
+            atomicExch(status, ERR_MMA_WAIT);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    const bool good = abort_flag == 0;
+    const int row = quarter * 32 + lane, n = n0 + row;
+    if (good && sick_flag && warp < CONVERTERS) {
+        // An operand is not finite: inf * 0 between its parts would be NaN where the product itself is not.  Once over
+        // with plain multiply-adds (slow; nothing but correctness matters here).
+        const int k1 = min(K, (first + blocks) * BK);
+#pragma unroll 1
+        for (int j = 0; j < HALF; ++j) {
+            const int m = m0 + half * HALF + j;
+            float s = 0.f;
+            if (n < N && m < M && half * HALF + j < bq)
+                for (int k = first * BK; k < k1; ++k) s = fmaf(A[(size_t)m * K + k], W[(size_t)n * K + k], s);
+#pragma unroll
+            for (int e = 0; e < HALF; ++e) if (e == j) acc[e] = s;
+        }
+    }
+    if (ksplit == 1) {
+        if (good && warp < CONVERTERS && n < N) {
+#pragma unroll
+            for (int j = 0; j < HALF; ++j) {
+                const int t = half * HALF + j;
+                if (t < bq && m0 + t < M) C[(size_t)(m0 + t) * N + n] = acc[j];
+            }
+        }
+    } else {
+        // The cluster's CTAs hold sums over their parts of K: each leaves its own in its shared memory (the stages are
+        // done with) and adds up every ksplit-th token's from all, in the order of the parts.  A CTA that gave up takes
+        // part in the barriers and leaves NaN.
+        float* sums = reinterpret_cast<float*>(tiles);                     // [token][row]
+        if (warp < CONVERTERS) {
+#pragma unroll
+            for (int j = 0; j < HALF; ++j) sums[(half * HALF + j) * BP + row] = good ? acc[j] : __int_as_float(0x7fffffff);
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (warp < CONVERTERS && n < N) {
+            for (int t = rank + half * ksplit; t < bq && m0 + t < M; t += 2 * ksplit) {
+                float v[8], s = 0.f;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    if (q < ksplit) {
+                        unsigned there;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_u32(&sums[t * BP + row])), "r"(q));
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[q]) : "r"(there) : "memory");
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 8; ++q) if (q < ksplit) s += v[q];
+                C[(size_t)(m0 + t) * N + n] = s;
+            }
+        }
+        // nobody leaves while another still reads its shared memory
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+    if (warp == CONVERTERS) {
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::COLS) : "memory");
+    }
+}
+
+template <int BQ, int AHEAD>
+int launch_parts(const float* A, const float* W, float* C, int* status, int M, int N, int K, cudaStream_t s) {
+    using S = Shape<BQ, AHEAD>;
+    const int token_tiles = (M + BQ - 1) / BQ;
+    const int bq = ((M + token_tiles - 1) / token_tiles + 15) / 16 * 16;       // tiles of equal size
+    const long long tiles = (long long)token_tiles * ((N + BP - 1) / BP);
+    auto kernel = gemm_f32_parts_kernel<BQ, AHEAD>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = S::SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    cfg.attrs = attr;
+    // how many clusters of q CTAs the GPU holds at a time: fewer than SMs / q, since a cluster stays inside a group of 16 to
+    // 18 SMs.  Asked for once (threads that ask at the same time write the same numbers).
+    static int fit[9];
+    if (fit[1] == 0) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+        cfg.numAttrs = 1;
+        for (int q = 8; q >= 1 && e == cudaSuccess; --q) {
+            cfg.gridDim = dim3(q);
+            attr[0].val.clusterDim.x = q;
+            int n = 0;
+            e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+            fit[q] = n < 1 ? 1 : n;
+        }
+        if (e != cudaSuccess) return (int)e;
+    }
+    // K is cut so that the tiles' parts come in as few and as short rounds as can be; a part has four stages at least
+    const int blocks = (K + BK - 1) / BK;
+    int ksplit = 1;
+    long long best = 1LL << 62;
+    for (int q = 1; q <= 8 && (q == 1 || blocks / q >= 4); ++q) {
+        const long long cost = (tiles + fit[q] - 1) / fit[q] * ((blocks + q - 1) / q + (q > 1 ? 3 : 2));
+        if (cost < best) best = cost, ksplit = q;
+    }
+    if (tiles * ksplit > 0x7fffffffLL) return TL_BAD_SIZE;
+    cfg.gridDim = dim3((unsigned)(tiles * ksplit));
+    attr[0].val.clusterDim.x = ksplit;
+    cfg.numAttrs = 2;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, A, W, C, status, M, N, K, bq, token_tiles, ksplit);
+}
+
+}  // namespace
+
+extern "C" int tl_gemm_f32_supports(const void* A, const void* W, int K) {
+    return K >= 4 && K % 4 == 0 && aligned16(A) && aligned16(W) ? 1 : 0;
+}
+
+// status: one int that is set to a non-zero code if a wait ran out.
+extern "C" int tl_gemm_f32(const void* A, const void* W, void* C, int M, int N, int K, int* status, void* stream) {
+    if (M <= 0 || N <= 0) return TL_OK;
+    if (!tl_gemm_f32_supports(A, W, K) || status == nullptr) return TL_BAD_ALIGN;
+    cudaStream_t s = (cudaStream_t)stream;
+    const float *a = (const float*)A, *w = (const float*)W;
+    float* c = (float*)C;
+    if (M == 1) return launch_rows<1>(a, w, c, M, N, K, s);
+    if (M == 2) return launch_rows<2>(a, w, c, M, N, K, s);
+    if (M <= 4) return launch_rows<4>(a, w, c, M, N, K, s);
+    if (M <= 8) return launch_rows<8>(a, w, c, M, N, K, s);
+    if (M <= 16) return launch_parts<16, 2>(a, w, c, status, M, N, K, s);
+    if (M <= 32) return launch_parts<32, 2>(a, w, c, status, M, N, K, s);
+    if (M <= 64) return launch_parts<64, 1>(a, w, c, status, M, N, K, s);
+    return launch_parts<128, 1>(a, w, c, status, M, N, K, s);
+}

@@ -155,7 +155,7 @@ class NativeOps:
     # ------------------------------------------------------------ libraries
     def prepare(self, dtype: torch.dtype, sampling: bool = True) -> None:
         """Compile, side by side, what a model of this dtype will call."""
-        names = ["elementwise", "sublayer", "rope", "attention", "gemm_simt", "recurrent", "moe", "matrix_state", "stream_sum", "conv_mixers", "matrix_recurrence"]
+        names = ["elementwise", "sublayer", "rope", "attention", "gemm_simt", "gemm_f32", "recurrent", "moe", "matrix_state", "stream_sum", "conv_mixers", "matrix_recurrence"]
         if dtype == torch.bfloat16:
             names += ["attention_mma", "attention_decode", "gemm_tcgen05"]
         if sampling:
@@ -1528,7 +1528,7 @@ class NativeOps:
     @_timed
     def linear(self, x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
                partials_ok: bool = False) -> torch.Tensor:
-        """``x [M, K] @ w[N, K]^T``.  float32 runs on the CUDA cores (true 32-bit).  bfloat16 with
+        """``x [M, K] @ w[N, K]^T``.  float32 is multiplied in true 32-bit.  bfloat16 with
         at most 64 rows (decode steps) runs on the tcgen05 kernel that streams the weight once;
         more rows use the library product, as the reference's ``nn.Linear`` does.
 
@@ -1655,12 +1655,19 @@ class NativeOps:
         return float(waited.item()) / 1e6
 
     def gemm_simt(self, x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
+        """Products without a reduced-precision mode, any size: float32 operands with 16-byte rows on the kernels of
+        ``gemm_f32``, everything else on the CUDA cores."""
         _cuda_contig(x, "gemm input")
         _cuda_contig(w, "gemm weight")
         _need(x.shape[1] == w.shape[1] and x.dtype == w.dtype and x.dtype in _DT, "gemm_simt: operands disagree")
         M, K = x.shape
         N = w.shape[0]
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
+        if x.dtype == torch.float32 and out_dtype == torch.float32 and self._lib("gemm_f32").tl_gemm_f32_supports(_ptr(x), _ptr(w), K) == 1:
+            rc = self._lib("gemm_f32").tl_gemm_f32(_ptr(x), _ptr(w), _ptr(out), M, N, K, ctypes.c_void_p(self._status.data_ptr()), _stream())
+            _check(rc, "gemm_f32")
+            self.launches += 1
+            return out
         rc = self._lib("gemm_simt").tl_gemm_simt(_ptr(x), _ptr(w), _ptr(out), _DT[x.dtype], _DT[out_dtype],
                                                 M, N, K, _stream())
         _check(rc, "gemm_simt")
