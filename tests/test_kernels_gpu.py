@@ -455,6 +455,31 @@ def test_paged_attention_matches_twin(ops, dtype, impl, case):
     torch.testing.assert_close(got.float(), want.float(), atol=t, rtol=t)
 
 
+@pytest.mark.parametrize("hd", [16, 32, 64, 128])
+@pytest.mark.parametrize("H,KV", [(1, 1), (4, 2), (9, 3), (32, 4), (9, 1), (32, 1), (33, 1)])
+@pytest.mark.parametrize("seq_lens,q_lens", [([1, 16, 17, 63, 129, 1000], [1] * 6), ([2500], [1]), ([1, 33, 65, 64, 300], [1, 33, 2, 64, 299]),
+                                             ([900, 31], [40, 31]), ([1500], [2])])
+def test_plain_float32_attention_at_the_edges_of_its_tiles(ops, hd, H, KV, seq_lens, q_lens):
+    """Groups that fill their rows and groups that do not, one token and many, whole ranges of keys and splits."""
+    a = build_paged(seq_lens, q_lens, H, KV, hd, 8, torch.float32, seed=hd + H)
+    want = torch.empty_like(a["q"], dtype=torch.float64)
+    for b, (L, n) in enumerate(zip(seq_lens, q_lens)):
+        pos = torch.arange(L, device="cuda")
+        pages = a["block_table"][b].long()[pos // 8]
+        k, v = (a[x][pages, :, pos % 8].double().repeat_interleave(H // KV, dim=1) for x in ("k_pages", "v_pages"))
+        rows = slice(int(a["q_start"][b]), int(a["q_start"][b]) + n)
+        s = torch.einsum("qhd,khd->hqk", a["q"][rows].double(), k) * hd ** -0.5
+        s = s.masked_fill(pos[None, None, :] > (torch.arange(n, device="cuda") + L - n)[None, :, None], float("-inf"))
+        want[rows] = torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), v)
+    # a score is hd products of N(0, 1) numbers, rounded hd times: its error, and with it a weight's relative error, is below
+    # (hd + 3) 2^-24 of the sum of the products' sizes (at most 128 * 0.64 * 128^-0.5, and less for the smaller heads), twice
+    # for the sum it is divided by; the results are of size 1
+    bound = 2 * (hd + 3) * 2.0 ** -24 * 0.64 * hd ** 0.5 * 4
+    for split in (True, False):
+        got = ops.paged_attention(**a, scale=hd ** -0.5, window=None, allow_split=split)
+        assert (got.double() - want).abs().max().item() <= bound
+
+
 @pytest.mark.parametrize("dtype,impl", IMPLS)
 @pytest.mark.parametrize("B,L", [(1, 2000), (2, 777), (3, 4100)])
 def test_decode_attention_split_over_keys(ops, dtype, impl, B, L):

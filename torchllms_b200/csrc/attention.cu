@@ -298,6 +298,8 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
                                        T* __restrict__ out, int n_splits, int head_dim,
                                        const T* __restrict__ gate, int gate_mode, int out_f32,
                                        const float* __restrict__ sinks, int n_heads, int sigmoid, long long out_pitch) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     const size_t row = blockIdx.x;
     const size_t out_at = row / n_heads * out_pitch + row % n_heads * head_dim;
     const float* ml = part_ml + row * n_splits * 2;
@@ -372,6 +374,381 @@ int launch_hd(const AttnParams& p, dim3 grid, cudaStream_t s) {
     if (widest <= 128) return launch<T, 128>(p, grid, s);
     if (widest <= 256) return launch<T, 256>(p, grid, s);
     return launch<T, 512>(p, grid, s);
+}
+
+// ---------------------------------------------------------------------------------------------- plain float32
+// Causal float32 attention without options, keys and values of one size (16, 32, 64 or 128), up to 32 heads a group: what the
+// true 32-bit path of a plain decoder calls.  Both kernels walk the same pages with the same partial results (and the same
+// number of splits) as the general kernel above, whose CTAs take 16 rows whatever there is to do, load a tile, wait, and fetch
+// five numbers from shared memory for every four multiply-adds.
+//
+// one token a request: bound by the latency of a few kilobytes a warp.  A CTA takes the heads of one group and one split of
+//   the keys; its eight warps take batches of keys by themselves, a key on head_dim / 4 lanes, all of a batch's keys and values
+//   (eight 16-byte loads of each a lane) under way at once, scores summed over the lanes by shuffles, one rescaling a batch.
+//   The warps' results meet in shared memory.
+// portions: bound by the multiply-adds' issue.  32 rows (token, head of the group) against tiles of 64 (head_dim 128: 32) keys
+//   that arrive through cp.async while the tile before is multiplied; a thread holds 4 x 4 scores and 4 x 4 results (4 x 2
+//   and 4 x 8), so that eight 16-byte loads from shared memory feed 64 multiply-adds.
+// In a 1B-shaped model (32 heads in groups of four, head_dim 64), a step of 4 requests with 50 to 700 keys 1,889 -> 1,468 us and 300
+// tokens scored 10.0 -> 8.95 ms: 25 us less a layer for the one (this kernel and the merge, which now starts early, took 35),
+// 65 us less for the other (94 before, 25 to 30 of it left).
+
+constexpr int DW = 8;              // warps of the one-token kernel
+constexpr int DU = 8;              // loads of keys (and as many of values) in flight per lane
+
+template <int HD, int G>
+__global__ void __launch_bounds__(DW * 32) decode_f32_kernel(const AttnParams p) {
+    constexpr int LPK = HD / 4, KPI = 32 / LPK, BATCH = KPI * DU;      // lanes a key, keys a load, keys a batch
+    __shared__ float part[DW][G][HD];
+    __shared__ float part_m[DW][G], part_l[DW][G];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / LPK, at = (lane % LPK) * 4;
+    const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int tok = p.q_start[b];
+    if (p.q_start[b + 1] == tok) return;
+    const int n_keys = p.kv_len[b];
+    const int chunk = ((n_keys + p.n_splits - 1) / p.n_splits + BATCH - 1) / BATCH * BATCH;
+    const int k_lo = split * chunk, k_hi = min(n_keys, k_lo + chunk);
+    const int* table = p.block_table + (size_t)b * p.table_stride;
+    const float* k_pages = reinterpret_cast<const float*>(p.k_pages);
+    const float* v_pages = reinterpret_cast<const float*>(p.v_pages);
+    const int head0 = kvh * p.group;
+    float4 q[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+        q[g] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.q) + ((size_t)tok * p.n_heads + head0 + min(g, p.group - 1)) * HD + at);
+    float m[G], l[G];
+    float4 acc[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        m[g] = -INFINITY;
+        l[g] = 0.f;
+        acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k0 = k_lo + warp * BATCH; k0 < k_hi; k0 += DW * BATCH) {
+        float4 k[DU], v[DU];
+#pragma unroll
+        for (int u = 0; u < DU; ++u) {
+            const int key = k0 + u * KPI + sub;
+            k[u] = v[u] = zero;
+            if (key < k_hi) {
+                const int page = table[key / p.page_size];
+                if (tl_check_page(page)) {
+                    const size_t from = (((size_t)page * p.n_kv_heads + kvh) * p.page_size + key % p.page_size) * HD + at;
+                    k[u] = *reinterpret_cast<const float4*>(k_pages + from);
+                    v[u] = *reinterpret_cast<const float4*>(v_pages + from);
+                }
+            }
+        }
+        float s[G][DU];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int u = 0; u < DU; ++u) {
+                float x = q[g].x * k[u].x;
+                x = fmaf(q[g].y, k[u].y, x);
+                x = fmaf(q[g].z, k[u].z, x);
+                s[g][u] = fmaf(q[g].w, k[u].w, x);
+            }
+#pragma unroll
+        for (int o = 1; o < LPK; o <<= 1)
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+#pragma unroll
+                for (int u = 0; u < DU; ++u) s[g][u] += __shfl_xor_sync(0xffffffffu, s[g][u], o);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            float top = m[g];
+#pragma unroll
+            for (int u = 0; u < DU; ++u) {
+                s[g][u] = k0 + u * KPI + sub < k_hi ? s[g][u] * p.scale : -INFINITY;
+                top = fmaxf(top, s[g][u]);
+            }
+            const float base = top == -INFINITY ? 0.f : top;       // (a lane group may have no key yet)
+            const float alpha = expf(m[g] - base);
+            m[g] = top;
+            l[g] *= alpha;
+            acc[g].x *= alpha; acc[g].y *= alpha; acc[g].z *= alpha; acc[g].w *= alpha;
+#pragma unroll
+            for (int u = 0; u < DU; ++u) {
+                const float w = expf(s[g][u] - base);
+                l[g] += w;
+                acc[g].x = fmaf(w, v[u].x, acc[g].x);
+                acc[g].y = fmaf(w, v[u].y, acc[g].y);
+                acc[g].z = fmaf(w, v[u].z, acc[g].z);
+                acc[g].w = fmaf(w, v[u].w, acc[g].w);
+            }
+        }
+    }
+    // the lane groups of a warp, then the warps
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+#pragma unroll
+        for (int o = LPK; o < 32; o <<= 1) {
+            const float mo = __shfl_xor_sync(0xffffffffu, m[g], o), lo = __shfl_xor_sync(0xffffffffu, l[g], o);
+            float4 ao;
+            ao.x = __shfl_xor_sync(0xffffffffu, acc[g].x, o);
+            ao.y = __shfl_xor_sync(0xffffffffu, acc[g].y, o);
+            ao.z = __shfl_xor_sync(0xffffffffu, acc[g].z, o);
+            ao.w = __shfl_xor_sync(0xffffffffu, acc[g].w, o);
+            const float top = fmaxf(m[g], mo), base = top == -INFINITY ? 0.f : top;
+            const float wa = expf(m[g] - base), wb = expf(mo - base);
+            m[g] = top;
+            l[g] = l[g] * wa + lo * wb;
+            acc[g].x = acc[g].x * wa + ao.x * wb;
+            acc[g].y = acc[g].y * wa + ao.y * wb;
+            acc[g].z = acc[g].z * wa + ao.z * wb;
+            acc[g].w = acc[g].w * wa + ao.w * wb;
+        }
+        if (sub == 0) *reinterpret_cast<float4*>(&part[warp][g][at]) = acc[g];
+        if (lane == 0) {
+            part_m[warp][g] = m[g];
+            part_l[warp][g] = l[g];
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < p.group * HD; i += DW * 32) {
+        const int g = i / HD, d = i % HD;
+        float top = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < DW; ++w) top = fmaxf(top, part_m[w][g]);
+        const float base = top == -INFINITY ? 0.f : top;
+        float num = 0.f, den = 0.f;
+#pragma unroll
+        for (int w = 0; w < DW; ++w) {
+            const float e = expf(part_m[w][g] - base);
+            num = fmaf(e, part[w][g][d], num);
+            den = fmaf(e, part_l[w][g], den);
+        }
+        const size_t row = (size_t)tok * p.n_heads + head0 + g;
+        if (p.n_splits == 1) {
+            reinterpret_cast<float*>(p.out)[(size_t)tok * p.out_pitch + (size_t)(head0 + g) * HD + d] = den > 0.f ? num / den : 0.f;
+        } else {
+            p.part_o[(row * p.n_splits + split) * HD + d] = num;
+            if (d == 0) {
+                p.part_ml[(row * p.n_splits + split) * 2] = top;
+                p.part_ml[(row * p.n_splits + split) * 2 + 1] = den;
+            }
+        }
+    }
+}
+
+constexpr int PR = 32;             // rows of the portion kernel's tile
+constexpr int PT = 128;            // threads: 8 groups of four rows x 16 groups of keys and of columns
+
+__device__ __forceinline__ void copy16_async(float* dst, const float* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+
+template <int HD>
+struct PortionShape {
+    static constexpr int KEYS = HD <= 64 ? 64 : 32, QP = HD + 4, PP = KEYS + 4;
+    static constexpr size_t SMEM = sizeof(float) * ((size_t)PR * QP + 2 * KEYS * QP + 2 * KEYS * HD + PR * PP);
+};
+
+template <int HD>
+__global__ void __launch_bounds__(PT) portion_f32_kernel(const AttnParams p) {
+    using S = PortionShape<HD>;
+    constexpr int KEYS = S::KEYS, QP = S::QP, PP = S::PP, KJ = KEYS / 16, CB = (HD + 63) / 64;
+    extern __shared__ __align__(16) float psm[];
+    float* Qs = psm;                            // [PR][QP]
+    float* Ks = Qs + PR * QP;                   // [2][KEYS][QP]
+    float* Vs = Ks + 2 * KEYS * QP;             // [2][KEYS][HD]
+    float* Ps = Vs + 2 * KEYS * HD;             // [PR][PP]
+    const int b = blockIdx.z, kvh = blockIdx.y, tid = threadIdx.x;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int qs = p.q_start[b], ql = p.q_start[b + 1] - qs, kl = p.kv_len[b];
+    const int split = blockIdx.x % p.n_splits;
+    // the last tokens see the most keys: their tiles start first
+    const int tile = gridDim.x / p.n_splits - 1 - blockIdx.x / p.n_splits;
+    const int tok0 = tile * p.tokens_per_tile;
+    if (tok0 >= ql) return;
+    const int ng = p.group, n_rows = min(p.tokens_per_tile, ql - tok0) * ng;
+    const int qpos0 = kl - ql + tok0, n_vis = qpos0 + (n_rows - 1) / ng + 1;
+    int k_lo = 0, k_hi = n_vis;
+    if (p.n_splits > 1) {
+        const int chunk = ((n_vis + p.n_splits - 1) / p.n_splits + KEYS - 1) / KEYS * KEYS;
+        k_lo = split * chunk;
+        k_hi = min(k_hi, k_lo + chunk);
+    }
+    const float* q = reinterpret_cast<const float*>(p.q);
+    const float* k_pages = reinterpret_cast<const float*>(p.k_pages);
+    const float* v_pages = reinterpret_cast<const float*>(p.v_pages);
+    const int* table = p.block_table + (size_t)b * p.table_stride;
+    for (int i = tid; i < PR * (HD / 4); i += PT) {
+        const int r = i / (HD / 4), d = i % (HD / 4) * 4;
+        const bool live = r < n_rows;
+        copy16_async(Qs + r * QP + d, q + ((size_t)(qs + tok0 + (live ? r / ng : 0)) * p.n_heads + kvh * ng + (live ? r % ng : 0)) * HD + d, live);
+    }
+    auto fetch = [&](int k0, int buf) {
+        for (int i = tid; i < KEYS * (HD / 4); i += PT) {
+            const int j = i / (HD / 4), d = i % (HD / 4) * 4, key = k0 + j;
+            const int page = key < k_hi ? table[key / p.page_size] : 0;
+            const bool live = key < k_hi && tl_check_page(page);
+            const size_t from = live ? (((size_t)page * p.n_kv_heads + kvh) * p.page_size + key % p.page_size) * HD + d : 0;
+            copy16_async(Ks + (buf * KEYS + j) * QP + d, k_pages + from, live);
+            copy16_async(Vs + (buf * KEYS + j) * HD + d, v_pages + from, live);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int tx = tid & 15, r0 = (tid >> 4) * 4;
+    int qpos[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) qpos[i] = r0 + i < n_rows ? qpos0 + (r0 + i) / ng : -1;
+    float m[4], l[4], acc[4][CB * 4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < CB * 4; ++c) acc[i][c] = 0.f;
+    }
+    if (k_lo < k_hi) fetch(k_lo, 0);
+    for (int k0 = k_lo, buf = 0; k0 < k_hi; k0 += KEYS, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();               // this tile is there, and nobody reads the one before it any more
+        if (k0 + KEYS < k_hi) fetch(k0 + KEYS, buf ^ 1);
+        const float* K = Ks + buf * KEYS * QP;
+        const float* V = Vs + buf * KEYS * HD;
+        float s[4][KJ];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < KJ; ++j) s[i][j] = 0.f;
+#pragma unroll 4
+        for (int d = 0; d < HD; d += 4) {
+            float4 x[4], y[KJ];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(Qs + (r0 + i) * QP + d);
+#pragma unroll
+            for (int j = 0; j < KJ; ++j) y[j] = *reinterpret_cast<const float4*>(K + (tx + 16 * j) * QP + d);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < KJ; ++j) {
+                    s[i][j] = fmaf(x[i].x, y[j].x, s[i][j]);
+                    s[i][j] = fmaf(x[i].y, y[j].y, s[i][j]);
+                    s[i][j] = fmaf(x[i].z, y[j].z, s[i][j]);
+                    s[i][j] = fmaf(x[i].w, y[j].w, s[i][j]);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float top = m[i], sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < KJ; ++j) {
+                const int key = k0 + tx + 16 * j;
+                s[i][j] = key < k_hi && key <= qpos[i] ? s[i][j] * p.scale : -INFINITY;
+                top = fmaxf(top, s[i][j]);
+            }
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+            const float base = top == -INFINITY ? 0.f : top;
+            const float alpha = expf(m[i] - base);
+            m[i] = top;
+#pragma unroll
+            for (int j = 0; j < KJ; ++j) {
+                const float w = expf(s[i][j] - base);
+                sum += w;
+                Ps[(r0 + i) * PP + tx + 16 * j] = w;
+            }
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            l[i] = l[i] * alpha + sum;
+#pragma unroll
+            for (int c = 0; c < CB * 4; ++c) acc[i][c] *= alpha;
+        }
+        __syncwarp();                  // (a row's probabilities are written and read by the same half of a warp)
+        if (tx * 4 < HD) {
+#pragma unroll 4
+            for (int j = 0; j < KEYS; j += 4) {
+                float4 w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(Ps + (r0 + i) * PP + j);
+#pragma unroll
+                for (int c = 0; c < CB; ++c) {
+                    float4 y[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) y[e] = *reinterpret_cast<const float4*>(V + (j + e) * HD + c * 64 + tx * 4);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float we[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            acc[i][c * 4] = fmaf(we[e], y[e].x, acc[i][c * 4]);
+                            acc[i][c * 4 + 1] = fmaf(we[e], y[e].y, acc[i][c * 4 + 1]);
+                            acc[i][c * 4 + 2] = fmaf(we[e], y[e].z, acc[i][c * 4 + 2]);
+                            acc[i][c * 4 + 3] = fmaf(we[e], y[e].w, acc[i][c * 4 + 3]);
+                        }
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");       // (a split without keys still has its queries under way)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = r0 + i;
+        if (r >= n_rows) continue;
+        const int tok = qs + tok0 + r / ng, head = kvh * ng + r % ng;
+        const size_t row = (size_t)tok * p.n_heads + head;
+        const float inv = p.n_splits > 1 ? 1.f : l[i] > 0.f ? 1.f / l[i] : 0.f;
+        float* o = p.n_splits > 1 ? p.part_o + (row * p.n_splits + split) * HD
+                                  : reinterpret_cast<float*>(p.out) + (size_t)tok * p.out_pitch + (size_t)head * HD;
+#pragma unroll
+        for (int c = 0; c < CB; ++c)
+            if (c * 64 + tx * 4 < HD)
+                *reinterpret_cast<float4*>(o + c * 64 + tx * 4) =
+                    make_float4(acc[i][c * 4] * inv, acc[i][c * 4 + 1] * inv, acc[i][c * 4 + 2] * inv, acc[i][c * 4 + 3] * inv);
+        if (p.n_splits > 1 && tx == 0) {
+            p.part_ml[(row * p.n_splits + split) * 2] = m[i];
+            p.part_ml[(row * p.n_splits + split) * 2 + 1] = l[i];
+        }
+    }
+}
+
+template <int HD>
+int launch_portion(AttnParams p, int n_seqs, int max_q_len, cudaStream_t s) {
+    using S = PortionShape<HD>;
+    static bool raised = false;
+    if (!raised) {
+        const cudaError_t e = cudaFuncSetAttribute(portion_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+        if (e != cudaSuccess) return (int)e;
+        raised = true;
+    }
+    p.tokens_per_tile = PR / p.group;
+    const int tiles = (max_q_len + p.tokens_per_tile - 1) / p.tokens_per_tile;
+    return (int)tl_launch(portion_f32_kernel<HD>, dim3(tiles * p.n_splits, p.n_kv_heads, n_seqs), dim3(PT), S::SMEM, s, p);
+}
+
+template <int HD>
+int launch_plain_f32_hd(const AttnParams& p, int n_seqs, int max_q_len, cudaStream_t s) {
+    if (max_q_len > 1 || p.group > 8) return launch_portion<HD>(p, n_seqs, max_q_len, s);
+    const dim3 grid(p.n_splits, p.n_kv_heads, n_seqs), block(DW * 32);
+    if (p.group == 1) return (int)tl_launch(decode_f32_kernel<HD, 1>, grid, block, 0, s, p);
+    if (p.group == 2) return (int)tl_launch(decode_f32_kernel<HD, 2>, grid, block, 0, s, p);
+    if (p.group <= 4) return (int)tl_launch(decode_f32_kernel<HD, 4>, grid, block, 0, s, p);
+    return (int)tl_launch(decode_f32_kernel<HD, 8>, grid, block, 0, s, p);
+}
+
+// What the two kernels above take (the rows of a result must start on 16 bytes: out_pitch is checked for it).
+bool plain_f32(const AttnParams& p, int dtype) {
+    return dtype == TL_F32 && (p.head_dim == 16 || p.head_dim == 32 || p.head_dim == 64 || p.head_dim == 128) && p.v_head_dim == p.head_dim &&
+           p.v_stride == p.head_dim && p.n_v_heads == p.n_kv_heads && p.group <= PR && p.window == 0 && p.chunk == 0 && p.keep_first == 0 &&
+           p.rel == nullptr && p.gate_mode == 0 && p.softcap == 0.f && p.sinks == nullptr && !p.sigmoid && p.out_pitch % 4 == 0 && aligned16(p.part_o);
+}
+
+int launch_plain_f32(const AttnParams& p, int n_seqs, int max_q_len, cudaStream_t s) {
+    switch (p.head_dim) {
+        case 16: return launch_plain_f32_hd<16>(p, n_seqs, max_q_len, s);
+        case 32: return launch_plain_f32_hd<32>(p, n_seqs, max_q_len, s);
+        case 64: return launch_plain_f32_hd<64>(p, n_seqs, max_q_len, s);
+        default: return launch_plain_f32_hd<128>(p, n_seqs, max_q_len, s);
+    }
 }
 
 }  // namespace
@@ -477,22 +854,22 @@ extern "C" int tl_paged_attention_ex(const void* q, const void* k_pages, const v
     cudaStream_t s = (cudaStream_t)stream;
     dim3 grid(pl.n_q_tiles * pl.n_splits, n_kv_heads * pl.n_gchunks, n_seqs);
     int rc;
-    if (dtype == TL_F32) rc = launch_hd<float>(p, grid, s);
+    if (plain_f32(p, dtype)) rc = launch_plain_f32(p, n_seqs, max_q_len, s);
+    else if (dtype == TL_F32) rc = launch_hd<float>(p, grid, s);
     else if (dtype == TL_BF16) rc = launch_hd<__nv_bfloat16>(p, grid, s);
     else return TL_BAD_DTYPE;
     if (rc != TL_OK) return rc;
     if (pl.n_splits > 1) {
         const int threads = o.v_head_dim >= 128 ? 128 : 64;
         const unsigned rows = (unsigned)n_tokens * n_heads;
+        cudaError_t e;
         if (dtype == TL_F32)
-            attention_merge_kernel<float><<<rows, threads, 0, s>>>(p.part_o, p.part_ml, (float*)out, pl.n_splits, o.v_head_dim,
-                                                                    (const float*)o.gate, o.gate_mode, o.out_f32, o.sinks, n_heads, o.sigmoid,
-                                                                    p.out_pitch);
+            e = tl_launch(attention_merge_kernel<float>, dim3(rows), dim3(threads), 0, s, p.part_o, p.part_ml, (float*)out, pl.n_splits, o.v_head_dim,
+                          (const float*)o.gate, o.gate_mode, o.out_f32, o.sinks, n_heads, o.sigmoid, p.out_pitch);
         else
-            attention_merge_kernel<__nv_bfloat16><<<rows, threads, 0, s>>>(p.part_o, p.part_ml, (__nv_bfloat16*)out, pl.n_splits,
-                                                                            o.v_head_dim, (const __nv_bfloat16*)o.gate, o.gate_mode, o.out_f32,
-                                                                            o.sinks, n_heads, o.sigmoid, p.out_pitch);
-        TL_LAUNCH_CHECK();
+            e = tl_launch(attention_merge_kernel<__nv_bfloat16>, dim3(rows), dim3(threads), 0, s, p.part_o, p.part_ml, (__nv_bfloat16*)out,
+                          pl.n_splits, o.v_head_dim, (const __nv_bfloat16*)o.gate, o.gate_mode, o.out_f32, o.sinks, n_heads, o.sigmoid, p.out_pitch);
+        if (e != cudaSuccess) return (int)e;
     }
     return TL_OK;
 }
