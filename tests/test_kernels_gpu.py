@@ -110,6 +110,19 @@ def test_gemm_f32_at_the_edges_of_its_tiles(ops, M, N, K):
     ops.check_status()
 
 
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("N,K", [(1, 1536), (2, 4096), (149, 1540), (295, 2304), (2369, 2060), (4737, 8196), (40000, 1536)])
+def test_gemm_f32_streams_rows(ops, M, N, K):
+    """Shares of one row, odd shares, shares of several blocks; pieces of K that no warp or two warps have, and ragged ones."""
+    x, w = rand((M, K), torch.float32, 25), rand((N, K), torch.float32, 26)
+    got = ops.gemm_simt(x, w, torch.float32)
+    want = x.double() @ w.double().t()
+    bound = (K + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())         # K rounded additions in any order
+    assert ((got.double() - want).abs() <= bound).all()
+    assert N < 100 or ((got.double() - want).norm() / want.norm()).item() < 8e-7      # as above
+    ops.check_status()
+
+
 @pytest.mark.parametrize("M", [4, 12, 70])
 def test_gemm_f32_with_numbers_that_are_not_finite(ops, M):
     x, w = rand((M, 512), torch.float32, 23), rand((300, 512), torch.float32, 24)

@@ -1,14 +1,16 @@
 // C[M, N] = A[M, K] . W[N, K]^T, everything float32: the projections of the true 32-bit path.  Both operands are K-major as
-// stored and 16-byte aligned with K % 4 == 0 (gemm_simt.cu takes the rest).  Two kernels; relative errors (2-norm, against
+// stored and 16-byte aligned with K % 4 == 0 (gemm_simt.cu takes the rest).  Relative errors (2-norm, against
 // 64 bits, K = 2,048 / 8,192) beside those of plain multiply-adds one after the other along K (gemm_simt.cu: 8.1e-7 / 1.6e-6).
 //
-// few rows (M <= 8, decode steps): bound by reading W once from HBM.  A warp owns four rows of W and a part of K; its lanes
-//   lie along K, 16 bytes each, with four 2 KB pieces of W in flight per warp (16 warps an SM: 128 KB, about twice what
-//   6.5 TB/s times the latency needs).  The sums over a warp's lanes are taken at the end by a transposing butterfly, those
-//   over the warps that share rows through shared memory, in a fixed order.  Error 1.0e-7 to 1.6e-7.
-//   4 rows against [16384, 2048] 29.5 us (4.6 TB/s), [2048, 8192] 16.5, [128256, 2048] 192 (5.5 TB/s); 210, 557 and 1,161 us
-//   before, when a 64 x 64 tile per CTA walked K alone.  (At 8 rows it is still ahead of the other kernel: 9.1 against 12.6 us
-//   for [2048, 2048], even for the head.)
+// few rows (M <= 8, decode steps): bound by reading W once from HBM; two kernels.  K >= 1,536: a CTA per SM streams an even share
+//   of W's rows through rings in shared memory (TMA copies of 2 KB, 96 KB in flight an SM, which start before the kernel ahead has
+//   ended); its eight warps split K.  Less: a warp owns four rows of W and a part of K, four 2 KB pieces in flight in registers.
+//   In both a warp's lanes lie along K, 16 bytes each; sums over lanes are taken by a transposing butterfly, those over
+//   warps through shared memory, in a fixed order.  Error 1.0e-7 to 1.6e-7.
+//   4 rows against [16384, 2048] 26.9 us (5.0 TB/s), [2048, 8192] 15.9, [128256, 2048] 177 (5.9 TB/s), [2048, 2048] 5.4; 30.0, 17.0,
+//   194 and 6.4 with the registers' kernel; 210, 557 and 1,161 us for the first three when a 64 x 64 tile per CTA walked K
+//   alone.  One row: 23.3, 13.5, 151 (7.0 TB/s) and 3.8.  What is left with 4 and 8 rows is the multiply-adds and the sums at the end of a block of rows, two warps a
+//   scheduler.
 //
 // more rows: bound by arithmetic, and the CUDA cores' multiply-adds give 75 TFLOP/s at most (64 x 128 register tiles: 28 to 45
 //   measured).  So each number is cut into three bfloat16 whose sum it is exactly (8 + 8 + 8 bits), and the tensor cores
@@ -23,6 +25,7 @@
 //
 // In both, the order in which a row's products are added depends on the shapes, never on the other rows' contents.
 #include "common.cuh"
+#include <cuda.h>
 
 namespace {
 
@@ -191,6 +194,175 @@ __device__ __forceinline__ void umma_commit(unsigned long long* bar) {
 __device__ __forceinline__ void tmem_load8(unsigned addr, unsigned (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(addr));
+}
+
+// ---------------------------------------------------------------------------------------------- few rows, large weights
+// A CTA per SM owns an even share of W's rows, a warp an eighth of K.  The warp copies its part of two rows at a time (2 KB, one
+// TMA instruction) into a ring of six in shared memory and reads what arrived while the others travel; the ring runs on through
+// the CTA's blocks of RB rows, over whose ends only the warps' sums meet.  So the copies never drain between one row and the
+// next, a part of A is read once for RB rows, and the first 96 KB of an SM's weights travel while the kernel before ends.
+constexpr int PK = 256;            // K positions of a piece
+constexpr int RING = 6;
+constexpr unsigned PIECE = 2 * PK * 4;
+enum : int { ERR_STREAM_WAIT = 124 };
+
+template <int MT, int RB>
+__global__ void __launch_bounds__(WARPS * 32, MT <= 2 ? 2 : 1) gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const float* __restrict__ A,
+                                                                        float* __restrict__ C, int* status, int M, int N, int K) {
+    extern __shared__ __align__(128) unsigned char ring_all[];
+    __shared__ __align__(8) unsigned long long full[WARPS][RING];
+    __shared__ float part[2][WARPS][MT * RB];
+    __shared__ int abort_flag;
+    constexpr int NV = MT * RB, VPL = NV > 32 ? NV / 32 : 1;        // sums of a block; per lane
+    static_assert(NV <= 32 || NV % 32 == 0, "whole warps of sums");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r0 = (int)((long long)N * blockIdx.x / gridDim.x), r1 = (int)((long long)N * (blockIdx.x + 1) / gridDim.x);
+    const int pieces = (K + PK - 1) / PK, p0 = pieces * warp / WARPS, p1 = pieces * (warp + 1) / WARPS;
+    const int n_blocks = (r1 - r0 + RB - 1) / RB;
+    unsigned char* ring = ring_all + warp * RING * PIECE;
+    if (threadIdx.x == 0) abort_flag = 0;
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < RING; ++i) mbar_init(&full[warp][i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    volatile int* aborted = &abort_flag;
+
+    // what is to be copied next: pair `pr` of block `pb` at piece `pp`, into place `ps` of the ring
+    int pb = p0 < p1 ? 0 : n_blocks, pp = p0, pr = 0, ps = 0;
+    auto issue = [&]() {
+        if (pb >= n_blocks) return;
+        if (lane == 0) {
+            const unsigned bar = smem_u32(&full[warp][ps]);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(PIECE) : "memory");
+            asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                         ::"r"(smem_u32(ring + ps * PIECE)), "l"(&map_w), "r"(bar), "r"(pp * PK), "r"(r0 + pb * RB + 2 * pr) : "memory");
+        }
+        ps = ps + 1 == RING ? 0 : ps + 1;
+        if (++pr == (min(RB, r1 - r0 - pb * RB) + 1) / 2) {
+            pr = 0;
+            if (++pp == p1) pp = p0, ++pb;
+        }
+    };
+    // (W is nobody's output)
+#pragma unroll
+    for (int i = 0; i < RING; ++i) issue();
+    grid_dependency_wait();
+    grid_launch_dependents();
+
+    int at = 0;
+    unsigned phase = 0;
+    bool ok = true;
+    float4 x[MT][2];
+    for (int b = 0; b < n_blocks; ++b) {
+        const int rows = min(RB, r1 - r0 - b * RB);
+        float acc[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) acc[i] = 0.f;
+        for (int pc = p0; pc < p1; ++pc) {
+            if (b == 0 || p1 - p0 > 1)          // (a warp whose part of A is one piece keeps it)
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int k = pc * PK + h * 128 + lane * 4;
+                    x[m][h] = k < K ? *reinterpret_cast<const float4*>(A + (size_t)min(m, M - 1) * K + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+            for (int g = 0; g < RB / 2; ++g) {
+                if (2 * g < rows) {
+                    ok = ok && warp_wait(&full[warp][at], phase, aborted);
+                    if (ok) {
+                        const float4* w = reinterpret_cast<const float4*>(ring + at * PIECE) + lane;
+                        float4 y[2][2];
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) y[r][h] = w[r * (PK / 4) + h * 32];
+#pragma unroll
+                        for (int m = 0; m < MT; ++m)
+#pragma unroll
+                            for (int r = 0; r < 2; ++r) {
+                                float& s = acc[m * RB + 2 * g + r];
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) {
+                                    s = fmaf(x[m][h].x, y[r][h].x, s);
+                                    s = fmaf(x[m][h].y, y[r][h].y, s);
+                                    s = fmaf(x[m][h].z, y[r][h].z, s);
+                                    s = fmaf(x[m][h].w, y[r][h].w, s);
+                                }
+                            }
+                        __syncwarp();              // all lanes have read the place before it is filled again
+                        issue();
+                    }
+                    if (++at == RING) at = 0, phase ^= 1u;
+                }
+            }
+        }
+        if (!ok && lane == 0) {
+            abort_flag = 1;
+            atomicExch(status, ERR_STREAM_WAIT);
+        }
+        if (NV <= 32) {
+            constexpr int NS = NV <= 32 ? NV : 32;
+            const float s = transposed_sum<NS>(reinterpret_cast<float (&)[NS]>(acc));
+            if (lane < NS) part[b & 1][warp][lane] = s;
+        } else {
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) {
+                float some[32];
+#pragma unroll
+                for (int i = 0; i < 32; ++i) some[i] = acc[(v * 32 + i) % NV];
+                const float s = transposed_sum<32>(some);
+                part[b & 1][warp][(v * 32 + lane) % NV] = s;
+            }
+        }
+        __syncthreads();          // (two sets of sums: those of the block before may still be read)
+        if (threadIdx.x < NV) {
+            float s = 0.f;
+#pragma unroll
+            for (int q = 0; q < WARPS; ++q) s += part[b & 1][q][threadIdx.x];
+            const int m = threadIdx.x / RB, r = threadIdx.x % RB;
+            if (m < M && r < rows && *aborted == 0) C[(size_t)m * N + r0 + b * RB + r] = s;
+        }
+    }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_tiled() {
+    static EncodeTiledFn fn = nullptr;
+    if (fn == nullptr) {
+        void* ptr = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<EncodeTiledFn>(ptr);
+    }
+    return fn;
+}
+
+template <int MT, int RB>
+int launch_stream(const float* A, const float* W, float* C, int* status, int M, int N, int K, cudaStream_t s) {
+    constexpr int SMEM = WARPS * RING * PIECE;
+    auto kernel = gemm_f32_stream_kernel<MT, RB>;
+    static bool raised = false;
+    if (!raised) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e != cudaSuccess) return (int)e;
+        raised = true;
+    }
+    EncodeTiledFn fn = encode_tiled();
+    if (fn == nullptr) return TL_BAD_SIZE;
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)N}, strides[1] = {(cuuint64_t)K * 4};
+    const cuuint32_t box[2] = {PK, 2}, elem[2] = {1, 1};
+    if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(W), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return TL_BAD_SIZE;
+    const int ctas = (N + 1) / 2 < kSMs ? (N + 1) / 2 : kSMs;
+    return (int)tl_launch(kernel, dim3(ctas), dim3(WARPS * 32), SMEM, s, map, A, C, status, M, N, K);
 }
 
 // Four numbers as three bfloat16 each, by truncation: v == hi + mid + lo exactly (8 + 8 + 8 bits of significand).  `sick`
@@ -517,6 +689,14 @@ extern "C" int tl_gemm_f32(const void* A, const void* W, void* C, int M, int N, 
     cudaStream_t s = (cudaStream_t)stream;
     const float *a = (const float*)A, *w = (const float*)W;
     float* c = (float*)C;
+    // (a warp of the streaming kernel owns an eighth of K in pieces of 256: below 1,536 half of the warps have nothing to do;
+    // 4 rows against [3072, 1024] 6.3 us, 5.7 in the other kernel, against [3072, 2048] 7.4 and 9.1)
+    if (M <= 8 && K >= 1536) {
+        if (M == 1) return launch_stream<1, 16>(a, w, c, status, M, N, K, s);
+        if (M == 2) return launch_stream<2, 16>(a, w, c, status, M, N, K, s);
+        if (M <= 4) return launch_stream<4, 16>(a, w, c, status, M, N, K, s);
+        return launch_stream<8, 8>(a, w, c, status, M, N, K, s);
+    }
     if (M == 1) return launch_rows<1>(a, w, c, M, N, K, s);
     if (M == 2) return launch_rows<2>(a, w, c, M, N, K, s);
     if (M <= 4) return launch_rows<4>(a, w, c, M, N, K, s);
