@@ -16,12 +16,18 @@
 //   measured).  So each number is cut into three bfloat16 whose sum it is exactly (8 + 8 + 8 bits), and the tensor cores
 //   multiply the parts: six of the nine products, the three that are left out being below 2^-23 of the whole each.  The leading
 //   products are added up in tensor memory over 128 positions of K only and then in registers, rounded to nearest; the small
-//   ones have an accumulator of their own.  Error 1.8e-7 to 4.6e-7.  Eight warps fetch both operands, cut them and
-//   store the parts as tiles of 128-byte-swizzled shared memory, while one warp issues the products of the stage before; the
-//   same eight drain the accumulators.  Tiles that are too few for 148 SMs are cut along K over a cluster of up to eight CTAs
-//   that add up through distributed shared memory.  Numbers that are not finite have no such parts: a CTA that meets one takes
-//   its sums again with plain multiply-adds.
-//   300 rows against [16384, 2048] 201 us (100 TFLOP/s), [2048, 8192] 128, [128256, 2048] 1,390; 866, 828 and 6,397 us before.
+//   ones have two accumulators of their own, that of a second-order product beside that of a third-order one: the tokens' parts
+//   lie one behind the other, so one instruction takes a part of W against two of them and reads it from shared memory once.
+//   Error 1.7e-7 to 3.0e-7.  Eight warps fetch W two or three stages ahead (registers that a third warp group hands over hold
+//   it), cut it and store the parts as tiles of 128-byte-swizzled shared memory, while one warp issues the products of the stage
+//   before; the same eight drain the accumulators.  From 33 rows on the tokens are cut once, by a kernel in front, into three planes
+//   that arrive by TMA; for fewer the eight warps cut them too, which saves a launch.  Tiles that are too few for 148 SMs are cut
+//   along K over a cluster of up to eight CTAs that add up through distributed shared memory.  Numbers that are not finite have no
+//   such parts: a CTA that meets one takes its sums again with plain multiply-adds.
+//   300 rows against [16384, 2048] 134 us (150 TFLOP/s), [2048, 8192] 84, [128256, 2048] 970; 204, 125 and 1,404 us with the tokens cut
+//   by every CTA again, W one stage ahead and six products a step (shared memory carried 270 KB a stage: 180 read by the
+//   products, 92 stored); 866, 828 and 6,397 us with multiply-adds.  64 rows against [16384, 2048] 45.6 and 50.9 us, [3072, 2048] 17.0
+//   and 16.4.
 //
 // In both, the order in which a row's products are added depends on the shapes, never on the other rows' contents.
 #include "common.cuh"
@@ -141,9 +147,13 @@ constexpr int BP = 128;                    // rows of W per CTA: the 128 rows of
 constexpr int BK = 64;                     // K per stage: 64 bfloat16, one 128-byte swizzle row
 constexpr int CHUNK = 2;                   // stages whose leading products are added up in tensor memory
 constexpr int CONVERTERS = 8;              // warps
-constexpr int THREADS = (CONVERTERS + 1) * 32;
+// A third warp group holds the issuing warp and hands its registers to the converters: the launch gives 168 a thread (with nine
+// warps it would give no more, three of them being on one scheduler).
+constexpr int THREADS = (CONVERTERS + 4) * 32;
+constexpr int REGS_LAUNCH = 168, REGS_CONVERT = 216, REGS_REST = 56;
+static_assert(2 * REGS_CONVERT + REGS_REST <= 3 * REGS_LAUNCH, "registers are traded, not made");
 constexpr unsigned long long WAIT_LIMIT_NS = 2000ull * 1000ull * 1000ull;
-enum : int { ERR_STAGE_WAIT = 121, ERR_MMA_WAIT = 122, ERR_SUM_WAIT = 123 };
+enum : int { ERR_STAGE_WAIT = 121, ERR_MMA_WAIT = 122, ERR_SUM_WAIT = 123, ERR_PLANES_WAIT = 125 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
@@ -365,6 +375,37 @@ int launch_stream(const float* A, const float* W, float* C, int* status, int M, 
     return (int)tl_launch(kernel, dim3(ctas), dim3(WARPS * 32), SMEM, s, map, A, C, status, M, N, K);
 }
 
+// sixteen of them with one wait
+__device__ __forceinline__ void tmem_load16(unsigned addr, unsigned (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(addr));
+}
+// acc[0 .. N) += N columns of this thread's lane
+template <int N>
+__device__ __forceinline__ void add_columns(float (&acc)[N], unsigned addr) {
+    constexpr int BIG = N / 16 * 16;
+#pragma unroll
+    for (int j = 0; j < BIG; j += 16) {
+        unsigned r[16];
+        tmem_load16(addr + (unsigned)j, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[j + e] += __uint_as_float(r[e]);
+    }
+    if (BIG < N) {
+        unsigned r[8];
+        tmem_load8(addr + (unsigned)BIG, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[(BIG + e) % N] += __uint_as_float(r[e]);
+    }
+}
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // Four numbers as three bfloat16 each, by truncation: v == hi + mid + lo exactly (8 + 8 + 8 bits of significand).  `sick`
 // becomes NaN where a number is not finite (its remainder is then NaN).
 struct Parts { uint2 hi, mid, lo; };
@@ -387,20 +428,23 @@ __device__ __forceinline__ Parts split4(const float4& v, float& sick) {
     return p;
 }
 
-// BQ: tokens per CTA at most (the launch says how many, a multiple of 16); AHEAD: stages of both operands in registers
+// BQ: tokens per CTA at most (the launch says how many, a multiple of 16); AHEAD: stages of W (and of tokens that are not cut
+// beforehand) in registers
 template <int BQ, int AHEAD>
 struct Shape {
-    static constexpr unsigned W_PART = BP * BK * 2, A_PART = BQ * BK * 2, STAGE = 3 * (W_PART + A_PART);
+    static constexpr bool PLANES = BQ > 32;
+    static constexpr unsigned W_PART = BP * BK * 2, STAGE = 3 * (W_PART + BQ * BK * 2);
     static constexpr unsigned SUMS = BQ * BP * 4;
     static constexpr unsigned SMEM = (2 * STAGE > SUMS ? 2 * STAGE : SUMS) + 1024;
-    static constexpr unsigned COLS = BQ == 128 ? 512 : BQ == 64 ? 256 : BQ == 32 ? 128 : 64;      // three accumulators, a power of two
+    static constexpr unsigned COLS = BQ > 64 ? 512 : BQ == 64 ? 256 : BQ == 32 ? 128 : 64;      // four accumulators, a power of two
 };
 
 template <int BQ, int AHEAD>
-__global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
+__global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_planes, const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
                                                                     int* status, int M, int N, int K, int bq, int token_tiles, int ksplit) {
     using S = Shape<BQ, AHEAD>;
-    constexpr int WL = BP / 16, AL = BQ / 16, HALF = BQ / 2;
+    constexpr bool PLANES = S::PLANES;
+    constexpr int WL = BP / 16, AL = PLANES ? 1 : BQ / 16, HALF = BQ / 2;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
     __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2], sum_full[2], sum_empty[2];
@@ -418,7 +462,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const float*
         abort_flag = 0;
         sick_flag = 0;
         for (int s = 0; s < 2; ++s) {
-            mbar_init(&full_bar[s], CONVERTERS);
+            mbar_init(&full_bar[s], CONVERTERS + (PLANES ? 1 : 0));
             mbar_init(&empty_bar[s], 1);
             mbar_init(&sum_full[s], 1);
             mbar_init(&sum_empty[s], CONVERTERS);
@@ -433,14 +477,15 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const float*
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const unsigned tmem = tmem_slot;
-    float acc[HALF];
-#pragma unroll
-    for (int j = 0; j < HALF; ++j) acc[j] = 0.f;
     bool ok = true;
-    const int quarter = warp & 3, half = warp >> 2;                        // a converter's share of the accumulators
-    const unsigned lanes = (unsigned)(quarter * 32) << 16;
 
     if (warp < CONVERTERS) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_CONVERT));
+        float acc[HALF];
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) acc[j] = 0.f;
+        const int quarter = warp & 3, half = warp >> 2;                    // a converter's share of the accumulators
+        const unsigned lanes = (unsigned)(quarter * 32) << 16;
         // rows warp * 2 + lane / 16 + 16 i of both tiles, 16 bytes at lane % 16 along K
         const int r0 = warp * 2 + (lane >> 4), kl = (lane & 15) * 4;
         const float *wp = W + (size_t)(n0 + r0) * K + kl, *ap = A + (size_t)(m0 + r0) * K + kl;
@@ -464,7 +509,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const float*
 #pragma unroll
         for (int d = 0; d < AHEAD; ++d)
 #pragma unroll
-            for (int i = 0; i < AL; ++i) ab[d][i] = a_at(i, d);
+            for (int i = 0; i < AL; ++i)
+                if (!PLANES) ab[d][i] = a_at(i, d);
         unsigned char* put = tiles + r0 * 128 + ((((lane & 15) >> 1) ^ (r0 & 7)) << 4) + (lane & 1) * 8;
         float sick = 0.f;
         int drained = 0;
@@ -473,14 +519,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const float*
             ok = ok && warp_wait(&sum_full[c & 1], (c >> 1) & 1, aborted);
             if (!ok) return;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < HALF; j += 8) {
-                unsigned r[8];
-                tmem_load8(tmem + lanes + (unsigned)((c & 1) * BQ + half * HALF + j), r);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(r[e]);
-            }
+            add_columns<HALF>(acc, tmem + lanes + (unsigned)((c & 1) * BQ + half * HALF));
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&sum_empty[c & 1]);
@@ -503,11 +542,13 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const float*
                     wb[d][i] = w_at(i, b + AHEAD);
                 }
 #pragma unroll
-                for (int i = 0; i < AL; ++i) {
-                    const Parts q = split4(ab[d][i], sick);
-                    *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART) = q.hi;
-                    *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + S::A_PART) = q.mid;
-                    *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + 2 * S::A_PART) = q.lo;
+                for (int i = 0; i < (PLANES ? 0 : AL); ++i) {
+                    if (16 * i < bq) {
+                        const Parts q = split4(ab[d][i], sick);
+                        *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART) = q.hi;
+                        *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + bq * 128) = q.mid;
+                        *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + bq * 256) = q.lo;
+                    }
                     ab[d][i] = a_at(i, b + AHEAD);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -519,109 +560,133 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const float*
         while (ok && drained < chunks) drain();
         if (ok && blocks > 0) {
             // the small products, added up over the whole range; the last chunk's signal covers them
+            add_columns<HALF>(acc, tmem + lanes + (unsigned)(2 * BQ + bq + half * HALF));
+            add_columns<HALF>(acc, tmem + lanes + (unsigned)(2 * BQ + half * HALF));
+        }
+        if (PLANES) {           // (parts of a number that is not finite make the sum NaN, whichever operand it is in)
+            sick = 0.f;
 #pragma unroll
-            for (int j = 0; j < HALF; j += 8) {
-                unsigned r[8];
-                tmem_load8(tmem + lanes + (unsigned)(2 * BQ + half * HALF + j), r);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[j + e] += __uint_as_float(r[e]);
-            }
+            for (int j = 0; j < HALF; ++j)
+                if (half * HALF + j < bq && m0 + half * HALF + j < M) sick += acc[j] != acc[j] ? acc[j] : 0.f;
         }
         if (sick != sick) sick_flag = 1;
         if (!ok && lane == 0) {
             abort_flag = 1;
             atomicExch(status, ERR_SUM_WAIT);
         }
-    } else {
-        // ---- tensor-core issuer: the whole warp in step, one elected lane issuing
-        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bq >> 3) << 17) | ((unsigned)(BP >> 4) << 24);
-        for (int b = 0; b < blocks; ++b) {
-            const int s = b & 1, c = b / CHUNK;
-            ok = warp_wait(&full_bar[s], (b >> 1) & 1, aborted);
-            if (ok && b % CHUNK == 0 && c >= 2) ok = warp_wait(&sum_empty[c & 1], ((c >> 1) - 1) & 1, aborted);
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const unsigned wt = smem_u32(tiles) + s * S::STAGE, at = wt + 3 * S::W_PART;
-            const unsigned lead = tmem + (unsigned)((c & 1) * BQ), small = tmem + 2 * BQ;
-#pragma unroll
-            for (int k = 0; k < BK / 16; ++k) {
-                unsigned long long w[3], a[3];
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    w[q] = umma_desc(wt + q * S::W_PART + k * 32);
-                    a[q] = umma_desc(at + q * S::A_PART + k * 32);
-                }
-                umma_bf16(small, w[2], a[0], idesc, b > 0 || k > 0);
-                umma_bf16(small, w[0], a[2], idesc, true);
-                umma_bf16(small, w[1], a[1], idesc, true);
-                umma_bf16(small, w[1], a[0], idesc, true);
-                umma_bf16(small, w[0], a[1], idesc, true);
-                umma_bf16(lead, w[0], a[0], idesc, b % CHUNK > 0 || k > 0);
-            }
-            umma_commit(&empty_bar[s]);
-            if (b % CHUNK == CHUNK - 1 || b == blocks - 1) umma_commit(&sum_full[c & 1]);
-        }
-        if (!ok && lane == 0) {
-            abort_flag = 1;
-            atomicExch(status, ERR_MMA_WAIT);
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    const bool good = abort_flag == 0;
-    const int row = quarter * 32 + lane, n = n0 + row;
-    if (good && sick_flag && warp < CONVERTERS) {
-        // An operand is not finite: inf * 0 between its parts would be NaN where the product itself is not.  Once over
-        // with plain multiply-adds (slow; nothing but correctness matters here).
-        const int k1 = min(K, (first + blocks) * BK);
+        asm volatile("tcgen05.fence::before_thread_sync;\nbar.sync 0;" ::: "memory");         // every role is done
+        const bool good = abort_flag == 0;
+        const int row = quarter * 32 + lane, n = n0 + row;
+        if (good && sick_flag) {
+            // An operand is not finite: inf * 0 between its parts would be NaN where the product itself is not.  Once over
+            // with plain multiply-adds (slow; nothing but correctness matters here).
+            const int k1 = min(K, (first + blocks) * BK);
 #pragma unroll 1
-        for (int j = 0; j < HALF; ++j) {
-            const int m = m0 + half * HALF + j;
-            float s = 0.f;
-            if (n < N && m < M && half * HALF + j < bq)
-                for (int k = first * BK; k < k1; ++k) s = fmaf(A[(size_t)m * K + k], W[(size_t)n * K + k], s);
-#pragma unroll
-            for (int e = 0; e < HALF; ++e) if (e == j) acc[e] = s;
-        }
-    }
-    if (ksplit == 1) {
-        if (good && warp < CONVERTERS && n < N) {
-#pragma unroll
             for (int j = 0; j < HALF; ++j) {
-                const int t = half * HALF + j;
-                if (t < bq && m0 + t < M) C[(size_t)(m0 + t) * N + n] = acc[j];
+                const int m = m0 + half * HALF + j;
+                float s = 0.f;
+                if (n < N && m < M && half * HALF + j < bq)
+                    for (int k = first * BK; k < k1; ++k) s = fmaf(A[(size_t)m * K + k], W[(size_t)n * K + k], s);
+#pragma unroll
+                for (int e = 0; e < HALF; ++e) if (e == j) acc[e] = s;
             }
         }
-    } else {
-        // The cluster's CTAs hold sums over their parts of K: each leaves its own in its shared memory (the stages are
-        // done with) and adds up every ksplit-th token's from all, in the order of the parts.  A CTA that gave up takes
-        // part in the barriers and leaves NaN.
-        float* sums = reinterpret_cast<float*>(tiles);                     // [token][row]
-        if (warp < CONVERTERS) {
+        if (ksplit == 1) {
+            if (good && n < N) {
+#pragma unroll
+                for (int j = 0; j < HALF; ++j) {
+                    const int t = half * HALF + j;
+                    if (t < bq && m0 + t < M) C[(size_t)(m0 + t) * N + n] = acc[j];
+                }
+            }
+        } else {
+            // The cluster's CTAs hold sums over their parts of K: each leaves its own in its shared memory (the stages are
+            // done with) and adds up every ksplit-th token's from all, in the order of the parts.  A CTA that gave up takes
+            // part in the barriers and leaves NaN.
+            float* sums = reinterpret_cast<float*>(tiles);                 // [token][row]
 #pragma unroll
             for (int j = 0; j < HALF; ++j) sums[(half * HALF + j) * BP + row] = good ? acc[j] : __int_as_float(0x7fffffff);
-        }
-        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        if (warp < CONVERTERS && n < N) {
-            for (int t = rank + half * ksplit; t < bq && m0 + t < M; t += 2 * ksplit) {
-                float v[8], s = 0.f;
+            cluster_sync();
+            if (n < N) {
+                for (int t = rank + half * ksplit; t < bq && m0 + t < M; t += 2 * ksplit) {
+                    float v[8], s = 0.f;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    if (q < ksplit) {
-                        unsigned there;
-                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_u32(&sums[t * BP + row])), "r"(q));
-                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[q]) : "r"(there) : "memory");
+                    for (int q = 0; q < 8; ++q) {
+                        if (q < ksplit) {
+                            unsigned there;
+                            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(smem_u32(&sums[t * BP + row])), "r"(q));
+                            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[q]) : "r"(there) : "memory");
+                        }
                     }
-                }
 #pragma unroll
-                for (int q = 0; q < 8; ++q) if (q < ksplit) s += v[q];
-                C[(size_t)(m0 + t) * N + n] = s;
+                    for (int q = 0; q < 8; ++q) if (q < ksplit) s += v[q];
+                    C[(size_t)(m0 + t) * N + n] = s;
+                }
+            }
+            cluster_sync();          // nobody leaves while another still reads its shared memory
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_REST));
+        if (warp == CONVERTERS) {
+            // ---- tensor-core issuer: the whole warp in step, one elected lane issuing
+            // The parts of the tokens lie one behind the other, and so do the accumulators of the products of the second and third
+            // order: a part of W meets two of them in one instruction, which reads it from shared memory once.
+            const unsigned one = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bq >> 3) << 17) | ((unsigned)(BP >> 4) << 24);
+            const unsigned pair = one + ((unsigned)(bq >> 3) << 17);
+            for (int b = 0; b < blocks; ++b) {
+                const int s = b & 1, c = b / CHUNK;
+                ok = warp_wait(&full_bar[s], (b >> 1) & 1, aborted);
+                if (ok && b % CHUNK == 0 && c >= 2) ok = warp_wait(&sum_empty[c & 1], ((c >> 1) - 1) & 1, aborted);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const unsigned wt = smem_u32(tiles) + s * S::STAGE, at = wt + 3 * S::W_PART;
+                const unsigned lead = tmem + (unsigned)((c & 1) * BQ), mid = tmem + 2 * BQ, low = mid + bq;
+#pragma unroll
+                for (int k = 0; k < BK / 16; ++k) {
+                    const unsigned long long w0 = umma_desc(wt + k * 32), w1 = umma_desc(wt + S::W_PART + k * 32), w2 = umma_desc(wt + 2 * S::W_PART + k * 32);
+                    const unsigned long long a0 = umma_desc(at + k * 32), a1 = umma_desc(at + bq * 128 + k * 32);
+                    umma_bf16(mid, w0, a1, pair, b > 0 || k > 0);          // w0 a1 | w0 a2
+                    umma_bf16(mid, w1, a0, pair, true);                    // w1 a0 | w1 a1
+                    umma_bf16(low, w2, a0, one, true);
+                    umma_bf16(lead, w0, a0, one, b % CHUNK > 0 || k > 0);
+                }
+                umma_commit(&empty_bar[s]);
+                if (b % CHUNK == CHUNK - 1 || b == blocks - 1) umma_commit(&sum_full[c & 1]);
+            }
+            if (!ok && lane == 0) {
+                abort_flag = 1;
+                atomicExch(status, ERR_MMA_WAIT);
             }
         }
-        // nobody leaves while another still reads its shared memory
-        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (PLANES && warp == CONVERTERS + 1) {
+            // ---- the tokens' parts, cut beforehand: [bq x 64] boxes of the three planes, one behind the other.  (Rows past
+            // the last token are another plane's or the zero fill; their sums are not stored.)
+            grid_dependency_wait();
+            for (int b = 0; b < blocks; ++b) {
+                const int s = b & 1;
+                if (b >= 2) ok = warp_wait(&empty_bar[s], ((b >> 1) - 1) & 1, aborted);
+                if (!ok) break;
+                if (lane == 0) {
+                    const unsigned bar = smem_u32(&full_bar[s]), to = smem_u32(tiles) + s * S::STAGE + 3 * S::W_PART;
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned)(3 * bq * 128)) : "memory");
+                    for (int q = 0; q < 3; ++q)
+                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                                     ::"r"(to + q * bq * 128), "l"(&map_planes), "r"(bar), "r"((first + b) * BK), "r"(q * M + m0) : "memory");
+                }
+                __syncwarp();
+            }
+            if (!ok && lane == 0) {
+                abort_flag = 1;
+                atomicExch(status, ERR_PLANES_WAIT);
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\nbar.sync 0;" ::: "memory");
+        if (ksplit > 1) {
+            cluster_sync();
+            cluster_sync();
+        }
     }
+    __syncthreads();
     if (warp == CONVERTERS) {
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -629,8 +694,26 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const float*
     }
 }
 
+// A [M, K] cut into three planes [M, KP] of bfloat16, KP = K rounded up to 8 (a tensor map's rows are multiples of 16 bytes)
+__global__ void __launch_bounds__(256) cut_planes_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ planes, int M, int K, int KP) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    const int per_row = KP / 8, m = (int)(i / per_row), k = (int)(i % per_row) * 8;
+    if (m >= M) return;
+    const float4 u = *reinterpret_cast<const float4*>(A + (size_t)m * K + k);
+    const float4 v = k + 4 < K ? *reinterpret_cast<const float4*>(A + (size_t)m * K + k + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float sick = 0.f;
+    const Parts p = split4(u, sick), q = split4(v, sick);
+    __nv_bfloat16* to = planes + (size_t)m * KP + k;
+    const size_t plane = (size_t)M * KP;
+    *reinterpret_cast<uint4*>(to) = make_uint4(p.hi.x, p.hi.y, q.hi.x, q.hi.y);
+    *reinterpret_cast<uint4*>(to + plane) = make_uint4(p.mid.x, p.mid.y, q.mid.x, q.mid.y);
+    *reinterpret_cast<uint4*>(to + 2 * plane) = make_uint4(p.lo.x, p.lo.y, q.lo.x, q.lo.y);
+}
+
 template <int BQ, int AHEAD>
-int launch_parts(const float* A, const float* W, float* C, int* status, int M, int N, int K, cudaStream_t s) {
+int launch_parts(const float* A, const float* W, float* C, void* planes, int* status, int M, int N, int K, cudaStream_t s) {
     using S = Shape<BQ, AHEAD>;
     const int token_tiles = (M + BQ - 1) / BQ;
     const int bq = ((M + token_tiles - 1) / token_tiles + 15) / 16 * 16;       // tiles of equal size
@@ -673,7 +756,19 @@ int launch_parts(const float* A, const float* W, float* C, int* status, int M, i
     cfg.gridDim = dim3((unsigned)(tiles * ksplit));
     attr[0].val.clusterDim.x = ksplit;
     cfg.numAttrs = 2;
-    return (int)cudaLaunchKernelEx(&cfg, kernel, A, W, C, status, M, N, K, bq, token_tiles, ksplit);
+    CUtensorMap map = {};
+    if (S::PLANES) {
+        const int KP = (K + 7) / 8 * 8;
+        const cudaError_t e = tl_launch(cut_planes_kernel, dim3((unsigned)(((long long)M * KP / 8 + 255) / 256)), dim3(256), 0, s, A, (__nv_bfloat16*)planes, M, K, KP);
+        if (e != cudaSuccess) return (int)e;
+        EncodeTiledFn fn = encode_tiled();
+        const cuuint64_t dims[2] = {(cuuint64_t)KP, (cuuint64_t)M * 3}, strides[1] = {(cuuint64_t)KP * 2};
+        const cuuint32_t box[2] = {BK, (cuuint32_t)bq}, elem[2] = {1, 1};
+        if (fn == nullptr || fn(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, planes, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return TL_BAD_SIZE;
+    }
+    return (int)cudaLaunchKernelEx(&cfg, kernel, map, A, W, C, status, M, N, K, bq, token_tiles, ksplit);
 }
 
 }  // namespace
@@ -682,10 +777,14 @@ extern "C" int tl_gemm_f32_supports(const void* A, const void* W, int K) {
     return K >= 4 && K % 4 == 0 && aligned16(A) && aligned16(W) ? 1 : 0;
 }
 
+// Bytes of scratch (16-byte aligned) that tl_gemm_f32 needs for M rows of K numbers.
+extern "C" long long tl_gemm_f32_scratch(int M, int K) { return M > 32 ? 6LL * M * ((K + 7) / 8 * 8) : 0; }
+
 // status: one int that is set to a non-zero code if a wait ran out.
-extern "C" int tl_gemm_f32(const void* A, const void* W, void* C, int M, int N, int K, int* status, void* stream) {
+extern "C" int tl_gemm_f32(const void* A, const void* W, void* C, void* scratch, int M, int N, int K, int* status, void* stream) {
     if (M <= 0 || N <= 0) return TL_OK;
     if (!tl_gemm_f32_supports(A, W, K) || status == nullptr) return TL_BAD_ALIGN;
+    if (M > 32 && (scratch == nullptr || !aligned16(scratch))) return TL_BAD_ALIGN;
     cudaStream_t s = (cudaStream_t)stream;
     const float *a = (const float*)A, *w = (const float*)W;
     float* c = (float*)C;
@@ -701,8 +800,8 @@ extern "C" int tl_gemm_f32(const void* A, const void* W, void* C, int M, int N, 
     if (M == 2) return launch_rows<2>(a, w, c, M, N, K, s);
     if (M <= 4) return launch_rows<4>(a, w, c, M, N, K, s);
     if (M <= 8) return launch_rows<8>(a, w, c, M, N, K, s);
-    if (M <= 16) return launch_parts<16, 2>(a, w, c, status, M, N, K, s);
-    if (M <= 32) return launch_parts<32, 2>(a, w, c, status, M, N, K, s);
-    if (M <= 64) return launch_parts<64, 1>(a, w, c, status, M, N, K, s);
-    return launch_parts<128, 1>(a, w, c, status, M, N, K, s);
+    if (M <= 16) return launch_parts<16, 2>(a, w, c, scratch, status, M, N, K, s);
+    if (M <= 32) return launch_parts<32, 2>(a, w, c, scratch, status, M, N, K, s);
+    if (M <= 64) return launch_parts<64, 3>(a, w, c, scratch, status, M, N, K, s);
+    return launch_parts<128, 2>(a, w, c, scratch, status, M, N, K, s);
 }

@@ -1664,9 +1664,13 @@ class NativeOps:
         N = w.shape[0]
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
         if x.dtype == torch.float32 and out_dtype == torch.float32 and self._lib("gemm_f32").tl_gemm_f32_supports(_ptr(x), _ptr(w), K) == 1:
-            rc = self._lib("gemm_f32").tl_gemm_f32(_ptr(x), _ptr(w), _ptr(out), M, N, K, ctypes.c_void_p(self._status.data_ptr()), _stream())
+            lib = self._lib("gemm_f32")
+            lib.tl_gemm_f32_scratch.restype = ctypes.c_longlong
+            scratch = lib.tl_gemm_f32_scratch(M, K)
+            planes = torch.empty(scratch, dtype=torch.uint8, device=x.device) if scratch else None
+            rc = lib.tl_gemm_f32(_ptr(x), _ptr(w), _ptr(out), _ptr(planes), M, N, K, ctypes.c_void_p(self._status.data_ptr()), _stream())
             _check(rc, "gemm_f32")
-            self.launches += 1
+            self.launches += 1 if planes is None else 2
             return out
         rc = self._lib("gemm_simt").tl_gemm_simt(_ptr(x), _ptr(w), _ptr(out), _DT[x.dtype], _DT[out_dtype],
                                                 M, N, K, _stream())
