@@ -24,9 +24,9 @@
 //   that arrive by TMA; for fewer the eight warps cut them too, which saves a launch.  Tiles that are too few for 148 SMs are cut
 //   along K over a cluster of up to eight CTAs that add up through distributed shared memory.  Numbers that are not finite have no
 //   such parts: a CTA that meets one takes its sums again with plain multiply-adds.
-//   300 rows against [16384, 2048] 134 us (150 TFLOP/s), [2048, 8192] 84, [128256, 2048] 970; 204, 125 and 1,404 us with the tokens cut
+//   300 rows against [16384, 2048] 132 us (152 TFLOP/s), [2048, 8192] 82, [128256, 2048] 940; 204, 125 and 1,404 us with the tokens cut
 //   by every CTA again, W one stage ahead and six products a step (shared memory carried 270 KB a stage: 180 read by the
-//   products, 92 stored); 866, 828 and 6,397 us with multiply-adds.  64 rows against [16384, 2048] 45.6 and 50.9 us, [3072, 2048] 17.0
+//   products, 92 stored); 866, 828 and 6,397 us with multiply-adds.  64 rows against [16384, 2048] 43.0 and 50.9 us, [3072, 2048] 16.7
 //   and 16.4.
 //
 // In both, the order in which a row's products are added depends on the shapes, never on the other rows' contents.
@@ -406,25 +406,39 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Four numbers as three bfloat16 each, by truncation: v == hi + mid + lo exactly (8 + 8 + 8 bits of significand).  `sick`
-// becomes NaN where a number is not finite (its remainder is then NaN).
+// Four numbers as three bfloat16 each, by truncation: v == hi + mid + lo exactly (8 + 8 + 8 bits of significand).  The parts of
+// a number that is not finite hold a NaN (its remainder); with CHECK, `sick` becomes NaN too.
 struct Parts { uint2 hi, mid, lo; };
+__device__ __forceinline__ float2 minus2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }       // exact where a - b is
+__device__ __forceinline__ float2 leading2(float2 v) {
+    return make_float2(__uint_as_float(__float_as_uint(v.x) & 0xffff0000u), __uint_as_float(__float_as_uint(v.y) & 0xffff0000u));
+}
+__device__ __forceinline__ unsigned upper2(float2 v) { return __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632); }
+template <bool CHECK>
 __device__ __forceinline__ Parts split4(const float4& v, float& sick) {
-    unsigned h[4], m[4], l[4];
-    const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        h[e] = __float_as_uint(x[e]) & 0xffff0000u;
-        const float r = x[e] - __uint_as_float(h[e]);
-        m[e] = __float_as_uint(r) & 0xffff0000u;
-        const float t = r - __uint_as_float(m[e]);
-        l[e] = __float_as_uint(t);
-        sick = fmaf(t, 0.f, sick);
-    }
     Parts p;
-    p.hi = make_uint2(__byte_perm(h[0], h[1], 0x7632), __byte_perm(h[2], h[3], 0x7632));
-    p.mid = make_uint2(__byte_perm(m[0], m[1], 0x7632), __byte_perm(m[2], m[3], 0x7632));
-    p.lo = make_uint2(__byte_perm(l[0], l[1], 0x7632), __byte_perm(l[2], l[3], 0x7632));
+    if (CHECK) {
+        unsigned m[4], l[4];
+        const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float r = x[e] - __uint_as_float(__float_as_uint(x[e]) & 0xffff0000u);
+            m[e] = __float_as_uint(r) & 0xffff0000u;
+            const float t = r - __uint_as_float(m[e]);
+            l[e] = __float_as_uint(t);
+            sick = fmaf(t, 0.f, sick);
+        }
+        p.hi = make_uint2(upper2(make_float2(v.x, v.y)), upper2(make_float2(v.z, v.w)));
+        p.mid = make_uint2(__byte_perm(m[0], m[1], 0x7632), __byte_perm(m[2], m[3], 0x7632));
+        p.lo = make_uint2(__byte_perm(l[0], l[1], 0x7632), __byte_perm(l[2], l[3], 0x7632));
+    } else {
+        // (two numbers an instruction: where the cutting sets the pace, 40 and 64 rows, 6 % faster; beside the check 2 % slower)
+        const float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w), xr = minus2(x, leading2(x)), yr = minus2(y, leading2(y));
+        p.hi = make_uint2(upper2(x), upper2(y));
+        p.mid = make_uint2(upper2(xr), upper2(yr));
+        const float2 xl = minus2(xr, leading2(xr)), yl = minus2(yr, leading2(yr));
+        p.lo = make_uint2(upper2(xl), upper2(yl));
+    }
     return p;
 }
 
@@ -535,7 +549,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
                 unsigned char* to = put + s * S::STAGE;
 #pragma unroll
                 for (int i = 0; i < WL; ++i) {
-                    const Parts q = split4(wb[d][i], sick);
+                    const Parts q = split4<!PLANES>(wb[d][i], sick);
                     *reinterpret_cast<uint2*>(to + i * 2048) = q.hi;
                     *reinterpret_cast<uint2*>(to + i * 2048 + S::W_PART) = q.mid;
                     *reinterpret_cast<uint2*>(to + i * 2048 + 2 * S::W_PART) = q.lo;
@@ -544,7 +558,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
 #pragma unroll
                 for (int i = 0; i < (PLANES ? 0 : AL); ++i) {
                     if (16 * i < bq) {
-                        const Parts q = split4(ab[d][i], sick);
+                        const Parts q = split4<true>(ab[d][i], sick);
                         *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART) = q.hi;
                         *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + bq * 128) = q.mid;
                         *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + bq * 256) = q.lo;
@@ -704,7 +718,7 @@ __global__ void __launch_bounds__(256) cut_planes_kernel(const float* __restrict
     const float4 u = *reinterpret_cast<const float4*>(A + (size_t)m * K + k);
     const float4 v = k + 4 < K ? *reinterpret_cast<const float4*>(A + (size_t)m * K + k + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
     float sick = 0.f;
-    const Parts p = split4(u, sick), q = split4(v, sick);
+    const Parts p = split4<false>(u, sick), q = split4<false>(v, sick);
     __nv_bfloat16* to = planes + (size_t)m * KP + k;
     const size_t plane = (size_t)M * KP;
     *reinterpret_cast<uint4*>(to) = make_uint4(p.hi.x, p.hi.y, q.hi.x, q.hi.y);
