@@ -110,6 +110,16 @@ def test_gemm_f32_at_the_edges_of_its_tiles(ops, M, N, K):
     ops.check_status()
 
 
+@pytest.mark.parametrize("M", [4096, 4097, 8193])
+def test_gemm_f32_of_more_rows_than_one_launch_takes(ops, M):
+    x, w = rand((M, 132), torch.float32, 27), rand((133, 132), torch.float32, 28)
+    got = ops.gemm_simt(x, w, torch.float32)
+    want = x.double() @ w.double().t()
+    bound = (132 + 16) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())       # K rounded additions in any order
+    assert ((got.double() - want).abs() <= bound).all()
+    ops.check_status()
+
+
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8])
 @pytest.mark.parametrize("N,K", [(1, 1536), (2, 4096), (149, 1540), (295, 2304), (2369, 2060), (4737, 8196), (40000, 1536)])
 def test_gemm_f32_streams_rows(ops, M, N, K):

@@ -104,6 +104,7 @@ def _timed(fn):
 class NativeOps:
     """The kernels as methods.  Libraries are compiled and loaded on first use."""
 
+    F32_ROWS = 4096         # rows of one float32 product
     PREFILL_MIN_Q = 96      # portions at least this long go to the tcgen05 prefill attention kernel
     FUSE_MAX_ROWS = 16      # steps of at most this many tokens let a product add itself to the residual stream and
                             # prepare the norm that follows in its own kernel; with more rows product + norm
@@ -1666,11 +1667,15 @@ class NativeOps:
         if x.dtype == torch.float32 and out_dtype == torch.float32 and self._lib("gemm_f32").tl_gemm_f32_supports(_ptr(x), _ptr(w), K) == 1:
             lib = self._lib("gemm_f32")
             lib.tl_gemm_f32_scratch.restype = ctypes.c_longlong
-            scratch = lib.tl_gemm_f32_scratch(M, K)
-            planes = torch.empty(scratch, dtype=torch.uint8, device=x.device) if scratch else None
-            rc = lib.tl_gemm_f32(_ptr(x), _ptr(w), _ptr(out), _ptr(planes), M, N, K, ctypes.c_void_p(self._status.data_ptr()), _stream())
-            _check(rc, "gemm_f32")
-            self.launches += 1 if planes is None else 2
+            # (so many rows at a time: they fill the GPU, and what the cut tokens take in memory stays bounded)
+            for a in range(0, M, self.F32_ROWS):
+                rows = min(M - a, self.F32_ROWS)
+                scratch = lib.tl_gemm_f32_scratch(rows, K)
+                planes = torch.empty(scratch, dtype=torch.uint8, device=x.device) if scratch else None
+                rc = lib.tl_gemm_f32(ctypes.c_void_p(x.data_ptr() + 4 * a * K), _ptr(w), ctypes.c_void_p(out.data_ptr() + 4 * a * N), _ptr(planes),
+                                     rows, N, K, ctypes.c_void_p(self._status.data_ptr()), _stream())
+                _check(rc, "gemm_f32")
+                self.launches += 1 if planes is None else 2
             return out
         rc = self._lib("gemm_simt").tl_gemm_simt(_ptr(x), _ptr(w), _ptr(out), _DT[x.dtype], _DT[out_dtype],
                                                 M, N, K, _stream())
