@@ -503,6 +503,50 @@ def test_plain_float32_attention_at_the_edges_of_its_tiles(ops, hd, H, KV, seq_l
         assert (got.double() - want).abs().max().item() <= bound
 
 
+def plain_attention_64(a, H, KV, hd):
+    """Causal attention over the pages of :func:`build_paged` (8 positions a page) as torch computes it in 64 bits."""
+    want = torch.empty_like(a["q"], dtype=torch.float64)
+    starts = a["q_start"].tolist()
+    for b, L in enumerate(a["kv_len"].tolist()):
+        pos, rows = torch.arange(L, device="cuda"), slice(starts[b], starts[b + 1])
+        pages, n = a["block_table"][b].long()[pos // 8], starts[b + 1] - starts[b]
+        k, v = (a[x][pages, :, pos % 8].double().repeat_interleave(H // KV, dim=1) for x in ("k_pages", "v_pages"))
+        s = torch.einsum("qhd,khd->hqk", a["q"][rows].double(), k) * hd ** -0.5
+        later = pos[None, :] > (torch.arange(n, device="cuda") + L - n)[:, None]
+        w = torch.softmax(s.masked_fill(later, float("-inf")), -1)
+        for i in range(n):                              # (a key that a query does not see takes no part, whatever its value)
+            m = L - n + i + 1
+            want[starts[b] + i] = torch.einsum("hk,khd->hd", w[:, i, :m], v[:m])
+    return want
+
+
+@pytest.mark.parametrize("seq_lens,q_lens", [([40, 1000, 200], [1, 1, 1]), ([40, 1000, 200], [2, 33, 1]), ([40, 200, 70], [40, 33, 1])])
+@pytest.mark.parametrize("H,KV", [(8, 2), (32, 1)])
+@pytest.mark.parametrize("where,value", [("q", "nan"), ("q", "inf"), ("k_pages", "nan"), ("k_pages", "inf"), ("v_pages", "nan"), ("v_pages", "inf")])
+def test_plain_float32_attention_keeps_what_is_not_finite(ops, seq_lens, q_lens, H, KV, where, value):
+    """A NaN or an infinity in a query, a key or a value gives what softmax gives, and leaves every other request's bits alone."""
+    hd = 64
+    a = build_paged(seq_lens, q_lens, H, KV, hd, 8, torch.float32, seed=H + len(where))
+    args = dict(scale=hd ** -0.5, window=None)
+    before = {split: ops.paged_attention(**a, **args, allow_split=split).clone() for split in (True, False)}
+    if where == "q":
+        a["q"][int(a["q_start"][1])][0, 5] = float(value)
+    else:
+        a[where][int(a["block_table"][1, 3 // 8]), 0, 3 % 8, 5] = float(value)      # (key 3 of request 1, first key head)
+    want = plain_attention_64(a, H, KV, hd)
+    fine = torch.isfinite(want)
+    # (an infinite key weighs nothing where the query's number is negative: then all is finite)
+    assert (where, value) == ("k_pages", "inf") or not fine.all()
+    others = torch.ones(want.shape[0], dtype=torch.bool, device="cuda")
+    others[int(a["q_start"][1]):int(a["q_start"][2])] = False
+    for split in (True, False):
+        got = ops.paged_attention(**a, **args, allow_split=split)
+        assert torch.equal(torch.isnan(got), torch.isnan(want))
+        assert torch.equal(got[torch.isinf(want)].double(), want[torch.isinf(want)])
+        assert (got[fine].double() - want[fine]).abs().max().item() < 2e-5
+        assert torch.equal(got[others], before[split][others])
+
+
 @pytest.mark.parametrize("dtype,impl", IMPLS)
 @pytest.mark.parametrize("B,L", [(1, 2000), (2, 777), (3, 4100)])
 def test_decode_attention_split_over_keys(ops, dtype, impl, B, L):

@@ -307,17 +307,19 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
     for (int i = 0; i < n_splits; ++i) M = fmaxf(M, ml[2 * i]);
     const float sink = sinks != nullptr ? sinks[row % n_heads] : -INFINITY;
     M = fmaxf(M, sink);
+    if (M == -INFINITY) M = 0.f;          // no score at all, or none but NaN: a difference of two infinities would be NaN by itself
     for (int d = threadIdx.x; d < head_dim; d += blockDim.x) {
         float num = 0.f, den = 0.f;
         for (int i = 0; i < n_splits; ++i) {
             const float mi = ml[2 * i];
-            if (mi == -INFINITY) continue;
+            if (mi == -INFINITY && ml[2 * i + 1] == 0.f) continue;   // no keys (the maximum passes over scores that are NaN; their sum does not)
             const float w = expf(mi - M);
             num = fmaf(w, part_o[(row * n_splits + i) * head_dim + d], num);
             den = fmaf(w, ml[2 * i + 1], den);
         }
         if (sinks != nullptr) den += expf(sink - M);
-        float o = sigmoid ? num : den > 0.f ? num / den : 0.f;       // (without a sum to divide by the partial results just add up)
+        // without a sum to divide by the partial results just add up; a sum that is NaN stays one
+        float o = sigmoid ? num : den == 0.f ? 0.f : num / den;
         if (gate_mode == 1) o *= to_float(gate[row]);
         else if (gate_mode == 2) o *= to_float(gate[row * head_dim + d]);
         if (out_f32) reinterpret_cast<float*>(out)[out_at + d] = o;
@@ -524,7 +526,7 @@ __global__ void __launch_bounds__(DW * 32) decode_f32_kernel(const AttnParams p)
         }
         const size_t row = (size_t)tok * p.n_heads + head0 + g;
         if (p.n_splits == 1) {
-            reinterpret_cast<float*>(p.out)[(size_t)tok * p.out_pitch + (size_t)(head0 + g) * HD + d] = den > 0.f ? num / den : 0.f;
+            reinterpret_cast<float*>(p.out)[(size_t)tok * p.out_pitch + (size_t)(head0 + g) * HD + d] = den == 0.f ? 0.f : num / den;   // (NaN stays NaN)
         } else {
             p.part_o[(row * p.n_splits + split) * HD + d] = num;
             if (d == 0) {
