@@ -547,6 +547,25 @@ def test_plain_float32_attention_keeps_what_is_not_finite(ops, seq_lens, q_lens,
         assert torch.equal(got[others], before[split][others])
 
 
+@pytest.mark.parametrize("hd", [16, 64, 128])
+@pytest.mark.parametrize("H,KV", [(1, 1), (9, 3), (32, 4)])
+@pytest.mark.parametrize("L,n,at", [(40, 40, 20), (40, 40, 39), (130, 130, 65), (900, 64, 870), (33, 33, 0)])
+def test_plain_float32_attention_does_not_see_later_values(ops, hd, H, KV, L, n, at):
+    """Values that are not finite at one token reach that token and those behind it; the ones ahead of it keep their bits."""
+    a = build_paged([L], [n], H, KV, hd, 8, torch.float32, seed=hd + L)
+    for split in (True, False):
+        before = ops.paged_attention(**a, scale=hd ** -0.5, window=None, allow_split=split).clone()
+        poisoned = dict(a, v_pages=a["v_pages"].clone(), k_pages=a["k_pages"].clone())
+        page = int(a["block_table"][0, at // 8])
+        poisoned["v_pages"][page, :, at % 8, 1::2] = float("nan")
+        poisoned["v_pages"][page, :, at % 8, 0::2] = float("inf")
+        poisoned["k_pages"][page, :, at % 8] *= 3.0
+        got = ops.paged_attention(**poisoned, scale=hd ** -0.5, window=None, allow_split=split)
+        ahead = at - (L - n)                       # tokens of the portion ahead of it
+        assert torch.equal(got[:ahead], before[:ahead])
+        assert torch.isnan(got[ahead:, :, 1::2]).all() and not torch.isfinite(got[ahead:, :, 0::2]).any()
+
+
 @pytest.mark.parametrize("dtype,impl", IMPLS)
 @pytest.mark.parametrize("B,L", [(1, 2000), (2, 777), (3, 4100)])
 def test_decode_attention_split_over_keys(ops, dtype, impl, B, L):

@@ -37,6 +37,7 @@
 // (decoding a few long requests), the key range is cut into splits whose partial (max, sum,
 // accumulator) go to a float32 workspace that tl_attention_merge combines.
 #include "common.cuh"
+#include <limits.h>
 #include <math.h>
 
 namespace {
@@ -597,9 +598,13 @@ __global__ void __launch_bounds__(PT) portion_f32_kernel(const AttnParams p) {
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int tx = tid & 15, r0 = (tid >> 4) * 4;
-    int qpos[4];
+    int qpos[4], first_q = INT_MAX, last_q = -1;       // (of this thread's rows)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) qpos[i] = r0 + i < n_rows ? qpos0 + (r0 + i) / ng : -1;
+    for (int i = 0; i < 4; ++i) {
+        qpos[i] = r0 + i < n_rows ? qpos0 + (r0 + i) / ng : -1;
+        last_q = max(last_q, qpos[i]);
+        if (qpos[i] >= 0) first_q = min(first_q, qpos[i]);
+    }
     float m[4], l[4], acc[4][CB * 4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -665,8 +670,11 @@ __global__ void __launch_bounds__(PT) portion_f32_kernel(const AttnParams p) {
         }
         __syncwarp();                  // (a row's probabilities are written and read by the same half of a warp)
         if (tx * 4 < HD) {
+            // up to the last key that one of the four rows sees; a term of a key that a row does not see is left out (its
+            // weight is 0, but 0 times a later token's value that is not finite would be NaN)
+            const int seen = min(KEYS, last_q + 1 - k0), seen_by_all = first_q + 1 - k0;
 #pragma unroll 4
-            for (int j = 0; j < KEYS; j += 4) {
+            for (int j = 0; j < seen; j += 4) {
                 float4 w[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(Ps + (r0 + i) * PP + j);
@@ -675,11 +683,13 @@ __global__ void __launch_bounds__(PT) portion_f32_kernel(const AttnParams p) {
                     float4 y[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) y[e] = *reinterpret_cast<const float4*>(V + (j + e) * HD + c * 64 + tx * 4);
+                    const bool all = j + 4 <= seen_by_all;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float we[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
+                            if (!all && k0 + j + e > qpos[i]) continue;
                             acc[i][c * 4] = fmaf(we[e], y[e].x, acc[i][c * 4]);
                             acc[i][c * 4 + 1] = fmaf(we[e], y[e].y, acc[i][c * 4 + 1]);
                             acc[i][c * 4 + 2] = fmaf(we[e], y[e].z, acc[i][c * 4 + 2]);
