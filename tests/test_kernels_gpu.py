@@ -145,6 +145,31 @@ def test_gemm_f32_with_numbers_that_are_not_finite(ops, M):
     assert torch.isfinite(got[fine]).all() and ((got - want)[fine].norm() / want[fine].norm()).item() < 8e-7
 
 
+@pytest.mark.parametrize("M", [4, 9, 20, 40, 70, 300])
+@pytest.mark.parametrize("value", ["nan", "inf", "largest"])
+def test_gemm_f32_sums_without_a_poisoned_number_keep_their_bits(ops, M, value):
+    """One token's and one weight row's numbers that are not finite (or overflow) change that token's and that column's sums alone."""
+    N, K = 300, 2048
+    x, w = rand((M, K), torch.float32, 29), rand((N, K), torch.float32, 30)
+    before = ops.gemm_simt(x, w, torch.float32)
+    bad = 3.4028234e38 if value == "largest" else float(value)
+    x[2, 1030], w[135, 700] = bad, -bad
+    got = ops.gemm_simt(x, w, torch.float32)
+    clean = torch.ones(M, N, dtype=torch.bool, device="cuda")
+    clean[2], clean[:, 135] = False, False
+    assert torch.equal(got[clean], before[clean])
+    want = x.double() @ w.double().t()
+    size = x.double().abs() @ w.double().abs().t()
+    sure = (want.abs() > 3.5e38) | ~torch.isfinite(want) | (size < 3.4e38)      # (in between, the order of additions decides what overflows)
+    want = torch.where(want.abs() > 3.5e38, want.sign() * float("inf"), want)
+    assert torch.equal(torch.isnan(got)[sure], torch.isnan(want)[sure])
+    assert torch.equal(got[torch.isinf(want)].double(), want[torch.isinf(want)])
+    fine = torch.isfinite(want) & sure
+    bound = (K + 16) * 2.0 ** -24 * size          # K rounded additions in any order
+    assert ((got.double() - want).abs() <= bound)[fine].all()
+    ops.check_status()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1000, 96), (7, 65, 17), (33, 130, 200)])
 @pytest.mark.parametrize("out_dtype", DTYPES)
 def test_gemm_simt_bfloat16_operands(ops, M, N, K, out_dtype):

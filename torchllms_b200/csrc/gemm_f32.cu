@@ -23,13 +23,15 @@
 //   before; the same eight drain the accumulators.  From 33 rows on the tokens are cut once, by a kernel in front, into three planes
 //   that arrive by TMA; for fewer the eight warps cut them too, which saves a launch.  Tiles that are too few for 148 SMs are cut
 //   along K over a cluster of up to eight CTAs that add up through distributed shared memory.  Numbers that are not finite have no
-//   such parts: a CTA that meets one takes its sums again with plain multiply-adds.
+//   such parts: the sums that one enters, and no others, are taken again with plain multiply-adds (300 rows against [16384, 2048]
+//   with one infinite token 239 us, without 138).
 //   300 rows against [16384, 2048] 132 us (152 TFLOP/s), [2048, 8192] 82, [128256, 2048] 940; 204, 125 and 1,404 us with the tokens cut
 //   by every CTA again, W one stage ahead and six products a step (shared memory carried 270 KB a stage: 180 read by the
 //   products, 92 stored); 866, 828 and 6,397 us with multiply-adds.  64 rows against [16384, 2048] 43.0 and 50.9 us, [3072, 2048] 16.7
 //   and 16.4.
 //
-// In both, the order in which a row's products are added depends on the shapes, never on the other rows' contents.
+// In both, the order in which a row's products are added depends on the shapes (the number of rows among them: a row's bits may
+// change where a batch grows from 8 to 9 rows, from 32 to 33, or K is cut otherwise), never on the other rows' contents.
 #include "common.cuh"
 #include <cuda.h>
 
@@ -407,40 +409,59 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 // Four numbers as three bfloat16 each, by truncation: v == hi + mid + lo exactly (8 + 8 + 8 bits of significand).  The parts of
-// a number that is not finite hold a NaN (its remainder); with CHECK, `sick` becomes NaN too.
+// a number that is not finite hold a NaN (its remainder).  (Two numbers an instruction: where the cutting sets the pace, 40 and
+// 64 rows, 6 % faster.)
 struct Parts { uint2 hi, mid, lo; };
 __device__ __forceinline__ float2 minus2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }       // exact where a - b is
 __device__ __forceinline__ float2 leading2(float2 v) {
     return make_float2(__uint_as_float(__float_as_uint(v.x) & 0xffff0000u), __uint_as_float(__float_as_uint(v.y) & 0xffff0000u));
 }
 __device__ __forceinline__ unsigned upper2(float2 v) { return __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632); }
-template <bool CHECK>
-__device__ __forceinline__ Parts split4(const float4& v, float& sick) {
+__device__ __forceinline__ Parts split4(const float4& v) {
     Parts p;
-    if (CHECK) {
-        unsigned m[4], l[4];
-        const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float r = x[e] - __uint_as_float(__float_as_uint(x[e]) & 0xffff0000u);
-            m[e] = __float_as_uint(r) & 0xffff0000u;
-            const float t = r - __uint_as_float(m[e]);
-            l[e] = __float_as_uint(t);
-            sick = fmaf(t, 0.f, sick);
-        }
-        p.hi = make_uint2(upper2(make_float2(v.x, v.y)), upper2(make_float2(v.z, v.w)));
-        p.mid = make_uint2(__byte_perm(m[0], m[1], 0x7632), __byte_perm(m[2], m[3], 0x7632));
-        p.lo = make_uint2(__byte_perm(l[0], l[1], 0x7632), __byte_perm(l[2], l[3], 0x7632));
-    } else {
-        // (two numbers an instruction: where the cutting sets the pace, 40 and 64 rows, 6 % faster; beside the check 2 % slower)
-        const float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w), xr = minus2(x, leading2(x)), yr = minus2(y, leading2(y));
-        p.hi = make_uint2(upper2(x), upper2(y));
-        p.mid = make_uint2(upper2(xr), upper2(yr));
-        const float2 xl = minus2(xr, leading2(xr)), yl = minus2(yr, leading2(yr));
-        p.lo = make_uint2(upper2(xl), upper2(yl));
-    }
+    const float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w), xr = minus2(x, leading2(x)), yr = minus2(y, leading2(y));
+    p.hi = make_uint2(upper2(x), upper2(y));
+    p.mid = make_uint2(upper2(xr), upper2(yr));
+    const float2 xl = minus2(xr, leading2(xr)), yl = minus2(yr, leading2(yr));
+    p.lo = make_uint2(upper2(xl), upper2(yl));
     return p;
 }
+
+// Products a . w of K numbers with plain multiply-adds for up to eight rows w (the lowest bits set in `rows`), by a whole warp in
+// step: 16 bytes a lane, over once all of them are NaN.  Lane r gets row r's; the others keep `mine`.
+__device__ __forceinline__ float plain_products(const float* __restrict__ a, const float* __restrict__ W, int K, unsigned rows, float mine) {
+    const int lane = threadIdx.x & 31;
+    int r[8];
+    float s[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        r[i] = rows != 0 ? __ffs(rows) - 1 : r[0];
+        rows &= rows - 1;
+        s[i] = 0.f;
+    }
+    for (int k = 0; k < K; k += 128) {
+        const int at = k + lane * 4;
+        bool nan = true;
+        if (at < K) {
+            const float4 x = *reinterpret_cast<const float4*>(a + at);
+            float4 y[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = *reinterpret_cast<const float4*>(W + (size_t)r[i] * K + at);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) s[i] = fmaf(x.w, y[i].w, fmaf(x.z, y[i].z, fmaf(x.y, y[i].y, fmaf(x.x, y[i].x, s[i]))));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) nan = __any_sync(0xffffffffu, s[i] != s[i]) && nan;
+        if (nan) break;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float sum = warp_sum(s[i]);
+        if (lane == r[i]) mine = sum;
+    }
+    return mine;
+}
+__device__ __forceinline__ bool is_finite(float v) { return fabsf(v) <= 3.402823466e38f; }
 
 // BQ: tokens per CTA at most (the launch says how many, a multiple of 16); AHEAD: stages of W (and of tokens that are not cut
 // beforehand) in registers
@@ -463,7 +484,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
     unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
     __shared__ __align__(8) unsigned long long full_bar[2], empty_bar[2], sum_full[2], sum_empty[2];
     __shared__ unsigned tmem_slot;
-    __shared__ int abort_flag, sick_flag;
+    __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = blockIdx.x % ksplit, tile = blockIdx.x / ksplit;
     const int m0 = (tile % token_tiles) * bq, n0 = (tile / token_tiles) * BP;      // the tiles that read a slab of W follow one another
@@ -474,7 +495,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
 
     if (threadIdx.x == 0) {
         abort_flag = 0;
-        sick_flag = 0;
         for (int s = 0; s < 2; ++s) {
             mbar_init(&full_bar[s], CONVERTERS + (PLANES ? 1 : 0));
             mbar_init(&empty_bar[s], 1);
@@ -526,7 +546,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
             for (int i = 0; i < AL; ++i)
                 if (!PLANES) ab[d][i] = a_at(i, d);
         unsigned char* put = tiles + r0 * 128 + ((((lane & 15) >> 1) ^ (r0 & 7)) << 4) + (lane & 1) * 8;
-        float sick = 0.f;
         int drained = 0;
         auto drain = [&]() {
             const int c = drained++;
@@ -549,7 +568,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
                 unsigned char* to = put + s * S::STAGE;
 #pragma unroll
                 for (int i = 0; i < WL; ++i) {
-                    const Parts q = split4<!PLANES>(wb[d][i], sick);
+                    const Parts q = split4(wb[d][i]);
                     *reinterpret_cast<uint2*>(to + i * 2048) = q.hi;
                     *reinterpret_cast<uint2*>(to + i * 2048 + S::W_PART) = q.mid;
                     *reinterpret_cast<uint2*>(to + i * 2048 + 2 * S::W_PART) = q.lo;
@@ -558,7 +577,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
 #pragma unroll
                 for (int i = 0; i < (PLANES ? 0 : AL); ++i) {
                     if (16 * i < bq) {
-                        const Parts q = split4<true>(ab[d][i], sick);
+                        const Parts q = split4(ab[d][i]);
                         *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART) = q.hi;
                         *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + bq * 128) = q.mid;
                         *reinterpret_cast<uint2*>(to + i * 2048 + 3 * S::W_PART + bq * 256) = q.lo;
@@ -577,13 +596,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
             add_columns<HALF>(acc, tmem + lanes + (unsigned)(2 * BQ + bq + half * HALF));
             add_columns<HALF>(acc, tmem + lanes + (unsigned)(2 * BQ + half * HALF));
         }
-        if (PLANES) {           // (parts of a number that is not finite make the sum NaN, whichever operand it is in)
-            sick = 0.f;
-#pragma unroll
-            for (int j = 0; j < HALF; ++j)
-                if (half * HALF + j < bq && m0 + half * HALF + j < M) sick += acc[j] != acc[j] ? acc[j] : 0.f;
-        }
-        if (sick != sick) sick_flag = 1;
         if (!ok && lane == 0) {
             abort_flag = 1;
             atomicExch(status, ERR_SUM_WAIT);
@@ -591,26 +603,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
         asm volatile("tcgen05.fence::before_thread_sync;\nbar.sync 0;" ::: "memory");         // every role is done
         const bool good = abort_flag == 0;
         const int row = quarter * 32 + lane, n = n0 + row;
-        if (good && sick_flag) {
-            // An operand is not finite: inf * 0 between its parts would be NaN where the product itself is not.  Once over
-            // with plain multiply-adds (slow; nothing but correctness matters here).
-            const int k1 = min(K, (first + blocks) * BK);
-#pragma unroll 1
-            for (int j = 0; j < HALF; ++j) {
-                const int m = m0 + half * HALF + j;
-                float s = 0.f;
-                if (n < N && m < M && half * HALF + j < bq)
-                    for (int k = first * BK; k < k1; ++k) s = fmaf(A[(size_t)m * K + k], W[(size_t)n * K + k], s);
-#pragma unroll
-                for (int e = 0; e < HALF; ++e) if (e == j) acc[e] = s;
-            }
-        }
+        float odd = 0.f;              // NaN if one of this thread's results is infinite or NaN
+        int t0 = half * HALF, t1 = min(min(bq, M - m0), t0 + HALF), dt = 1;      // its tokens
         if (ksplit == 1) {
+            float o[4] = {0.f, 0.f, 0.f, 0.f};        // (four short chains, and no look at which of them count: those are looked at again)
+#pragma unroll
+            for (int j = 0; j < HALF; ++j) o[j & 3] = fmaf(acc[j], 0.f, o[j & 3]);
+            odd = (o[0] + o[1]) + (o[2] + o[3]);
             if (good && n < N) {
 #pragma unroll
                 for (int j = 0; j < HALF; ++j) {
-                    const int t = half * HALF + j;
-                    if (t < bq && m0 + t < M) C[(size_t)(m0 + t) * N + n] = acc[j];
+                    if (t0 + j < t1) C[(size_t)(m0 + t0 + j) * N + n] = acc[j];
                 }
             }
         } else {
@@ -621,8 +624,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
 #pragma unroll
             for (int j = 0; j < HALF; ++j) sums[(half * HALF + j) * BP + row] = good ? acc[j] : __int_as_float(0x7fffffff);
             cluster_sync();
+            t0 = rank + half * ksplit, t1 = min(bq, M - m0), dt = 2 * ksplit;
             if (n < N) {
-                for (int t = rank + half * ksplit; t < bq && m0 + t < M; t += 2 * ksplit) {
+                for (int t = t0; t < t1; t += dt) {
                     float v[8], s = 0.f;
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
@@ -635,9 +639,28 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
 #pragma unroll
                     for (int q = 0; q < 8; ++q) if (q < ksplit) s += v[q];
                     C[(size_t)(m0 + t) * N + n] = s;
+                    odd = fmaf(s, 0.f, odd);
                 }
             }
             cluster_sync();          // nobody leaves while another still reads its shared memory
+        }
+        // An operand that is not finite makes every sum that it enters NaN (inf * 0 between its parts, where the product itself
+        // may be infinite), and a sum may have overflowed on its way.  Such a result is taken again with plain multiply-adds, by
+        // the whole warp; the others keep their bits.
+        if (good && __any_sync(0xffffffffu, odd != odd)) {
+            for (int t = t0; t < t1; t += dt) {
+                const float* a = A + (size_t)(m0 + t) * K;
+                float* c = C + (size_t)(m0 + t) * N + n;
+                float v = n < N ? *c : 0.f;
+                unsigned again = __ballot_sync(0xffffffffu, !is_finite(v));
+                if (again == 0) continue;
+                while (again != 0) {
+                    v = plain_products(a, W + (size_t)(n0 + quarter * 32) * K, K, again, v);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) again &= again - 1;
+                }
+                if (n < N) *c = v;
+            }
         }
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_REST));
@@ -717,8 +740,7 @@ __global__ void __launch_bounds__(256) cut_planes_kernel(const float* __restrict
     if (m >= M) return;
     const float4 u = *reinterpret_cast<const float4*>(A + (size_t)m * K + k);
     const float4 v = k + 4 < K ? *reinterpret_cast<const float4*>(A + (size_t)m * K + k + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-    float sick = 0.f;
-    const Parts p = split4<false>(u, sick), q = split4<false>(v, sick);
+    const Parts p = split4(u), q = split4(v);
     __nv_bfloat16* to = planes + (size_t)m * KP + k;
     const size_t plane = (size_t)M * KP;
     *reinterpret_cast<uint4*>(to) = make_uint4(p.hi.x, p.hi.y, q.hi.x, q.hi.y);
