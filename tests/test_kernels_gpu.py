@@ -145,6 +145,45 @@ def test_gemm_f32_with_numbers_that_are_not_finite(ops, M):
     assert torch.isfinite(got[fine]).all() and ((got - want)[fine].norm() / want[fine].norm()).item() < 8e-7
 
 
+def multiply_adds(x, w):
+    """``x @ w^T`` by one float32 multiply-add after the other along K (a product of two float32 is exact in 64 bits)."""
+    total = torch.zeros(x.shape[0], w.shape[0], device="cuda")
+    for k in range(x.shape[1]):
+        total = (total.double() + x[:, k].double()[:, None] * w[:, k].double()[None, :]).float()
+    return total
+
+
+@pytest.mark.parametrize("M", [3, 9, 40, 130])
+@pytest.mark.parametrize("K", [4, 8, 60, 128, 188, 192, 256, 516, 2048])
+@pytest.mark.parametrize("numbers", ["normal", "positive", "wide", "large first"])
+def test_gemm_f32_is_no_further_off_than_multiply_adds(ops, M, K, numbers):
+    x, w = rand((M, K), torch.float32, 31), rand((1000, K), torch.float32, 32)
+    if numbers == "positive":
+        x, w = x.abs(), w.abs()
+    elif numbers == "wide":
+        x, w = x * torch.exp(2 * rand((M, K), torch.float32, 33)), w * torch.exp(2 * rand((1000, K), torch.float32, 34))
+    elif numbers == "large first":
+        x[:, 0] *= 300
+        w[:, 0] *= 30
+    # errors as parts of the products' sizes: of numbers of very different size the largest results would decide alone
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    off = ((ops.gemm_simt(x, w, torch.float32).double() - want) / size).norm()
+    assert off <= 1.01 * ((multiply_adds(x, w).double() - want) / size).norm()       # (1.01: chance, where both round alike)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("M", [3, 12, 40, 130])
+@pytest.mark.parametrize("size_x,size_w", [(1e-36, 1.0), (1e-38, 1e20), (1e-42, 1e30), (1e30, 1e-40), (1e-20, 1e-20), (1e34, 1e-30), (3e38, 1e-38)])
+def test_gemm_f32_of_very_small_and_very_large_numbers(ops, M, size_x, size_w):
+    """Numbers whose parts would lie below the smallest bfloat16 or above the largest."""
+    x = (rand((M, 512), torch.float32, 35).double().clamp(-1, 1) * size_x).float()
+    w = (rand((300, 512), torch.float32, 36).double().clamp(-1, 1) * size_w).float()
+    want = x.double() @ w.double().t()
+    off = (ops.gemm_simt(x, w, torch.float32).double() - want).norm()
+    assert off <= 1.01 * (multiply_adds(x, w).double() - want).norm()
+    ops.check_status()
+
+
 @pytest.mark.parametrize("M", [4, 9, 20, 40, 70, 300])
 @pytest.mark.parametrize("value", ["nan", "inf", "largest"])
 def test_gemm_f32_sums_without_a_poisoned_number_keep_their_bits(ops, M, value):

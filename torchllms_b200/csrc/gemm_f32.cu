@@ -1,29 +1,39 @@
 // C[M, N] = A[M, K] . W[N, K]^T, everything float32: the projections of the true 32-bit path.  Both operands are K-major as
-// stored and 16-byte aligned with K % 4 == 0 (gemm_simt.cu takes the rest).  Relative errors (2-norm, against
-// 64 bits, K = 2,048 / 8,192) beside those of plain multiply-adds one after the other along K (gemm_simt.cu: 8.1e-7 / 1.6e-6).
+// stored and 16-byte aligned with K % 4 == 0 and, for more than 8 rows, K >= 192 (gemm_simt.cu takes the rest).
 //
 // few rows (M <= 8, decode steps): bound by reading W once from HBM; two kernels.  K >= 1,536: a CTA per SM streams an even share
 //   of W's rows through rings in shared memory (TMA copies of 2 KB, 96 KB in flight an SM, which start before the kernel ahead has
 //   ended); its eight warps split K.  Less: a warp owns four rows of W and a part of K, four 2 KB pieces in flight in registers.
 //   In both a warp's lanes lie along K, 16 bytes each; sums over lanes are taken by a transposing butterfly, those over
-//   warps through shared memory, in a fixed order.  Error 1.0e-7 to 1.6e-7.
+//   warps through shared memory, in a fixed order.  Relative error (2-norm, against 64 bits) 1.0e-7 to
+//   1.6e-7.
 //   4 rows against [16384, 2048] 26.9 us (5.0 TB/s), [2048, 8192] 15.9, [128256, 2048] 177 (5.9 TB/s), [2048, 2048] 5.4; 30.0, 17.0,
 //   194 and 6.4 with the registers' kernel; 210, 557 and 1,161 us for the first three when a 64 x 64 tile per CTA walked K
 //   alone.  One row: 23.3, 13.5, 151 (7.0 TB/s) and 3.8.  What is left with 4 and 8 rows is the multiply-adds and the sums at the end of a block of rows, two warps a
 //   scheduler.
 //
 // more rows: bound by arithmetic, and the CUDA cores' multiply-adds give 75 TFLOP/s at most (64 x 128 register tiles: 28 to 45
-//   measured).  So each number is cut into three bfloat16 whose sum it is exactly (8 + 8 + 8 bits), and the tensor cores
-//   multiply the parts: six of the nine products, the three that are left out being below 2^-23 of the whole each.  The leading
-//   products are added up in tensor memory over 128 positions of K only and then in registers, rounded to nearest; the small
-//   ones have two accumulators of their own, that of a second-order product beside that of a third-order one: the tokens' parts
-//   lie one behind the other, so one instruction takes a part of W against two of them and reads it from shared memory once.
-//   Error 1.7e-7 to 3.0e-7.  Eight warps fetch W two or three stages ahead (registers that a third warp group hands over hold
+//   measured).  So each number, times 2^16, is cut into three bfloat16 whose sum it is exactly, each rounded to nearest, and the
+//   tensor cores multiply the parts: six of the nine products.  The three that are left out are below 2^-25 of the whole
+//   (twice) and 2^-34, and as often above zero as below.  The leading products are added up in tensor memory over 128 positions of K only
+//   and then in registers, rounded to nearest; the small ones have two accumulators of their own, that of a second-order product
+//   beside that of a third-order one: the tokens' parts lie one behind the other, so one instruction takes a part of W against two
+//   of them and reads it from shared memory once.  Relative errors (2-norm, against 64 bits, times 10^-8) beside those of one multiply-add
+//   after the other (gemm_simt.cu), 300 rows:
+//     K                           64     128     192     256    2048    8192   14336
+//     N(0, 1) . N(0, 0.02)      7.5/14  12/20   11/25   13/29  13/81  15/162  16/215
+//     |N(0, 1)| . |N(0, 1)|     9.3/12  18/17   15/19   18/25  17/70  17/140  17/178
+//     a large product first      16/19  28/27   27/32   27/36  21/79  15/105
+//   From 192 on they are the smaller ones whatever the numbers, so there the line lies.  (What remains is mostly that the tensor cores
+//   cut what they add up instead of rounding it: the mean error is -0.9 to -1.6e-7 of the result, towards zero.)  The factor keeps the parts
+//   of the smallest numbers (1e-42 against 1e30: 9e-8) above the smallest bfloat16.  Cut to the leading bits without it, the parts
+//   cost 1 to 2 % less time; products of K = 4 were off by 7e-8 (multiply-adds 4e-8), and numbers below 2^-110 lost bits or vanished.
+//   Eight warps fetch W two or three stages ahead (registers that a third warp group hands over hold
 //   it), cut it and store the parts as tiles of 128-byte-swizzled shared memory, while one warp issues the products of the stage
 //   before; the same eight drain the accumulators.  From 33 rows on the tokens are cut once, by a kernel in front, into three planes
 //   that arrive by TMA; for fewer the eight warps cut them too, which saves a launch.  Tiles that are too few for 148 SMs are cut
-//   along K over a cluster of up to eight CTAs that add up through distributed shared memory.  Numbers that are not finite have no
-//   such parts: the sums that one enters, and no others, are taken again with plain multiply-adds (300 rows against [16384, 2048]
+//   along K over a cluster of up to eight CTAs that add up through distributed shared memory.  Numbers of 2^111 and more and those that are not
+//   finite have no such parts: the sums that one enters, and no others, are taken again with plain multiply-adds (300 rows against [16384, 2048]
 //   with one infinite token 239 us, without 138).
 //   300 rows against [16384, 2048] 132 us (152 TFLOP/s), [2048, 8192] 82, [128256, 2048] 940; 204, 125 and 1,404 us with the tokens cut
 //   by every CTA again, W one stage ahead and six products a step (shared memory carried 270 KB a stage: 180 read by the
@@ -408,22 +418,26 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Four numbers as three bfloat16 each, by truncation: v == hi + mid + lo exactly (8 + 8 + 8 bits of significand).  The parts of
-// a number that is not finite hold a NaN (its remainder).  (Two numbers an instruction: where the cutting sets the pace, 40 and
-// 64 rows, 6 % faster.)
+// Four numbers, each times 2^16, as three bfloat16: v 2^16 == hi + mid + lo exactly, each part the one before's remainder rounded
+// to nearest (|mid| <= 2^-8, |lo| <= 2^-17 of the power of two below |v|; what is left after mid has 7 bits at most).  With the factor
+// the last bit of the smallest number there is (2^-149) is the last bit of the smallest bfloat16 (2^-133).  A number of
+// 2^111 and more, or one that is infinite or NaN, has an infinite or NaN part.
+constexpr float CUT_SCALE = 65536.f, CUT_UNSCALE = 1.f / (65536.f * 65536.f);
 struct Parts { uint2 hi, mid, lo; };
-__device__ __forceinline__ float2 minus2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }       // exact where a - b is
-__device__ __forceinline__ float2 leading2(float2 v) {
-    return make_float2(__uint_as_float(__float_as_uint(v.x) & 0xffff0000u), __uint_as_float(__float_as_uint(v.y) & 0xffff0000u));
+__device__ __forceinline__ float2 minus2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ unsigned round2(float2 v) {
+    const __nv_bfloat162 r = __floats2bfloat162_rn(v.x, v.y);
+    return *reinterpret_cast<const unsigned*>(&r);
 }
-__device__ __forceinline__ unsigned upper2(float2 v) { return __byte_perm(__float_as_uint(v.x), __float_as_uint(v.y), 0x7632); }
+__device__ __forceinline__ float2 rest2(float2 v, unsigned r) { return minus2(v, make_float2(__uint_as_float(r << 16), __uint_as_float(r & 0xffff0000u))); }
 __device__ __forceinline__ Parts split4(const float4& v) {
     Parts p;
-    const float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w), xr = minus2(x, leading2(x)), yr = minus2(y, leading2(y));
-    p.hi = make_uint2(upper2(x), upper2(y));
-    p.mid = make_uint2(upper2(xr), upper2(yr));
-    const float2 xl = minus2(xr, leading2(xr)), yl = minus2(yr, leading2(yr));
-    p.lo = make_uint2(upper2(xl), upper2(yl));
+    float2 x = __fmul2_rn(make_float2(v.x, v.y), make_float2(CUT_SCALE, CUT_SCALE)), y = __fmul2_rn(make_float2(v.z, v.w), make_float2(CUT_SCALE, CUT_SCALE));
+    p.hi = make_uint2(round2(x), round2(y));
+    x = rest2(x, p.hi.x), y = rest2(y, p.hi.y);
+    p.mid = make_uint2(round2(x), round2(y));
+    x = rest2(x, p.mid.x), y = rest2(y, p.mid.y);
+    p.lo = make_uint2(round2(x), round2(y));
     return p;
 }
 
@@ -613,7 +627,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
             if (good && n < N) {
 #pragma unroll
                 for (int j = 0; j < HALF; ++j) {
-                    if (t0 + j < t1) C[(size_t)(m0 + t0 + j) * N + n] = acc[j];
+                    if (t0 + j < t1) C[(size_t)(m0 + t0 + j) * N + n] = acc[j] * CUT_UNSCALE;
                 }
             }
         } else {
@@ -638,7 +652,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
                     }
 #pragma unroll
                     for (int q = 0; q < 8; ++q) if (q < ksplit) s += v[q];
-                    C[(size_t)(m0 + t) * N + n] = s;
+                    C[(size_t)(m0 + t) * N + n] = s * CUT_UNSCALE;
                     odd = fmaf(s, 0.f, odd);
                 }
             }
@@ -809,8 +823,9 @@ int launch_parts(const float* A, const float* W, float* C, void* planes, int* st
 
 }  // namespace
 
-extern "C" int tl_gemm_f32_supports(const void* A, const void* W, int K) {
-    return K >= 4 && K % 4 == 0 && aligned16(A) && aligned16(W) ? 1 : 0;
+// (a short product of many rows is less exact in parts than in multiply-adds: see the top)
+extern "C" int tl_gemm_f32_supports(const void* A, const void* W, int M, int K) {
+    return K >= (M > 8 ? 192 : 4) && K % 4 == 0 && aligned16(A) && aligned16(W) ? 1 : 0;
 }
 
 // Bytes of scratch (16-byte aligned) that tl_gemm_f32 needs for M rows of K numbers.
@@ -819,7 +834,7 @@ extern "C" long long tl_gemm_f32_scratch(int M, int K) { return M > 32 ? 6LL * M
 // status: one int that is set to a non-zero code if a wait ran out.
 extern "C" int tl_gemm_f32(const void* A, const void* W, void* C, void* scratch, int M, int N, int K, int* status, void* stream) {
     if (M <= 0 || N <= 0) return TL_OK;
-    if (!tl_gemm_f32_supports(A, W, K) || status == nullptr) return TL_BAD_ALIGN;
+    if (!tl_gemm_f32_supports(A, W, M, K) || status == nullptr) return TL_BAD_ALIGN;
     if (M > 32 && (scratch == nullptr || !aligned16(scratch))) return TL_BAD_ALIGN;
     cudaStream_t s = (cudaStream_t)stream;
     const float *a = (const float*)A, *w = (const float*)W;

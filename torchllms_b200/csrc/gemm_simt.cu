@@ -1,6 +1,6 @@
 // C[M, N] = A[M, K] . W[N, K]^T with float32 multiply-adds on the CUDA cores (no tensor cores,
-// hence no reduced-precision matrix mode): float32 operands whose rows are not 16-byte aligned (gemm_f32.cu
-// takes the others), a fallback for bfloat16 operands, and products per head.  Both operands are K-major as stored: activations row-major and
+// hence no reduced-precision matrix mode): float32 operands whose rows are not 16-byte aligned, and those of
+// short products of many rows (gemm_f32.cu takes the others), a fallback for bfloat16 operands, and products per head.  Both operands are K-major as stored: activations row-major and
 // weights in the [out, in] layout of nn.Linear (torchllms/models/networks.py:474-493, :600-602).
 //
 // 64 x 64 output tile per CTA, K walked 16 at a time through shared memory, 4 x 4 outputs per

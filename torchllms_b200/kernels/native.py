@@ -1529,7 +1529,7 @@ class NativeOps:
     @_timed
     def linear(self, x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
                partials_ok: bool = False) -> torch.Tensor:
-        """``x [M, K] @ w[N, K]^T``.  float32 is multiplied in true 32-bit.  bfloat16 with
+        """``x [M, K] @ w[N, K]^T``.  float32 is multiplied in true 32-bit (see :meth:`gemm_simt`).  bfloat16 with
         at most 64 rows (decode steps) runs on the tcgen05 kernel that streams the weight once;
         more rows use the library product, as the reference's ``nn.Linear`` does.
 
@@ -1656,15 +1656,16 @@ class NativeOps:
         return float(waited.item()) / 1e6
 
     def gemm_simt(self, x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
-        """Products without a reduced-precision mode, any size: float32 operands with 16-byte rows on the kernels of
-        ``gemm_f32``, everything else on the CUDA cores."""
+        """Products without a reduced-precision mode, any size: float32 operands with 16-byte rows on the kernels of ``gemm_f32``
+        (with more than 8 rows from K = 192 on: exact three-part products on the tensor cores, whose error is below that of
+        multiply-adds from there), everything else with multiply-adds on the CUDA cores."""
         _cuda_contig(x, "gemm input")
         _cuda_contig(w, "gemm weight")
         _need(x.shape[1] == w.shape[1] and x.dtype == w.dtype and x.dtype in _DT, "gemm_simt: operands disagree")
         M, K = x.shape
         N = w.shape[0]
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
-        if x.dtype == torch.float32 and out_dtype == torch.float32 and self._lib("gemm_f32").tl_gemm_f32_supports(_ptr(x), _ptr(w), K) == 1:
+        if x.dtype == torch.float32 and out_dtype == torch.float32 and self._lib("gemm_f32").tl_gemm_f32_supports(_ptr(x), _ptr(w), M, K) == 1:
             lib = self._lib("gemm_f32")
             lib.tl_gemm_f32_scratch.restype = ctypes.c_longlong
             # (so many rows at a time: they fill the GPU, and what the cut tokens take in memory stays bounded)
