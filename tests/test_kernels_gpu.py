@@ -798,6 +798,20 @@ def test_a_wait_that_nothing_satisfies_gives_up_and_reports(ops):
     ops.check_status()
 
 
+def test_a_warp_that_gives_up_lets_its_copies_land(ops):
+    """The float32 product's streaming warp with a full ring and a wait that nothing ends."""
+    from torchllms_b200.kernels.native import KernelError
+    ops.check_status()
+    w = rand((12, 256), torch.float32, 37)
+    for limit in (0.0, 1.0):
+        assert torch.equal(ops.give_up_selftest(w, limit_ms=limit), w)
+        with pytest.raises(KernelError, match="gave up waiting"):
+            ops.check_status()
+    x, w = rand((3, 2048), torch.float32, 38), rand((300, 2048), torch.float32, 39)
+    torch.testing.assert_close(ops.linear(x, w), x @ w.t(), atol=1e-3, rtol=1e-4)        # the kernels still run
+    ops.check_status()
+
+
 # -------------------------------------------------------------------------------- sampling
 
 def test_greedy_is_first_argmax(ops):

@@ -165,6 +165,7 @@ constexpr int THREADS = (CONVERTERS + 4) * 32;
 constexpr int REGS_LAUNCH = 168, REGS_CONVERT = 216, REGS_REST = 56;
 static_assert(2 * REGS_CONVERT + REGS_REST <= 3 * REGS_LAUNCH, "registers are traded, not made");
 constexpr unsigned long long WAIT_LIMIT_NS = 2000ull * 1000ull * 1000ull;
+constexpr int SETTLE_POLLS = 1 << 20;      // tens of milliseconds
 enum : int { ERR_STAGE_WAIT = 121, ERR_MMA_WAIT = 122, ERR_SUM_WAIT = 123, ERR_PLANES_WAIT = 125 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -185,14 +186,23 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
+// A role that ends, given up or not, first waits (without a look at the others) for the copies and products that it has under way:
+// shared and tensor memory must not be another CTA's while they land.
+__device__ __forceinline__ void settle(unsigned long long* bar, unsigned parity) {
+    unsigned ok = 0;
+    for (int i = 0; i < SETTLE_POLLS && ok == 0; ++i)
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    __syncwarp();
+}
 // by a whole warp: false (for all its lanes) once the limit has passed or another role has given up
-__device__ __forceinline__ bool warp_wait(unsigned long long* bar, unsigned parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool warp_wait(unsigned long long* bar, unsigned parity, volatile int* abort_flag, unsigned long long limit_ns = WAIT_LIMIT_NS) {
     bool ok = mbar_try_wait(bar, parity);
     if (!ok) {
         const unsigned long long t0 = global_ns();
         for (unsigned i = 1; !ok; ++i) {
             ok = mbar_try_wait(bar, parity);
-            if (!ok && (i & 255u) == 0u && (*abort_flag || global_ns() - t0 > WAIT_LIMIT_NS)) break;
+            if (!ok && (i & 255u) == 0u && (*abort_flag || global_ns() - t0 > limit_ns)) break;
         }
     }
     return __all_sync(0xffffffffu, ok);
@@ -228,6 +238,21 @@ constexpr int RING = 6;
 constexpr unsigned PIECE = 2 * PK * 4;
 enum : int { ERR_STREAM_WAIT = 124 };
 
+// a warp's copies under way, from place `at` of its ring (whose next phase is `phase`) up to place `end`; there is one at least
+__device__ __forceinline__ void settle_ring(unsigned long long* full, int at, unsigned phase, int end) {
+    for (int left = end > at ? end - at : end - at + RING; left > 0; --left) {
+        settle(&full[at], phase);
+        if (++at == RING) at = 0, phase ^= 1u;
+    }
+}
+
+__device__ __forceinline__ void copy_piece(const CUtensorMap* map, unsigned char* to, unsigned long long* full, int k, int row) {
+    const unsigned bar = smem_u32(full);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(PIECE) : "memory");
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(smem_u32(to)), "l"(map), "r"(bar), "r"(k), "r"(row) : "memory");
+}
+
 template <int MT, int RB>
 __global__ void __launch_bounds__(WARPS * 32, MT <= 2 ? 2 : 1) gemm_f32_stream_kernel(const __grid_constant__ CUtensorMap map_w, const float* __restrict__ A,
                                                                         float* __restrict__ C, int* status, int M, int N, int K) {
@@ -255,12 +280,7 @@ __global__ void __launch_bounds__(WARPS * 32, MT <= 2 ? 2 : 1) gemm_f32_stream_k
     int pb = p0 < p1 ? 0 : n_blocks, pp = p0, pr = 0, ps = 0;
     auto issue = [&]() {
         if (pb >= n_blocks) return;
-        if (lane == 0) {
-            const unsigned bar = smem_u32(&full[warp][ps]);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(PIECE) : "memory");
-            asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                         ::"r"(smem_u32(ring + ps * PIECE)), "l"(&map_w), "r"(bar), "r"(pp * PK), "r"(r0 + pb * RB + 2 * pr) : "memory");
-        }
+        if (lane == 0) copy_piece(&map_w, ring + ps * PIECE, &full[warp][ps], pp * PK, r0 + pb * RB + 2 * pr);
         ps = ps + 1 == RING ? 0 : ps + 1;
         if (++pr == (min(RB, r1 - r0 - pb * RB) + 1) / 2) {
             pr = 0;
@@ -273,7 +293,7 @@ __global__ void __launch_bounds__(WARPS * 32, MT <= 2 ? 2 : 1) gemm_f32_stream_k
     grid_dependency_wait();
     grid_launch_dependents();
 
-    int at = 0;
+    int at = 0, lost = -1;            // lost: the place, and its phase, whose copy was not waited for to the end
     unsigned phase = 0;
     bool ok = true;
     float4 x[MT][2];
@@ -317,6 +337,8 @@ __global__ void __launch_bounds__(WARPS * 32, MT <= 2 ? 2 : 1) gemm_f32_stream_k
                             }
                         __syncwarp();              // all lanes have read the place before it is filled again
                         issue();
+                    } else if (lost < 0) {
+                        lost = at + (int)phase * RING;
                     }
                     if (++at == RING) at = 0, phase ^= 1u;
                 }
@@ -349,6 +371,32 @@ __global__ void __launch_bounds__(WARPS * 32, MT <= 2 ? 2 : 1) gemm_f32_stream_k
             if (m < M && r < rows && *aborted == 0) C[(size_t)m * N + r0 + b * RB + r] = s;
         }
     }
+    if (!ok) settle_ring(full[warp], lost % RING, (unsigned)(lost / RING), ps);
+}
+
+// What a warp of the kernel above does when a wait runs out, with a wait that nothing ends: it fills its ring, gives up after
+// limit_ns, lets its copies land, and writes out what they brought (RING pieces, [2 RING, PK] of W).
+__global__ void __launch_bounds__(32) give_up_selftest_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__ out, int* status, unsigned long long limit_ns) {
+    __shared__ __align__(128) unsigned char ring[RING * PIECE];
+    __shared__ __align__(8) unsigned long long full[RING], never;
+    __shared__ int abort_flag;
+    const int lane = threadIdx.x;
+    grid_dependency_wait();
+    if (lane == 0) {
+        abort_flag = 0;
+        mbar_init(&never, 1);
+        for (int i = 0; i < RING; ++i) mbar_init(&full[i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int i = 0; i < RING; ++i) copy_piece(&map_w, ring + i * PIECE, &full[i], 0, 2 * i);
+    }
+    __syncwarp();
+    const bool ok = warp_wait(&never, 0, &abort_flag, limit_ns);
+    if (!ok && lane == 0) {
+        abort_flag = 1;
+        atomicExch(status, ERR_STREAM_WAIT);
+    }
+    if (!ok) settle_ring(full, 0, 0, 0);
+    for (int i = lane; i < RING * 2 * PK; i += 32) out[i] = reinterpret_cast<const float*>(ring)[i];
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -365,6 +413,14 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
+bool map_pieces(CUtensorMap* map, const float* W, int N, int K) {
+    EncodeTiledFn fn = encode_tiled();
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)N}, strides[1] = {(cuuint64_t)K * 4};
+    const cuuint32_t box[2] = {PK, 2}, elem[2] = {1, 1};
+    return fn != nullptr && fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(W), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int MT, int RB>
 int launch_stream(const float* A, const float* W, float* C, int* status, int M, int N, int K, cudaStream_t s) {
     constexpr int SMEM = WARPS * RING * PIECE;
@@ -375,14 +431,8 @@ int launch_stream(const float* A, const float* W, float* C, int* status, int M, 
         if (e != cudaSuccess) return (int)e;
         raised = true;
     }
-    EncodeTiledFn fn = encode_tiled();
-    if (fn == nullptr) return TL_BAD_SIZE;
     CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)N}, strides[1] = {(cuuint64_t)K * 4};
-    const cuuint32_t box[2] = {PK, 2}, elem[2] = {1, 1};
-    if (fn(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(W), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return TL_BAD_SIZE;
+    if (!map_pieces(&map, W, N, K)) return TL_BAD_SIZE;
     const int ctas = (N + 1) / 2 < kSMs ? (N + 1) / 2 : kSMs;
     return (int)tl_launch(kernel, dim3(ctas), dim3(WARPS * 32), SMEM, s, map, A, C, status, M, N, K);
 }
@@ -684,7 +734,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
             // order: a part of W meets two of them in one instruction, which reads it from shared memory once.
             const unsigned one = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(bq >> 3) << 17) | ((unsigned)(BP >> 4) << 24);
             const unsigned pair = one + ((unsigned)(bq >> 3) << 17);
-            for (int b = 0; b < blocks; ++b) {
+            int b = 0;
+            for (; b < blocks; ++b) {
                 const int s = b & 1, c = b / CHUNK;
                 ok = warp_wait(&full_bar[s], (b >> 1) & 1, aborted);
                 if (ok && b % CHUNK == 0 && c >= 2) ok = warp_wait(&sum_empty[c & 1], ((c >> 1) - 1) & 1, aborted);
@@ -708,12 +759,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
                 abort_flag = 1;
                 atomicExch(status, ERR_MMA_WAIT);
             }
+            if (b > 0) settle(&empty_bar[(b - 1) & 1], ((b - 1) >> 1) & 1);       // its last products
         }
         if (PLANES && warp == CONVERTERS + 1) {
             // ---- the tokens' parts, cut beforehand: [bq x 64] boxes of the three planes, one behind the other.  (Rows past
             // the last token are another plane's or the zero fill; their sums are not stored.)
             grid_dependency_wait();
-            for (int b = 0; b < blocks; ++b) {
+            int b = 0;
+            for (; b < blocks; ++b) {
                 const int s = b & 1;
                 if (b >= 2) ok = warp_wait(&empty_bar[s], ((b >> 1) - 1) & 1, aborted);
                 if (!ok) break;
@@ -730,6 +783,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
                 abort_flag = 1;
                 atomicExch(status, ERR_PLANES_WAIT);
             }
+            // its last copies; converters that have given up never signal these stages: then it waits as long as copies may take
+            for (int q = b > 2 ? b - 2 : 0; q < b; ++q) settle(&full_bar[q & 1], (q >> 1) & 1);
         }
         asm volatile("tcgen05.fence::before_thread_sync;\nbar.sync 0;" ::: "memory");
         if (ksplit > 1) {
@@ -826,6 +881,13 @@ int launch_parts(const float* A, const float* W, float* C, void* planes, int* st
 // (a short product of many rows is less exact in parts than in multiply-adds: see the top)
 extern "C" int tl_gemm_f32_supports(const void* A, const void* W, int M, int K) {
     return K >= (M > 8 ? 192 : 4) && K % 4 == 0 && aligned16(A) && aligned16(W) ? 1 : 0;
+}
+
+// W: 12 rows of 256 numbers on 16 bytes; out receives them; status is set.
+extern "C" int tl_gemm_f32_give_up_selftest(const void* W, void* out, int* status, unsigned long long limit_ns, void* stream) {
+    CUtensorMap map;
+    if (!aligned16(W) || !map_pieces(&map, (const float*)W, 2 * RING, PK)) return TL_BAD_ALIGN;
+    return (int)tl_launch(give_up_selftest_kernel, dim3(1), dim3(32), 0, (cudaStream_t)stream, map, (float*)out, status, limit_ns);
 }
 
 // Bytes of scratch (16-byte aligned) that tl_gemm_f32 needs for M rows of K numbers.

@@ -1655,6 +1655,18 @@ class NativeOps:
         torch.cuda.synchronize()
         return float(waited.item()) / 1e6
 
+    def give_up_selftest(self, w: torch.Tensor, limit_ms: float = 1.0) -> torch.Tensor:
+        """The same for a warp of the float32 product with copies under way: it gives up, lets them land and returns what they
+        brought, ``w`` (``[12, 256]`` float32) itself."""
+        _cuda_contig(w, "gemm weight", torch.float32)
+        _need(tuple(w.shape) == (12, 256), "give_up_selftest takes 12 rows of 256 numbers")
+        out = torch.empty_like(w)
+        rc = self._lib("gemm_f32").tl_gemm_f32_give_up_selftest(_ptr(w), _ptr(out), ctypes.c_void_p(self._status.data_ptr()),
+                                                                ctypes.c_ulonglong(int(limit_ms * 1e6)), _stream())
+        _check(rc, "give_up_selftest")
+        torch.cuda.synchronize()
+        return out
+
     def gemm_simt(self, x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
         """Products without a reduced-precision mode, any size: float32 operands with 16-byte rows on the kernels of ``gemm_f32``
         (with more than 8 rows from K = 192 on: exact three-part products on the tensor cores, whose error is below that of
