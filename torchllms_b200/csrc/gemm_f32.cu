@@ -162,8 +162,7 @@ constexpr int CONVERTERS = 8;              // warps
 // A third warp group holds the issuing warp and hands its registers to the converters: the launch gives 168 a thread (with nine
 // warps it would give no more, three of them being on one scheduler).
 constexpr int THREADS = (CONVERTERS + 4) * 32;
-constexpr int REGS_LAUNCH = 168, REGS_CONVERT = 216, REGS_REST = 56;
-static_assert(2 * REGS_CONVERT + REGS_REST <= 3 * REGS_LAUNCH, "registers are traded, not made");
+constexpr int REGS_LAUNCH = 168;
 constexpr unsigned long long WAIT_LIMIT_NS = 2000ull * 1000ull * 1000ull;
 constexpr int SETTLE_POLLS = 1 << 20;      // tens of milliseconds
 enum : int { ERR_STAGE_WAIT = 121, ERR_MMA_WAIT = 122, ERR_SUM_WAIT = 123, ERR_PLANES_WAIT = 125 };
@@ -535,6 +534,10 @@ struct Shape {
     static constexpr unsigned W_PART = BP * BK * 2, STAGE = 3 * (W_PART + BQ * BK * 2);
     static constexpr unsigned SUMS = BQ * BP * 4;
     static constexpr unsigned SMEM = (2 * STAGE > SUMS ? 2 * STAGE : SUMS) + 1024;
+    // what the converters get and what the others keep: three stages of W take more of the former (else 24 bytes are spilled), the
+    // products of long tiles of tokens more of the latter (32 bytes, 4 % of the time)
+    static constexpr int REGS_CONVERT = AHEAD > 2 ? 224 : 216, REGS_REST = AHEAD > 2 ? 56 : 72;
+    static_assert(2 * REGS_CONVERT + REGS_REST <= 3 * REGS_LAUNCH, "registers are traded, not made");
     static constexpr unsigned COLS = BQ > 64 ? 512 : BQ == 64 ? 256 : BQ == 32 ? 128 : 64;      // four accumulators, a power of two
 };
 
@@ -578,7 +581,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
     bool ok = true;
 
     if (warp < CONVERTERS) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_CONVERT));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S::REGS_CONVERT));
         float acc[HALF];
 #pragma unroll
         for (int j = 0; j < HALF; ++j) acc[j] = 0.f;
@@ -727,7 +730,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
             }
         }
     } else {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_REST));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::REGS_REST));
         if (warp == CONVERTERS) {
             // ---- tensor-core issuer: the whole warp in step, one elected lane issuing
             // The parts of the tokens lie one behind the other, and so do the accumulators of the products of the second and third
