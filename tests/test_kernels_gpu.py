@@ -805,7 +805,7 @@ def test_a_warp_that_gives_up_lets_its_copies_land(ops):
     w = rand((12, 256), torch.float32, 37)
     for limit in (0.0, 1.0):
         assert torch.equal(ops.give_up_selftest(w, limit_ms=limit), w)
-        with pytest.raises(KernelError, match="gave up waiting"):
+        with pytest.raises(KernelError, match="gave up waiting .code 124."):      # (the wait that ran out, not the one that stopped with it)
             ops.check_status()
     x, w = rand((3, 2048), torch.float32, 38), rand((300, 2048), torch.float32, 39)
     torch.testing.assert_close(ops.linear(x, w), x @ w.t(), atol=1e-3, rtol=1e-4)        # the kernels still run

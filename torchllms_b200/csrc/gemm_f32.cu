@@ -165,7 +165,7 @@ constexpr int THREADS = (CONVERTERS + 4) * 32;
 constexpr int REGS_LAUNCH = 168;
 constexpr unsigned long long WAIT_LIMIT_NS = 2000ull * 1000ull * 1000ull;
 constexpr int SETTLE_POLLS = 1 << 20;      // tens of milliseconds
-enum : int { ERR_STAGE_WAIT = 121, ERR_MMA_WAIT = 122, ERR_SUM_WAIT = 123, ERR_PLANES_WAIT = 125 };
+enum : int { ERR_MMA_WAIT = 122, ERR_CONVERTER_WAIT = 123 /* for a free stage or for a sum */, ERR_PLANES_WAIT = 125 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
@@ -205,6 +205,10 @@ __device__ __forceinline__ bool warp_wait(unsigned long long* bar, unsigned pari
         }
     }
     return __all_sync(0xffffffffu, ok);
+}
+// by one thread of a role whose wait ended so: the first one's reason is what the host reads, the others stopped because of it
+__device__ __forceinline__ void give_up(int* abort_flag, int* status, int code) {
+    if (atomicExch(abort_flag, 1) == 0) atomicExch(status, code);
 }
 
 // shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024 bytes apart
@@ -343,10 +347,7 @@ __global__ void __launch_bounds__(WARPS * 32, MT <= 2 ? 2 : 1) gemm_f32_stream_k
                 }
             }
         }
-        if (!ok && lane == 0) {
-            abort_flag = 1;
-            atomicExch(status, ERR_STREAM_WAIT);
-        }
+        if (!ok && lane == 0) give_up(&abort_flag, status, ERR_STREAM_WAIT);
         if (NV <= 32) {
             constexpr int NS = NV <= 32 ? NV : 32;
             const float s = transposed_sum<NS>(reinterpret_cast<float (&)[NS]>(acc));
@@ -374,28 +375,29 @@ __global__ void __launch_bounds__(WARPS * 32, MT <= 2 ? 2 : 1) gemm_f32_stream_k
 }
 
 // What a warp of the kernel above does when a wait runs out, with a wait that nothing ends: it fills its ring, gives up after
-// limit_ns, lets its copies land, and writes out what they brought (RING pieces, [2 RING, PK] of W).
-__global__ void __launch_bounds__(32) give_up_selftest_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__ out, int* status, unsigned long long limit_ns) {
+// limit_ns, lets its copies land, and writes out what they brought (RING pieces, [2 RING, PK] of W).  A second warp waits for the
+// same and ends when the first one has given up.
+__global__ void __launch_bounds__(64) give_up_selftest_kernel(const __grid_constant__ CUtensorMap map_w, float* __restrict__ out, int* status, unsigned long long limit_ns) {
     __shared__ __align__(128) unsigned char ring[RING * PIECE];
     __shared__ __align__(8) unsigned long long full[RING], never;
     __shared__ int abort_flag;
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31;
     grid_dependency_wait();
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
         abort_flag = 0;
         mbar_init(&never, 1);
         for (int i = 0; i < RING; ++i) mbar_init(&full[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         for (int i = 0; i < RING; ++i) copy_piece(&map_w, ring + i * PIECE, &full[i], 0, 2 * i);
     }
-    __syncwarp();
-    const bool ok = warp_wait(&never, 0, &abort_flag, limit_ns);
-    if (!ok && lane == 0) {
-        abort_flag = 1;
-        atomicExch(status, ERR_STREAM_WAIT);
+    __syncthreads();
+    const bool first = threadIdx.x < 32;
+    const bool ok = warp_wait(&never, 0, &abort_flag, first ? limit_ns : WAIT_LIMIT_NS);
+    if (!ok && lane == 0) give_up(&abort_flag, status, first ? ERR_STREAM_WAIT : ERR_PLANES_WAIT);
+    if (first) {
+        if (!ok) settle_ring(full, 0, 0, 0);
+        for (int i = lane; i < RING * 2 * PK; i += 32) out[i] = reinterpret_cast<const float*>(ring)[i];
     }
-    if (!ok) settle_ring(full, 0, 0, 0);
-    for (int i = lane; i < RING * 2 * PK; i += 32) out[i] = reinterpret_cast<const float*>(ring)[i];
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -663,10 +665,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
             add_columns<HALF>(acc, tmem + lanes + (unsigned)(2 * BQ + bq + half * HALF));
             add_columns<HALF>(acc, tmem + lanes + (unsigned)(2 * BQ + half * HALF));
         }
-        if (!ok && lane == 0) {
-            abort_flag = 1;
-            atomicExch(status, ERR_SUM_WAIT);
-        }
+        if (!ok && lane == 0) give_up(&abort_flag, status, ERR_CONVERTER_WAIT);
         asm volatile("tcgen05.fence::before_thread_sync;\nbar.sync 0;" ::: "memory");         // every role is done
         const bool good = abort_flag == 0;
         const int row = quarter * 32 + lane, n = n0 + row;
@@ -758,10 +757,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
                 umma_commit(&empty_bar[s]);
                 if (b % CHUNK == CHUNK - 1 || b == blocks - 1) umma_commit(&sum_full[c & 1]);
             }
-            if (!ok && lane == 0) {
-                abort_flag = 1;
-                atomicExch(status, ERR_MMA_WAIT);
-            }
+            if (!ok && lane == 0) give_up(&abort_flag, status, ERR_MMA_WAIT);
             if (b > 0) settle(&empty_bar[(b - 1) & 1], ((b - 1) >> 1) & 1);       // its last products
         }
         if (PLANES && warp == CONVERTERS + 1) {
@@ -782,10 +778,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_parts_kernel(const __grid
                 }
                 __syncwarp();
             }
-            if (!ok && lane == 0) {
-                abort_flag = 1;
-                atomicExch(status, ERR_PLANES_WAIT);
-            }
+            if (!ok && lane == 0) give_up(&abort_flag, status, ERR_PLANES_WAIT);
             // its last copies; converters that have given up never signal these stages: then it waits as long as copies may take
             for (int q = b > 2 ? b - 2 : 0; q < b; ++q) settle(&full_bar[q & 1], (q >> 1) & 1);
         }
@@ -890,7 +883,7 @@ extern "C" int tl_gemm_f32_supports(const void* A, const void* W, int M, int K) 
 extern "C" int tl_gemm_f32_give_up_selftest(const void* W, void* out, int* status, unsigned long long limit_ns, void* stream) {
     CUtensorMap map;
     if (!aligned16(W) || !map_pieces(&map, (const float*)W, 2 * RING, PK)) return TL_BAD_ALIGN;
-    return (int)tl_launch(give_up_selftest_kernel, dim3(1), dim3(32), 0, (cudaStream_t)stream, map, (float*)out, status, limit_ns);
+    return (int)tl_launch(give_up_selftest_kernel, dim3(1), dim3(64), 0, (cudaStream_t)stream, map, (float*)out, status, limit_ns);
 }
 
 // Bytes of scratch (16-byte aligned) that tl_gemm_f32 needs for M rows of K numbers.
