@@ -71,7 +71,9 @@ class LLM:
         build a model with random weights on the device.  ``max_bsz`` is the number of requests
         that may run at once; the cache holds ``max_bsz * max_len`` tokens unless ``kv_memory_fraction``
         (a share of the device memory that is free once the weights are loaded) or ``kv_memory_gb``
-        gives its size in GiB (torchllms/models/networks.py:872-884)."""
+        gives its size in GiB (torchllms/models/networks.py:872-884).  What a step needs besides comes out
+        of the rest: its activations, and in float32 up to 6 bytes a number for the cut inputs of 4,096 rows
+        (50 to 350 MB at 2,048 to 14,336 numbers a row)."""
         if prefix_cache is not None:
             # the reference's argument at its place in the list; this engine keeps no cache of prefixes
             raise ValueError("prefix_cache: this engine has no prefix cache; leave it None")

@@ -1680,15 +1680,16 @@ class NativeOps:
         if x.dtype == torch.float32 and out_dtype == torch.float32 and self._lib("gemm_f32").tl_gemm_f32_supports(_ptr(x), _ptr(w), M, K) == 1:
             lib = self._lib("gemm_f32")
             lib.tl_gemm_f32_scratch.restype = ctypes.c_longlong
-            # (so many rows at a time: they fill the GPU, and what the cut tokens take in memory stays bounded)
+            # so many rows at a time: they fill the GPU, and what the cut tokens take in memory stays bounded (one buffer for
+            # all launches, which follow one another on the stream)
+            scratch = lib.tl_gemm_f32_scratch(min(M, self.F32_ROWS), K)
+            planes = torch.empty(scratch, dtype=torch.uint8, device=x.device) if scratch else None
             for a in range(0, M, self.F32_ROWS):
                 rows = min(M - a, self.F32_ROWS)
-                scratch = lib.tl_gemm_f32_scratch(rows, K)
-                planes = torch.empty(scratch, dtype=torch.uint8, device=x.device) if scratch else None
                 rc = lib.tl_gemm_f32(ctypes.c_void_p(x.data_ptr() + 4 * a * K), _ptr(w), ctypes.c_void_p(out.data_ptr() + 4 * a * N), _ptr(planes),
                                      rows, N, K, ctypes.c_void_p(self._status.data_ptr()), _stream())
                 _check(rc, "gemm_f32")
-                self.launches += 1 if planes is None else 2
+                self.launches += 2 if lib.tl_gemm_f32_scratch(rows, K) else 1
             return out
         rc = self._lib("gemm_simt").tl_gemm_simt(_ptr(x), _ptr(w), _ptr(out), _DT[x.dtype], _DT[out_dtype],
                                                 M, N, K, _stream())
