@@ -125,7 +125,7 @@ def test_gemm_f32_of_more_rows_than_one_launch_takes(ops, M):
 
 
 @pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8])
-@pytest.mark.parametrize("N,K", [(1, 1536), (2, 4096), (149, 1540), (295, 2304), (2369, 2060), (4737, 8196), (40000, 1536)])
+@pytest.mark.parametrize("N,K", [(1, 1536), (2, 4096), (149, 1540), (295, 2304), (2369, 2060), (4737, 8196), (40000, 1536), (8191, 2304), (8192, 2304), (8200, 3076)])
 def test_gemm_f32_streams_rows(ops, M, N, K):
     """Shares of one row, odd shares, shares of several blocks; pieces of K that no warp or two warps have, and ragged ones."""
     x, w = rand((M, K), torch.float32, 25), rand((N, K), torch.float32, 26)

@@ -1,7 +1,7 @@
 // C[M, N] = A[M, K] . W[N, K]^T, everything float32: the projections of the true 32-bit path.  Both operands are K-major as
 // stored and 16-byte aligned with K % 4 == 0 and, for more than 8 rows, K >= 192 (gemm_simt.cu takes the rest).
 //
-// few rows (M <= 8, decode steps): bound by reading W once from HBM; two kernels.  K >= 1,536: a CTA per SM streams an even share
+// few rows (M <= 8, decode steps): bound by reading W once from HBM; two kernels.  K >= 1,536 (save for some lengths, see the end): a CTA per SM streams an even share
 //   of W's rows through rings in shared memory (TMA copies of 2 KB, 96 KB in flight an SM, which start before the kernel ahead has
 //   ended); its eight warps split K.  Less: a warp owns four rows of W and a part of K, four 2 KB pieces in flight in registers.
 //   In both a warp's lanes lie along K, 16 bytes each; sums over lanes are taken by a transposing butterfly, those over
@@ -897,9 +897,14 @@ extern "C" int tl_gemm_f32(const void* A, const void* W, void* C, void* scratch,
     cudaStream_t s = (cudaStream_t)stream;
     const float *a = (const float*)A, *w = (const float*)W;
     float* c = (float*)C;
-    // (a warp of the streaming kernel owns an eighth of K in pieces of 256: below 1,536 half of the warps have nothing to do;
-    // 4 rows against [3072, 1024] 6.3 us, 5.7 in the other kernel, against [3072, 2048] 7.4 and 9.1)
-    if (M <= 8 && K >= 1536) {
+    // A warp of the streaming kernel owns an eighth of K in pieces of 256.  Below 1,536 half of the warps have nothing to do (4 rows
+    // against [3072, 1024] 6.3 us, 5.7 in the other kernel; against [3072, 1536] 6.5 and 7.4).  With nine to twelve pieces some
+    // warps have two and the others, which wait for them, one: a CTA with many rows to go through loses more by that than the
+    // rings gain (4 rows against [16384, 2304] 42.3 and 32.7, [16384, 3072] 47.0 and 41.8, [9216, 3072] 27.6 and 24.3; the other way round
+    // [5120, 3072] 16.7 and 20.0, [3072, 2304] 10.1 and 10.4, [16384, 3328] 46.9 and 45.1 with 4 rows, 40.2 and 42.8 with one; 1 and
+    // 8 rows lie alike).
+    const int pieces = (K + PK - 1) / PK;
+    if (M <= 8 && K >= 1536 && !(pieces > 8 && pieces <= 12 && N >= 8192)) {
         if (M == 1) return launch_stream<1, 16>(a, w, c, status, M, N, K, s);
         if (M == 2) return launch_stream<2, 16>(a, w, c, status, M, N, K, s);
         if (M <= 4) return launch_stream<4, 16>(a, w, c, status, M, N, K, s);
