@@ -388,10 +388,11 @@ int launch_hd(const AttnParams& p, dim3 grid, cudaStream_t s) {
 // one token a request: bound by the latency of a few kilobytes a warp.  A CTA takes the heads of one group and one split of
 //   the keys; its eight warps take batches of keys by themselves, a key on head_dim / 4 lanes, all of a batch's keys and values
 //   (eight 16-byte loads of each a lane) under way at once, scores summed over the lanes by shuffles, one rescaling a batch.
-//   The warps' results meet in shared memory.
+//   The warps' results meet in shared memory.  (Groups of five to eight heads take all 255 registers, nothing is spilled.)
 // portions: bound by the multiply-adds' issue.  32 rows (token, head of the group) against tiles of 64 (head_dim 128: 32) keys
 //   that arrive through cp.async while the tile before is multiplied; a thread holds 4 x 4 scores and 4 x 4 results (4 x 2
-//   and 4 x 8), so that eight 16-byte loads from shared memory feed 64 multiply-adds.
+//   and 4 x 8), so that eight 16-byte loads from shared memory feed 64 multiply-adds.  (The splits are planned for the general
+//   kernel's tiles of 16 rows, so portions get half as many CTAs as the plan aims at.)
 // In a 1B-shaped model (32 heads in groups of four, head_dim 64), a step of 4 requests with 50 to 700 keys 1,889 -> 1,468 us and 300
 // tokens scored 10.0 -> 8.95 ms: 25 us less a layer for the one (this kernel and the merge, which now starts early, took 35),
 // 65 us less for the other (94 before, 25 to 30 of it left).

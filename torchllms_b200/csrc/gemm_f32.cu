@@ -7,7 +7,7 @@
 //   In both a warp's lanes lie along K, 16 bytes each; sums over lanes are taken by a transposing butterfly, those over
 //   warps through shared memory, in a fixed order.  Relative error (2-norm, against 64 bits) 1.0e-7 to
 //   1.6e-7.
-//   4 rows against [16384, 2048] 26.9 us (5.0 TB/s), [2048, 8192] 15.9, [128256, 2048] 177 (5.9 TB/s), [2048, 2048] 5.4; 30.0, 17.0,
+//   4 rows against [16384, 2048] 25.5 us (5.3 TB/s), [2048, 8192] 14.1, [128256, 2048] 177 (5.9 TB/s), [2048, 2048] 5.4; 30.0, 17.0,
 //   194 and 6.4 with the registers' kernel; 210, 557 and 1,161 us for the first three when a 64 x 64 tile per CTA walked K
 //   alone.  One row: 23.3, 13.5, 151 (7.0 TB/s) and 3.8.  What is left with 4 and 8 rows is the multiply-adds and the sums at the end of a block of rows, two warps a
 //   scheduler.
@@ -35,9 +35,9 @@
 //   along K over a cluster of up to eight CTAs that add up through distributed shared memory.  Numbers of 2^111 and more and those that are not
 //   finite have no such parts: the sums that one enters, and no others, are taken again with plain multiply-adds (300 rows against [16384, 2048]
 //   with one infinite token 239 us, without 138).
-//   300 rows against [16384, 2048] 132 us (152 TFLOP/s), [2048, 8192] 82, [128256, 2048] 940; 204, 125 and 1,404 us with the tokens cut
+//   300 rows against [16384, 2048] 127 us (158 TFLOP/s), [2048, 8192] 77, [128256, 2048] 940; 204, 125 and 1,404 us with the tokens cut
 //   by every CTA again, W one stage ahead and six products a step (shared memory carried 270 KB a stage: 180 read by the
-//   products, 92 stored); 866, 828 and 6,397 us with multiply-adds.  64 rows against [16384, 2048] 43.0 and 50.9 us, [3072, 2048] 16.7
+//   products, 92 stored); 866, 828 and 6,397 us with multiply-adds.  64 rows against [16384, 2048] 41.3 and 50.9 us, [3072, 2048] 16.2
 //   and 16.4.
 //
 // In both, the order in which a row's products are added depends on the shapes (the number of rows among them: a row's bits may

@@ -3,6 +3,7 @@
     python -m torchllms_b200.kernels.microbench attention_decode
     python -m torchllms_b200.kernels.microbench attention_prefill --lengths 2048,8192 --impls mma,prefill
     python -m torchllms_b200.kernels.microbench gemm
+    python -m torchllms_b200.kernels.microbench float32 --rows 1,4,8,12,64,300 --tokens 300
     python -m torchllms_b200.kernels.microbench elementwise --tokens 2048
     python -m torchllms_b200.kernels.microbench peaks
     python -m torchllms_b200.kernels.microbench selective_scan --tokens 2048 --channels 4096 --state 16
@@ -19,6 +20,7 @@ summaries under ``profiles/`` quote them.
 from __future__ import annotations
 
 import argparse
+import ctypes
 from typing import Callable, List
 
 import torch
@@ -124,6 +126,45 @@ def gemm(args) -> None:
             ops.check_status()
             print(f"gemm M {M:3d} {name:9s} {N:6d} x {K:5d}: tcgen05 {ours:7.1f} us ({N * K * 2 / ours / 1e6:4.2f} TB/s)   "
                   f"torch.mm {lib:7.1f} us")
+
+
+def float32(args) -> None:
+    """The true 32-bit path of a 1B-shaped decoder: its products beside plain multiply-adds, with both errors against 64
+    bits, and its attention for decoded tokens and for a portion beside the general kernel."""
+    ops = get_ops()
+
+    def plain(x, w, out):
+        M, K = x.shape
+        assert ops._lib("gemm_simt").tl_gemm_simt(*(ctypes.c_void_p(t.data_ptr()) for t in (x, w, out)), 0, 0, M, w.shape[0], K,
+                                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        return out
+
+    for N, K in ((3072, 2048), (16384, 2048), (2048, 8192), (16384, 3072), (512, 192)):
+        copies = max(2, int(300e6 // (N * K * 4)) + 1)
+        ws = [torch.randn(N, K, device="cuda") * 0.02 for _ in range(copies)]
+        for M in (int(x) for x in args.rows.split(",")):
+            x, out = torch.randn(M, K, device="cuda"), torch.empty(M, N, device="cuda")
+            us = _time(_graphed([(lambda w=w: ops.linear(x, w)) for w in ws]), 5) / copies
+            base = _time(_graphed([(lambda w=w: plain(x, w, out)) for w in ws[:2]]), 3) / 2
+            want = x.double() @ ws[0].double().t()
+            off = [((y.double() - want).norm() / want.norm()).item() for y in (ops.linear(x, ws[0]), plain(x, ws[0], out))]
+            ops.check_status()
+            print(f"float32 product M {M:4d} {N:6d} x {K:5d}: {us:7.1f} us ({N * K * 4 / us / 1e6:4.2f} TB/s of weight, {2 * M * N * K / us / 1e6:6.1f} "
+                  f"TFLOP/s) off {off[0]:.1e}   multiply-adds {base:7.1f} us off {off[1]:.1e}")
+        del ws
+    heads, kv, hd, page = 32, 8, 64, 16
+    for B, L, n in ((4, 700, 1), (4, 50, 1), (64, 600, 1), (1, args.tokens, args.tokens), (1, 2048, 2048)):
+        blocks = -(-L // page)
+        table = torch.randperm(B * blocks).int().view(B, blocks).cuda()
+        k, v = (torch.randn(B * blocks, kv, page, hd, device="cuda") for _ in range(2))
+        q = torch.randn(B * n, heads, hd, device="cuda")
+        q_start = torch.arange(0, B * n + 1, n, dtype=torch.int32, device="cuda")
+        kv_len = torch.full((B,), L, dtype=torch.int32, device="cuda")
+        how = dict(n_seqs=B, max_q_len=n, max_kv_len=L, scale=hd ** -0.5, page_size=page)
+        # (a window that holds every key takes the call to the general kernel)
+        us, base = (_time(_graphed([lambda: ops.paged_attention(q, k, v, table, q_start, kv_len, window=window, **how)] * 10), 5) / 10
+                    for window in (None, 1 << 20))
+        print(f"float32 attention {B:3d} x {n:5d} tokens behind {L - n:5d}: {us:7.1f} us   general kernel {base:7.1f} us")
 
 
 def elementwise(args) -> None:
@@ -351,6 +392,10 @@ def main(argv=None) -> None:
     p = sub.add_parser("gemm")
     p.add_argument("--rows", default="8,64")
     p.set_defaults(run=gemm)
+    p = sub.add_parser("float32")
+    p.add_argument("--rows", default="1,4,8,12,64,300")
+    p.add_argument("--tokens", type=int, default=300)
+    p.set_defaults(run=float32)
     p = sub.add_parser("peaks")
     p.set_defaults(run=peaks)
     p = sub.add_parser("selective_scan")
