@@ -1,5 +1,6 @@
 """Each CUDA kernel alone against its plain PyTorch twin, at sizes other than the engine's."""
 
+import ctypes
 import math
 
 import numpy as np
@@ -670,6 +671,38 @@ def test_decode_attention_with_a_given_number_of_splits(ops, case, n_splits):
     ops.check_status()
     torch.testing.assert_close(got.float(), want.float(), atol=2e-2, rtol=2e-2)
     torch.testing.assert_close(got.float(), whole.float(), atol=1e-2, rtol=1e-2)
+
+
+@pytest.mark.parametrize("case", [
+    (64, 600, 1, 32, 8, 128, 16, None),          # a batch of short chats
+    (61, 2500, 1, 32, 8, 64, 16, None),
+    (40, 900, 4, 32, 8, 128, 32, None),          # 16 rows to a tile, requests of one to four tokens
+    (60, 1300, 1, 24, 8, 128, 64, 333),          # behind a window
+    (80, 65, 2, 16, 8, 64, 16, None),            # one piece a request, or two
+    (90, 150, 1, 16, 16, 128, 8, 77),            # more than 64 requests, a head to a group
+], ids=["8b", "hd64", "rows16", "window", "short", "many"])
+def test_decode_attention_in_shares(ops, case):
+    """With more pieces of requests than CTAs run at a time, CTAs take shares of the pieces: bit for bit what a CTA
+    to a piece and the merge give, also a second time (the counters are zero again)."""
+    B, longest, most, H, KV, hd, P, window = case
+    g = torch.Generator().manual_seed(B)
+    q_lens = torch.randint(1, most + 1, (B,), generator=g).tolist()
+    seq_lens = [max(n, int(v)) for n, v in zip(q_lens, torch.randint(1, longest + 1, (B,), generator=g))]
+    seq_lens[3] = longest
+    a = build_paged(seq_lens, q_lens, H, KV, hd, P, torch.bfloat16, seed=B)
+    a["max_kv_len"] = 8192
+    a["block_table"] = torch.nn.functional.pad(a["block_table"], (0, 8192 // P - a["block_table"].shape[1]))
+    n, floats, counters = ctypes.c_int(0), ctypes.c_longlong(0), ctypes.c_longlong(0)
+    rc = ops._lib("attention_decode").tl_attention_decode_plan(sum(q_lens), B, H, KV, hd, a["max_q_len"], 8192, 1, ctypes.byref(n),
+                                                               ctypes.byref(floats), ctypes.byref(counters))
+    assert rc == 0 and n.value > 1 and counters.value == B * KV
+    args = dict(scale=hd ** -0.5, window=window, impl="decode")
+    pieces = ops.paged_attention(**a, **args, allow_split=n.value)
+    for _ in range(2):
+        assert torch.equal(ops.paged_attention(**a, **args), pieces)
+    want = TWIN.paged_attention(**a, scale=hd ** -0.5, window=window)
+    ops.check_status()
+    torch.testing.assert_close(pieces.float(), want.float(), atol=2e-2, rtol=2e-2)       # bfloat16 results of unit values, as above
 
 
 @pytest.mark.parametrize("dtype,impl", IMPLS)

@@ -7,12 +7,21 @@
 // the TMA unit instead of by every thread: the decode step is bound by streaming K and V once
 // from HBM, and issuing 16-byte copies from all threads cost more instructions than the math.
 //
-// A CTA serves one (request, kv head, key split).  Warp 4 is the producer: for every 64-key tile it
-// looks up the pages, and issues cp.async.bulk.tensor copies (no multicast) of [page rows x 64
-// elements] boxes into 128-byte-swizzled shared memory, completing on an mbarrier per stage.
-// Warps 0-3 share the rows and each takes 16 keys of every tile; they hand a stage back through a
-// second mbarrier.  No CTA-wide barrier is used until the four partial results are merged.  Key
-// splits over CTAs write float32 partials that merge_partials_kernel combines.
+// A request's keys may be cut into several pieces (whole tiles, as many pieces as the host plans for the
+// longest context there could be; a shorter request has shorter pieces, or fewer).  Warp 4 of a CTA is the
+// producer: for every 64-key tile it looks up the pages, and issues cp.async.bulk.tensor copies (no
+// multicast) of [page rows x 64 elements] boxes into 128-byte-swizzled shared memory, completing on an
+// mbarrier per stage.  Warps 0-3 share the rows and each takes 16 keys of every tile; they hand a stage back
+// through a second mbarrier.  A piece leaves float32 partials; the pieces of a request are added up in order.
+//
+// Two ways to hand the pieces out.  Where one CTA to a piece fits the GPU in one wave, that is what is
+// launched, and merge_partials_kernel adds up (the weights of the product that follows stream in
+// meanwhile).  With more pieces than CTAs fit (many requests; most pieces are short or empty then) as many
+// CTAs as fit take even shares of the pieces, found on the device from the requests' lengths; the producer
+// runs ahead across the borders of pieces and requests, and the CTA that is last to finish with a request adds
+// its pieces up (a counter per request and kv head).  The sums are the same bit for bit.
+// (64 requests of 320 tokens, 32 / 8 heads of 128, planned for 8,192: 3,072 CTAs, half of them empty, 29.0 us;
+// 444 with shares 23.4 us; 40 requests of 1,000: 31.7 and 31.5; 64 of 2,048, where every piece is long: 86.7 and 86.9.)
 //
 // The products are taken transposed: scores^T = K Q^T and out^T = V^T P^T, so that the 16 rows of
 // a tensor-core tile are keys (or value columns), all of them real, and the few query rows (four
@@ -36,7 +45,8 @@ constexpr int BN = 64;                  // keys per tile
 constexpr int NCW = 4;                  // consumer warps
 constexpr int NTHREADS = (NCW + 1) * 32;
 constexpr int MIN_SPLIT = 128;
-constexpr int MERGE_MAX_SPLITS = 64;
+constexpr int MERGE_MAX_SPLITS = 64;    // pieces of one request's keys, at most
+constexpr int FAILED_PART = 1 << 16;    // what a CTA that gave up adds to a counter beside its 1
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
 constexpr unsigned long long WAIT_NS = 2000ull * 1000ull * 1000ull;
@@ -48,16 +58,19 @@ struct DecodeParams {
     const int* block_table;
     const int* q_start;
     const int* kv_len;
-    float* part_o;   // [T * H, n_splits, head_dim]
-    float* part_ml;  // [T * H, n_splits, 2]
+    float* part_o;   // a CTA to a piece: [T * H, n_splits, head_dim]; shares: [n_seqs * units, n_splits, rows, head_dim]
+    float* part_ml;  // the same with 2 in the place of head_dim: maximum (natural-log scale) and sum
+    int* counters;   // shares: [n_seqs * units], zero between launches
     int* status;
     int table_stride;
     int n_heads, n_kv_heads, page_size, page_shift, box_rows;
     int total_rows;             // rows of the page tensor: a copy that starts there reads only the zero fill
-    int group, ng, n_gchunks, tpw;
+    int group, ng, n_gchunks, units;    // units: kv heads x chunks of a group's heads
+    int n_seqs, max_tokens;     // requests; tokens of a request
+    int rows;                   // rows of a tile in use: max_tokens * ng
+    int n_splits;
     int window;
     int streamed;               // the call reads more keys and values than L2 holds: their copies are marked to leave it first
-    int n_splits;
     float scale_log2;
 };
 
@@ -132,8 +145,120 @@ __device__ __forceinline__ unsigned movmatrix_trans(unsigned a) {     // 8 x 8 b
     return d;
 }
 
+__device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(NCW * 32) : "memory"); }
+
+// What a launch reads of one request's keys.
+struct Span {
+    int lo, hi;      // visible keys lo .. hi - 1 (of any of its tokens)
+    int base;        // position of its first new token
+    int n_tokens;    // 0: the request brings none
+    int piece;       // keys of a piece: whole tiles, or all of them
+    int pieces;      // how many of them have keys (at least one)
+};
+__device__ __forceinline__ Span span_of(const DecodeParams& p, int b) {
+    Span s;
+    const int ql = p.q_start[b + 1] - p.q_start[b];
+    s.base = p.kv_len[b] - ql;
+    s.n_tokens = max(0, min(ql, p.max_tokens));
+    s.lo = p.window > 0 ? max(0, s.base - p.window + 1) : 0;
+    s.hi = s.base + s.n_tokens;
+    const int len = max(s.hi - s.lo, 0);
+    s.piece = p.n_splits > 1 ? max(((len + p.n_splits - 1) / p.n_splits + BN - 1) / BN * BN, BN) : max(len, 1);
+    s.pieces = p.n_splits > 1 ? max((len + s.piece - 1) / s.piece, 1) : 1;
+    return s;
+}
+
+// The pieces a CTA works on, one after the other (every warp walks on its own).
+struct Walk {
+    int b, unit, split;  // request; kv head and chunk of its heads; piece
+    Span span;
+    int lo, hi;          // keys of the piece
+    int start, tiles;    // its tiles: the first starts on a box (page) boundary; keys below lo are masked
+    int at, end;         // shares: places on the line of tiles, of the piece and where the share ends
+    int first_split;     // shares: the first piece of this (request, unit) in the share
+};
+__device__ __forceinline__ void walk_piece(const DecodeParams& p, Walk& w) {
+    w.lo = w.span.lo + w.split * w.span.piece;
+    w.hi = min(w.span.hi, w.lo + w.span.piece);
+    w.start = w.lo & ~(p.box_rows - 1);
+    w.tiles = w.hi > w.start ? (w.hi - w.start + BN - 1) / BN : 0;
+}
+// On to the next piece of the line; false: it belongs to the next share, or there is none.
+__device__ __forceinline__ bool walk_next(const DecodeParams& p, Walk& w) {
+    w.at += w.span.piece / BN;
+    if (++w.split == w.span.pieces) {
+        w.split = 0;
+        if (++w.unit == p.units) {
+            w.unit = 0;
+            do {
+                if (++w.b >= p.n_seqs) return false;
+                w.span = span_of(p, w.b);
+            } while (w.span.n_tokens == 0);
+        }
+        w.first_split = 0;
+    }
+    if (w.at >= w.end) return false;
+    walk_piece(p, w);
+    return true;
+}
+// The first piece of this CTA's share.  All pieces of a request's first unit, of its second and so on, then the next
+// request's, lie on one line, a piece as long as it has tiles; a share is every piece that starts in an equal
+// part of the line.  false: there is none.
+__device__ __forceinline__ bool walk_share(const DecodeParams& p, Walk& w, int lane) {
+    int total = 0;
+    for (int b = lane; b < p.n_seqs; b += 32) {
+        const Span s = span_of(p, b);
+        if (s.n_tokens > 0) total += s.pieces * (s.piece / BN);
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    const int share = (total * p.units + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int begin = blockIdx.x * share;
+    w.end = begin + share;
+    if (begin >= total * p.units) return false;
+    int before = 0;                                     // tiles (of one unit) of the requests before this block of 32
+    for (int b0 = 0; b0 < p.n_seqs; b0 += 32) {
+        int t = 0;
+        if (b0 + lane < p.n_seqs) {
+            const Span s = span_of(p, b0 + lane);
+            if (s.n_tokens > 0) t = s.pieces * (s.piece / BN);
+        }
+        int upto = t;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += v;
+        }
+        const unsigned here = __ballot_sync(0xffffffffu, (before + upto) * p.units > begin);
+        if (here) {
+            const int src = __ffs(here) - 1;            // the first request that reaches beyond the share's start
+            w.b = b0 + src;
+            w.span = span_of(p, w.b);
+            const int request = (before + __shfl_sync(0xffffffffu, upto - t, src)) * p.units;
+            const int wide = w.span.piece / BN, all = w.span.pieces * wide;
+            w.unit = (begin - request) / all;
+            w.split = (begin - request - w.unit * all) / wide;
+            w.at = request + w.unit * all + w.split * wide;
+            w.first_split = w.split;
+            if (w.at == begin) {
+                walk_piece(p, w);
+                return true;
+            }
+            // the piece that the share's start falls into belongs to the share before
+            const int u = w.unit;
+            const int b = w.b;
+            const bool got = walk_next(p, w);
+            if (w.b == b && w.unit == u) w.first_split = w.split;
+            return got;
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return false;
+}
+
 // NT: 8-row blocks of query rows (1: up to 8 rows, 2: up to 16)
-template <int HD, int STAGES, int NT>
+// SHARES: a CTA takes a share of all pieces and the last one adds a request's up; else a CTA to a piece
+// (blockIdx: request z, unit y, piece x), and merge_partials_kernel follows
+template <int HD, int STAGES, int NT, bool SHARES>
 __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                                   const __grid_constant__ CUtensorMap map_v,
                                                                                   const DecodeParams p) {
@@ -147,140 +272,159 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
     constexpr int OPITCH = HD + 4;                      // of the merge buffer: rows two apart fall on different banks
     extern __shared__ unsigned char smem_raw[];
     unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
-    __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(tiles + STAGES * STAGE_BYTES);   // [16][QPITCH]
+    // behind the stages: the queries [NROWS][QPITCH] and, with shares in the same place one after the other, the four
+    // warps' results Om [NCW][rows][OPITCH] and the weights of the pieces [rows][MERGE_MAX_SPLITS].  (With one piece to
+    // a CTA the results lie where the tiles were.)
+    __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(tiles + STAGES * STAGE_BYTES);
+    float* Om = reinterpret_cast<float*>(tiles + (SHARES ? STAGES * STAGE_BYTES : 0));
+    __shared__ float Mm[NCW][NROWS], Lm[NCW][NROWS];
     __shared__ __align__(8) unsigned long long full_bar[STAGES];
     __shared__ __align__(8) unsigned long long empty_bar[STAGES];
     __shared__ int failed_flag;
+    __shared__ int arrived;
 
     grid_launch_dependents();
     // What follows, down to the dependency wait, reads nothing that the kernels just before this one
     // write: the step's index data were uploaded before its first kernel, and keys and values of
     // positions before the step's own tokens were written by earlier steps.  Under programmatic
     // dependent launch this part runs while the predecessor is still at work.
-    const int b = blockIdx.z;
-    const int qs = p.q_start[b];
-    const int ql = p.q_start[b + 1] - qs;
-    const int kl = p.kv_len[b];
-    const int tile = blockIdx.x / p.n_splits;
-    const int split = blockIdx.x - tile * p.n_splits;
-    const int tok0 = tile * p.tpw;
-    if (tok0 >= ql) return;
-    const int kvh = blockIdx.y / p.n_gchunks;
-    const int g0 = (blockIdx.y - kvh * p.n_gchunks) * p.ng;
-    const int ng = min(p.ng, p.group - g0);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     volatile int* failed = &failed_flag;
-
-    // ---- which keys this CTA walks: its share of the request's visible keys, in whole tiles
-    const int cta_tok_hi = min(ql, tok0 + p.tpw);
-    const int qpos_base = kl - ql;
-    int k_lo = p.window > 0 ? max(0, qpos_base + tok0 - p.window + 1) : 0;
-    int k_hi = qpos_base + cta_tok_hi;
-    if (p.n_splits > 1) {
-        const int len = max(k_hi - k_lo, 0);
-        const int chunk = ((len + p.n_splits - 1) / p.n_splits + BN - 1) / BN * BN;
-        const int lo = k_lo + split * chunk;
-        k_hi = min(k_hi, lo + chunk);
-        k_lo = lo;
-    }
-    const int k_start = k_lo & ~(p.box_rows - 1);      // copies start on a box (page) boundary; keys below k_lo are masked
-    const int n_tiles = k_hi > k_start ? (k_hi - k_start + BN - 1) / BN : 0;
-    const int* table = p.block_table + (size_t)b * p.table_stride;
-
-    // one tile: a box per page (or per 64 rows of a larger page) and 64-element column block, K and V.
-    // The whole producer warp issues it, a lane to a box: the page lookups go side by side.
-    auto issue_tile = [&](int it) {
-        const int s = it % STAGES;
-        const int k0 = k_start + it * BN;
-        if (lane == 0) mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-        __syncwarp();
-        unsigned char* kt = tiles + s * STAGE_BYTES;
-        for (int c = lane; c < BN / p.box_rows; c += 32) {
-            const int kpos = k0 + c * p.box_rows;
-            // boxes past the last key start outside the tensor: the copy writes the zero fill, so
-            // that what is multiplied by probability 0 there is finite
-            int row = p.total_rows;
-            if (kpos < k_hi) {
-                const int page = table[kpos >> p.page_shift];
-                if (tl_check_page(page))                           // (debug builds: a bad page reads as the zero fill)
-                    row = (page * p.n_kv_heads + kvh) * p.page_size + (kpos & (p.page_size - 1));
-            }
-#pragma unroll
-            for (int h = 0; h < HALVES; ++h) {
-                unsigned char* dst = kt + h * HALF_BYTES + c * p.box_rows * 128;
-                if (p.streamed) {
-                    tma_load_2d_streamed(dst, &map_k, &full_bar[s], h * 64, row);
-                    tma_load_2d_streamed(dst + KV_BYTES, &map_v, &full_bar[s], h * 64, row);
-                } else {
-                    tma_load_2d(dst, &map_k, &full_bar[s], h * 64, row);
-                    tma_load_2d(dst + KV_BYTES, &map_v, &full_bar[s], h * 64, row);
-                }
-            }
-        }
-        __syncwarp();
-    };
-
-    if (warp == NCW) {
-        // the producer warp sets the barriers up and sends the first tiles on their way while the
-        // other warps are still fetching the queries
-        if (lane == 0) {
-            failed_flag = 0;
-            for (int s = 0; s < STAGES; ++s) {
-                mbar_init(&full_bar[s], 1);
-                mbar_init(&empty_bar[s], NCW);
-            }
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        __syncwarp();
-        // tiles that end before the step's first new position can go now; a tile that may hold a key
-        // written by the predecessor (only the last tile of the last split can) waits for it
-        int it = 0;
-        for (; it < STAGES && it < n_tiles && k_start + (it + 1) * BN <= qpos_base; ++it) issue_tile(it);
-        grid_dependency_wait();
-        for (; it < STAGES && it < n_tiles; ++it) issue_tile(it);
+    Walk w;
+    if (SHARES) {
+        if (!walk_share(p, w, lane)) return;            // (the same for all warps)
     } else {
-        grid_dependency_wait();
+        w.b = blockIdx.z;
+        w.unit = blockIdx.y;
+        w.split = blockIdx.x;
+        w.span = span_of(p, w.b);
+        if (w.span.n_tokens == 0) return;
+        walk_piece(p, w);
     }
-    // queries (zero rows where the tile has none)
-    for (int c = tid; c < 16 * (HD / 8); c += NTHREADS) {
-        const int rr = c / (HD / 8), part = c - rr * (HD / 8);
-        const int tok = tok0 + rr / ng;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (rr < p.tpw * ng && tok < ql) {
-            const int head = kvh * p.group + g0 + rr % ng;
-            v = *reinterpret_cast<const uint4*>(p.q + ((size_t)(qs + tok) * p.n_heads + head) * HD + part * 8);
+    if (tid == NCW * 32) {
+        failed_flag = 0;
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], NCW);
         }
-        *reinterpret_cast<uint4*>(Qs + rr * QPITCH + part * 8) = v;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
 
-    // this thread's two query rows of every 8-row block are 2t and 2t + 1: of the scores^T tile it
-    // holds keys g and g + 8 for them, of the out^T tile value columns g and g + 8
-    float m[NT][2], l[NT][2];
-    float o[NT][KSTEPS][4];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt) {
-        m[nt][0] = m[nt][1] = -INFINITY;
-        l[nt][0] = l[nt][1] = 0.f;
-#pragma unroll
-        for (int i = 0; i < KSTEPS; ++i) o[nt][i][0] = o[nt][i][1] = o[nt][i][2] = o[nt][i][3] = 0.f;
-    }
-    const int g = lane >> 2, t = lane & 3;
-
     if (warp == NCW) {
-        // ---- producer: the first tiles are on their way; keep the ring full
-        for (int it = STAGES; it < n_tiles; ++it) {
-            if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[it % STAGES], ((it / STAGES) - 1) & 1, failed))) {
-                if (lane == 0) {
-                    failed_flag = 1;
-                    atomicExch(p.status, ERR_PRODUCER_WAIT);
+        // ---- producer: a box per page (or per 64 rows of a larger page) and 64-element column block,
+        // K and V.  The whole warp issues a tile, a lane to a box: the page lookups go side by side.
+        bool waited = false;
+        int it = 0;
+        bool ok = true;
+        do {
+            const int kvh = w.unit / p.n_gchunks;
+            const int* table = p.block_table + (size_t)w.b * p.table_stride;
+            for (int i = 0; i < w.tiles && ok; ++i, ++it) {
+                const int s = it % STAGES;
+                const int k0 = w.start + i * BN;
+                // the first tiles go at once, up to one that may hold a key written by the predecessor
+                if (!waited && (it >= STAGES || k0 + BN > w.span.base)) {
+                    grid_dependency_wait();
+                    waited = true;
                 }
-                break;
+                if (it >= STAGES && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ((it / STAGES) - 1) & 1, failed))) {
+                    if (lane == 0) {
+                        failed_flag = 1;
+                        atomicExch(p.status, ERR_PRODUCER_WAIT);
+                    }
+                    ok = false;
+                    break;
+                }
+                if (lane == 0) mbar_expect_tx(&full_bar[s], STAGE_BYTES);
+                __syncwarp();
+                unsigned char* kt = tiles + s * STAGE_BYTES;
+                for (int c = lane; c < BN / p.box_rows; c += 32) {
+                    const int kpos = k0 + c * p.box_rows;
+                    // boxes past the last key start outside the tensor: the copy writes the zero fill, so
+                    // that what is multiplied by probability 0 there is finite
+                    int row = p.total_rows;
+                    if (kpos < w.hi) {
+                        const int page = table[kpos >> p.page_shift];
+                        if (tl_check_page(page))                       // (debug builds: a bad page reads as the zero fill)
+                            row = (page * p.n_kv_heads + kvh) * p.page_size + (kpos & (p.page_size - 1));
+                    }
+#pragma unroll
+                    for (int h = 0; h < HALVES; ++h) {
+                        unsigned char* dst = kt + h * HALF_BYTES + c * p.box_rows * 128;
+                        if (p.streamed) {
+                            tma_load_2d_streamed(dst, &map_k, &full_bar[s], h * 64, row);
+                            tma_load_2d_streamed(dst + KV_BYTES, &map_v, &full_bar[s], h * 64, row);
+                        } else {
+                            tma_load_2d(dst, &map_k, &full_bar[s], h * 64, row);
+                            tma_load_2d(dst + KV_BYTES, &map_v, &full_bar[s], h * 64, row);
+                        }
+                    }
+                }
+                __syncwarp();
             }
-            issue_tile(it);
+        } while (SHARES && ok && walk_next(p, w));
+        if (!waited) grid_dependency_wait();
+        // (nothing that is still on its way may land in shared memory that is no longer this CTA's)
+        int never = 0;
+        for (int k = max(0, it - STAGES); k < it; ++k) mbar_wait(&full_bar[k % STAGES], (k / STAGES) & 1, &never);
+        return;
+    }
+
+    // ---- consumers: the same rows, 16 keys of every tile each
+    grid_dependency_wait();
+    const int g = lane >> 2, t = lane & 3, mi = lane >> 3;
+    const int key_off = warp * 16;
+    // this lane's row and first chunk inside a tile: K as the 16-row operand [keys x 16 columns],
+    // V through a transposing load as [16 columns x keys]
+    const int k_row = key_off + (lane & 7) + ((mi & 1) ? 8 : 0);
+    const int v_row = key_off + (lane & 7) + ((mi & 2) ? 8 : 0);
+    const unsigned k_lane_off = swz(k_row, (mi & 2) ? 1 : 0);
+    const unsigned v_lane_off = swz(v_row, mi & 1);
+    bool ok = true, fresh = true;
+    unsigned qf[NT][KSTEPS][2];
+    int it = 0;
+    do {
+        const int kvh = w.unit / p.n_gchunks;
+        const int g0 = (w.unit - kvh * p.n_gchunks) * p.ng;
+        const int ng = min(p.ng, p.group - g0);
+        const int n_rows = w.span.n_tokens * ng;
+        const int qs = p.q_start[w.b];
+        const int k_lo = w.lo, k_hi = w.hi, base = w.span.base;
+        // queries (zero rows where the tile has none); the next pieces of a request find them in registers
+        if (fresh) {
+            for (int c = tid; c < NROWS * (HD / 8); c += NCW * 32) {
+                const int rr = c / (HD / 8), part = c - rr * (HD / 8);
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (rr < n_rows) {
+                    const int head = kvh * p.group + g0 + rr % ng;
+                    v = *reinterpret_cast<const uint4*>(p.q + ((size_t)(qs + rr / ng) * p.n_heads + head) * HD + part * 8);
+                }
+                *reinterpret_cast<uint4*>(Qs + rr * QPITCH + part * 8) = v;
+            }
+            consumers_sync();
+            // Q^T as the 8-wide operand: this thread holds columns 2t, 2t + 1 (and + 8) of row g
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int kd2 = 0; kd2 < KSTEPS / 2; ++kd2) {
+                    unsigned r[4];
+                    ldmatrix_x4(r, smem_u32(Qs + (nt * 8 + (lane & 7)) * QPITCH + (kd2 * 4 + mi) * 8));
+                    qf[nt][2 * kd2][0] = r[0]; qf[nt][2 * kd2][1] = r[1];
+                    qf[nt][2 * kd2 + 1][0] = r[2]; qf[nt][2 * kd2 + 1][1] = r[3];
+                }
         }
-    } else {
-        // ---- consumers: the same rows, 16 keys of every tile each
+        // this thread's two query rows of every 8-row block are 2t and 2t + 1: of the scores^T tile it
+        // holds keys g and g + 8 for them, of the out^T tile value columns g and g + 8
+        float m[NT][2], l[NT][2];
+        float o[NT][KSTEPS][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            m[nt][0] = m[nt][1] = -INFINITY;
+            l[nt][0] = l[nt][1] = 0.f;
+#pragma unroll
+            for (int i = 0; i < KSTEPS; ++i) o[nt][i][0] = o[nt][i][1] = o[nt][i][2] = o[nt][i][3] = 0.f;
+        }
         int qpos[NT][2];
         int qmax = -1, qmin = INT_MAX;
 #pragma unroll
@@ -288,41 +432,23 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int rr = nt * 8 + 2 * t + j;
-                const int tok = tok0 + rr / ng;
-                const int qp = (rr < p.tpw * ng && tok < ql) ? qpos_base + tok : -1;
+                const int qp = rr < n_rows ? base + rr / ng : -1;
                 qpos[nt][j] = qp;
                 qmax = max(qmax, qp);
                 if (qp >= 0) qmin = min(qmin, qp);
             }
         const int warp_qmax = __reduce_max_sync(0xffffffffu, qmax);
         const int warp_qmin = __reduce_min_sync(0xffffffffu, qmin);
-        // Q^T as the 8-wide operand: this thread holds columns 2t, 2t + 1 (and + 8) of row g
-        unsigned qf[NT][KSTEPS][2];
-        const int mi = lane >> 3;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int kd2 = 0; kd2 < KSTEPS / 2; ++kd2) {
-                unsigned r[4];
-                ldmatrix_x4(r, smem_u32(Qs + (nt * 8 + (lane & 7)) * QPITCH + (kd2 * 4 + mi) * 8));
-                qf[nt][2 * kd2][0] = r[0]; qf[nt][2 * kd2][1] = r[1];
-                qf[nt][2 * kd2 + 1][0] = r[2]; qf[nt][2 * kd2 + 1][1] = r[3];
-            }
-        const int key_off = warp * 16;
-        // this lane's row and first chunk inside a tile: K as the 16-row operand [keys x 16 columns],
-        // V through a transposing load as [16 columns x keys]
-        const int k_row = key_off + (lane & 7) + ((mi & 1) ? 8 : 0);
-        const int v_row = key_off + (lane & 7) + ((mi & 2) ? 8 : 0);
-        const unsigned k_lane_off = swz(k_row, (mi & 2) ? 1 : 0);
-        const unsigned v_lane_off = swz(v_row, mi & 1);
-        bool ok = true;
-        for (int it = 0; it < n_tiles; ++it) {
+        for (int i = 0; i < w.tiles; ++i, ++it) {
             const int s = it % STAGES;
-            if (!mbar_wait(&full_bar[s], (it / STAGES) & 1, failed)) {
+            if (ok && !mbar_wait(&full_bar[s], (it / STAGES) & 1, failed)) {
                 ok = false;
-                break;
+                failed_flag = 1;
+                if (lane == 0) atomicExch(p.status, ERR_CONSUMER_WAIT);
             }
-            const int share_lo = k_start + it * BN + key_off;
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            const int share_lo = w.start + i * BN + key_off;
             if (share_lo <= warp_qmax && share_lo + 16 > k_lo) {
                 const unsigned kt = smem_u32(tiles + s * STAGE_BYTES);
                 // rows are 128 bytes and tiles 1024-byte aligned, so bits 4-6 of a row's address are the
@@ -375,9 +501,9 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                     }
                     if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
-                        for (int i = 0; i < KSTEPS; ++i) {
-                            o[nt][i][0] *= alpha[0]; o[nt][i][1] *= alpha[1];
-                            o[nt][i][2] *= alpha[0]; o[nt][i][3] *= alpha[1];
+                        for (int d = 0; d < KSTEPS; ++d) {
+                            o[nt][d][0] *= alpha[0]; o[nt][d][1] *= alpha[1];
+                            o[nt][d][2] *= alpha[0]; o[nt][d][3] *= alpha[1];
                         }
                     }
                     // probabilities as value + remainder in bfloat16 (the product keeps 16 bits of them),
@@ -405,10 +531,6 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_bar[s]);     // this warp is done with the stage
         }
-        if (!__all_sync(0xffffffffu, ok) && lane == 0) {
-            failed_flag = 1;
-            atomicExch(p.status, ERR_CONSUMER_WAIT);
-        }
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -417,67 +539,133 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                 l[nt][j] += __shfl_xor_sync(0xffffffffu, l[nt][j], 8);
                 l[nt][j] += __shfl_xor_sync(0xffffffffu, l[nt][j], 16);
             }
-    }
 
-    // ---- merge the four warps' partials through shared memory (the stages are done with)
-    __syncthreads();
-    if (failed_flag) return;
-    float* Om = reinterpret_cast<float*>(tiles);          // [NCW][NROWS][OPITCH]
-    float* Mm = Om + NCW * NROWS * OPITCH;                // [NCW][NROWS]
-    float* Lm = Mm + NCW * NROWS;                         // [NCW][NROWS]
-    if (warp < NCW) {
+        // ---- the four warps' results, through shared memory (all have read the queries and the tiles)
+        consumers_sync();
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-            for (int dp = 0; dp < KSTEPS; ++dp)
+            for (int j = 0; j < 2; ++j) {
+                const int rr = nt * 8 + 2 * t + j;
+                if (rr < n_rows) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    Om[(warp * NROWS + nt * 8 + 2 * t + (e & 1)) * OPITCH + dp * 16 + g + 8 * (e >> 1)] = o[nt][dp][e];
-            if (g == 0) {
+                    for (int dp = 0; dp < KSTEPS; ++dp) {
+                        Om[(warp * p.rows + rr) * OPITCH + dp * 16 + g] = o[nt][dp][j];
+                        Om[(warp * p.rows + rr) * OPITCH + dp * 16 + g + 8] = o[nt][dp][j + 2];
+                    }
+                    if (g == 0) {
+                        Mm[warp][rr] = m[nt][j];
+                        Lm[warp][rr] = l[nt][j];
+                    }
+                }
+            }
+        consumers_sync();
+        const bool sound = !*failed;
+        const int parts = SHARES ? w.span.pieces : p.n_splits;
+        if (sound) {
+            for (int idx = tid; idx < n_rows * (HD / 4); idx += NCW * 32) {      // four columns of a row per turn
+                const int rr = idx / (HD / 4), d = (idx - rr * (HD / 4)) * 4;
+                float M = -INFINITY;
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    Mm[warp * NROWS + nt * 8 + 2 * t + j] = m[nt][j];
-                    Lm[warp * NROWS + nt * 8 + 2 * t + j] = l[nt][j];
+                for (int v = 0; v < NCW; ++v) M = fmaxf(M, Mm[v][rr]);
+                float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+                float den = 0.f;
+#pragma unroll
+                for (int v = 0; v < NCW; ++v) {
+                    const float mv = Mm[v][rr], lv = Lm[v][rr];
+                    if (mv == -INFINITY) continue;
+                    const float f = exp2f(mv - M);
+                    const float4 o4 = *reinterpret_cast<const float4*>(Om + (v * p.rows + rr) * OPITCH + d);
+                    num.x = fmaf(f, o4.x, num.x); num.y = fmaf(f, o4.y, num.y);
+                    num.z = fmaf(f, o4.z, num.z); num.w = fmaf(f, o4.w, num.w);
+                    den = fmaf(f, lv, den);
+                }
+                if (parts == 1) {
+                    const float inv = den > 0.f ? 1.f / den : 0.f;
+                    uint2 w2;
+                    w2.x = pack_bf16(num.x * inv, num.y * inv);
+                    w2.y = pack_bf16(num.z * inv, num.w * inv);
+                    const int head = kvh * p.group + g0 + rr % ng;
+                    *reinterpret_cast<uint2*>(p.out + ((size_t)(qs + rr / ng) * p.n_heads + head) * HD + d) = w2;
+                } else {
+                    const int head = kvh * p.group + g0 + rr % ng;
+                    const size_t place = SHARES ? (((size_t)w.b * p.units + w.unit) * p.n_splits + w.split) * p.rows + rr
+                                                : ((size_t)(qs + rr / ng) * p.n_heads + head) * p.n_splits + w.split;
+                    __stcg(reinterpret_cast<float4*>(p.part_o + place * HD + d), num);
+                    if (d == 0) __stcg(reinterpret_cast<float2*>(p.part_ml + place * 2), make_float2(M == -INFINITY ? -INFINITY : M * LN2, den));   // natural-log scale
                 }
             }
         }
-    }
-    __syncthreads();
-    const int n_rows = min(p.tpw, ql - tok0) * ng;
-    for (int idx = tid; idx < n_rows * (HD / 4); idx += NTHREADS) {      // four columns of a row per turn
-        const int rr = idx / (HD / 4), d = (idx - rr * (HD / 4)) * 4;
-        float M = -INFINITY;
+        // ---- whoever is last with a request's pieces adds them up (in order, as merge_partials_kernel does)
+        const bool last_here = SHARES && (w.split + 1 == parts || w.at + w.span.piece / BN >= w.end);
+        if (SHARES && parts > 1 && last_here) {
+            consumers_sync();
+            const int mine = w.split + 1 - w.first_split;
+            int seen = mine;
+            if (mine < parts) {
+                int* counter = p.counters + (size_t)w.b * p.units + w.unit;
+                if (tid == 0) {
+                    // (release what the barrier has gathered of all threads' stores, acquire what the others released)
+                    const int add = sound ? mine : mine + FAILED_PART;
+                    int before;
+                    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(before) : "l"(counter), "r"(add) : "memory");
+                    arrived = before + add;
+                    if (((before + add) & (FAILED_PART - 1)) == parts) *counter = 0;
+                }
+                consumers_sync();
+                seen = arrived;
+            } else if (!sound) {
+                seen = FAILED_PART;
+            }
+            if (seen == parts) {
+                float* weight = Om;                                          // [rows][MERGE_MAX_SPLITS]
+                const size_t place0 = ((size_t)w.b * p.units + w.unit) * p.n_splits * p.rows;
+                for (int rr = warp; rr < n_rows; rr += NCW) {
+                    float2 ml[MERGE_MAX_SPLITS / 32];
+                    float M = -INFINITY, den = 0.f;
 #pragma unroll
-        for (int w = 0; w < NCW; ++w) M = fmaxf(M, Mm[w * NROWS + rr]);
-        float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
-        float den = 0.f;
+                    for (int i = 0; i < MERGE_MAX_SPLITS / 32; ++i) {
+                        const int c = i * 32 + lane;
+                        ml[i] = make_float2(-INFINITY, 0.f);
+                        if (c < parts) ml[i] = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (place0 + (size_t)c * p.rows + rr) * 2));
+                        M = fmaxf(M, ml[i].x);
+                    }
+                    M = warp_max(M);
 #pragma unroll
-        for (int w = 0; w < NCW; ++w) {
-            const float mw = Mm[w * NROWS + rr];
-            if (mw == -INFINITY) continue;
-            const float f = exp2f(mw - M);
-            const float4 o4 = *reinterpret_cast<const float4*>(Om + (w * NROWS + rr) * OPITCH + d);
-            num.x = fmaf(f, o4.x, num.x); num.y = fmaf(f, o4.y, num.y);
-            num.z = fmaf(f, o4.z, num.z); num.w = fmaf(f, o4.w, num.w);
-            den = fmaf(f, Lm[w * NROWS + rr], den);
-        }
-        const int tok = qs + tok0 + rr / ng;
-        const int head = kvh * p.group + g0 + rr % ng;
-        const size_t row = (size_t)tok * p.n_heads + head;
-        if (p.n_splits == 1) {
-            const float inv = den > 0.f ? 1.f / den : 0.f;
-            uint2 w2;
-            w2.x = pack_bf16(num.x * inv, num.y * inv);
-            w2.y = pack_bf16(num.z * inv, num.w * inv);
-            *reinterpret_cast<uint2*>(p.out + row * HD + d) = w2;
-        } else {
-            *reinterpret_cast<float4*>(p.part_o + (row * p.n_splits + split) * HD + d) = num;
-            if (d == 0) {
-                p.part_ml[(row * p.n_splits + split) * 2] = (M == -INFINITY) ? -INFINITY : M * LN2;   // natural-log scale
-                p.part_ml[(row * p.n_splits + split) * 2 + 1] = den;
+                    for (int i = 0; i < MERGE_MAX_SPLITS / 32; ++i) {
+                        const int c = i * 32 + lane;
+                        const float f = ml[i].x == -INFINITY ? 0.f : __expf(ml[i].x - M);
+                        if (c < parts) weight[rr * MERGE_MAX_SPLITS + c] = f;
+                        den = fmaf(f, ml[i].y, den);
+                    }
+                    den = warp_sum(den);
+                    if (lane == 0) Lm[0][rr] = den;
+                }
+                consumers_sync();
+                for (int idx = tid; idx < n_rows * (HD / 4); idx += NCW * 32) {
+                    const int rr = idx / (HD / 4), d = (idx - rr * (HD / 4)) * 4;
+                    float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+                    for (int c = 0; c < parts; ++c) {
+                        const float f = weight[rr * MERGE_MAX_SPLITS + c];
+                        const float4 o4 = __ldcg(reinterpret_cast<const float4*>(p.part_o + (place0 + (size_t)c * p.rows + rr) * HD + d));
+                        num.x = fmaf(f, o4.x, num.x); num.y = fmaf(f, o4.y, num.y);
+                        num.z = fmaf(f, o4.z, num.z); num.w = fmaf(f, o4.w, num.w);
+                    }
+                    const float den = Lm[0][rr];
+                    const float inv = den > 0.f ? 1.f / den : 0.f;
+                    uint2 w2;
+                    w2.x = pack_bf16(num.x * inv, num.y * inv);
+                    w2.y = pack_bf16(num.z * inv, num.w * inv);
+                    const int head = kvh * p.group + g0 + rr % ng;
+                    *reinterpret_cast<uint2*>(p.out + ((size_t)(qs + rr / ng) * p.n_heads + head) * HD + d) = w2;
+                }
             }
         }
-    }
+        if (!SHARES) return;
+        fresh = w.split + 1 == parts;
+        consumers_sync();            // the place behind the stages is the next piece's
+    } while (walk_next(p, w));
 }
 
 // out[row, d] = sum_i e^{m_i - M} o_i[d] / sum_i e^{m_i - M} l_i,  M = max_i m_i: the weights are
@@ -565,8 +753,31 @@ template <int HD> constexpr size_t smem_for() {
     return (size_t)stages_for<HD>() * 2 * (HD / 64) * BN * 128 + 16 * (HD + 8) * 2 + 1024;
 }
 
+// with shares: the warps' results lie behind the stages (`rows`: rows of a tile in use)
+template <int HD> constexpr size_t smem_shares(int rows) {
+    const size_t queries = (size_t)(rows <= 8 ? 8 : 16) * (HD + 8) * 2, results = (size_t)NCW * rows * (HD + 4) * 4;
+    return (size_t)stages_for<HD>() * 2 * (HD / 64) * BN * 128 + (queries > results ? queries : results) + 1024;
+}
+static_assert(NCW * (64 + 4) >= MERGE_MAX_SPLITS, "the pieces' weights lie where the warps' results were");
+
+template <int HD, int NT> int shares_per_sm(int rows) {
+    static int known[17] = {};                     // (threads that come here at the same time write the same)
+    if (known[rows] == 0) {
+        auto kern = attention_decode_kernel<HD, stages_for<HD>(), NT, true>;
+        int n = 0;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_shares<HD>(8 * NT)) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, NTHREADS, smem_shares<HD>(rows)) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            n = 1;
+        }
+        known[rows] = n;
+    }
+    return known[rows];
+}
+
 struct Plan {
     int ng, n_gchunks, tpw, n_q_tiles, n_splits;
+    int shares;        // CTAs that take shares of the pieces; 0: a CTA to a piece
 };
 
 bool takes(int n_heads, int n_kv_heads, int head_dim, int page_size, int max_q_len) {
@@ -576,6 +787,12 @@ bool takes(int n_heads, int n_kv_heads, int head_dim, int page_size, int max_q_l
     const int group = n_heads / n_kv_heads;
     const int ng = group < 16 ? group : 16;
     return max_q_len >= 1 && max_q_len <= 16 / ng;
+}
+
+// with a CTA to a piece
+int ctas_per_sm(int head_dim) {
+    const int fit = (int)((size_t)224 * 1024 / ((head_dim == 128 ? smem_for<128>() : smem_for<64>()) + 1024));
+    return fit > 6 ? 6 : fit;
 }
 
 Plan make_plan(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int max_q_len, int max_kv_len, int allow_split) {
@@ -595,10 +812,7 @@ Plan make_plan(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int max_q_
         // CTAs with long walks leave most of the memory system idle: one request of 8,192 keys
         // takes 21.8 us in 8 splits and 11.2 us in 32); beyond one wave each split is charged
         // for its partial results and the merge.
-        const size_t per_cta = head_dim == 128 ? smem_for<128>() : smem_for<64>();
-        int per_sm = (int)((size_t)224 * 1024 / (per_cta + 1024));
-        if (per_sm > 6) per_sm = 6;
-        const long long slots = 148LL * per_sm;
+        const long long slots = 148LL * ctas_per_sm(head_dim);
         const long long base = (long long)pl.n_q_tiles * n_kv_heads * pl.n_gchunks * n_seqs;
         int most = max_kv_len / MIN_SPLIT;
         if (most > MERGE_MAX_SPLITS) most = MERGE_MAX_SPLITS;
@@ -612,20 +826,31 @@ Plan make_plan(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int max_q_
             }
         }
     }
+    // More than one wave of CTAs, planned for the longest context there could be: most of them would find few keys, or
+    // none.  (Within one wave shares lose: 24 requests of up to 1,900 tokens, 32 / 8 heads of 64, 576 CTAs: a step of 3,335
+    // us took 3,433.)
+    pl.shares = 0;
+    if (allow_split == 1 && pl.n_splits > 1 && (long long)n_kv_heads * pl.n_gchunks * n_seqs * pl.n_splits > 148LL * ctas_per_sm(head_dim)) {
+        const int rows = max_q_len * pl.ng;
+        pl.shares = 148 * (head_dim == 128 ? (rows <= 8 ? shares_per_sm<128, 1>(rows) : shares_per_sm<128, 2>(rows))
+                                           : (rows <= 8 ? shares_per_sm<64, 1>(rows) : shares_per_sm<64, 2>(rows)));
+    }
     return pl;
 }
 
 template <int HD, int NT>
-int launch(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, dim3 grid, cudaStream_t s) {
+int launch(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, const Plan& pl, cudaStream_t s) {
+    if (pl.shares > 0)          // (shares_per_sm has raised the limit on shared memory)
+        return (int)tl_launch(attention_decode_kernel<HD, stages_for<HD>(), NT, true>, dim3(pl.shares), dim3(NTHREADS), smem_shares<HD>(p.rows), s, mk, mv, p);
     constexpr size_t smem = smem_for<HD>();
-    auto kern = attention_decode_kernel<HD, stages_for<HD>(), NT>;
+    auto kern = attention_decode_kernel<HD, stages_for<HD>(), NT, false>;
     static bool raised = false;
     if (!raised) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         raised = true;
     }
-    return (int)tl_launch(kern, grid, dim3(NTHREADS), smem, s, mk, mv, p);
+    return (int)tl_launch(kern, dim3(pl.n_splits, p.units, p.n_seqs), dim3(NTHREADS), smem, s, mk, mv, p);
 }
 
 }  // namespace
@@ -636,20 +861,25 @@ extern "C" int tl_attention_decode_supports(int n_heads, int n_kv_heads, int hea
     return takes(n_heads, n_kv_heads, head_dim, page_size, max_q_len) ? 1 : 0;
 }
 
+// What a call needs beside its operands: n_splits pieces of a request's keys, workspace_floats of scratch, and
+// n_counters ints that are zero (and are zero again when the call has run); with counters there is one launch, else
+// there are two when n_splits is over 1.
 extern "C" int tl_attention_decode_plan(int n_tokens, int n_seqs, int n_heads, int n_kv_heads, int head_dim,
                                         int max_q_len, int max_kv_len, int allow_split,
-                                        int* n_splits, long long* workspace_floats) {
+                                        int* n_splits, long long* workspace_floats, long long* n_counters) {
     if (!takes(n_heads, n_kv_heads, head_dim, 16, max_q_len)) return TL_BAD_SIZE;
     const Plan pl = make_plan(n_seqs, n_heads, n_kv_heads, head_dim, max_q_len, max_kv_len, allow_split);
+    const long long units = (long long)n_kv_heads * pl.n_gchunks * n_seqs;
     *n_splits = pl.n_splits;
-    *workspace_floats = pl.n_splits > 1 ? (long long)n_tokens * n_heads * pl.n_splits * (head_dim + 2) : 0;
+    *workspace_floats = pl.n_splits <= 1 ? 0 : (pl.shares > 0 ? units * max_q_len * pl.ng : (long long)n_tokens * n_heads) * pl.n_splits * (head_dim + 2);
+    *n_counters = pl.shares > 0 ? units : 0;
     return TL_OK;
 }
 
 // Same arguments as tl_paged_attention_mma; n_pages is the first extent of the page tensors.
 extern "C" int tl_paged_attention_decode(const void* q, const void* k_pages, const void* v_pages, void* out,
                                          const int* block_table, int table_stride, const int* q_start,
-                                         const int* kv_len, float* workspace, int* status, int n_tokens, int n_seqs,
+                                         const int* kv_len, float* workspace, int* counters, int* status, int n_tokens, int n_seqs,
                                          int n_heads, int n_kv_heads, int head_dim, int page_size, long long n_pages,
                                          int max_q_len, int max_kv_len, int window, float scale, int allow_split,
                                          void* stream) {
@@ -658,19 +888,21 @@ extern "C" int tl_paged_attention_decode(const void* q, const void* k_pages, con
     if (n_pages * n_kv_heads * page_size >= (1LL << 31)) return TL_BAD_SIZE;
     if (!aligned16(q) || !aligned16(k_pages) || !aligned16(v_pages) || !aligned16(out) || status == nullptr) return TL_BAD_ALIGN;
     const Plan pl = make_plan(n_seqs, n_heads, n_kv_heads, head_dim, max_q_len, max_kv_len, allow_split);
-    if (pl.n_splits > 1 && workspace == nullptr) return TL_BAD_SIZE;
+    if (pl.n_splits > 1 && (workspace == nullptr || !aligned16(workspace))) return TL_BAD_SIZE;
+    if (pl.shares > 0 && counters == nullptr) return TL_BAD_SIZE;
     if (n_seqs > 65535 || (long long)n_kv_heads * pl.n_gchunks > 65535) return TL_BAD_SIZE;
 
     DecodeParams p;
     p.q = (const __nv_bfloat16*)q; p.out = (__nv_bfloat16*)out;
     p.block_table = block_table; p.q_start = q_start; p.kv_len = kv_len; p.table_stride = table_stride;
-    p.status = status;
+    p.status = status; p.counters = counters;
     p.n_heads = n_heads; p.n_kv_heads = n_kv_heads; p.page_size = page_size;
     p.page_shift = 0;
     while ((1 << p.page_shift) < page_size) ++p.page_shift;
     p.box_rows = page_size < BN ? page_size : BN;
     p.total_rows = (int)(n_pages * n_kv_heads * page_size);
-    p.group = n_heads / n_kv_heads; p.ng = pl.ng; p.n_gchunks = pl.n_gchunks; p.tpw = pl.tpw;
+    p.group = n_heads / n_kv_heads; p.ng = pl.ng; p.n_gchunks = pl.n_gchunks; p.units = n_kv_heads * pl.n_gchunks;
+    p.n_seqs = n_seqs; p.max_tokens = max_q_len; p.rows = max_q_len * pl.ng;
     p.window = window > 0 ? window : 0;
     {
         // (an upper bound of what the call reads: every request's keys and values up to the longest context)
@@ -682,7 +914,7 @@ extern "C" int tl_paged_attention_decode(const void* q, const void* k_pages, con
     p.n_splits = pl.n_splits;
     p.scale_log2 = scale * LOG2E;
     p.part_o = workspace;
-    p.part_ml = workspace ? workspace + (size_t)n_tokens * n_heads * pl.n_splits * head_dim : nullptr;
+    p.part_ml = workspace ? workspace + (pl.shares > 0 ? (size_t)n_seqs * p.units * p.rows : (size_t)n_tokens * n_heads) * pl.n_splits * head_dim : nullptr;
 
     const long long rows = n_pages * n_kv_heads * page_size;
     CUtensorMap mk, mv;
@@ -692,15 +924,13 @@ extern "C" int tl_paged_attention_decode(const void* q, const void* k_pages, con
     if (rc != TL_OK) return rc;
 
     cudaStream_t s = (cudaStream_t)stream;
-    dim3 grid(pl.n_q_tiles * pl.n_splits, n_kv_heads * pl.n_gchunks, n_seqs);
     // query rows a CTA can meet: one 8-row block is enough for them, or two
-    const int rows_used = (max_q_len < pl.tpw ? max_q_len : pl.tpw) * pl.ng;
-    if (rows_used <= 8)
-        rc = head_dim == 128 ? launch<128, 1>(mk, mv, p, grid, s) : launch<64, 1>(mk, mv, p, grid, s);
+    if (p.rows <= 8)
+        rc = head_dim == 128 ? launch<128, 1>(mk, mv, p, pl, s) : launch<64, 1>(mk, mv, p, pl, s);
     else
-        rc = head_dim == 128 ? launch<128, 2>(mk, mv, p, grid, s) : launch<64, 2>(mk, mv, p, grid, s);
+        rc = head_dim == 128 ? launch<128, 2>(mk, mv, p, pl, s) : launch<64, 2>(mk, mv, p, pl, s);
     if (rc != TL_OK) return rc;
-    if (pl.n_splits > 1) {
+    if (pl.n_splits > 1 && pl.shares == 0) {
         cudaError_t e = tl_launch(merge_partials_kernel, dim3((unsigned)n_tokens * (unsigned)n_heads),
                                   dim3(head_dim >= 128 ? 128u : 64u), 0, s, (const float*)p.part_o, (const float*)p.part_ml,
                                   p.out, pl.n_splits, head_dim);

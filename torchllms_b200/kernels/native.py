@@ -1755,6 +1755,19 @@ class NativeOps:
             self._workspace[key] = buf
         return buf
 
+    def _counters(self, device: torch.device, n: int) -> Optional[torch.Tensor]:
+        """At least ``n`` ints that are zero between launches (whoever counts with them sets them back)."""
+        if n <= 0:
+            return None
+        key = (device.index or 0, "counters")
+        buf = self._workspace.get(key)
+        if buf is None or buf.numel() < n:
+            if buf is not None:
+                self._retired.append(buf)      # a captured graph may still point into it
+            buf = torch.zeros(max(n, 1 << 16), dtype=torch.int32, device=device)
+            self._workspace[key] = buf
+        return buf
+
     @_timed
     def paged_attention(self, q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
                         block_table: torch.Tensor, q_start: torch.Tensor, kv_len: torch.Tensor, *,
@@ -1861,18 +1874,22 @@ class NativeOps:
             return out
         if decode_ok:
             lib = self._lib("attention_decode")
+            counters = ctypes.c_longlong(0)
             rc = lib.tl_attention_decode_plan(T, n_seqs, n_heads, n_kv_heads, head_dim, max_q_len, max_kv_len,
-                                              int(allow_split), ctypes.byref(n_splits), ctypes.byref(floats))
+                                              int(allow_split), ctypes.byref(n_splits), ctypes.byref(floats), ctypes.byref(counters))
             _check(rc, "attention_decode_plan")
             ws = self._scratch(q.device, floats.value)
             self._debug_limit("attention_decode", 0, k_pages.shape[0])
             rc = lib.tl_paged_attention_decode(
                 _ptr(q), _ptr(k_pages), _ptr(v_pages), _ptr(out), _ptr(block_table), block_table.stride(0),
-                _ptr(q_start), _ptr(kv_len), _ptr(ws), ctypes.c_void_p(self._status.data_ptr()), T, n_seqs,
+                _ptr(q_start), _ptr(kv_len), _ptr(ws), _ptr(self._counters(q.device, counters.value)),
+                ctypes.c_void_p(self._status.data_ptr()), T, n_seqs,
                 n_heads, n_kv_heads, head_dim, page_size, ctypes.c_longlong(k_pages.shape[0]), max_q_len, max_kv_len,
                 int(window or 0), ctypes.c_float(scale), int(allow_split), _stream())
             _check(rc, "paged_attention_decode")
-        elif use_mma:
+            self.launches += 2 if n_splits.value > 1 and not counters.value else 1
+            return out
+        if use_mma:
             lib = self._lib("attention_mma")
             rc = lib.tl_attention_mma_plan(T, n_seqs, n_heads, n_kv_heads, head_dim, max_q_len, max_kv_len,
                                            1 if allow_split else 0, ctypes.byref(n_splits), ctypes.byref(floats))
