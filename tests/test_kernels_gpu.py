@@ -783,6 +783,20 @@ def test_window_edge_is_exact(ops, dtype, impl):
         torch.testing.assert_close(got, want, atol=tol(dtype, 2e-5, 2e-2), rtol=tol(dtype, 2e-5, 2e-2))
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("q_len", [1, 128, 129, 256, 257])
+@pytest.mark.parametrize("window", [None, 130])
+def test_prefill_attention_rings_wrap(ops, hd, q_len, window):
+    """One to nine key tiles, ends of tiles and one key beside them: every state of the rings of K and V and of the score
+    buffer, query tiles that take part in different key tiles, and a second query tile without rows."""
+    seq_lens = [q_len + behind for behind in (0, 1, 127, 255, 384, 511, 640, 897, 1024)]
+    a = build_paged(seq_lens, [q_len] * len(seq_lens), 4, 2, hd, 16, torch.bfloat16, seed=q_len)
+    want = TWIN.paged_attention(**a, scale=hd ** -0.5, window=window).float()
+    got = ops.paged_attention(**a, scale=hd ** -0.5, window=window, impl="prefill").float()
+    ops.check_status()
+    torch.testing.assert_close(got, want, atol=2e-2, rtol=2e-2)          # probabilities and results rounded to bfloat16
+
+
 @pytest.mark.parametrize("seed", [0, 1, 2])
 def test_prefill_attention_on_random_shapes(ops, seed):
     """Both tcgen05 prefill kernels on shapes nobody picked: heads and groups, page sizes from 4 to 256, up to

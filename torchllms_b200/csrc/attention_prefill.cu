@@ -8,8 +8,7 @@
 // Two kernels.  The one that is used by default is the second in this file: one bfloat16 per
 // probability, a thread to a query row, 512 threads.  The first, described next, multiplies every
 // probability as value + remainder (half the rounding error, a third slower); it has two threads
-// to a query row that exchange one number per key tile.  Both share the tiling, the producer and
-// the issuers' order of work.
+// to a query row that exchange one number per key tile.  Both share the tiling.
 //
 // A CTA serves 256 consecutive tokens of one request and one query head as two query tiles of
 // 128 rows (M = 128 each), walking the visible keys in tiles of 128.  Every K and V tile that is
@@ -661,42 +660,51 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_prefill_kernel(const __
 //                    thread, which reads the 128 scores of a key tile into registers once (192
 //                    registers a thread: the warp groups trade registers at the start with
 //                    setmaxnreg), takes their maximum, tells the correction warps by how much the
-//                    row's accumulator has to shrink, and writes the probabilities where the scores were.
+//                    row's accumulator has to shrink, and writes the probabilities into tensor memory.
 //   warps 8-11     : correction.  When a row's maximum in use has grown they rescale its accumulator
 //                    (a round trip through registers) off the softmax's path; at the end they divide
 //                    by the row's sum and store it.
-//   warp 12        : TMA producer (the two query tiles through a three-dimensional map of q, then K and V);
-//                    warps 13, 14 : the issuers of the two query tiles (the whole warp
-//                    runs in step and one elected lane issues: a lone lane inside a divergent branch
-//                    cannot keep the descriptors in uniform registers, and issued a fifth slower);
-//                    warp 15 is there to complete the warp group.
-// Barriers beside those of the kernel above: alpha_ready (softmax -> correction: factors are in
-// shared memory), o_ready (correction -> issuer: the accumulator may take the next product),
-// p_half (softmax -> issuer: the probabilities of the tile's first 64 keys are in place, the product may
-// start on them), l_ready (softmax -> correction: the row sums are in shared memory), turn (softmax ->
-// the other tile's softmax: the exponential unit is yours).
+//   warp 12        : brings the two query tiles (through a three-dimensional map of q) and K; warp 13 issues the scores of
+//                    both query tiles, warp 14 their products with V (the whole warp runs in step and one elected lane
+//                    issues: a lone lane inside a divergent branch cannot keep the descriptors in uniform
+//                    registers, and issued a fifth slower); warp 15 brings V.  Pages are looked up a tile ahead.
+// Scores, probabilities and accumulators have tensor memory of their own, so that the scores of a tile's next 128
+// keys are made while the exponentials of these are taken; where they shared it the chain scores, softmax, both
+// products, scores (3,460 cycles for 128 x 128 pairs, of which the softmax is 2,025) set the pace of a tile, and the
+// other tile only filled its gaps (tensor pipe 47 % active).  With head_dim 128 there is room for one score buffer, which the tiles use
+// in turn; it is free as soon as the scores are in registers.  One warp issues both tiles' products with V, in
+// order: that keeps the tiles half a period apart (a warp to a tile let them fall into step, 222 us where this takes 168,
+// and an explicit turn for the exponentials, 171).  What bounds it now: the way of the score buffer between the tiles (read, free,
+// scores, seen: 1,400 cycles of a period of 3,000) and the exponential unit (2,048).
+//     2,000 tokens behind 5,001, 24 / 8 heads of 128, pages of 16:  200 -> 168 us
+//     a prompt of 2,048, 32 / 8 heads of 128:                      51.8 -> 46.5
+//     two portions of 611, 32 / 8 heads of 64:                     24.4 -> 22.5
+// Barriers beside those of the kernel above: s_free (softmax -> scores: the buffer has been read), alpha_ready
+// (softmax -> correction: factors are in shared memory; not before the product of the key tile before is over, when
+// the correction has taken the word of that tile), o_ready (correction -> issuer: the accumulator may take the
+// next product), p_half (softmax -> issuer: the probabilities of the tile's first 64 keys are in place, the
+// product may start on them), l_ready (softmax -> correction: the row sums are in shared memory).
 constexpr int NTHREADS_ROWS = 512;
 // Registers a thread after the trade: softmax / correction / the rest.  A warp group can only be given
 // what another has handed back, so the sum stays within what the launch allots (128 a thread).
 constexpr int REGS_SOFTMAX = 192, REGS_CORRECTION = 72, REGS_REST = 40;
 static_assert(QT * REGS_SOFTMAX + REGS_CORRECTION + REGS_REST <= 4 * 128, "registers are traded, not made");
-constexpr int WR_CORR = 4 * QT, WR_COPY = 4 * QT + 4, WR_ISSUE = 4 * QT + 5;
+constexpr int WR_CORR = 4 * QT, WR_COPY = 4 * QT + 4, WR_ISSUE = 4 * QT + 5, WR_COPY_V = 4 * QT + 7;
 
-template <int STAGES>
+template <int KSTAGES, int STAGES>
 struct TailRows {
-    unsigned long long q_full, k_full[STAGES], k_empty[STAGES], v_full[STAGES], v_empty[STAGES];
-    unsigned long long s_full[QT], p_half[QT], p_full[QT], pv_done[QT], alpha_ready[QT], o_ready[QT], l_ready[QT], turn[QT];
+    unsigned long long q_full, k_full[KSTAGES], k_empty[KSTAGES], v_full[STAGES], v_empty[STAGES];
+    unsigned long long s_full[QT], s_free[QT], p_half[QT], p_full[QT], pv_done[QT], alpha_ready[QT], o_ready[QT], l_ready[QT];
     unsigned tmem_base_slot;
     int failed_flag;
     int grow_any[QT][2][4];     // [tile][parity of the tile's step][warp of the tile]: did a row of the warp grow
-    float alpha[QT][2][BM];     // [tile][parity of the tile's step][row]: what the row's accumulator shrinks by
-    float l_final[QT][BM];
+    float alpha[QT][2][BM];     // [tile][parity of the tile's step][row]: what the row's accumulator shrinks by; at the end, the row's sum
 };
 
 template <int N> __device__ __forceinline__ void regs_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-template <int HD, int STAGES>
+template <int HD, int KSTAGES, int STAGES>
 __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                                  const __grid_constant__ CUtensorMap map_v,
                                                                                  const __grid_constant__ CUtensorMap map_q,
@@ -704,23 +712,28 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
     constexpr int HALVES = HD / 64;
     constexpr unsigned HALF_BYTES = BN * 128;
     constexpr unsigned KV_BYTES = HALVES * HALF_BYTES;
+    // Tensor memory: scores, probabilities (two to a column) and accumulators lie apart.  With head_dim 64 every tile has
+    // a score buffer, with 128 both use one in turn (it is free again as soon as they are in registers).
+    constexpr int NS = HD == 64 ? 2 : 1;
+    constexpr unsigned COL_S = 0, COL_P = NS * BN, COL_O = COL_P + QT * (BN / 2);
+    static_assert(COL_O + QT * HD <= TMEM_COLS, "scores, probabilities and accumulators must fit the tensor memory of a CTA");
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* Qs = smem_raw;
     unsigned char* tiles = Qs + QT * KV_BYTES;
-    TailRows<STAGES>& tail = *reinterpret_cast<TailRows<STAGES>*>(tiles + 2 * STAGES * KV_BYTES);
+    TailRows<KSTAGES, STAGES>& tail = *reinterpret_cast<TailRows<KSTAGES, STAGES>*>(tiles + (KSTAGES + STAGES) * KV_BYTES);
     unsigned long long& q_full = tail.q_full;
-    unsigned long long (&k_full)[STAGES] = tail.k_full;
-    unsigned long long (&k_empty)[STAGES] = tail.k_empty;
+    unsigned long long (&k_full)[KSTAGES] = tail.k_full;
+    unsigned long long (&k_empty)[KSTAGES] = tail.k_empty;
     unsigned long long (&v_full)[STAGES] = tail.v_full;
     unsigned long long (&v_empty)[STAGES] = tail.v_empty;
     unsigned long long (&s_full)[QT] = tail.s_full;
+    unsigned long long (&s_free)[QT] = tail.s_free;
     unsigned long long (&p_full)[QT] = tail.p_full;
     unsigned long long (&p_half)[QT] = tail.p_half;
     unsigned long long (&pv_done)[QT] = tail.pv_done;
     unsigned long long (&alpha_ready)[QT] = tail.alpha_ready;
     unsigned long long (&o_ready)[QT] = tail.o_ready;
     unsigned long long (&l_ready)[QT] = tail.l_ready;
-    unsigned long long (&turn)[QT] = tail.turn;
     unsigned& tmem_base_slot = tail.tmem_base_slot;
     int& failed_flag = tail.failed_flag;
 
@@ -728,21 +741,23 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
     if (tid == 0) {
         failed_flag = 0;
         mbar_init(&q_full, 1);
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < KSTAGES; ++s) {
             mbar_init(&k_full[s], 1);
             mbar_init(&k_empty[s], QT);
+        }
+        for (int s = 0; s < STAGES; ++s) {
             mbar_init(&v_full[s], 1);
             mbar_init(&v_empty[s], QT);
         }
         for (int t = 0; t < QT; ++t) {
             mbar_init(&s_full[t], 1);
+            mbar_init(&s_free[t], 4);
             mbar_init(&p_full[t], 4);
             mbar_init(&p_half[t], 4);
             mbar_init(&pv_done[t], 1);
             mbar_init(&alpha_ready[t], 4);
             mbar_init(&o_ready[t], 4);
             mbar_init(&l_ready[t], 4);
-            mbar_init(&turn[t], 4);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -787,9 +802,10 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
 
     if (warp >= WR_COPY) {
         regs_down<REGS_REST>();
-        if (warp == WR_COPY) {
+        if (warp == WR_COPY || warp == WR_COPY_V) {
             if (active) {
-                // ---- producer: as in the kernel above
+                // ---- producers, one for the queries and K, one for V (scores run ahead of the products with V: neither
+                // may wait for the other's room); the pages of the next tile are looked up while this one's room is waited for
                 bool sound = (smem_u32(Qs) & 1023u) == 0u;
                 if (!sound && lane == 0) {
                     failed_flag = 1;
@@ -798,7 +814,7 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
                 // the queries of both tiles: [128 tokens x 64 elements] boxes of this head, which land in the
                 // layout of a K tile (rows past the request's own are another request's or the zero fill:
                 // their results are never stored)
-                if (sound && lane == 0) {
+                if (sound && warp == WR_COPY && lane == 0) {
                     int tiles_q = 0;
                     for (int t = 0; t < QT; ++t) tiles_q += (t ? range[1].rows : range[0].rows) > 0 ? 1 : 0;
                     mbar_expect_tx(&q_full, tiles_q * KV_BYTES);
@@ -808,116 +824,133 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
                                 tma_load_3d(Qs + t * KV_BYTES + h * HALF_BYTES, &map_q, &q_full, h * 64, head, qs + tok0 + t * BM);
                 }
                 __syncwarp();
+                const bool is_k = warp == WR_COPY;
+                const CUtensorMap* map = is_k ? &map_k : &map_v;
+                unsigned long long* full = is_k ? k_full : v_full;
+                unsigned long long* empty = is_k ? k_empty : v_empty;
+                const int stages = is_k ? KSTAGES : STAGES;
+                unsigned char* ring = is_k ? tiles : tiles + KSTAGES * KV_BYTES;
                 const int* table = p.block_table + (size_t)b * p.table_stride;
                 const int n_boxes = BN / p.box_rows;
+                // the row of the page tensor where the box at this position starts.  Boxes past the last key start outside
+                // the tensor: the copy writes the zero fill, so that what is multiplied by probability 0 there is finite.
+                // So do boxes that end before the first key of a window (their pages may have been given back).
+                auto box_row = [&](int kpos) {
+                    int row = p.total_rows;
+                    if (kpos < k_hi && kpos + p.box_rows > k_lo) {
+                        const int page = table[kpos >> p.page_shift];
+                        if (tl_check_page(page))
+                            row = (page * p.n_kv_heads + kvh) * p.page_size + (kpos & (p.page_size - 1));
+                    }
+                    return row;
+                };
+                int next_row = lane < n_boxes && n_tiles > 0 ? box_row(k_start + lane * p.box_rows) : 0;
+                int s = 0, round = 0;
                 for (int j = 0; j < n_tiles && sound; ++j) {
-                    const int s = j % STAGES;
                     const int k0 = k_start + j * BN;
-                    for (int which = 0; which < 2 && sound; ++which) {
-                        unsigned long long* full = which == 0 ? &k_full[s] : &v_full[s];
-                        unsigned long long* empty = which == 0 ? &k_empty[s] : &v_empty[s];
-                        if (j >= STAGES && !__all_sync(0xffffffffu, mbar_wait(empty, ((j / STAGES) - 1) & 1, failed))) {
-                            if (lane == 0) {
-                                failed_flag = 1;
-                                atomicExch(p.status, ERR_PRODUCER_WAIT);
-                            }
-                            sound = false;
-                            break;
+                    const int first_row = next_row;
+                    if (lane < n_boxes && j + 1 < n_tiles) next_row = box_row(k0 + BN + lane * p.box_rows);
+                    if (round > 0 && !__all_sync(0xffffffffu, mbar_wait(&empty[s], (round - 1) & 1, failed))) {
+                        if (lane == 0) {
+                            failed_flag = 1;
+                            atomicExch(p.status, ERR_PRODUCER_WAIT);
                         }
-                        if (lane == 0) mbar_expect_tx(full, KV_BYTES);
-                        __syncwarp();
-                        unsigned char* dst0 = tiles + (which * STAGES + s) * KV_BYTES;
-                        const CUtensorMap* map = which == 0 ? &map_k : &map_v;
-                        for (int c = lane; c < n_boxes; c += 32) {
-                            const int kpos = k0 + c * p.box_rows;
-                            int row = p.total_rows;
-                            if (kpos < k_hi && kpos + p.box_rows > k_lo) {
-                                const int page = table[kpos >> p.page_shift];
-                                if (tl_check_page(page))
-                                    row = (page * p.n_kv_heads + kvh) * p.page_size + (kpos & (p.page_size - 1));
-                            }
+                        sound = false;
+                        break;
+                    }
+                    if (lane == 0) mbar_expect_tx(&full[s], KV_BYTES);
+                    __syncwarp();
+                    for (int c = lane; c < n_boxes; c += 32) {
+                        const int row = c == lane ? first_row : box_row(k0 + c * p.box_rows);
 #pragma unroll
-                            for (int h = 0; h < HALVES; ++h) {
-                                unsigned char* dst = dst0 + h * HALF_BYTES + c * p.box_rows * 128;
-                                if (!copy_is_sound(dst, h * 64, row)) {
-                                    failed_flag = 1;
-                                    atomicExch(p.status, ERR_BAD_COPY);
-                                    continue;
-                                }
-                                tma_load_2d(dst, map, full, h * 64, row);
+                        for (int h = 0; h < HALVES; ++h) {
+                            unsigned char* dst = ring + s * KV_BYTES + h * HALF_BYTES + c * p.box_rows * 128;
+                            if (!copy_is_sound(dst, h * 64, row)) {
+                                failed_flag = 1;
+                                atomicExch(p.status, ERR_BAD_COPY);
+                                continue;
                             }
+                            tma_load_2d(dst, map, &full[s], h * 64, row);
                         }
-                        __syncwarp();
+                    }
+                    __syncwarp();
+                    if (++s == stages) {
+                        s = 0;
+                        ++round;
                     }
                 }
             }
         } else if (warp < WR_ISSUE + QT) {
             if (active) {
-                // ---- issuers, one per query tile; the whole warp runs in step and one elected lane issues.
-                // As in the kernel above, with two differences.  The product into the accumulator also waits
-                // for the correction warps' word that the accumulator is ready for it.  And the scores of the
-                // next key tile are queued right behind that product (the tensor core takes its instructions
-                // in order, so the scores overwrite the probabilities only after the product has read them):
-                // everything else the two wait for (K, V) is waited for before the probabilities are, so
-                // that nothing but the products themselves stands between one softmax and the next.
-                constexpr unsigned id_s = idesc(BN, 1u, 1u, 0u);
-                constexpr unsigned id_o = idesc(HD, 1u, 1u, 1u);
-                const int t = warp - WR_ISSUE;
-                const int first = t ? range[1].first : range[0].first, last = t ? range[1].last : range[0].last;
-                bool ok = __all_sync(0xffffffffu, mbar_wait(&q_full, 0, failed));
-                tc_fence_after();
-                const unsigned long long qd0 = desc_k_major(smem_u32(Qs + t * KV_BYTES));
-                const unsigned d_s = tmem + COL_S + t * BN, d_o = tmem + COL_O + t * BN;
-                // scores of key tile j (its K stage has arrived), or this tile's leave to reuse the stage
-                auto scores = [&](int j) {
-                    const int s = j % STAGES;
-                    if (j >= first && j < last) {
-                        tc_fence_after();
+                // ---- issuers: one for the scores, one for the products into the accumulators; the whole warp runs
+                // in step and one elected lane issues.  Both go through the key tiles in order, query tile 0 before 1.
+                bool ok = true;
+                if (warp == WR_ISSUE) {
+                    // S_j = Q K_j^T, as soon as the scores that lie in the buffer have been read: well before the
+                    // probabilities of the key tile before are multiplied.
+                    constexpr unsigned id_s = idesc(BN, 1u, 1u, 0u);
+                    ok = __all_sync(0xffffffffu, mbar_wait(&q_full, 0, failed));
+                    int used = 0;
+                    for (int j = 0; j < n_tiles && ok; ++j) {
+                        const int s = j % KSTAGES;
+                        ok = __all_sync(0xffffffffu, mbar_wait(&k_full[s], (j / KSTAGES) & 1, failed));
                         const unsigned long long kd0 = desc_k_major(smem_u32(tiles + s * KV_BYTES));
 #pragma unroll
-                        for (int kd = 0; kd < HD / 16; ++kd) {
-                            const unsigned off = ((kd / 4) * HALF_BYTES + (kd % 4) * 32) >> 4;
-                            umma_ss_elect(d_s, qd0 + off, kd0 + off, id_s, kd > 0 ? 1u : 0u);
+                        for (int t = 0; t < QT; ++t) {
+                            if (!ok) break;
+                            if (j >= range[t].first && j < range[t].last) {
+                                const int before = NS == 1 ? used : j - range[t].first;
+                                if (before > 0) ok = __all_sync(0xffffffffu, mbar_wait(&s_free[NS == 1 ? 0 : t], (before - 1) & 1, failed));
+                                if (!ok) break;
+                                tc_fence_after();
+                                const unsigned long long qd0 = desc_k_major(smem_u32(Qs + t * KV_BYTES));
+#pragma unroll
+                                for (int kd = 0; kd < HD / 16; ++kd) {
+                                    const unsigned off = ((kd / 4) * HALF_BYTES + (kd % 4) * 32) >> 4;
+                                    umma_ss_elect(tmem + COL_S + (NS == 1 ? 0 : t * BN), qd0 + off, kd0 + off, id_s, kd > 0 ? 1u : 0u);
+                                }
+                                umma_commit_elect(&s_full[t]);
+                                umma_commit_elect(&k_empty[s]);
+                                ++used;
+                            } else if (lane == 0) {
+                                mbar_arrive(&k_empty[s]);          // not this tile's keys: nothing to wait for
+                            }
                         }
-                        umma_commit_elect(&s_full[t]);
-                        umma_commit_elect(&k_empty[s]);
-                    } else if (lane == 0) {
-                        mbar_arrive(&k_empty[s]);
                     }
-                };
-                if (ok && n_tiles > 0) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(&k_full[0], 0, failed));
-                    if (ok) scores(0);
-                }
-                for (int j = 0; j < n_tiles && ok; ++j) {
-                    const int s = j % STAGES;
-                    const unsigned ring = (j / STAGES) & 1;
-                    const bool mine = j >= first && j < last;
-                    ok = __all_sync(0xffffffffu, mbar_wait(&v_full[s], ring, failed));
-                    if (ok && j + 1 < n_tiles) ok = __all_sync(0xffffffffu, mbar_wait(&k_full[(j + 1) % STAGES], ((j + 1) / STAGES) & 1, failed));
-                    if (!ok) break;
-                    if (mine) {
-                        // the product starts on the first half of the probabilities while the second is still being taken
-                        ok = __all_sync(0xffffffffu, mbar_wait(&p_half[t], (j - first) & 1, failed) && mbar_wait(&o_ready[t], (j - first) & 1, failed));
-                        if (!ok) break;
-                        tc_fence_after();
-                        const unsigned long long vd0 = desc_mn_major(smem_u32(tiles + (STAGES + s) * KV_BYTES), HALF_BYTES);
-                        const unsigned acc = j > first ? 1u : 0u;
+                } else {
+                    // O += P_j V_j, with the probabilities read from tensor memory: the product starts on the first half of
+                    // the keys while the second half's probabilities are still being taken.
+                    constexpr unsigned id_o = idesc(HD, 1u, 1u, 1u);
+                    for (int j = 0; j < n_tiles && ok; ++j) {
+                        const int s = j % STAGES;
+                        ok = __all_sync(0xffffffffu, mbar_wait(&v_full[s], (j / STAGES) & 1, failed));
+                        const unsigned long long vd0 = desc_mn_major(smem_u32(tiles + (KSTAGES + s) * KV_BYTES), HALF_BYTES);
 #pragma unroll
-                        for (int kk = 0; kk < BN / 32; ++kk)
-                            umma_ts_elect(d_o, d_s + kk * 8, vd0 + kk * (2048 >> 4), id_o, kk > 0 ? 1u : acc);
-                        ok = __all_sync(0xffffffffu, mbar_wait(&p_full[t], (j - first) & 1, failed));
-                        if (!ok) break;
-                        tc_fence_after();
+                        for (int t = 0; t < QT; ++t) {
+                            if (!ok) break;
+                            if (j >= range[t].first && j < range[t].last) {
+                                const unsigned par = (j - range[t].first) & 1;
+                                const unsigned d_p = tmem + COL_P + t * (BN / 2), d_o = tmem + COL_O + t * HD;
+                                ok = __all_sync(0xffffffffu, mbar_wait(&p_half[t], par, failed) && mbar_wait(&o_ready[t], par, failed));
+                                if (!ok) break;
+                                tc_fence_after();
+                                const unsigned acc = j > range[t].first ? 1u : 0u;
 #pragma unroll
-                        for (int kk = BN / 32; kk < BN / 16; ++kk)
-                            umma_ts_elect(d_o, d_s + kk * 8, vd0 + kk * (2048 >> 4), id_o, 1u);
-                        umma_commit_elect(&pv_done[t]);
-                        umma_commit_elect(&v_empty[s]);
-                    } else if (lane == 0) {
-                        mbar_arrive(&v_empty[s]);
+                                for (int kk = 0; kk < BN / 32; ++kk)
+                                    umma_ts_elect(d_o, d_p + kk * 8, vd0 + kk * (2048 >> 4), id_o, kk > 0 ? 1u : acc);
+                                ok = __all_sync(0xffffffffu, mbar_wait(&p_full[t], par, failed));
+                                if (!ok) break;
+                                tc_fence_after();
+#pragma unroll
+                                for (int kk = BN / 32; kk < BN / 16; ++kk)
+                                    umma_ts_elect(d_o, d_p + kk * 8, vd0 + kk * (2048 >> 4), id_o, 1u);
+                                umma_commit_elect(&pv_done[t]);
+                                umma_commit_elect(&v_empty[s]);
+                            } else if (lane == 0) {
+                                mbar_arrive(&v_empty[s]);
+                            }
+                        }
                     }
-                    if (j + 1 < n_tiles) scores(j + 1);
                 }
                 if (!ok && lane == 0) {
                     failed_flag = 1;
@@ -950,11 +983,11 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
 #pragma unroll
                         for (int c = 0; c < HD / PIECE; ++c) {
                             unsigned v[PIECE];
-                            tmem_ld<PIECE>(lane_addr + COL_O + t * BN + c * PIECE, v);
+                            tmem_ld<PIECE>(lane_addr + COL_O + t * HD + c * PIECE, v);
                             tmem_wait_ld();
 #pragma unroll
                             for (int i = 0; i < PIECE; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * a);
-                            tmem_st<PIECE>(lane_addr + COL_O + t * BN + c * PIECE, v);
+                            tmem_st<PIECE>(lane_addr + COL_O + t * HD + c * PIECE, v);
                         }
                         tmem_wait_st();
                     }
@@ -972,7 +1005,7 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
                 ok = __all_sync(0xffffffffu, mbar_wait(&l_ready[t], 0, failed) && mbar_wait(&pv_done[t], (n - 1) & 1, failed));
                 if (!ok) break;
                 tc_fence_after();
-                const float l = tail.l_final[t][r];
+                const float l = tail.alpha[t][n & 1][r];       // (the parity that the last key tile did not use)
                 const float inv = l > 0.f ? 1.f / l : 0.f;
                 // The rows leave through shared memory (the query tile's place: its last product is over), in
                 // the swizzled layout the queries had, so that they are written to global memory a row
@@ -981,7 +1014,7 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
 #pragma unroll
                 for (int c = 0; c < HD / PIECE; ++c) {
                     unsigned v[PIECE];
-                    tmem_ld<PIECE>(lane_addr + COL_O + t * BN + c * PIECE, v);
+                    tmem_ld<PIECE>(lane_addr + COL_O + t * HD + c * PIECE, v);
                     tmem_wait_ld();
 #pragma unroll
                     for (int i = 0; i < PIECE / 8; ++i) {
@@ -1019,23 +1052,13 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
             const unsigned lane_addr = tmem + ((unsigned)(sw * 32) << 16);
             const int rows = t ? range[1].rows : range[0].rows;
             const int first = t ? range[1].first : range[0].first, last = t ? range[1].last : range[0].last;
-            const unsigned col_s = COL_S + t * BN;
+            const unsigned col_s = COL_S + (NS == 1 ? 0 : t * BN), col_p = COL_P + t * (BN / 2);
             float m_used = -INFINITY, l_sum = 0.f;
             const int t0 = qpos_base + tok0 + t * BM;
             const int qpos = t0 + (r < rows ? r : rows - 1);
             const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
             bool ok = true;
-            // The exponentials of the two query tiles take turns (turn[t]: tile t may go), so that one tile's
-            // softmax has the exponential unit to itself while the tensor core works for the other tile;
-            // side by side they would both wait for the unit and then both for the tensor core.
-            if (t == 1 && lane == 0) mbar_arrive(&turn[0]);
-            for (int j = 0; j < n_tiles; ++j) {
-                if (j < first || j >= last) {      // not this tile's keys: pass the turn on
-                    ok = __all_sync(0xffffffffu, mbar_wait(&turn[t], j & 1, failed));
-                    if (!ok) break;
-                    if (lane == 0) mbar_arrive(&turn[t ^ 1]);
-                    continue;
-                }
+            for (int j = first; j < last; ++j) {
                 const int k0 = k_start + j * BN;
                 const int it = j - first, par = it & 1;
                 ok = __all_sync(0xffffffffu, mbar_wait(&s_full[t], par, failed));
@@ -1044,6 +1067,9 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
                 unsigned raw[BN];
                 tmem_ld<BN>(lane_addr + col_s, raw);
                 tmem_wait_ld();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s_free[NS == 1 ? 0 : t]);      // the buffer may take the next scores
                 const bool clear = k0 + BN - 1 <= t0 && (p.window <= 0 || k0 > t0 + rows - 1 - p.window);
                 if (!clear) {
 #pragma unroll
@@ -1066,12 +1092,17 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
                 if (grow) m_used = m_new;
                 // the correction warps learn what this row's accumulator shrinks by, and whether any row of the warp does
                 const bool any = __any_sync(0xffffffffu, grow);
+                // (not before the product of the key tile before is over: the correction warps have then taken the word
+                // of that tile, and its probabilities have been read)
+                if (it > 0) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[t], (it - 1) & 1, failed));
+                    if (!ok) break;
+                    tc_fence_after();
+                }
                 tail.alpha[t][par][r] = alpha;
                 if (lane == 0) tail.grow_any[t][par][sw] = any ? 1 : 0;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&alpha_ready[t]);
-                ok = __all_sync(0xffffffffu, mbar_wait(&turn[t], j & 1, failed));
-                if (!ok) break;
                 l_sum *= alpha;
                 const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
                 const float2 nm2 = make_float2(-m_safe, -m_safe);
@@ -1090,7 +1121,7 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
                         packed[i / 2] = pack_bf16(ea.x, ea.y);
                         packed[i / 2 + 1] = pack_bf16(eb.x, eb.y);
                     }
-                    tmem_st<16>(lane_addr + col_s + c * 16, packed);      // (all scores are in registers: nothing is overwritten unread)
+                    tmem_st<16>(lane_addr + col_p + c * 16, packed);
                     if (c == BN / 64 - 1) {          // half of the keys' probabilities are in place
                         tmem_wait_st();
                         tc_fence_before();
@@ -1099,15 +1130,13 @@ __global__ void __launch_bounds__(NTHREADS_ROWS, 1) attention_prefill_rows_kerne
                     }
                 }
                 l_sum += (la.x + la.y) + (lb.x + lb.y);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&turn[t ^ 1]);
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&p_full[t]);
             }
             if (ok) {
-                tail.l_final[t][r] = l_sum;
+                tail.alpha[t][(last - first) & 1][r] = l_sum;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&l_ready[t]);
             } else if (lane == 0) {
@@ -1216,15 +1245,16 @@ bool takes(int n_heads, int n_kv_heads, int head_dim, int page_size) {
 
 bool p_blocks_too_many(int max_q_len) { return (max_q_len + QT * BM - 1) / (QT * BM) > 65535; }
 
+template <int HD> constexpr int k_stages_for() { return HD == 128 ? 3 : 4; }
 template <int HD> constexpr size_t smem_rows_for() {
-    return (size_t)(QT + 2 * stages_for<HD>()) * (HD / 64) * BN * 128 + sizeof(TailRows<stages_for<HD>()>);
+    return (size_t)(QT + k_stages_for<HD>() + stages_for<HD>()) * (HD / 64) * BN * 128 + sizeof(TailRows<k_stages_for<HD>(), stages_for<HD>()>);
 }
 static_assert(smem_rows_for<128>() <= 227 * 1024 && smem_rows_for<64>() <= 227 * 1024, "a CTA has 227 KB of shared memory");
 
 template <int HD>
 int launch_rows(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mq, const PrefillParams& p, dim3 grid, cudaStream_t s) {
     constexpr size_t smem = smem_rows_for<HD>();
-    auto kern = attention_prefill_rows_kernel<HD, stages_for<HD>()>;
+    auto kern = attention_prefill_rows_kernel<HD, k_stages_for<HD>(), stages_for<HD>()>;
     static bool raised = false;
     if (!raised) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
