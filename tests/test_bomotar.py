@@ -529,6 +529,39 @@ def test_delta_rule_with_a_decay_per_channel(backend):
 
 
 @pytest.mark.parametrize("backend", BACKENDS)
+@pytest.mark.parametrize("d", [65, 128])
+def test_delta_rule_at_the_edges_of_blocks(backend, d):
+    """Portions that end one token before, at and behind the blocks of 8 tokens and the buffers of 32 that keys of 65 to 128 walk in."""
+    ops, dev = _ops(backend)
+    g = torch.Generator().manual_seed(d)
+    dt, H, dv = _dt(backend), 1, 18
+    lens = [7, 8, 9, 31, 32, 33, 64, 71]
+    T, n = sum(lens), len(lens)
+    q = torch.nn.functional.normalize(torch.randn(T, 1, d, generator=g), dim=-1) * d ** -0.5
+    k = torch.nn.functional.normalize(torch.randn(T, 1, d, generator=g), dim=-1)
+    v, beta = torch.randn(T, dv, generator=g).to(dt), torch.randn(T, 1, generator=g).to(dt)
+    z, rate, bias = torch.randn(T, d, generator=g).to(dt), torch.rand(1, generator=g) + 0.1, torch.randn(d, generator=g) - 2.0
+    decay = torch.exp(-rate.double() * torch.nn.functional.softplus(z.double() + bias.double()))
+    held = torch.randn(n, d, dv, generator=g)
+    state = held.transpose(1, 2).unsqueeze(1).contiguous().to(dev)
+    want, at = [], 0
+    for b, length in enumerate(lens):
+        S = held[b].double()
+        for t in range(at, at + length):
+            S = decay[t][:, None] * S
+            S = S + torch.outer(k[t, 0].double(), torch.sigmoid(beta[t].double()) * (v[t].double() - S.T @ k[t, 0].double()))
+            want.append(S.T @ q[t, 0].double())
+        held[b] = S.float()
+        at += length
+    (q_start, slot_t, fresh_t), how = _steps(lens, list(range(n)), [0] * n, dev)
+    got = ops.linear_recurrence(q.flatten(1).to(dev), k.flatten(1).to(dev), v.to(dev), state, q_start, slot_t, fresh_t, beta_logits=beta.to(dev),
+                                decay_logits=z.to(dev), decay_rate=rate.to(dev), decay_bias=bias.to(dev), **how)
+    want = torch.stack(want)
+    torch.testing.assert_close(got.cpu().double(), want, atol=2e-5 * float(want.abs().max()), rtol=1e-4)      # as above
+    torch.testing.assert_close(state[:, 0].transpose(1, 2).cpu(), held, atol=2e-5 * float(held.abs().max()), rtol=1e-4)
+
+
+@pytest.mark.parametrize("backend", BACKENDS)
 def test_results_that_are_columns_of_wider_rows(backend):
     """The head norm with a sigmoid gate, and attention with a gate in one key split and in several, writing into a column
     range of wider rows: the same numbers as into a tensor of their own, and nothing beside the range."""

@@ -10,25 +10,25 @@
 // that a token needs (two per column, taken from the decayed state before its update, and k . q:
 // o = S^T q + u (k . q)) are one round of shuffles.
 //
-// Steps with long portions: recurrence_blocks_kernel, four tokens at a time.  With S the state before a block, g_t a
-// token's decay, P_j = g_0 .. g_j, and D_ij = g_(i+1) .. g_j (so that P_j = g_0 D_0j):
+// Steps with long portions: recurrence_blocks_kernel, a block of four or eight tokens at a time.  With S the state before a
+// block, g_t a token's decay, P_j = g_0 .. g_j, D_ij = g_(i+1) .. g_j (so that P_j = g_0 D_0j), E the block's last token:
 //     d_j = (P_j k_j)^T S,   A_ij = (D_ij k_j) . k_i  (i < j),   u_j = beta_j (v_j - d_j - sum_(i<j) A_ij u_i)
 //     o_j = (P_j q_j)^T S + sum_(i<=j) B_ij u_i,                 B_ij = (D_ij q_j) . k_i
-//     S  <- P_3 S + sum_i (D_i3 k_i) u_i^T
+//     S  <- P_E S + sum_i (D_iE k_i) u_i^T
 // which is the token-by-token rule written out (no division, no approximation: only the order of additions differs);
 // for the fixed decay u_j = v_j.  The sums over the key size that a block needs are all taken from one and the same S:
-// one round of shuffles for four tokens instead of four rounds one after the other.
+// one round of shuffles for the block instead of a round per token one after the other.
 //
 // A CTA per (4 * 32 / KS * NC columns, head, request).  Four of its warps walk blocks: their lanes are 32 / KS groups of NC
 // columns x KS slices of the key size, and lane (group, s) keeps S[s R + r][its NC columns], r < R, in registers, in pairs
-// of neighbouring r (fma.rn.f32x2).  Four other warps prepare the next 16 tokens meanwhile: each turns the four tokens of a
-// block into P_j k_j, P_j q_j, D_i3 k_i and P_3 (rows in shared memory, slices padded so that they start in different
+// of neighbouring r (fma.rn.f32x2).  Four other warps prepare the next four blocks meanwhile: each turns the tokens of a
+// block into P_j k_j, P_j q_j, D_iE k_i and P_E (rows in shared memory, slices padded so that they start in different
 // banks) and the scalars A, B, beta, while the tokens after those are on their way from global memory.
 #include "common.cuh"
 
 namespace {
 
-constexpr int WALKERS = 128, NT = 256, BLOCK = 4, CHUNK = 16, NC = 2;      // (threads that walk; of a CTA)
+constexpr int WALKERS = 128, NT = 256, NC = 2;       // threads that walk; of a CTA; columns of a lane
 constexpr int STEP_NT = 128, STEP_COLS = 8;
 
 enum Decay : int { FIXED = 0, HEAD = 1, CHANNEL = 2 };
@@ -77,49 +77,52 @@ __device__ __forceinline__ pair_t mul2(pair_t a, pair_t b) {
 }
 __device__ __forceinline__ ulonglong2 row4(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
 
-// 16 values over the W lanes of a group: lane s of the group ends with the sums of values s * (16 / W) ... in v[0] ... (of a
-// whole warp: with sum s / 2)
-template <int W>
-__device__ __forceinline__ void reduce_scatter(float (&v)[16], int lane) {
+// N values over the W lanes of a group: with N >= W lane s of the group ends with the sums of values s * (N / W) ... in v[0] ...,
+// else with sum s / (W / N)
+template <int W, int N>
+__device__ __forceinline__ void reduce_scatter(float (&v)[N], int lane) {
 #pragma unroll
-    for (int mask = W / 2, m = 8; mask >= 1; mask >>= 1, m >>= 1) {
+    for (int mask = W / 2, m = N / 2; mask >= 1; mask >>= 1, m >>= 1) {
         const bool up = (lane & mask) != 0;
+        if (m == 0) v[0] += __shfl_xor_sync(0xffffffffu, v[0], mask);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < N / 2; ++i) {
             if (i >= m) break;
             const float send = up ? v[i] : v[i + m], keep = up ? v[i + m] : v[i];
             v[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
         }
     }
-    if (W == 32) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-template <int R, int KS, int MODE>
+// BLOCK tokens are one step of the walk; a buffer holds one block per warp that prepares
+template <int R, int KS, int MODE, int BLOCK>
 struct BlocksLayout {
     static constexpr bool DELTA = MODE != FIXED;
+    static constexpr int CHUNK = WALKERS / 32 * BLOCK;
     static constexpr int SLOT = R + 4;                   // a slice in shared memory
     static constexpr int PITCH = KS * SLOT;
     static constexpr int COLS = (WALKERS / 32) * (32 / KS) * NC;      // columns of a CTA
-    // one buffer of 16 tokens, in floats
+    // one buffer of CHUNK tokens, in floats
     static constexpr int KP = 0;                                     // [CHUNK][PITCH]: P_j k_j (delta rule)
     static constexpr int QP = KP + (DELTA ? CHUNK * PITCH : 0);      // [CHUNK][PITCH]: P_j q_j
-    static constexpr int KN = QP + CHUNK * PITCH;                    // [CHUNK][PITCH]: D_i3 k_i
-    static constexpr int P3 = KN + CHUNK * PITCH;                    // [CHUNK / BLOCK][PITCH]
-    static constexpr int V = P3 + CHUNK / BLOCK * PITCH;             // [CHUNK][COLS]
-    static constexpr int AB = V + CHUNK * COLS;                      // [CHUNK][8]: A_0j A_1j A_2j beta_j B_0j B_1j B_2j B_3j (B_ij = 0 for i > j)
-    static constexpr int SIZE = AB + CHUNK * 8;
+    static constexpr int KN = QP + CHUNK * PITCH;                    // [CHUNK][PITCH]: D_iE k_i, E the block's last token
+    static constexpr int PE = KN + CHUNK * PITCH;                    // [CHUNK / BLOCK][PITCH]: P_E
+    static constexpr int V = PE + CHUNK / BLOCK * PITCH;             // [CHUNK][COLS]
+    static constexpr int AB = V + CHUNK * COLS;                      // [CHUNK][2 BLOCK]: A_0j .. A_(BLOCK-2)j beta_j B_0j .. B_(BLOCK-1)j (0 for i > j)
+    static constexpr int SIZE = AB + CHUNK * 2 * BLOCK;
 };
 
 // The warps that prepare: tokens from global memory into registers, a chunk ahead, and from there into a buffer.
-template <int R, int KS, int MODE, typename TV>
+template <int R, int KS, int MODE, int BLOCK, typename TV>
 struct Preparer {
-    using L = BlocksLayout<R, KS, MODE>;
+    using L = BlocksLayout<R, KS, MODE, BLOCK>;
+    static constexpr int CHUNK = L::CHUNK;
     static constexpr int XN = (KS * R + 31) / 32;        // coordinates of a row that a lane brings
     static constexpr int V_EACH = (CHUNK * L::COLS + WALKERS - 1) / WALKERS;
     float fq[BLOCK][XN], fk[BLOCK][XN], fd[MODE == CHANNEL ? BLOCK : 1][XN];
     TV fv[V_EACH], fa, fb;                               // (converted when they are used: a conversion would wait for the load)
 
-    // the 16 tokens from t0 on: a warp brings the four of its block (past the portion's end: zeros, and decays of one)
+    // the CHUNK tokens from t0 on: a warp brings those of its block (past the portion's end: zeros, and decays of one)
     __device__ __forceinline__ void fetch(const RecurrenceParams& p, int start, int len, int t0, int tid, int h, int hq) {
         const int lane = tid & 31, warp = tid >> 5, n = min(len - t0, CHUNK), qk_row = p.G * p.dk;
 #pragma unroll
@@ -161,81 +164,65 @@ struct Preparer {
 #pragma unroll
             for (int w = 0; w < BLOCK; ++w) gs[w] = warp * BLOCK + w < n ? d : 1.f;
         }
-        float ab[16];                                   // A01 A02 A12 A03 A13 A23 | B00 B01 B11 B02 B12 B22 B03 B13 B23 B33
+        float ab[BLOCK * BLOCK];                        // of token j, from j * j on: A_0j .. A_(j-1)j, B_0j .. B_jj
 #pragma unroll
-        for (int i = 0; i < 16; ++i) ab[i] = 0.f;
+        for (int i = 0; i < BLOCK * BLOCK; ++i) ab[i] = 0.f;
 #pragma unroll
         for (int it = 0; it < XN; ++it) {
             const int d = lane + 32 * it;
-            constexpr int C = MODE == CHANNEL ? 1 : 0;
-            const float g0 = C ? fd[0][it] : gs[0], g1 = C ? fd[C][it] : gs[1], g2 = C ? fd[2 * C][it] : gs[2], g3 = C ? fd[3 * C][it] : gs[3];
-            const float k0 = fk[0][it], k1 = fk[1][it], k2 = fk[2][it], k3 = fk[3][it];
-            const float q0 = fq[0][it], q1 = fq[1][it], q2 = fq[2][it], q3 = fq[3][it];
-            const float p1 = g0 * g1, p2 = p1 * g2, p3 = p2 * g3;
-            const float e01 = g1 * k0, e02 = g2 * e01, e03 = g3 * e02, e12 = g2 * k1, e13 = g3 * e12, e23 = g3 * k2;
-            if (L::DELTA) {
-                ab[0] = fmaf(k1, e01, ab[0]);
-                ab[1] = fmaf(k2, e02, ab[1]);
-                ab[2] = fmaf(k2, e12, ab[2]);
-                ab[3] = fmaf(k3, e03, ab[3]);
-                ab[4] = fmaf(k3, e13, ab[4]);
-                ab[5] = fmaf(k3, e23, ab[5]);
-            }
-            ab[6] = fmaf(q0, k0, ab[6]);
-            ab[7] = fmaf(q1, e01, ab[7]);
-            ab[8] = fmaf(q1, k1, ab[8]);
-            ab[9] = fmaf(q2, e02, ab[9]);
-            ab[10] = fmaf(q2, e12, ab[10]);
-            ab[11] = fmaf(q2, k2, ab[11]);
-            ab[12] = fmaf(q3, e03, ab[12]);
-            ab[13] = fmaf(q3, e13, ab[13]);
-            ab[14] = fmaf(q3, e23, ab[14]);
-            ab[15] = fmaf(q3, k3, ab[15]);
-            if (d < KS * R) {
-                const int at = (d / R) * L::SLOT + (d & (R - 1)), row = warp * BLOCK * L::PITCH + at;
-                if (L::DELTA) {
-                    buf[L::KP + row] = g0 * k0;
-                    buf[L::KP + row + L::PITCH] = p1 * k1;
-                    buf[L::KP + row + 2 * L::PITCH] = p2 * k2;
-                    buf[L::KP + row + 3 * L::PITCH] = p3 * k3;
+            const int at = (d / R) * L::SLOT + (d & (R - 1)), row = warp * BLOCK * L::PITCH + at;
+            const bool in = d < KS * R;
+            float e[BLOCK], P = 1.f;                    // D_ij k_i; P_j
+#pragma unroll
+            for (int j = 0; j < BLOCK; ++j) {
+                const float gj = MODE == CHANNEL ? fd[MODE == CHANNEL ? j : 0][it] : gs[j], kj = fk[j][it], qj = fq[j][it];
+                P = j == 0 ? gj : P * gj;
+#pragma unroll
+                for (int i = 0; i < j; ++i) {
+                    e[i] *= gj;
+                    if (L::DELTA) ab[j * j + i] = fmaf(kj, e[i], ab[j * j + i]);
+                    ab[j * j + j + i] = fmaf(qj, e[i], ab[j * j + j + i]);
                 }
-                buf[L::QP + row] = g0 * q0;
-                buf[L::QP + row + L::PITCH] = p1 * q1;
-                buf[L::QP + row + 2 * L::PITCH] = p2 * q2;
-                buf[L::QP + row + 3 * L::PITCH] = p3 * q3;
-                buf[L::KN + row] = e03;
-                buf[L::KN + row + L::PITCH] = e13;
-                buf[L::KN + row + 2 * L::PITCH] = e23;
-                buf[L::KN + row + 3 * L::PITCH] = k3;
-                buf[L::P3 + warp * L::PITCH + at] = p3;
+                e[j] = kj;
+                ab[j * j + 2 * j] = fmaf(qj, kj, ab[j * j + 2 * j]);
+                if (in) {
+                    if (L::DELTA) buf[L::KP + row + j * L::PITCH] = P * kj;
+                    buf[L::QP + row + j * L::PITCH] = P * qj;
+                }
+            }
+            if (in) {
+#pragma unroll
+                for (int i = 0; i < BLOCK; ++i) buf[L::KN + row + i * L::PITCH] = e[i];
+                buf[L::PE + warp * L::PITCH + at] = P;
             }
         }
-        reduce_scatter<32>(ab, lane);                   // lane l ends with sum l / 2
-        const int i = lane >> 1;
-        int at;                                         // where sum i belongs
-        if (i < 6) {                                    // A_ij in the order 01 02 12 03 13 23
-            const int jj = i < 1 ? 1 : i < 3 ? 2 : 3, ii = i < 1 ? 0 : i < 3 ? i - 1 : i - 3;
-            at = jj * 8 + ii;
-        } else {                                        // B_ij in the order 00 01 11 02 12 22 03 13 23 33
-            const int x = i - 6, jj = x < 1 ? 0 : x < 3 ? 1 : x < 6 ? 2 : 3, ii = x - jj * (jj + 1) / 2;
-            at = jj * 8 + 4 + ii;
+        reduce_scatter<32>(ab, lane);                   // with 16 sums lane l ends with sum l / 2, with 64 with 2 l and 2 l + 1
+        constexpr int EACH = BLOCK * BLOCK > 32 ? BLOCK * BLOCK / 32 : 1;
+#pragma unroll
+        for (int x = 0; x < EACH; ++x) {
+            const int i = BLOCK * BLOCK >= 32 ? lane * EACH + x : lane / (32 / (BLOCK * BLOCK));
+            int j = 0;                                  // where sum i belongs: j * j <= i
+#pragma unroll
+            for (int c = 1; c < BLOCK; ++c) j += i >= c * c ? 1 : 0;
+            const int r = i - j * j;
+            if (L::DELTA || r >= j) buf[L::AB + (warp * BLOCK + j) * 2 * BLOCK + (r < j ? r : BLOCK + r - j)] = ab[x];
         }
-        if ((lane & 1) == 0) buf[L::AB + warp * BLOCK * 8 + at] = ab[0];
-        if (L::DELTA && lane < BLOCK) buf[L::AB + (warp * BLOCK + lane) * 8 + 3] = warp * BLOCK + lane < n ? 1.f / (1.f + expf(-to_float(fb))) : 0.f;
+        if (L::DELTA && lane < BLOCK) buf[L::AB + (warp * BLOCK + lane) * 2 * BLOCK + BLOCK - 1] = warp * BLOCK + lane < n ? 1.f / (1.f + expf(-to_float(fb))) : 0.f;
 #pragma unroll
         for (int i2 = 0; i2 < V_EACH; ++i2)
             if (tid + i2 * WALKERS < CHUNK * L::COLS) buf[L::V + tid + i2 * WALKERS] = to_float(fv[i2]);
     }
 };
 
-template <int R, int KS, int MODE, typename TV>
+template <int R, int KS, int MODE, int BLOCK, typename TV>
 __global__ void __launch_bounds__(NT) recurrence_blocks_kernel(const RecurrenceParams p) {
     extern __shared__ __align__(16) float smem[];
-    using L = BlocksLayout<R, KS, MODE>;
+    using L = BlocksLayout<R, KS, MODE, BLOCK>;
+    constexpr int CHUNK = L::CHUNK, AB_ROW = 2 * BLOCK;
     grid_launch_dependents();
-    constexpr int M = 16 / KS;                           // sums that a lane is left with
+    constexpr int N_SUMS = 2 * BLOCK * NC, M = N_SUMS / KS;            // sums that a lane is left with
     const int h = blockIdx.y, b = blockIdx.z, hq = h / (p.H / p.G);
-    for (int i = threadIdx.x; i < 2 * CHUNK * 8; i += NT) smem[(i / (CHUNK * 8)) * L::SIZE + L::AB + i % (CHUNK * 8)] = 0.f;
+    for (int i = threadIdx.x; i < 2 * CHUNK * AB_ROW; i += NT) smem[(i / (CHUNK * AB_ROW)) * L::SIZE + L::AB + i % (CHUNK * AB_ROW)] = 0.f;
     grid_dependency_wait();
     const int start = p.q_start[b], len = p.q_start[b + 1] - start;
     if (len <= 0) return;
@@ -244,7 +231,7 @@ __global__ void __launch_bounds__(NT) recurrence_blocks_kernel(const RecurrenceP
     if (threadIdx.x >= WALKERS) {
         // ---- the warps that prepare stay one chunk ahead; both sides meet at one barrier per chunk
         const int tid = threadIdx.x - WALKERS;
-        Preparer<R, KS, MODE, TV> prep;
+        Preparer<R, KS, MODE, BLOCK, TV> prep;
         prep.fetch(p, start, len, 0, tid, h, hq);
         for (int c = 0; c < n_chunks; ++c) {
             prep.put(p, smem + (c & 1) * L::SIZE, min(len - c * CHUNK, CHUNK), tid, h);
@@ -292,14 +279,14 @@ __global__ void __launch_bounds__(NT) recurrence_blocks_kernel(const RecurrenceP
                         for (int c = 0; c < NC; ++c) d2[j][c] = fma2(S[c][2 * r + 1], kv.y, fma2(S[c][2 * r], kv.x, d2[j][c]));
                     }
                 }
-            float sums[16];                             // d_jc at 2 j + c, o_jc at 8 + 2 j + c
+            float sums[N_SUMS];                         // d_jc at 2 j + c, o_jc at 2 BLOCK + 2 j + c
 #pragma unroll
             for (int j = 0; j < BLOCK; ++j)
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     const float2 x = unpack2(d2[j][c]), y = unpack2(o2[j][c]);
                     sums[2 * j + c] = x.x + x.y;
-                    sums[8 + 2 * j + c] = y.x + y.y;
+                    sums[2 * BLOCK + 2 * j + c] = y.x + y.y;
                 }
             reduce_scatter<KS>(sums, lane);             // lane s of a group holds sums s * M ... s * M + M - 1
             float u[BLOCK][NC];
@@ -310,19 +297,23 @@ __global__ void __launch_bounds__(NT) recurrence_blocks_kernel(const RecurrenceP
                 u[j][1] = vj.y;
             }
             if (L::DELTA) {
-                float dj[8];
+                float dj[2 * BLOCK];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) dj[i] = __shfl_sync(0xffffffffu, sums[i % M], i / M, KS);
+                for (int i = 0; i < 2 * BLOCK; ++i) dj[i] = __shfl_sync(0xffffffffu, sums[i % M], i / M, KS);
 #pragma unroll
                 for (int j = 0; j < BLOCK; ++j) {
-                    const float4 a = *reinterpret_cast<const float4*>(buf + L::AB + (w * BLOCK + j) * 8);
+                    float a[BLOCK];
+#pragma unroll
+                    for (int i = 0; i < BLOCK; i += 4) {
+                        const float4 a4 = *reinterpret_cast<const float4*>(buf + L::AB + (w * BLOCK + j) * AB_ROW + i);
+                        a[i] = a4.x; a[i + 1] = a4.y; a[i + 2] = a4.z; a[i + 3] = a4.w;
+                    }
 #pragma unroll
                     for (int c = 0; c < NC; ++c) {
                         float x = u[j][c] - dj[2 * j + c];
-                        if (j > 0) x = fmaf(-a.x, u[0][c], x);
-                        if (j > 1) x = fmaf(-a.y, u[1][c], x);
-                        if (j > 2) x = fmaf(-a.z, u[2][c], x);
-                        u[j][c] = a.w * x;
+#pragma unroll
+                        for (int i = 0; i < j; ++i) x = fmaf(-a[i], u[i][c], x);
+                        u[j][c] = a[BLOCK - 1] * x;
                     }
                 }
             }
@@ -333,7 +324,7 @@ __global__ void __launch_bounds__(NT) recurrence_blocks_kernel(const RecurrenceP
                 for (int c = 0; c < NC; ++c) uu[j][c] = pack2(u[j][c], u[j][c]);
 #pragma unroll
             for (int r = 0; r < R / 4; ++r) {
-                const ulonglong2 pv = row4(buf + L::P3 + w * L::PITCH + s * L::SLOT + 4 * r);
+                const ulonglong2 pv = row4(buf + L::PE + w * L::PITCH + s * L::SLOT + 4 * r);
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
                     S[c][2 * r] = mul2(S[c][2 * r], pv.x);
@@ -349,16 +340,19 @@ __global__ void __launch_bounds__(NT) recurrence_blocks_kernel(const RecurrenceP
                     }
                 }
             }
-            if (s * M >= 8) {                           // the lanes that hold o
+            if (s * M >= 2 * BLOCK) {                   // the lanes that hold o
 #pragma unroll
                 for (int i = 0; i < M; ++i) {
-                    const int x = s * M + i - 8, j = x >> 1, c = x & 1;
-                    const float4 bj = *reinterpret_cast<const float4*>(buf + L::AB + (w * BLOCK + j) * 8 + 4);
+                    const int x = s * M + i - 2 * BLOCK, j = x >> 1, c = x & 1;
                     float o = sums[i];
-                    o = fmaf(bj.x, c ? u[0][1] : u[0][0], o);
-                    o = fmaf(bj.y, c ? u[1][1] : u[1][0], o);
-                    o = fmaf(bj.z, c ? u[2][1] : u[2][0], o);
-                    o = fmaf(bj.w, c ? u[3][1] : u[3][0], o);
+#pragma unroll
+                    for (int y = 0; y < BLOCK; y += 4) {
+                        const float4 bj = *reinterpret_cast<const float4*>(buf + L::AB + (w * BLOCK + j) * AB_ROW + BLOCK + y);
+                        o = fmaf(bj.x, c ? u[y][1] : u[y][0], o);
+                        o = fmaf(bj.y, c ? u[y + 1][1] : u[y + 1][0], o);
+                        o = fmaf(bj.z, c ? u[y + 2][1] : u[y + 2][0], o);
+                        o = fmaf(bj.w, c ? u[y + 3][1] : u[y + 3][0], o);
+                    }
                     if (w * BLOCK + j < n && j0 + c < p.dv)
                         p.out[((size_t)(start + t0 + w * BLOCK + j) * p.H + h) * p.dv + j0 + c] = o;
                 }
@@ -488,23 +482,27 @@ __global__ void __launch_bounds__(STEP_NT) recurrence_steps_kernel(const Recurre
         }
 }
 
-template <int R, int KS, int MODE, typename TV>
+template <int R, int KS, int MODE, int BLOCK, typename TV>
 cudaError_t launch_blocks(const RecurrenceParams& p, int n_seqs, cudaStream_t s) {
-    using L = BlocksLayout<R, KS, MODE>;
+    using L = BlocksLayout<R, KS, MODE, BLOCK>;
     constexpr size_t smem = 2 * L::SIZE * sizeof(float);
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(recurrence_blocks_kernel<R, KS, MODE, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(recurrence_blocks_kernel<R, KS, MODE, BLOCK, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    return tl_launch(recurrence_blocks_kernel<R, KS, MODE, TV>, dim3((p.dv + L::COLS - 1) / L::COLS, p.H, n_seqs), dim3(NT), smem, s, p);
+    return tl_launch(recurrence_blocks_kernel<R, KS, MODE, BLOCK, TV>, dim3((p.dv + L::COLS - 1) / L::COLS, p.H, n_seqs), dim3(NT), smem, s, p);
 }
 
 template <int MODE, typename TV>
 cudaError_t launch_block_sizes(const RecurrenceParams& p, int n_seqs, cudaStream_t s) {
-    if (p.dk <= 32) return launch_blocks<8, 4, MODE, TV>(p, n_seqs, s);
-    if (p.dk <= 64) return launch_blocks<8, 8, MODE, TV>(p, n_seqs, s);
-    if (p.dk <= 128) return launch_blocks<8, 16, MODE, TV>(p, n_seqs, s);
-    return launch_blocks<16, 16, MODE, TV>(p, n_seqs, s);
+    // A walk of 8 tokens a block takes fewer rounds of sums over the lanes, and gives each warp more that does not depend
+    // on what came before: 601 tokens, 16 heads of 128, a decay per channel: 97.1 us in blocks of 4, 89.0 in blocks
+    // of 8.  (One column a lane with two CTAs an SM: 131.7.)  The other decays and sizes keep blocks of 4: theirs is the
+    // only form that has been measured.
+    if (p.dk <= 32) return launch_blocks<8, 4, MODE, 4, TV>(p, n_seqs, s);
+    if (p.dk <= 64) return launch_blocks<8, 8, MODE, 4, TV>(p, n_seqs, s);
+    if (p.dk <= 128) return launch_blocks<8, 16, MODE, MODE == CHANNEL ? 8 : 4, TV>(p, n_seqs, s);
+    return launch_blocks<16, 16, MODE, 4, TV>(p, n_seqs, s);
 }
 
 template <int MODE, typename TV>
@@ -536,7 +534,7 @@ int launch_mode(const RecurrenceParams& p, int n_seqs, int mode, bool blocks, cu
 // logits (of v's dtype), decay is exp(A_log) per head.  mode 1: gate are rows of pitch ldz with `heads` columns and
 // decay_bias [heads] the bias inside the softplus.  mode 2, a decay per channel: gate has heads * dk columns and decay_bias
 // heads * dk numbers, or, with blocks != 0, gate is float32 [n_tokens][heads * dk], the decays themselves.
-// blocks != 0: for steps with long portions, four tokens at a time.
+// blocks != 0: for steps with long portions, blocks of tokens at a time.
 extern "C" int tl_linear_recurrence(const float* q, const float* k, const void* v, int v_dtype, long long ldv, const void* beta,
                                     long long ldg, const void* gate, long long ldz, const float* decay, const float* decay_bias, float* state,
                                     long long state_pitch, const int* q_start, const int* state_slot, const int* fresh,

@@ -1079,7 +1079,7 @@ class NativeOps:
         self.launches += 2 if (max_q_len > 4 and w_conv.shape[0] > 1) else 1
         return q, k, v, small, low
 
-    BLOCKS_MIN_Q = 9      # steps with portions at least this long run a matrix recurrence four tokens at a time
+    BLOCKS_MIN_Q = 9      # steps with portions at least this long run a matrix recurrence in blocks of tokens
 
     @_timed
     def recurrence_prep(self, x: torch.Tensor, *, scale: float, n_heads: int, head_dim: int,
@@ -1123,7 +1123,7 @@ class NativeOps:
         per head and key coordinate: ``decay_logits`` ``[T, H * dk]`` and ``decay_bias`` ``[H * dk]``, each acting on its row of ``S``.
         ``q``, ``k``: float32 ``[T, G * dk]``, ``G`` heads each shared by ``H / G`` value heads; ``v``: ``[T, H * dv]``;
         ``state``: ``[slots, H, dv, dk]`` (a head's matrix with a column's keys side by side), read (zeros where
-        ``fresh``) and left updated.  Returns float32 ``[T, H * dv]``.  Steps with long portions take four tokens at a time
+        ``fresh``) and left updated.  Returns float32 ``[T, H * dv]``.  Steps with long portions take blocks of tokens
         (the same rule written out), others one."""
         _cuda_contig(q, "q", torch.float32)
         _cuda_contig(k, "k", torch.float32)
