@@ -935,3 +935,22 @@ def test_sampling_follows_the_softmax(ops):
     p3 = torch.softmax(base[[0, 1, 6]] / 0.8, -1).numpy()
     f3 = np.array([(got3 == i).mean() for i in (0, 1, 6)])
     assert np.abs(f3 - p3).max() < 0.02
+
+
+def test_tokens_read_back_several_at_a_time(ops):
+    """Buffers of tokens on their way to the host are used again only when they have been read: sizes around the smallest
+    buffer, more in flight than are kept, finished out of order, and asked for twice."""
+    from torchllms_b200.sampling.sampler import Sampler
+    sampler = Sampler(ops, "cuda")
+    for round_ in range(3):
+        rows = [torch.arange(n, dtype=torch.int32, device="cuda") + 1000 * n + round_ for n in (1, 64, 65, 3, 200, 64, 7)]
+        pending = [sampler.read_back(r) for r in rows]
+        for i in (3, 0, 6, 5, 1, 2, 4):
+            assert sampler.finish(pending[i]) == rows[i].tolist()
+        for p, r in zip(pending, rows):
+            assert sampler.finish(p) == r.tolist()
+        assert len(sampler._rooms) <= Sampler.ROOMS
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        got = sampler.read_back(torch.full((5,), 9, dtype=torch.int32, device="cuda"))
+        assert sampler.finish(got) == [9] * 5

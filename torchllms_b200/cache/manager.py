@@ -303,7 +303,7 @@ class CacheManager:
 
         Returns each request's length before the call (the position of its
         first new token) and advances the lengths."""
-        seen = set()
+        seen, reqs = set(), []
         for handle, n in wants:
             if handle in seen:
                 raise CacheError(f"request handle {handle} appears twice in one batch")
@@ -314,17 +314,17 @@ class CacheManager:
             if req.length + n > self.max_len:
                 raise CacheError(
                     f"request {handle}: {req.length} + {n} tokens exceed the longest sequence ({self.max_len})")
-        need = [sum(self._blocks_wanted(self._req(h), gi, n) for h, n in wants) for gi in range(len(self.groups))]
+            reqs.append((req, n))
+        blocks = [[self._blocks_wanted(req, gi, n) for req, n in reqs] for gi in range(len(self.groups))]
         for gi, g in enumerate(self.groups):
-            if need[gi] > g.allocator.n_free:
+            if sum(blocks[gi]) > g.allocator.n_free:
                 raise OutOfPages(
-                    f"group {gi} ({g.need.kind}): {need[gi]} pages wanted, {g.allocator.n_free} of "
+                    f"group {gi} ({g.need.kind}): {sum(blocks[gi])} pages wanted, {g.allocator.n_free} of "
                     f"{g.allocator.n_pages} free")
         starts = []
-        for handle, n in wants:
-            req = self._req(handle)
+        for i, (req, n) in enumerate(reqs):
             for gi, g in enumerate(self.groups):
-                k = self._blocks_wanted(req, gi, n)
+                k = blocks[gi][i]
                 if k:
                     new = g.allocator.alloc(k)
                     lo = len(req.blocks[gi])

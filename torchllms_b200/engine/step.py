@@ -26,6 +26,7 @@ import numpy as np
 import torch
 
 from ..cache.manager import CacheManager, OutOfPages
+from ..kernels.streams import current_stream
 from .model import Model
 
 
@@ -144,7 +145,7 @@ class _StepBuffers:
         self.uploaded_bytes = 4 * (end - start)
         self.dev[start:end].copy_(self.host[start:end], non_blocking=True)
         if self.copied is not None:
-            self.copied.record()
+            self.copied.record(current_stream())
             self._pending = True
 
 
@@ -166,6 +167,7 @@ class Engine:
         self._buf = _StepBuffers(self.cache, self.max_step_tokens, self.device)
         self._has_window = any(g.gives_back for g in self.cache.groups)
         self.vocab_size = model.spec.vocab_size
+        self._count = np.arange(self.cache.max_num_seqs + 1, dtype=np.int64)
         self.steps_run = 0
         self.tokens_run = 0
         # A step's launch shapes depend only on (tokens, requests, wanted rows, longest portion) and, for
@@ -322,15 +324,19 @@ class Engine:
         # Inside the batch, requests that bring one token stand before those that bring more (each kind
         # in the caller's order): the mixer sends the two kinds to kernels made for them.  The wanted
         # rows keep the caller's order, so nothing of this shows outside.
-        order = sorted(range(B), key=lambda i: shape[i][1] != 1)
-        identity = order == list(range(B))
-        handles = [shape[i][0] for i in order]
-        q_lens = [shape[i][1] for i in order]
-        base_of = [0] * B                       # caller's entry -> its first row in the batch
-        base = 0
-        for i in order:
-            base_of[i] = base
-            base += shape[i][1]
+        if T == B:                              # one token each: as given
+            order, identity = None, True
+            handles, q_lens, base_of = [h for h, _n, _w in shape], [1] * B, range(B)
+        else:
+            order = sorted(range(B), key=lambda i: shape[i][1] != 1)
+            identity = order == list(range(B))
+            handles = [shape[i][0] for i in order]
+            q_lens = [shape[i][1] for i in order]
+            base_of = [0] * B                   # caller's entry -> its first row in the batch
+            base = 0
+            for i in order:
+                base_of[i] = base
+                base += shape[i][1]
         want_rows: List[int] = []
         for i, (_h, n, want) in enumerate(shape):
             want_rows += [base_of[i] + w for w in ([n - 1] if want is None else want)]
@@ -341,15 +347,19 @@ class Engine:
             buf = self._buf
             buf.wait_host_free()
             buf.lay_out(T, B)
-            lens = np.asarray(q_lens, dtype=np.int64)
             first = np.asarray(starts, dtype=np.int64)
-            q_start = np.zeros(B + 1, dtype=np.int64)
-            np.cumsum(lens, out=q_start[1:])
-            kv_lens = (first + lens).tolist()
             slots = [cache.slot(h) for h in handles]
             # per token: which request it belongs to and its absolute position (no loop over requests)
-            seq_of = np.repeat(np.arange(B, dtype=np.int64), lens)
-            pos_all = np.arange(T, dtype=np.int64) - q_start[seq_of] + first[seq_of]
+            if T == B:
+                q_start, seq_of, pos_all = self._count[:B + 1], self._count[:B], first
+                kv_lens = [n + 1 for n in starts]
+            else:
+                lens = np.asarray(q_lens, dtype=np.int64)
+                q_start = np.zeros(B + 1, dtype=np.int64)
+                np.cumsum(lens, out=q_start[1:])
+                kv_lens = (first + lens).tolist()
+                seq_of = np.repeat(self._count[:B], lens)
+                pos_all = np.arange(T, dtype=np.int64) - q_start[seq_of] + first[seq_of]
             buf.host_view("positions")[:T] = pos_all
             buf.host_view("seq_of_token")[:T] = seq_of
             buf.host_view("q_start")[:B + 1] = q_start

@@ -16,6 +16,8 @@ from typing import List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..kernels.streams import current_stream
+
 MASK64 = (1 << 64) - 1
 GOLDEN = 0x9E3779B97F4A7C15
 
@@ -46,16 +48,21 @@ class SamplingParams:
 class PendingTokens:
     """Sampled tokens on their way to the host."""
 
-    __slots__ = ("host", "done")
+    __slots__ = ("host", "done", "room")
 
-    def __init__(self, host: torch.Tensor, done):
-        self.host, self.done = host, done
+    def __init__(self, host, done, room: Optional[torch.Tensor] = None):
+        self.host, self.done, self.room = host, done, room      # room: the pinned buffer that ``host`` is the start of
 
 
 class Sampler:
+    ROOMS = 4
+
     def __init__(self, ops, device):
         self.ops = ops
         self.device = torch.device(device)
+        # pinned buffers that are free again, with their events (allocating the two takes as long as the copy): at most
+        # ROOMS, as many as steps in flight want
+        self._rooms: List[tuple] = []
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], requests: Sequence[int],
                token_indices: Sequence[int]) -> List[int]:
@@ -90,18 +97,29 @@ class Sampler:
         this call does not delay :meth:`finish`, which waits for this copy alone."""
         if tokens.device.type != "cuda":
             return PendingTokens(tokens, None)
-        host = torch.empty(tokens.shape, dtype=tokens.dtype, pin_memory=True)
+        n = tokens.numel()
+        try:
+            room, done = self._rooms.pop()
+        except IndexError:
+            room = None
+        if room is None or room.numel() < n or room.dtype != tokens.dtype or tokens.dim() != 1:
+            room, done = torch.empty(max(n, 64), dtype=tokens.dtype, pin_memory=True), torch.cuda.Event()
+        host = room[:n].view(tokens.shape)
         host.copy_(tokens, non_blocking=True)
-        done = torch.cuda.Event()
-        done.record()
-        return PendingTokens(host, done)
+        done.record(current_stream())
+        return PendingTokens(host, done, room)
 
     def finish(self, tokens) -> List[int]:
         """The tokens of :meth:`launch` (or of :meth:`read_back`) on the host; this waits for them."""
         if isinstance(tokens, PendingTokens):
-            if tokens.done is not None:
-                tokens.done.synchronize()
-            return self._checked(tokens.host.tolist())
+            if isinstance(tokens.host, torch.Tensor):
+                if tokens.done is not None:
+                    tokens.done.synchronize()
+                room, tokens.host = tokens.room, tokens.host.tolist()
+                if room is not None and len(self._rooms) < self.ROOMS:
+                    self._rooms.append((room, tokens.done))         # (read: nothing is on its way into it any more)
+                tokens.room = tokens.done = None
+            return self._checked(list(tokens.host))
         return self._checked(tokens.tolist())
 
     def _checked(self, tokens: List[int]) -> List[int]:
