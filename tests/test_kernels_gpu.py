@@ -74,7 +74,7 @@ def test_rmsnorm_rows_leaves_stream_alone(ops, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("n,hidden", [(1, 8), (5, 192), (64, 1000), (3, 14336), (7, 166), (3, 5)])
+@pytest.mark.parametrize("n,hidden", [(1, 8), (5, 192), (64, 1000), (3, 14336), (7, 166), (3, 5), (300, 4088), (2, 4096), (70, 4104)])
 def test_swiglu(ops, dtype, n, hidden):
     x = rand((n, 2 * hidden), dtype, 8, 3.0)
     got, want = ops.swiglu(x), TWIN.swiglu(x)
