@@ -446,6 +446,26 @@ def test_rope_kv_write(ops, dtype, H, KV, hd, P, interleaved):
     assert torch.equal(q1, q3)
 
 
+@pytest.mark.parametrize("H,KV,hd", [(32, 8, 128), (24, 8, 128), (3, 1, 64), (40, 2, 8), (5, 5, 48)])
+def test_rope_of_many_tokens_is_that_of_few(ops, H, KV, hd):
+    """From 256 tokens on another kernel rotates heads of a power of two: bit for bit the one for fewer tokens."""
+    T, P, parts, max_pos = 300, 16, 4, 999
+    qkv, ssq = rand((T, (H + 2 * KV) * hd), torch.bfloat16, 51), rand((T, parts), torch.float32, 52).abs() + 0.1
+    pos = torch.randint(0, max_pos, (T,), dtype=torch.int32).cuda()
+    table = rand((max_pos, hd // 2, 2), torch.float32, 53)
+    slots = torch.randperm(32 * P)[:T].to(torch.int32).cuda()
+    kw = dict(n_heads=H, n_kv_heads=KV, head_dim=hd, interleaved=True, page_size=P)
+    from torchllms_b200.kernels.lazy import RowScaled
+    for scaled in (False, True):
+        of = lambda a, b: RowScaled(qkv[a:b], ssq[a:b], 64, 1e-5) if scaled else qkv[a:b]  # noqa: E731
+        pages = [torch.full((32, KV, P, hd), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+        whole = ops.rope_kv_write(of(0, T), pos, table, k_pages=pages[0], v_pages=pages[1], slot_mapping=slots, **kw)
+        cut = [ops.rope_kv_write(of(a, b), pos[a:b], table, k_pages=pages[2], v_pages=pages[3], slot_mapping=slots[a:b], **kw)
+               for a, b in ((0, 200), (200, T))]
+        assert torch.equal(whole, torch.cat(cut)) and torch.equal(pages[0], pages[2]) and torch.equal(pages[1], pages[3])
+        assert torch.equal(whole, ops.rope_kv_write(of(0, T), pos, table, k_pages=None, v_pages=None, slot_mapping=None, **kw))
+
+
 # ------------------------------------------------------------------------------- attention
 
 def build_paged(seq_lens, q_lens, H, KV, hd, P, dtype, seed, n_extra_pages=3, peak=None):

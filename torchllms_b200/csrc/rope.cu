@@ -179,6 +179,80 @@ __global__ void rope_kv_write_vec_kernel(const TI* __restrict__ qkv, int splits,
     }
 }
 
+// The same for the many tokens of a prompt, bfloat16 in and out, one plane, heads of a power of two up to 1,024: a
+// thread's runs of eight lanes lie a multiple of the head size apart, so that one run of the rotation table serves them all,
+// heads come by a shift, and all loads of a token are under way together.  The kernel above loads, divides and
+// rotates one run after the other (1,209 tokens, 48 heads of 64, in 16 layers of a 1B step: 3,213 us -> 3,182 for the step;
+// prompts of 2,000 and more at the power cap's clock: within what two runs differ by).  With fewer than 256 tokens a
+// token's heads are spread over more CTAs, and a thread has one run at most.
+constexpr int ROPE_EACH = 3;
+__global__ void __launch_bounds__(128) rope_kv_write_rows_kernel(const __nv_bfloat16* __restrict__ qkv, const int* __restrict__ positions,
+                                                                 const float* __restrict__ table, const int* __restrict__ slot_mapping,
+                                                                 __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_pages,
+                                                                 __nv_bfloat16* __restrict__ v_pages, int n_heads, int n_kv_heads,
+                                                                 int head_dim, int log_runs, int page_size, int table_rows, const RowScale rs) {
+    grid_launch_dependents();
+    const int t = blockIdx.x;
+    const int heads = n_heads + 2 * n_kv_heads, runs = heads << log_runs, stride = gridDim.y * blockDim.x;
+    int pos = positions[t];
+    (void)TL_CHECK(pos >= 0 && pos < table_rows, TL_DBG_POSITION);
+    pos = pos < 0 ? 0 : (pos >= table_rows ? table_rows - 1 : pos);
+    bool write = k_pages != nullptr;
+    int page = 0, slot = 0;
+    if (write) {
+        const int sm = slot_mapping[t];
+        page = sm / page_size;
+        slot = sm - page * page_size;
+        if (!(TL_CHECK(sm >= 0, TL_DBG_SLOT) && tl_check_page(page))) write = false;    // (debug builds: nothing is written there)
+    }
+    const int c_first = blockIdx.y * blockDim.x + threadIdx.x;
+    const int off = (c_first & ((1 << log_runs) - 1)) << 3;
+    float r[8];
+    load8(table + (size_t)pos * head_dim + off, r);      // (cos, sin) of the four pairs
+    grid_dependency_wait();
+    const __nv_bfloat16* src = qkv + (size_t)t * heads * head_dim;
+    uint4 raw[ROPE_EACH];
+    auto fetch = [&](int c0) {
+#pragma unroll
+        for (int e = 0; e < ROPE_EACH; ++e)
+            if (c0 + e * stride < runs) raw[e] = *reinterpret_cast<const uint4*>(src + (size_t)(c0 + e * stride) * 8);
+    };
+    fetch(c_first);
+    const float sc = warp_row_scale(rs, t);            // (a CTA's threads all work on token t; all of a warp take part)
+    for (int c0 = c_first; c0 < runs; c0 += ROPE_EACH * stride) {
+        if (c0 != c_first) fetch(c0);
+#pragma unroll
+        for (int e = 0; e < ROPE_EACH; ++e) {
+            const int c = c0 + e * stride;
+            if (c >= runs) break;
+            const int head = c >> log_runs;
+            float x[8];
+            const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(&raw[e]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 v = __bfloat1622float2(x2[i]);
+                x[2 * i] = v.x * sc;
+                x[2 * i + 1] = v.y * sc;
+            }
+            if (head < n_heads + n_kv_heads) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float a = x[2 * i], b = x[2 * i + 1], co = r[2 * i], si = r[2 * i + 1];
+                    x[2 * i] = a * co - b * si;
+                    x[2 * i + 1] = b * co + a * si;
+                }
+            }
+            if (head < n_heads) {
+                store8(q_out + ((size_t)t * n_heads + head) * head_dim + off, x);
+            } else if (write) {
+                const bool is_k = head < n_heads + n_kv_heads;
+                const int kvh = is_k ? head - n_heads : head - n_heads - n_kv_heads;
+                store8((is_k ? k_pages : v_pages) + (((size_t)page * n_kv_heads + kvh) * page_size + slot) * head_dim + off, x);
+            }
+        }
+    }
+}
+
 // k_pages / v_pages may both be null: then only q is produced (a run that reads another run's cache).
 // qkv: [splits, n_tokens, row] of in_dtype (splits > 1 only for float32 partial sums); q, pages: dtype.
 // in_ssq may be null; else [n_tokens, in_parts] floats give every token's row scale (see the top of the file).
@@ -208,6 +282,14 @@ extern "C" int tl_rope_kv_write(const void* qkv, int in_dtype, int splits, const
         const int vthreads = 128;
         int by = (chunks8 + vthreads - 1) / vthreads;
         if (n_tokens >= 256 && by > 2) by = 2;        // many tokens: fewer, fatter CTAs
+        const int head_runs = head_dim / 8;
+        if (in_dtype == TL_BF16 && dtype == TL_BF16 && splits == 1 && n_tokens >= 256 && head_runs <= vthreads && (head_runs & (head_runs - 1)) == 0) {
+            int log_runs = 0;
+            while ((1 << log_runs) < head_runs) ++log_runs;
+            return (int)tl_launch(rope_kv_write_rows_kernel, dim3(n_tokens, by), dim3(vthreads), 0, s, (const __nv_bfloat16*)qkv, positions,
+                                  table, slot_mapping, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, n_heads,
+                                  n_kv_heads, head_dim, log_runs, page_size, table_rows, rs);
+        }
 #define TL_ROPE_VEC(TI, T)                                                                                      \
     tl_launch(rope_kv_write_vec_kernel<TI, T>, dim3(n_tokens, by), dim3(vthreads), 0, s,                        \
               (const TI*)qkv, splits, plane, positions, table, slot_mapping, (T*)q_out, (T*)k_pages, (T*)v_pages, \
