@@ -725,6 +725,38 @@ def test_decode_attention_in_shares(ops, case):
     torch.testing.assert_close(pieces.float(), want.float(), atol=2e-2, rtol=2e-2)       # bfloat16 results of unit values, as above
 
 
+def test_decode_attention_in_shares_gives_up(ops):
+    """A third of the CTAs wait for room that nobody makes.  They give up, say so and go on to their end, the others write what
+    they write anyway, no row is made of parts of which one is missing, and the counters are zero again."""
+    from torchllms_b200.kernels.native import KernelError, _ptr, _stream
+    B, H, KV, hd, P = 40, 32, 8, 64, 16
+    g = torch.Generator().manual_seed(5)
+    seq_lens = torch.randint(1, 1500, (B,), generator=g).tolist()
+    a = build_paged(seq_lens, [1] * B, H, KV, hd, P, torch.bfloat16, seed=5)
+    a["max_kv_len"] = 8192
+    a["block_table"] = torch.nn.functional.pad(a["block_table"], (0, 8192 // P - a["block_table"].shape[1]))
+    want = ops.paged_attention(**a, scale=hd ** -0.5, window=None, impl="decode")
+    lib = ops._lib("attention_decode")
+    n, floats, counters = ctypes.c_int(0), ctypes.c_longlong(0), ctypes.c_longlong(0)
+    assert lib.tl_attention_decode_plan(B, B, H, KV, hd, 1, 8192, 1, ctypes.byref(n), ctypes.byref(floats), ctypes.byref(counters)) == 0
+    counts = torch.zeros(counters.value, dtype=torch.int32, device="cuda")
+    ws, out = torch.full((floats.value,), float("nan"), device="cuda"), torch.full_like(want, float("nan"))
+    rc = lib.tl_attention_decode_give_up_selftest(
+        _ptr(a["q"]), _ptr(a["k_pages"]), _ptr(a["v_pages"]), _ptr(out), _ptr(a["block_table"]), a["block_table"].stride(0), _ptr(a["q_start"]),
+        _ptr(a["kv_len"]), _ptr(ws), _ptr(counts), ctypes.c_void_p(ops._status.data_ptr()), B, B, H, KV, hd, P,
+        ctypes.c_longlong(a["k_pages"].shape[0]), 1, 8192, 0, ctypes.c_float(hd ** -0.5), ctypes.c_ulonglong(5_000_000), _stream())
+    assert rc == 0
+    torch.cuda.synchronize()
+    with pytest.raises(KernelError, match="gave up waiting .code 21[12]."):
+        ops.check_status()
+    written = ~out.isnan().any(-1)
+    assert 0 < int(written.sum()) < B * H
+    assert torch.equal(out[written], want[written]) and bool(out[~written].isnan().all())
+    assert not counts.any()
+    assert torch.equal(ops.paged_attention(**a, scale=hd ** -0.5, window=None, impl="decode"), want)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("dtype,impl", IMPLS)
 @pytest.mark.parametrize("key_pos", [0, 15, 16, 511, 640])
 def test_attention_finds_one_far_key_among_hundreds(ops, dtype, impl, key_pos):

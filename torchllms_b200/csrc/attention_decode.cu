@@ -30,7 +30,8 @@
 // probabilities change sides between the two products (result columns -> operand columns),
 // which is one movmatrix per 8 x 8 block.
 // Every mbarrier wait is bounded in time; on a time-out the CTA records a code in the status
-// word, writes nothing and returns.
+// word and writes no results from there on.  With shares it still goes through its pieces: the other CTAs
+// of a request count on it, and whoever is last learns from the count that a part is missing.
 #include "common.cuh"
 #include <cuda.h>
 #include <limits.h>
@@ -72,6 +73,7 @@ struct DecodeParams {
     int window;
     int streamed;               // the call reads more keys and values than L2 holds: their copies are marked to leave it first
     float scale_log2;
+    unsigned long long limit_ns;    // self-test only: how long a wait may take
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -90,7 +92,7 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, volatile int* failed) {
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, volatile int* failed, unsigned long long limit_ns = WAIT_NS) {
     if (mbar_try_wait(bar, parity)) return true;
     unsigned long long t0;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
@@ -99,7 +101,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
         if ((i & 255u) == 0u) {
             unsigned long long t1;
             asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-            if (*failed || t1 - t0 > WAIT_NS) return false;
+            if (*failed || t1 - t0 > limit_ns) return false;
         }
     }
 }
@@ -258,7 +260,8 @@ __device__ __forceinline__ bool walk_share(const DecodeParams& p, Walk& w, int l
 // NT: 8-row blocks of query rows (1: up to 8 rows, 2: up to 16)
 // SHARES: a CTA takes a share of all pieces and the last one adds a request's up; else a CTA to a piece
 // (blockIdx: request z, unit y, piece x), and merge_partials_kernel follows
-template <int HD, int STAGES, int NT, bool SHARES>
+// SELFTEST: every third CTA never hands back its first stage, so that its producer's wait for room runs out
+template <int HD, int STAGES, int NT, bool SHARES, bool SELFTEST = false>
 __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                                   const __grid_constant__ CUtensorMap map_v,
                                                                                   const DecodeParams p) {
@@ -281,7 +284,7 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
     __shared__ __align__(8) unsigned long long full_bar[STAGES];
     __shared__ __align__(8) unsigned long long empty_bar[STAGES];
     __shared__ int failed_flag;
-    __shared__ int arrived;
+    __shared__ int arrived, gave_up;
 
     grid_launch_dependents();
     // What follows, down to the dependency wait, reads nothing that the kernels just before this one
@@ -290,6 +293,7 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
     // dependent launch this part runs while the predecessor is still at work.
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     volatile int* failed = &failed_flag;
+    const unsigned long long limit_ns = SELFTEST ? p.limit_ns : WAIT_NS;
     Walk w;
     if (SHARES) {
         if (!walk_share(p, w, lane)) return;            // (the same for all warps)
@@ -328,11 +332,8 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                     grid_dependency_wait();
                     waited = true;
                 }
-                if (it >= STAGES && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ((it / STAGES) - 1) & 1, failed))) {
-                    if (lane == 0) {
-                        failed_flag = 1;
-                        atomicExch(p.status, ERR_PRODUCER_WAIT);
-                    }
+                if (it >= STAGES && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ((it / STAGES) - 1) & 1, failed, limit_ns))) {
+                    if (lane == 0 && atomicExch(&failed_flag, 1) == 0) atomicExch(p.status, ERR_PRODUCER_WAIT);
                     ok = false;
                     break;
                 }
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
         if (!waited) grid_dependency_wait();
         // (nothing that is still on its way may land in shared memory that is no longer this CTA's)
         int never = 0;
-        for (int k = max(0, it - STAGES); k < it; ++k) mbar_wait(&full_bar[k % STAGES], (k / STAGES) & 1, &never);
+        for (int k = max(0, it - STAGES); k < it; ++k) mbar_wait(&full_bar[k % STAGES], (k / STAGES) & 1, &never, limit_ns);
         return;
     }
 
@@ -441,13 +442,12 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
         const int warp_qmin = __reduce_min_sync(0xffffffffu, qmin);
         for (int i = 0; i < w.tiles; ++i, ++it) {
             const int s = it % STAGES;
-            if (ok && !mbar_wait(&full_bar[s], (it / STAGES) & 1, failed)) {
-                ok = false;
-                failed_flag = 1;
-                if (lane == 0) atomicExch(p.status, ERR_CONSUMER_WAIT);
+            ok = __all_sync(0xffffffffu, ok && mbar_wait(&full_bar[s], (it / STAGES) & 1, failed, limit_ns));
+            if (!ok) {
+                // (whichever lane's wait ran out; one that only stopped with another's has nothing to report)
+                if (lane == 0 && atomicExch(&failed_flag, 1) == 0) atomicExch(p.status, ERR_CONSUMER_WAIT);
+                break;
             }
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
             const int share_lo = w.start + i * BN + key_off;
             if (share_lo <= warp_qmax && share_lo + 16 > k_lo) {
                 const unsigned kt = smem_u32(tiles + s * STAGE_BYTES);
@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&empty_bar[s]);     // this warp is done with the stage
+            if (lane == 0 && !(SELFTEST && it == 0 && blockIdx.x % 3 == 1)) mbar_arrive(&empty_bar[s]);     // this warp is done with the stage
         }
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
@@ -559,8 +559,11 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                     }
                 }
             }
+        // (the producer may give up at any moment: one thread reads the flag for all, so that all take the same way
+        // through the barriers below; what this piece is made of has arrived by now, or a consumer has set the flag)
+        if (tid == 0) gave_up = *failed;
         consumers_sync();
-        const bool sound = !*failed;
+        const bool sound = gave_up == 0;
         const int parts = SHARES ? w.span.pieces : p.n_splits;
         if (sound) {
             for (int idx = tid; idx < n_rows * (HD / 4); idx += NCW * 32) {      // four columns of a row per turn
@@ -838,6 +841,15 @@ Plan make_plan(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int max_q_
     return pl;
 }
 
+// A self-test of the waits: shares of 148 CTAs (a first stage that is not handed back stops each third of them once it
+// has more tiles than stages), heads of 64, up to 8 rows.
+int launch_selftest(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, cudaStream_t s) {
+    auto kern = attention_decode_kernel<64, stages_for<64>(), 1, true, true>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_shares<64>(8));
+    if (e != cudaSuccess) return (int)e;
+    return (int)tl_launch(kern, dim3(148), dim3(NTHREADS), smem_shares<64>(p.rows), s, mk, mv, p);
+}
+
 template <int HD, int NT>
 int launch(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, const Plan& pl, cudaStream_t s) {
     if (pl.shares > 0)          // (shares_per_sm has raised the limit on shared memory)
@@ -876,13 +888,13 @@ extern "C" int tl_attention_decode_plan(int n_tokens, int n_seqs, int n_heads, i
     return TL_OK;
 }
 
-// Same arguments as tl_paged_attention_mma; n_pages is the first extent of the page tensors.
-extern "C" int tl_paged_attention_decode(const void* q, const void* k_pages, const void* v_pages, void* out,
-                                         const int* block_table, int table_stride, const int* q_start,
-                                         const int* kv_len, float* workspace, int* counters, int* status, int n_tokens, int n_seqs,
-                                         int n_heads, int n_kv_heads, int head_dim, int page_size, long long n_pages,
-                                         int max_q_len, int max_kv_len, int window, float scale, int allow_split,
-                                         void* stream) {
+// limit_ns: 0, or the limit of the self-test's waits
+static int attention_decode(const void* q, const void* k_pages, const void* v_pages, void* out,
+                            const int* block_table, int table_stride, const int* q_start,
+                            const int* kv_len, float* workspace, int* counters, int* status, int n_tokens, int n_seqs,
+                            int n_heads, int n_kv_heads, int head_dim, int page_size, long long n_pages,
+                            int max_q_len, int max_kv_len, int window, float scale, int allow_split,
+                            unsigned long long limit_ns, void* stream) {
     if (n_tokens <= 0 || n_seqs <= 0) return TL_OK;
     if (!takes(n_heads, n_kv_heads, head_dim, page_size, max_q_len) || max_kv_len <= 0 || n_pages <= 0) return TL_BAD_SIZE;
     if (n_pages * n_kv_heads * page_size >= (1LL << 31)) return TL_BAD_SIZE;
@@ -913,6 +925,7 @@ extern "C" int tl_paged_attention_decode(const void* q, const void* k_pages, con
     }
     p.n_splits = pl.n_splits;
     p.scale_log2 = scale * LOG2E;
+    p.limit_ns = limit_ns;
     p.part_o = workspace;
     p.part_ml = workspace ? workspace + (pl.shares > 0 ? (size_t)n_seqs * p.units * p.rows : (size_t)n_tokens * n_heads) * pl.n_splits * head_dim : nullptr;
 
@@ -924,6 +937,7 @@ extern "C" int tl_paged_attention_decode(const void* q, const void* k_pages, con
     if (rc != TL_OK) return rc;
 
     cudaStream_t s = (cudaStream_t)stream;
+    if (limit_ns != 0) return pl.shares > 0 && head_dim == 64 && p.rows <= 8 ? launch_selftest(mk, mv, p, s) : TL_BAD_SIZE;
     // query rows a CTA can meet: one 8-row block is enough for them, or two
     if (p.rows <= 8)
         rc = head_dim == 128 ? launch<128, 1>(mk, mv, p, pl, s) : launch<64, 1>(mk, mv, p, pl, s);
@@ -937,4 +951,29 @@ extern "C" int tl_paged_attention_decode(const void* q, const void* k_pages, con
         if (e != cudaSuccess) return (int)e;
     }
     return TL_OK;
+}
+
+// Same arguments as tl_paged_attention_mma; n_pages is the first extent of the page tensors.
+extern "C" int tl_paged_attention_decode(const void* q, const void* k_pages, const void* v_pages, void* out,
+                                         const int* block_table, int table_stride, const int* q_start,
+                                         const int* kv_len, float* workspace, int* counters, int* status, int n_tokens, int n_seqs,
+                                         int n_heads, int n_kv_heads, int head_dim, int page_size, long long n_pages,
+                                         int max_q_len, int max_kv_len, int window, float scale, int allow_split,
+                                         void* stream) {
+    return attention_decode(q, k_pages, v_pages, out, block_table, table_stride, q_start, kv_len, workspace, counters, status, n_tokens,
+                            n_seqs, n_heads, n_kv_heads, head_dim, page_size, n_pages, max_q_len, max_kv_len, window, scale, allow_split,
+                            0, stream);
+}
+
+// The same call as a self-test of the bounded waits (shares, heads of 64, at most 8 rows): a third of the CTAs wait for room that
+// nobody makes, give up after limit_ns and set status; the rest of the results are those of the call.
+extern "C" int tl_attention_decode_give_up_selftest(const void* q, const void* k_pages, const void* v_pages, void* out,
+                                                    const int* block_table, int table_stride, const int* q_start,
+                                                    const int* kv_len, float* workspace, int* counters, int* status, int n_tokens, int n_seqs,
+                                                    int n_heads, int n_kv_heads, int head_dim, int page_size, long long n_pages,
+                                                    int max_q_len, int max_kv_len, int window, float scale, unsigned long long limit_ns,
+                                                    void* stream) {
+    if (limit_ns == 0) return TL_BAD_SIZE;
+    return attention_decode(q, k_pages, v_pages, out, block_table, table_stride, q_start, kv_len, workspace, counters, status, n_tokens,
+                            n_seqs, n_heads, n_kv_heads, head_dim, page_size, n_pages, max_q_len, max_kv_len, window, scale, 1, limit_ns, stream);
 }
