@@ -725,6 +725,78 @@ def test_decode_attention_in_shares(ops, case):
     torch.testing.assert_close(pieces.float(), want.float(), atol=2e-2, rtol=2e-2)       # bfloat16 results of unit values, as above
 
 
+def test_decode_attention_in_shares_on_several_streams(ops):
+    """Calls on two streams, and graphs of one capture stream that are replayed on two, run beside each other and do not meet in
+    their scratch or their counters; nor does a call whose first sight of the GPU is a capture leave them undefined."""
+    from torchllms_b200.kernels.native import NativeOps
+    own, cases = NativeOps(), []
+    for B, H, KV, hd, seed in ((64, 32, 8, 128, 61), (48, 16, 8, 64, 62)):
+        g = torch.Generator().manual_seed(seed)
+        a = build_paged(torch.randint(1, 900, (B,), generator=g).tolist(), [1] * B, H, KV, hd, 16, torch.bfloat16, seed=seed)
+        a["max_kv_len"] = 8192
+        a["block_table"] = torch.nn.functional.pad(a["block_table"], (0, 512 - a["block_table"].shape[1]))
+        n, floats, counters = ctypes.c_int(0), ctypes.c_longlong(0), ctypes.c_longlong(0)
+        rc = ops._lib("attention_decode").tl_attention_decode_plan(B, B, H, KV, hd, 1, 8192, 1, ctypes.byref(n), ctypes.byref(floats),
+                                                                   ctypes.byref(counters))
+        assert rc == 0 and counters.value > 0
+        a.update(scale=hd ** -0.5, window=None, impl="decode")
+        cases.append((a, ops.paged_attention(**a, allow_split=n.value), [torch.empty_like(a["q"]) for _ in range(24)]))
+    torch.cuda.synchronize()
+
+    def unwritten(a, want, outs):
+        for o in outs:
+            o.fill_(float("nan"))
+
+    # memory that a graph's pool hands out again is not zero
+    filled = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(filled):
+        used = torch.full((1 << 20,), -1, dtype=torch.int32, device="cuda")
+    filled.replay()
+    torch.cuda.synchronize()
+    del used
+    graphs = []
+    for a, want, outs in cases:
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], pool=filled.pool() if len(graphs) == 1 else None):
+            for o in outs:
+                own.paged_attention(**a, out=o)
+    for a, want, outs in cases:
+        unwritten(a, want, outs)
+        own.paged_attention(**a, out=outs[0])            # before any replay
+        assert torch.equal(outs[0], want)
+    streams = [torch.cuda.Stream() for _ in cases]
+    for replayed in (True, False):
+        for _ in range(10):
+            for case in cases:
+                unwritten(*case)
+            torch.cuda.synchronize()
+            if replayed:
+                for s, graph in zip(streams, graphs):
+                    with torch.cuda.stream(s):
+                        graph.replay()
+            else:
+                for i in range(24):
+                    for s, (a, want, outs) in zip(streams, cases):
+                        with torch.cuda.stream(s):
+                            own.paged_attention(**a, out=outs[i])
+            torch.cuda.synchronize()
+            for a, want, outs in cases:
+                assert all(torch.equal(o, want) for o in outs)
+    # counters that somebody else has counted with are found out, and are right again after that
+    a, want, outs = cases[0]
+    own.paged_attention(**a, out=outs[0])
+    for _capture, counts in own._counts.values():
+        counts.fill_(1000)
+    own.paged_attention(**a, out=outs[0])
+    torch.cuda.synchronize()
+    with pytest.raises(RuntimeError, match="gave up waiting .code 213."):
+        own.check_status()
+    outs[0].fill_(float("nan"))
+    own.paged_attention(**a, out=outs[0])
+    own.check_status()
+    assert torch.equal(outs[0], want)
+
+
 def test_decode_attention_in_shares_gives_up(ops):
     """A third of the CTAs wait for room that nobody makes.  They give up, say so and go on to their end, the others write what
     they write anyway, no row is made of parts of which one is missing, and the counters are zero again."""

@@ -51,7 +51,7 @@ constexpr int FAILED_PART = 1 << 16;    // what a CTA that gave up adds to a cou
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LN2 = 0.6931471805599453f;
 constexpr unsigned long long WAIT_NS = 2000ull * 1000ull * 1000ull;
-enum : int { ERR_PRODUCER_WAIT = 211, ERR_CONSUMER_WAIT = 212 };
+enum : int { ERR_PRODUCER_WAIT = 211, ERR_CONSUMER_WAIT = 212, ERR_COUNT = 213 };
 
 struct DecodeParams {
     const __nv_bfloat16* q;
@@ -613,7 +613,9 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                     int before;
                     asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(before) : "l"(counter), "r"(add) : "memory");
                     arrived = before + add;
-                    if (((before + add) & (FAILED_PART - 1)) == parts) *counter = 0;
+                    const int pieces = arrived & (FAILED_PART - 1);
+                    if (pieces >= parts) *counter = 0;
+                    if (pieces > parts) atomicExch(p.status, ERR_COUNT);      // (another call counts in the same place)
                 }
                 consumers_sync();
                 seen = arrived;
@@ -873,9 +875,19 @@ extern "C" int tl_attention_decode_supports(int n_heads, int n_kv_heads, int hea
     return takes(n_heads, n_kv_heads, head_dim, page_size, max_q_len) ? 1 : 0;
 }
 
+// Which capture the stream takes part in: 0 where it is in none, else a number that no other capture has.
+extern "C" int tl_stream_capture_id(void* stream, unsigned long long* id) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    *id = 0;
+    const cudaError_t e = cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, id);
+    if (e != cudaSuccess) return (int)e;
+    if (status != cudaStreamCaptureStatusActive) *id = 0;
+    return TL_OK;
+}
+
 // What a call needs beside its operands: n_splits pieces of a request's keys, workspace_floats of scratch, and
-// n_counters ints that are zero (and are zero again when the call has run); with counters there is one launch, else
-// there are two when n_splits is over 1.
+// n_counters ints that are zero (and are zero again when the call has run); no call that may run at the same time may have
+// either.  With counters there is one launch, else there are two when n_splits is over 1.
 extern "C" int tl_attention_decode_plan(int n_tokens, int n_seqs, int n_heads, int n_kv_heads, int head_dim,
                                         int max_q_len, int max_kv_len, int allow_split,
                                         int* n_splits, long long* workspace_floats, long long* n_counters) {

@@ -118,8 +118,8 @@ class NativeOps:
                 "torchllms_b200 runs on a CUDA GPU (sm_100a) only: torch.cuda.is_available() is False "
                 "and there is no CPU implementation")
         self.launches = 0          # kernels of this library launched so far (a bench counts with it)
-        self._workspace: Dict[Tuple[int, str], torch.Tensor] = {}
-        self._retired: list = []
+        # (device, stream, inside a capture) -> ints that are zero between launches, and the capture they belong to
+        self._counts: Dict[Tuple[int, int, bool], Tuple[int, torch.Tensor]] = {}
         self.use_tcgen05 = True
         # SwiGLU in the epilogue of the gate/up product (TORCHLLMS_B200_NO_GATED=1 keeps the two kernels, for comparisons)
         self.use_gated = os.environ.get("TORCHLLMS_B200_NO_GATED", "") not in ("1", "true")
@@ -929,7 +929,7 @@ class NativeOps:
             _need(bias.numel() == 3 * W, "bias must have 3 * width elements")
         lib = self._lib("recurrent")
         lib.tl_mingru_scan_scratch.restype = ctypes.c_longlong
-        ws = self._scratch(proj.device, lib.tl_mingru_scan_scratch(n_seqs, W, max_q_len), "recurrent")
+        ws = self._scratch(proj.device, lib.tl_mingru_scan_scratch(n_seqs, W, max_q_len))
         out = torch.empty((T, W), dtype=out_dtype, device=proj.device)
         rc = lib.tl_mingru_scan(_ptr(proj), _DT[proj.dtype], splits, ctypes.c_longlong(proj.stride(0) if splits > 1 else 0),
                                 _ptr(bias), _ptr(state), _ptr(q_start), _ptr(state_slot), _ptr(fresh), _ptr(out), _DT[out_dtype],
@@ -1632,6 +1632,11 @@ class NativeOps:
         code = int(self._status[0])
         if code != 0:
             self._status[0] = 0
+            torch.cuda.synchronize()
+            for capture, counts in list(self._counts.values()):
+                if not capture:
+                    counts.zero_()               # (whatever happened, the next call counts from zero; a graph's replay does so itself)
+            torch.cuda.synchronize()
             raise KernelError(f"a kernel gave up waiting (code {code}); its output is not valid")
         if self.debug:
             from .build import loaded_libraries
@@ -1743,29 +1748,26 @@ class NativeOps:
         return q
 
     # --------------------------------------------------------------- attention
-    def _scratch(self, device: torch.device, floats: int, tag: str = "attention") -> Optional[torch.Tensor]:
-        if floats <= 0:
-            return None
-        key = (device.index or 0, tag)
-        buf = self._workspace.get(key)
-        if buf is None or buf.numel() < floats:
-            if buf is not None:
-                self._retired.append(buf)      # a captured graph may still point into it
-            buf = torch.empty(max(floats, 1 << 22), dtype=torch.float32, device=device)
-            self._workspace[key] = buf
-        return buf
+    @staticmethod
+    def _scratch(device: torch.device, floats: int) -> Optional[torch.Tensor]:
+        """Scratch of one call.  The allocator gives it to the next call on the same stream and to none on another, and inside a
+        capture it is the graph's own: calls of several threads, streams and graphs may run at the same time."""
+        return torch.empty(floats, dtype=torch.float32, device=device) if floats > 0 else None
 
     def _counters(self, device: torch.device, n: int) -> Optional[torch.Tensor]:
-        """At least ``n`` ints that are zero between launches (whoever counts with them sets them back)."""
+        """At least ``n`` ints that are zero between launches (whoever counts with them sets them back) and that no other stream's
+        work uses.  A graph may be replayed on any stream, beside whatever its capture's stream does then: a capture has
+        counters of its own, and setting them to zero is the first thing it records of them."""
         if n <= 0:
             return None
-        key = (device.index or 0, "counters")
-        buf = self._workspace.get(key)
-        if buf is None or buf.numel() < n:
-            if buf is not None:
-                self._retired.append(buf)      # a captured graph may still point into it
-            buf = torch.zeros(max(n, 1 << 16), dtype=torch.int32, device=device)
-            self._workspace[key] = buf
+        stream, capture = _stream(), ctypes.c_ulonglong(0)
+        _check(self._lib("attention_decode").tl_stream_capture_id(stream, ctypes.byref(capture)), "stream_capture_id")
+        key = (device.index or 0, stream.value or 0, capture.value != 0)
+        of, buf = self._counts.get(key, (0, None))
+        if buf is None or of != capture.value or buf.numel() < n:
+            # (what is replaced goes back to the allocator, which hands it out again behind this stream's work)
+            buf = torch.zeros(max(n, 1 << 12), dtype=torch.int32, device=device)
+            self._counts[key] = (capture.value, buf)
         return buf
 
     @_timed
@@ -2048,7 +2050,7 @@ class NativeOps:
         if top_k is None and vocab > 8192:
             # no rank filter: spread every row over many CTAs, then pick among their candidates
             lib.tl_sample_wide_scratch.restype = ctypes.c_longlong
-            ws = self._scratch(logits.device, lib.tl_sample_wide_scratch(n, vocab), "sampling")
+            ws = self._scratch(logits.device, lib.tl_sample_wide_scratch(n, vocab))
             rc = lib.tl_sample_wide(_ptr(logits), ctypes.c_longlong(logits.stride(0)), n, vocab, _ptr(temperature),
                                     _ptr(row_keys), _ptr(ws), _ptr(out), _stream())
             _check(rc, "sample_wide")
