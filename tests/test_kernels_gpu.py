@@ -725,12 +725,36 @@ def test_decode_attention_in_shares(ops, case):
     torch.testing.assert_close(pieces.float(), want.float(), atol=2e-2, rtol=2e-2)       # bfloat16 results of unit values, as above
 
 
+def test_decode_attention_in_shares_of_other_groups(ops):
+    """Groups of more heads than a tile has rows (the last chunk of a group smaller than the others), requests that bring no token,
+    and calls of several shapes in turn, which count in the same places: bit for bit a CTA to a piece."""
+    made = []
+    for B, longest, H, KV, hd, empty in ((100, 700, 48, 2, 64, (0, 41, 99)), (130, 500, 32, 1, 128, (7, 8, 128, 129)), (64, 300, 16, 8, 128, ())):
+        g = torch.Generator().manual_seed(B)
+        q_lens = [0 if b in empty else 1 for b in range(B)]
+        a = build_paged(torch.randint(1, longest + 1, (B,), generator=g).tolist(), q_lens, H, KV, hd, 16, torch.bfloat16, seed=B)
+        a["max_kv_len"] = 8192
+        a["block_table"] = torch.nn.functional.pad(a["block_table"], (0, 512 - a["block_table"].shape[1]))
+        n, floats, counters = ctypes.c_int(0), ctypes.c_longlong(0), ctypes.c_longlong(0)
+        rc = ops._lib("attention_decode").tl_attention_decode_plan(sum(q_lens), B, H, KV, hd, 1, 8192, 1, ctypes.byref(n), ctypes.byref(floats),
+                                                                   ctypes.byref(counters))
+        assert rc == 0 and n.value > 1 and counters.value == B * KV * -(-(H // KV) // 16)
+        a.update(scale=hd ** -0.5, window=None, impl="decode")
+        made.append((a, ops.paged_attention(**a, allow_split=n.value)))
+        want = TWIN.paged_attention(**{k: v for k, v in a.items() if k != "impl"})
+        torch.testing.assert_close(made[-1][1].float(), want.float(), atol=2e-2, rtol=2e-2)       # bfloat16 results of unit values, as above
+    for _ in range(3):
+        for a, pieces in made:
+            assert torch.equal(ops.paged_attention(**a, out=torch.full_like(pieces, float("nan"))), pieces)
+    ops.check_status()
+
+
 def test_decode_attention_in_shares_on_several_streams(ops):
     """Calls on two streams, and graphs of one capture stream that are replayed on two, run beside each other and do not meet in
     their scratch or their counters; nor does a call whose first sight of the GPU is a capture leave them undefined."""
     from torchllms_b200.kernels.native import NativeOps
     own, cases = NativeOps(), []
-    for B, H, KV, hd, seed in ((64, 32, 8, 128, 61), (48, 16, 8, 64, 62)):
+    for B, H, KV, hd, seed in ((64, 32, 8, 128, 61), (64, 16, 8, 64, 62)):
         g = torch.Generator().manual_seed(seed)
         a = build_paged(torch.randint(1, 900, (B,), generator=g).tolist(), [1] * B, H, KV, hd, 16, torch.bfloat16, seed=seed)
         a["max_kv_len"] = 8192
@@ -801,7 +825,7 @@ def test_decode_attention_in_shares_gives_up(ops):
     """A third of the CTAs wait for room that nobody makes.  They give up, say so and go on to their end, the others write what
     they write anyway, no row is made of parts of which one is missing, and the counters are zero again."""
     from torchllms_b200.kernels.native import KernelError, _ptr, _stream
-    B, H, KV, hd, P = 40, 32, 8, 64, 16
+    B, H, KV, hd, P = 64, 32, 8, 64, 16
     g = torch.Generator().manual_seed(5)
     seq_lens = torch.randint(1, 1500, (B,), generator=g).tolist()
     a = build_paged(seq_lens, [1] * B, H, KV, hd, P, torch.bfloat16, seed=5)

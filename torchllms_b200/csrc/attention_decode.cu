@@ -14,14 +14,13 @@
 // mbarrier per stage.  Warps 0-3 share the rows and each takes 16 keys of every tile; they hand a stage back
 // through a second mbarrier.  A piece leaves float32 partials; the pieces of a request are added up in order.
 //
-// Two ways to hand the pieces out.  Where one CTA to a piece fits the GPU in one wave, that is what is
-// launched, and merge_partials_kernel adds up (the weights of the product that follows stream in
-// meanwhile).  With more pieces than CTAs fit (many requests; most pieces are short or empty then) as many
-// CTAs as fit take even shares of the pieces, found on the device from the requests' lengths; the producer
-// runs ahead across the borders of pieces and requests, and the CTA that is last to finish with a request adds
-// its pieces up (a counter per request and kv head).  The sums are the same bit for bit.
-// (64 requests of 320 tokens, 32 / 8 heads of 128, planned for 8,192: 3,072 CTAs, half of them empty, 29.0 us;
-// 444 with shares 23.4 us; 40 requests of 1,000: 31.7 and 31.5; 64 of 2,048, where every piece is long: 86.7 and 86.9.)
+// Two ways to hand the pieces out, each a kernel.  A CTA to a piece, and merge_partials_kernel adds up (the weights of the
+// product that follows stream in meanwhile).  Or, where there are many more pieces than CTAs fit (many requests; most
+// pieces are short or empty then), as many CTAs as fit take even shares of the pieces, found on the device from the requests'
+// lengths; the producer runs ahead across the borders of pieces and requests, and the CTA that is last to finish with a
+// request adds its pieces up (a counter per request and kv head).  The sums are the same bit for bit; where the line between
+// the two lies, and what both take on either side of it, stands at make_plan.  What bounds both is the latency of a tile: 24 requests
+// of 130 to 1,900 tokens read 50 MB in 14 us.
 //
 // The products are taken transposed: scores^T = K Q^T and out^T = V^T P^T, so that the 16 rows of
 // a tensor-core tile are keys (or value columns), all of them real, and the few query rows (four
@@ -92,7 +91,7 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, volatile int* failed, unsigned long long limit_ns = WAIT_NS) {
+__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, const volatile int* failed, unsigned long long limit_ns = WAIT_NS) {
     if (mbar_try_wait(bar, parity)) return true;
     unsigned long long t0;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
@@ -153,13 +152,15 @@ __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;
 struct Span {
     int lo, hi;      // visible keys lo .. hi - 1 (of any of its tokens)
     int base;        // position of its first new token
+    int first;       // the row of that token
     int n_tokens;    // 0: the request brings none
     int piece;       // keys of a piece: whole tiles, or all of them
     int pieces;      // how many of them have keys (at least one)
 };
 __device__ __forceinline__ Span span_of(const DecodeParams& p, int b) {
     Span s;
-    const int ql = p.q_start[b + 1] - p.q_start[b];
+    s.first = p.q_start[b];
+    const int ql = p.q_start[b + 1] - s.first;
     s.base = p.kv_len[b] - ql;
     s.n_tokens = max(0, min(ql, p.max_tokens));
     s.lo = p.window > 0 ? max(0, s.base - p.window + 1) : 0;
@@ -176,7 +177,7 @@ struct Walk {
     Span span;
     int lo, hi;          // keys of the piece
     int start, tiles;    // its tiles: the first starts on a box (page) boundary; keys below lo are masked
-    int at, end;         // shares: places on the line of tiles, of the piece and where the share ends
+    int at, end;         // shares: places on the line of pieces, of the piece and where the share ends
     int first_split;     // shares: the first piece of this (request, unit) in the share
 };
 __device__ __forceinline__ void walk_piece(const DecodeParams& p, Walk& w) {
@@ -185,9 +186,14 @@ __device__ __forceinline__ void walk_piece(const DecodeParams& p, Walk& w) {
     w.start = w.lo & ~(p.box_rows - 1);
     w.tiles = w.hi > w.start ? (w.hi - w.start + BN - 1) / BN : 0;
 }
+// What a piece is worth on the line, in tiles: the queries, the four warps' results and the parts take as long as two or
+// (more than 8 rows) three tiles.  By its tiles alone a share of many short pieces took far longer than one of few long ones:
+// 64 requests of 130 to 1,900 tokens, 32 / 8 heads of 128, 63 us where pieces by themselves take 52 and shares by this measure 50;
+// 128 / 8 heads 163, 93 and 89.
+template <int NT> __device__ __forceinline__ int worth(const Span& s) { return s.piece / BN + (NT == 1 ? 2 : 3); }
 // On to the next piece of the line; false: it belongs to the next share, or there is none.
-__device__ __forceinline__ bool walk_next(const DecodeParams& p, Walk& w) {
-    w.at += w.span.piece / BN;
+template <int NT> __device__ __forceinline__ bool walk_next(const DecodeParams& p, Walk& w) {
+    w.at += worth<NT>(w.span);
     if (++w.split == w.span.pieces) {
         w.split = 0;
         if (++w.unit == p.units) {
@@ -204,25 +210,25 @@ __device__ __forceinline__ bool walk_next(const DecodeParams& p, Walk& w) {
     return true;
 }
 // The first piece of this CTA's share.  All pieces of a request's first unit, of its second and so on, then the next
-// request's, lie on one line, a piece as long as it has tiles; a share is every piece that starts in an equal
+// request's, lie on one line, a piece as long as it is worth; a share is every piece that starts in an equal
 // part of the line.  false: there is none.
-__device__ __forceinline__ bool walk_share(const DecodeParams& p, Walk& w, int lane) {
+template <int NT> __device__ __forceinline__ bool walk_share(const DecodeParams& p, Walk& w, int lane) {
     int total = 0;
     for (int b = lane; b < p.n_seqs; b += 32) {
         const Span s = span_of(p, b);
-        if (s.n_tokens > 0) total += s.pieces * (s.piece / BN);
+        if (s.n_tokens > 0) total += s.pieces * worth<NT>(s);
     }
     total = __reduce_add_sync(0xffffffffu, total);
     const int share = (total * p.units + (int)gridDim.x - 1) / (int)gridDim.x;
     const int begin = blockIdx.x * share;
     w.end = begin + share;
     if (begin >= total * p.units) return false;
-    int before = 0;                                     // tiles (of one unit) of the requests before this block of 32
+    int before = 0;                                     // worth (of one unit) of the requests before this block of 32
     for (int b0 = 0; b0 < p.n_seqs; b0 += 32) {
         int t = 0;
         if (b0 + lane < p.n_seqs) {
             const Span s = span_of(p, b0 + lane);
-            if (s.n_tokens > 0) t = s.pieces * (s.piece / BN);
+            if (s.n_tokens > 0) t = s.pieces * worth<NT>(s);
         }
         int upto = t;
 #pragma unroll
@@ -236,7 +242,7 @@ __device__ __forceinline__ bool walk_share(const DecodeParams& p, Walk& w, int l
             w.b = b0 + src;
             w.span = span_of(p, w.b);
             const int request = (before + __shfl_sync(0xffffffffu, upto - t, src)) * p.units;
-            const int wide = w.span.piece / BN, all = w.span.pieces * wide;
+            const int wide = worth<NT>(w.span), all = w.span.pieces * wide;
             w.unit = (begin - request) / all;
             w.split = (begin - request - w.unit * all) / wide;
             w.at = request + w.unit * all + w.split * wide;
@@ -248,7 +254,7 @@ __device__ __forceinline__ bool walk_share(const DecodeParams& p, Walk& w, int l
             // the piece that the share's start falls into belongs to the share before
             const int u = w.unit;
             const int b = w.b;
-            const bool got = walk_next(p, w);
+            const bool got = walk_next<NT>(p, w);
             if (w.b == b && w.unit == u) w.first_split = w.split;
             return got;
         }
@@ -257,168 +263,91 @@ __device__ __forceinline__ bool walk_share(const DecodeParams& p, Walk& w, int l
     return false;
 }
 
-// NT: 8-row blocks of query rows (1: up to 8 rows, 2: up to 16)
-// SHARES: a CTA takes a share of all pieces and the last one adds a request's up; else a CTA to a piece
-// (blockIdx: request z, unit y, piece x), and merge_partials_kernel follows
-// SELFTEST: every third CTA never hands back its first stage, so that its producer's wait for room runs out
-template <int HD, int STAGES, int NT, bool SHARES, bool SELFTEST = false>
-__global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_kernel(const __grid_constant__ CUtensorMap map_k,
-                                                                                  const __grid_constant__ CUtensorMap map_v,
-                                                                                  const DecodeParams p) {
+// ---- what the two kernels below have in common.  HD: head size; NT: 8-row blocks of query rows (1: up to 8 rows, 2: up to 16)
+
+// A tile's keys and values on their way: a box per page (or per 64 rows of a larger page) and 64-element column block.  The whole
+// producer warp issues it, a lane to a box: the page lookups go side by side.
+template <int HD>
+__device__ __forceinline__ void issue_tile(const DecodeParams& p, const CUtensorMap& map_k, const CUtensorMap& map_v, unsigned char* kt,
+                                           unsigned long long* bar, const int* table, int kvh, int k0, int k_hi, int lane) {
     constexpr int HALVES = HD / 64;                     // 64-element (128-byte) column blocks of a row
-    constexpr unsigned HALF_BYTES = BN * 128;           // one [64 keys x 128 B] block
-    constexpr unsigned KV_BYTES = HALVES * HALF_BYTES;  // K (or V) of a tile
-    constexpr unsigned STAGE_BYTES = 2 * KV_BYTES;
-    constexpr int QPITCH = HD + 8;
-    constexpr int KSTEPS = HD / 16;
-    constexpr int NROWS = 8 * NT;
-    constexpr int OPITCH = HD + 4;                      // of the merge buffer: rows two apart fall on different banks
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
-    // behind the stages: the queries [NROWS][QPITCH] and, with shares in the same place one after the other, the four
-    // warps' results Om [NCW][rows][OPITCH] and the weights of the pieces [rows][MERGE_MAX_SPLITS].  (With one piece to
-    // a CTA the results lie where the tiles were.)
-    __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(tiles + STAGES * STAGE_BYTES);
-    float* Om = reinterpret_cast<float*>(tiles + (SHARES ? STAGES * STAGE_BYTES : 0));
-    __shared__ float Mm[NCW][NROWS], Lm[NCW][NROWS];
-    __shared__ __align__(8) unsigned long long full_bar[STAGES];
-    __shared__ __align__(8) unsigned long long empty_bar[STAGES];
-    __shared__ int failed_flag;
-    __shared__ int arrived, gave_up;
-
-    grid_launch_dependents();
-    // What follows, down to the dependency wait, reads nothing that the kernels just before this one
-    // write: the step's index data were uploaded before its first kernel, and keys and values of
-    // positions before the step's own tokens were written by earlier steps.  Under programmatic
-    // dependent launch this part runs while the predecessor is still at work.
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    volatile int* failed = &failed_flag;
-    const unsigned long long limit_ns = SELFTEST ? p.limit_ns : WAIT_NS;
-    Walk w;
-    if (SHARES) {
-        if (!walk_share(p, w, lane)) return;            // (the same for all warps)
-    } else {
-        w.b = blockIdx.z;
-        w.unit = blockIdx.y;
-        w.split = blockIdx.x;
-        w.span = span_of(p, w.b);
-        if (w.span.n_tokens == 0) return;
-        walk_piece(p, w);
-    }
-    if (tid == NCW * 32) {
-        failed_flag = 0;
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], NCW);
+    constexpr unsigned HALF_BYTES = BN * 128, KV_BYTES = HALVES * HALF_BYTES;
+    if (lane == 0) mbar_expect_tx(bar, 2 * KV_BYTES);
+    __syncwarp();
+    for (int c = lane; c < BN / p.box_rows; c += 32) {
+        const int kpos = k0 + c * p.box_rows;
+        // boxes past the last key start outside the tensor: the copy writes the zero fill, so
+        // that what is multiplied by probability 0 there is finite
+        int row = p.total_rows;
+        if (kpos < k_hi) {
+            const int page = table[kpos >> p.page_shift];
+            if (tl_check_page(page))                           // (debug builds: a bad page reads as the zero fill)
+                row = (page * p.n_kv_heads + kvh) * p.page_size + (kpos & (p.page_size - 1));
         }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-
-    if (warp == NCW) {
-        // ---- producer: a box per page (or per 64 rows of a larger page) and 64-element column block,
-        // K and V.  The whole warp issues a tile, a lane to a box: the page lookups go side by side.
-        bool waited = false;
-        int it = 0;
-        bool ok = true;
-        do {
-            const int kvh = w.unit / p.n_gchunks;
-            const int* table = p.block_table + (size_t)w.b * p.table_stride;
-            for (int i = 0; i < w.tiles && ok; ++i, ++it) {
-                const int s = it % STAGES;
-                const int k0 = w.start + i * BN;
-                // the first tiles go at once, up to one that may hold a key written by the predecessor
-                if (!waited && (it >= STAGES || k0 + BN > w.span.base)) {
-                    grid_dependency_wait();
-                    waited = true;
-                }
-                if (it >= STAGES && !__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], ((it / STAGES) - 1) & 1, failed, limit_ns))) {
-                    if (lane == 0 && atomicExch(&failed_flag, 1) == 0) atomicExch(p.status, ERR_PRODUCER_WAIT);
-                    ok = false;
-                    break;
-                }
-                if (lane == 0) mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-                __syncwarp();
-                unsigned char* kt = tiles + s * STAGE_BYTES;
-                for (int c = lane; c < BN / p.box_rows; c += 32) {
-                    const int kpos = k0 + c * p.box_rows;
-                    // boxes past the last key start outside the tensor: the copy writes the zero fill, so
-                    // that what is multiplied by probability 0 there is finite
-                    int row = p.total_rows;
-                    if (kpos < w.hi) {
-                        const int page = table[kpos >> p.page_shift];
-                        if (tl_check_page(page))                       // (debug builds: a bad page reads as the zero fill)
-                            row = (page * p.n_kv_heads + kvh) * p.page_size + (kpos & (p.page_size - 1));
-                    }
 #pragma unroll
-                    for (int h = 0; h < HALVES; ++h) {
-                        unsigned char* dst = kt + h * HALF_BYTES + c * p.box_rows * 128;
-                        if (p.streamed) {
-                            tma_load_2d_streamed(dst, &map_k, &full_bar[s], h * 64, row);
-                            tma_load_2d_streamed(dst + KV_BYTES, &map_v, &full_bar[s], h * 64, row);
-                        } else {
-                            tma_load_2d(dst, &map_k, &full_bar[s], h * 64, row);
-                            tma_load_2d(dst + KV_BYTES, &map_v, &full_bar[s], h * 64, row);
-                        }
-                    }
-                }
-                __syncwarp();
+        for (int h = 0; h < HALVES; ++h) {
+            unsigned char* dst = kt + h * HALF_BYTES + c * p.box_rows * 128;
+            if (p.streamed) {
+                tma_load_2d_streamed(dst, &map_k, bar, h * 64, row);
+                tma_load_2d_streamed(dst + KV_BYTES, &map_v, bar, h * 64, row);
+            } else {
+                tma_load_2d(dst, &map_k, bar, h * 64, row);
+                tma_load_2d(dst + KV_BYTES, &map_v, bar, h * 64, row);
             }
-        } while (SHARES && ok && walk_next(p, w));
-        if (!waited) grid_dependency_wait();
-        // (nothing that is still on its way may land in shared memory that is no longer this CTA's)
-        int never = 0;
-        for (int k = max(0, it - STAGES); k < it; ++k) mbar_wait(&full_bar[k % STAGES], (k / STAGES) & 1, &never, limit_ns);
-        return;
-    }
-
-    // ---- consumers: the same rows, 16 keys of every tile each
-    grid_dependency_wait();
-    const int g = lane >> 2, t = lane & 3, mi = lane >> 3;
-    const int key_off = warp * 16;
-    // this lane's row and first chunk inside a tile: K as the 16-row operand [keys x 16 columns],
-    // V through a transposing load as [16 columns x keys]
-    const int k_row = key_off + (lane & 7) + ((mi & 1) ? 8 : 0);
-    const int v_row = key_off + (lane & 7) + ((mi & 2) ? 8 : 0);
-    const unsigned k_lane_off = swz(k_row, (mi & 2) ? 1 : 0);
-    const unsigned v_lane_off = swz(v_row, mi & 1);
-    bool ok = true, fresh = true;
-    unsigned qf[NT][KSTEPS][2];
-    int it = 0;
-    do {
-        const int kvh = w.unit / p.n_gchunks;
-        const int g0 = (w.unit - kvh * p.n_gchunks) * p.ng;
-        const int ng = min(p.ng, p.group - g0);
-        const int n_rows = w.span.n_tokens * ng;
-        const int qs = p.q_start[w.b];
-        const int k_lo = w.lo, k_hi = w.hi, base = w.span.base;
-        // queries (zero rows where the tile has none); the next pieces of a request find them in registers
-        if (fresh) {
-            for (int c = tid; c < NROWS * (HD / 8); c += NCW * 32) {
-                const int rr = c / (HD / 8), part = c - rr * (HD / 8);
-                uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (rr < n_rows) {
-                    const int head = kvh * p.group + g0 + rr % ng;
-                    v = *reinterpret_cast<const uint4*>(p.q + ((size_t)(qs + rr / ng) * p.n_heads + head) * HD + part * 8);
-                }
-                *reinterpret_cast<uint4*>(Qs + rr * QPITCH + part * 8) = v;
-            }
-            consumers_sync();
-            // Q^T as the 8-wide operand: this thread holds columns 2t, 2t + 1 (and + 8) of row g
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                for (int kd2 = 0; kd2 < KSTEPS / 2; ++kd2) {
-                    unsigned r[4];
-                    ldmatrix_x4(r, smem_u32(Qs + (nt * 8 + (lane & 7)) * QPITCH + (kd2 * 4 + mi) * 8));
-                    qf[nt][2 * kd2][0] = r[0]; qf[nt][2 * kd2][1] = r[1];
-                    qf[nt][2 * kd2 + 1][0] = r[2]; qf[nt][2 * kd2 + 1][1] = r[3];
-                }
         }
-        // this thread's two query rows of every 8-row block are 2t and 2t + 1: of the scores^T tile it
-        // holds keys g and g + 8 for them, of the out^T tile value columns g and g + 8
-        float m[NT][2], l[NT][2];
-        float o[NT][KSTEPS][4];
+    }
+    __syncwarp();
+}
+
+// The consumers' queries into shared memory, [8 NT][HD + 8] (zero rows where there are none).
+template <int HD, int NT>
+__device__ __forceinline__ void fetch_queries(const DecodeParams& p, __nv_bfloat16* Qs, int first, int head0, int ng, int n_rows) {
+    for (int c = threadIdx.x; c < 8 * NT * (HD / 8); c += NCW * 32) {
+        const int rr = c / (HD / 8), part = c - rr * (HD / 8);
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (rr < n_rows)
+            v = *reinterpret_cast<const uint4*>(p.q + ((size_t)(first + rr / ng) * p.n_heads + head0 + rr % ng) * HD + part * 8);
+        *reinterpret_cast<uint4*>(Qs + rr * (HD + 8) + part * 8) = v;
+    }
+}
+
+// What a consumer thread keeps of a piece.  Its two query rows of every 8-row block are 2t and 2t + 1: of the scores^T
+// tile it holds keys g and g + 8 for them, of the out^T tile value columns g and g + 8.
+template <int HD, int NT>
+struct Consumer {
+    static constexpr int KSTEPS = HD / 16;
+    static constexpr unsigned HALF_BYTES = BN * 128, KV_BYTES = HD / 64 * HALF_BYTES;
+    static constexpr int OPITCH = HD + 4;               // of the results in shared memory: rows two apart fall on different banks
+    unsigned qf[NT][KSTEPS][2];                         // Q^T as the 8-wide operand: columns 2t, 2t + 1 (and + 8) of row g
+    float m[NT][2], l[NT][2], o[NT][KSTEPS][4];
+    int qpos[NT][2], warp_qmax, warp_qmin;
+    int g, t, key_off;
+    unsigned k_lane_off, v_lane_off;
+
+    __device__ __forceinline__ void place(int warp, int lane) {
+        const int mi = lane >> 3;
+        g = lane >> 2;
+        t = lane & 3;
+        key_off = warp * 16;
+        // this lane's row and first chunk inside a tile: K as the 16-row operand [keys x 16 columns],
+        // V through a transposing load as [16 columns x keys]
+        const int k_row = key_off + (lane & 7) + ((mi & 1) ? 8 : 0);
+        const int v_row = key_off + (lane & 7) + ((mi & 2) ? 8 : 0);
+        k_lane_off = swz(k_row, (mi & 2) ? 1 : 0);
+        v_lane_off = swz(v_row, mi & 1);
+    }
+    __device__ __forceinline__ void take_queries(const __nv_bfloat16* Qs, int lane) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int kd2 = 0; kd2 < KSTEPS / 2; ++kd2) {
+                unsigned r[4];
+                ldmatrix_x4(r, smem_u32(Qs + (nt * 8 + (lane & 7)) * (HD + 8) + (kd2 * 4 + (lane >> 3)) * 8));
+                qf[nt][2 * kd2][0] = r[0]; qf[nt][2 * kd2][1] = r[1];
+                qf[nt][2 * kd2 + 1][0] = r[2]; qf[nt][2 * kd2 + 1][1] = r[3];
+            }
+    }
+    __device__ __forceinline__ void begin(int base, int ng, int n_rows) {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             m[nt][0] = m[nt][1] = -INFINITY;
@@ -426,7 +355,6 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
 #pragma unroll
             for (int i = 0; i < KSTEPS; ++i) o[nt][i][0] = o[nt][i][1] = o[nt][i][2] = o[nt][i][3] = 0.f;
         }
-        int qpos[NT][2];
         int qmax = -1, qmin = INT_MAX;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
@@ -438,99 +366,91 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                 qmax = max(qmax, qp);
                 if (qp >= 0) qmin = min(qmin, qp);
             }
-        const int warp_qmax = __reduce_max_sync(0xffffffffu, qmax);
-        const int warp_qmin = __reduce_min_sync(0xffffffffu, qmin);
-        for (int i = 0; i < w.tiles; ++i, ++it) {
-            const int s = it % STAGES;
-            ok = __all_sync(0xffffffffu, ok && mbar_wait(&full_bar[s], (it / STAGES) & 1, failed, limit_ns));
-            if (!ok) {
-                // (whichever lane's wait ran out; one that only stopped with another's has nothing to report)
-                if (lane == 0 && atomicExch(&failed_flag, 1) == 0) atomicExch(p.status, ERR_CONSUMER_WAIT);
-                break;
-            }
-            const int share_lo = w.start + i * BN + key_off;
-            if (share_lo <= warp_qmax && share_lo + 16 > k_lo) {
-                const unsigned kt = smem_u32(tiles + s * STAGE_BYTES);
-                // rows are 128 bytes and tiles 1024-byte aligned, so bits 4-6 of a row's address are the
-                // swizzled chunk: xor-ing a constant chunk number in is all it takes to move along a row
-                const unsigned ka = kt + k_lane_off, va = kt + KV_BYTES + v_lane_off;
-                float sc[NT][4];
+        warp_qmax = __reduce_max_sync(0xffffffffu, qmax);
+        warp_qmin = __reduce_min_sync(0xffffffffu, qmin);
+    }
+    // the warp's 16 keys of the tile at kt, which begins with key k0; keys lo .. hi - 1 are the piece's
+    __device__ __forceinline__ void tile(const DecodeParams& p, unsigned kt, int k0, int lo, int hi) {
+        const int share_lo = k0 + key_off;
+        if (share_lo > warp_qmax || share_lo + 16 <= lo) return;
+        // rows are 128 bytes and tiles 1024-byte aligned, so bits 4-6 of a row's address are the
+        // swizzled chunk: xor-ing a constant chunk number in is all it takes to move along a row
+        const unsigned ka = kt + k_lane_off, va = kt + KV_BYTES + v_lane_off;
+        float sc[NT][4];
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
+        for (int nt = 0; nt < NT; ++nt) sc[nt][0] = sc[nt][1] = sc[nt][2] = sc[nt][3] = 0.f;
 #pragma unroll
-                for (int kd = 0; kd < KSTEPS; ++kd) {
-                    unsigned kf[4];
-                    ldmatrix_x4(kf, (ka ^ (unsigned)(((kd * 2) & 7) << 4)) + (kd / 4) * HALF_BYTES);
+        for (int kd = 0; kd < KSTEPS; ++kd) {
+            unsigned kf[4];
+            ldmatrix_x4(kf, (ka ^ (unsigned)(((kd * 2) & 7) << 4)) + (kd / 4) * HALF_BYTES);
 #pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) mma_bf16(sc[nt], kf, qf[nt][kd][0], qf[nt][kd][1]);
-                }
-                const bool all_visible = share_lo >= k_lo && share_lo + 16 <= k_hi && share_lo + 15 <= warp_qmin &&
-                                         (p.window <= 0 || share_lo > warp_qmax - p.window);
-                if (!all_visible) {
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int qp = qpos[nt][e & 1];
-                            const int kpos = share_lo + g + 8 * (e >> 1);
-                            const bool vis = kpos >= k_lo && kpos < k_hi && kpos <= qp && (p.window <= 0 || kpos > qp - p.window);
-                            if (!vis) sc[nt][e] = -INFINITY;
-                        }
-                }
-                unsigned ph[NT][2], pl[NT][2];
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    float m_safe[2], alpha[2];
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) {
-                        float mx = fmaxf(sc[nt][j], sc[nt][j + 2]);            // over the 16 keys: the lanes that share t
-                        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-                        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-                        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-                        const float m_new = fmaxf(m[nt][j], mx * p.scale_log2);   // maxima live on the base-2 scale
-                        m_safe[j] = (m_new == -INFINITY) ? 0.f : m_new;           // no key seen yet: keep exponents finite
-                        alpha[j] = ex2(m[nt][j] - m_safe[j]);
-                        m[nt][j] = m_new;
-                        l[nt][j] *= alpha[j];
-                    }
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float pv = ex2(fmaf(sc[nt][e], p.scale_log2, -m_safe[e & 1]));
-                        sc[nt][e] = pv;
-                        l[nt][e & 1] += pv;
-                    }
-                    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
-#pragma unroll
-                        for (int d = 0; d < KSTEPS; ++d) {
-                            o[nt][d][0] *= alpha[0]; o[nt][d][1] *= alpha[1];
-                            o[nt][d][2] *= alpha[0]; o[nt][d][3] *= alpha[1];
-                        }
-                    }
-                    // probabilities as value + remainder in bfloat16 (the product keeps 16 bits of them),
-                    // moved from result layout [key g][rows 2t, 2t+1] to operand layout [keys 2t, 2t+1][row g]
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const float a = sc[nt][2 * h], c = sc[nt][2 * h + 1];
-                        const __nv_bfloat162 hi = __floats2bfloat162_rn(a, c);
-                        const float2 back = __bfloat1622float2(hi);
-                        ph[nt][h] = movmatrix_trans(*reinterpret_cast<const unsigned*>(&hi));
-                        pl[nt][h] = movmatrix_trans(pack_bf16(a - back.x, c - back.y));
-                    }
-                }
-#pragma unroll
-                for (int dp = 0; dp < KSTEPS; ++dp) {
-                    unsigned vf[4];
-                    ldmatrix_x4_trans(vf, (va ^ (unsigned)(((dp * 2) & 7) << 4)) + (dp / 4) * HALF_BYTES);
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) {
-                        mma_bf16(o[nt][dp], vf, ph[nt][0], ph[nt][1]);
-                        mma_bf16(o[nt][dp], vf, pl[nt][0], pl[nt][1]);
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0 && !(SELFTEST && it == 0 && blockIdx.x % 3 == 1)) mbar_arrive(&empty_bar[s]);     // this warp is done with the stage
+            for (int nt = 0; nt < NT; ++nt) mma_bf16(sc[nt], kf, qf[nt][kd][0], qf[nt][kd][1]);
         }
+        const bool all_visible = share_lo >= lo && share_lo + 16 <= hi && share_lo + 15 <= warp_qmin &&
+                                 (p.window <= 0 || share_lo > warp_qmax - p.window);
+        if (!all_visible) {
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int qp = qpos[nt][e & 1];
+                    const int kpos = share_lo + g + 8 * (e >> 1);
+                    const bool vis = kpos >= lo && kpos < hi && kpos <= qp && (p.window <= 0 || kpos > qp - p.window);
+                    if (!vis) sc[nt][e] = -INFINITY;
+                }
+        }
+        unsigned ph[NT][2], pl[NT][2];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            float m_safe[2], alpha[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float mx = fmaxf(sc[nt][j], sc[nt][j + 2]);            // over the 16 keys: the lanes that share t
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                const float m_new = fmaxf(m[nt][j], mx * p.scale_log2);   // maxima live on the base-2 scale
+                m_safe[j] = (m_new == -INFINITY) ? 0.f : m_new;           // no key seen yet: keep exponents finite
+                alpha[j] = ex2(m[nt][j] - m_safe[j]);
+                m[nt][j] = m_new;
+                l[nt][j] *= alpha[j];
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float pv = ex2(fmaf(sc[nt][e], p.scale_log2, -m_safe[e & 1]));
+                sc[nt][e] = pv;
+                l[nt][e & 1] += pv;
+            }
+            if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+                for (int d = 0; d < KSTEPS; ++d) {
+                    o[nt][d][0] *= alpha[0]; o[nt][d][1] *= alpha[1];
+                    o[nt][d][2] *= alpha[0]; o[nt][d][3] *= alpha[1];
+                }
+            }
+            // probabilities as value + remainder in bfloat16 (the product keeps 16 bits of them),
+            // moved from result layout [key g][rows 2t, 2t+1] to operand layout [keys 2t, 2t+1][row g]
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float a = sc[nt][2 * h], c = sc[nt][2 * h + 1];
+                const __nv_bfloat162 hi2 = __floats2bfloat162_rn(a, c);
+                const float2 back = __bfloat1622float2(hi2);
+                ph[nt][h] = movmatrix_trans(*reinterpret_cast<const unsigned*>(&hi2));
+                pl[nt][h] = movmatrix_trans(pack_bf16(a - back.x, c - back.y));
+            }
+        }
+#pragma unroll
+        for (int dp = 0; dp < KSTEPS; ++dp) {
+            unsigned vf[4];
+            ldmatrix_x4_trans(vf, (va ^ (unsigned)(((dp * 2) & 7) << 4)) + (dp / 4) * HALF_BYTES);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                mma_bf16(o[nt][dp], vf, ph[nt][0], ph[nt][1]);
+                mma_bf16(o[nt][dp], vf, pl[nt][0], pl[nt][1]);
+            }
+        }
+    }
+    __device__ __forceinline__ void end() {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -539,9 +459,9 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                 l[nt][j] += __shfl_xor_sync(0xffffffffu, l[nt][j], 8);
                 l[nt][j] += __shfl_xor_sync(0xffffffffu, l[nt][j], 16);
             }
-
-        // ---- the four warps' results, through shared memory (all have read the queries and the tiles)
-        consumers_sync();
+    }
+    // the warp's results: Om [NCW][om_rows][OPITCH], Mm and Lm [NCW][8 NT]
+    __device__ __forceinline__ void leave(float* Om, float* Mm, float* Lm, int warp, int om_rows, int n_rows) const {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -550,58 +470,293 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                 if (rr < n_rows) {
 #pragma unroll
                     for (int dp = 0; dp < KSTEPS; ++dp) {
-                        Om[(warp * p.rows + rr) * OPITCH + dp * 16 + g] = o[nt][dp][j];
-                        Om[(warp * p.rows + rr) * OPITCH + dp * 16 + g + 8] = o[nt][dp][j + 2];
+                        Om[(warp * om_rows + rr) * OPITCH + dp * 16 + g] = o[nt][dp][j];
+                        Om[(warp * om_rows + rr) * OPITCH + dp * 16 + g + 8] = o[nt][dp][j + 2];
                     }
                     if (g == 0) {
-                        Mm[warp][rr] = m[nt][j];
-                        Lm[warp][rr] = l[nt][j];
+                        Mm[warp * 8 * NT + rr] = m[nt][j];
+                        Lm[warp * 8 * NT + rr] = l[nt][j];
                     }
                 }
             }
+    }
+    // the four warps' results of row rr, columns d .. d + 3, added up: sums, and the maximum (base-2 scale) and sum of the weights
+    static __device__ __forceinline__ float4 add_up(const float* Om, const float* Mm, const float* Lm, int om_rows, int rr, int d, float& M, float& den) {
+        M = -INFINITY;
+#pragma unroll
+        for (int v = 0; v < NCW; ++v) M = fmaxf(M, Mm[v * 8 * NT + rr]);
+        float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
+        den = 0.f;
+#pragma unroll
+        for (int v = 0; v < NCW; ++v) {
+            const float mv = Mm[v * 8 * NT + rr], lv = Lm[v * 8 * NT + rr];
+            if (mv == -INFINITY) continue;
+            const float f = exp2f(mv - M);
+            const float4 o4 = *reinterpret_cast<const float4*>(Om + (v * om_rows + rr) * OPITCH + d);
+            num.x = fmaf(f, o4.x, num.x); num.y = fmaf(f, o4.y, num.y);
+            num.z = fmaf(f, o4.z, num.z); num.w = fmaf(f, o4.w, num.w);
+            den = fmaf(f, lv, den);
+        }
+        return num;
+    }
+};
+__device__ __forceinline__ void store_row(__nv_bfloat16* out, float4 num, float den) {
+    const float inv = den > 0.f ? 1.f / den : 0.f;
+    uint2 w2;
+    w2.x = pack_bf16(num.x * inv, num.y * inv);
+    w2.y = pack_bf16(num.z * inv, num.w * inv);
+    *reinterpret_cast<uint2*>(out) = w2;
+}
+__device__ __forceinline__ float natural(float M) { return M == -INFINITY ? -INFINITY : M * LN2; }     // a maximum on the natural-log scale
+
+template <int STAGES>
+__device__ __forceinline__ void set_up_barriers(unsigned long long* full_bar, unsigned long long* empty_bar) {
+    for (int s = 0; s < STAGES; ++s) {
+        mbar_init(&full_bar[s], 1);
+        mbar_init(&empty_bar[s], NCW);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+// The first in the CTA whose wait runs out reports (one that only stopped with another's has nothing to say).
+__device__ __forceinline__ void report(int* failed_flag, int* status, int code) {
+    if (atomicExch(failed_flag, 1) == 0) atomicExch(status, code);
+}
+// The wait of a whole warp: false for all lanes if it ran out for any.
+__device__ __forceinline__ bool warp_wait(unsigned long long* bar, unsigned parity, int* failed_flag, int* status, int code, int lane,
+                                          unsigned long long limit_ns) {
+    if (__all_sync(0xffffffffu, mbar_wait(bar, parity, failed_flag, limit_ns))) return true;
+    if (lane == 0) report(failed_flag, status, code);
+    return false;
+}
+
+// ---- a CTA to a piece (blockIdx: request z, unit y, piece x); merge_partials_kernel follows where there are several.
+// The CTA's one barrier stands right behind the set-up, so that the queries are fetched while the producer looks the first pages
+// up (behind the first tiles and the queries: 4 requests of 2,000 tokens and 4 new ones each, 32 / 8 heads of 128, 19.5 us, this
+// order 18.4; one request of 333 5.3 and 5.0).  It is a kernel of its own because the loops of the shares cost it: 24 requests of 130 to 1,900,
+// heads of 64, 14.8 us in one body with them, 14.3 here; 4 of 5,000 to 7,900, 24 / 8 heads of 128, 20.9 and 20.6.
+template <int HD, int STAGES, int NT>
+__global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_kernel(const __grid_constant__ CUtensorMap map_k,
+                                                                                  const __grid_constant__ CUtensorMap map_v,
+                                                                                  const DecodeParams p) {
+    using C = Consumer<HD, NT>;
+    constexpr unsigned STAGE_BYTES = 2 * C::KV_BYTES;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
+    __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(tiles + STAGES * STAGE_BYTES);
+    // (the four warps' results lie where the tiles were)
+    float* Om = reinterpret_cast<float*>(tiles);
+    float* Mm = Om + NCW * 8 * NT * C::OPITCH;
+    float* Lm = Mm + NCW * 8 * NT;
+    __shared__ __align__(8) unsigned long long full_bar[STAGES];
+    __shared__ __align__(8) unsigned long long empty_bar[STAGES];
+    __shared__ int failed_flag, gave_up;
+
+    grid_launch_dependents();
+    // What follows, down to the dependency wait, reads nothing that the kernels just before this one
+    // write: the step's index data were uploaded before its first kernel, and keys and values of
+    // positions before the step's own tokens were written by earlier steps.  Under programmatic
+    // dependent launch this part runs while the predecessor is still at work.
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int b = blockIdx.z, split = blockIdx.x;
+    const Span span = span_of(p, b);
+    if (span.n_tokens == 0) return;
+    const int kvh = blockIdx.y / p.n_gchunks;
+    const int g0 = (blockIdx.y - kvh * p.n_gchunks) * p.ng;
+    const int ng = min(p.ng, p.group - g0);
+    const int k_lo = span.lo + split * span.piece, k_hi = min(span.hi, k_lo + span.piece);
+    const int k_start = k_lo & ~(p.box_rows - 1);      // copies start on a box (page) boundary; keys below k_lo are masked
+    const int n_tiles = k_hi > k_start ? (k_hi - k_start + BN - 1) / BN : 0;
+    if (tid == NCW * 32) {
+        failed_flag = 0;
+        set_up_barriers<STAGES>(full_bar, empty_bar);
+    }
+    __syncthreads();
+
+    if (warp == NCW) {
+        const int* table = p.block_table + (size_t)b * p.table_stride;
+        auto issue = [&](int it) {
+            issue_tile<HD>(p, map_k, map_v, tiles + (it % STAGES) * STAGE_BYTES, &full_bar[it % STAGES], table, kvh, k_start + it * BN, k_hi, lane);
+        };
+        // tiles that end before the step's first new position can go now; a tile that may hold a key
+        // written by the predecessor (only the last tile of the last piece can) waits for it
+        int it = 0;
+        for (; it < STAGES && it < n_tiles && k_start + (it + 1) * BN <= span.base; ++it) issue(it);
+        grid_dependency_wait();
+        for (; it < STAGES && it < n_tiles; ++it) issue(it);
+        for (; it < n_tiles; ++it) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[it % STAGES], ((it / STAGES) - 1) & 1, &failed_flag))) {
+                if (lane == 0) report(&failed_flag, p.status, ERR_PRODUCER_WAIT);
+                break;
+            }
+            issue(it);
+        }
+        // (nothing that is still on its way may land in shared memory that is no longer this CTA's)
+        int never = 0;
+        for (int k = max(0, it - STAGES); k < it; ++k) mbar_wait(&full_bar[k % STAGES], (k / STAGES) & 1, &never);
+        return;
+    }
+
+    // ---- consumers: the same rows, 16 keys of every tile each
+    grid_dependency_wait();
+    const int n_rows = span.n_tokens * ng, head0 = kvh * p.group + g0;
+    fetch_queries<HD, NT>(p, Qs, span.first, head0, ng, n_rows);
+    consumers_sync();
+    C c;
+    c.place(warp, lane);
+    c.begin(span.base, ng, n_rows);
+    c.take_queries(Qs, lane);
+    bool ok = true;
+    for (int it = 0; it < n_tiles; ++it) {
+        const int s = it % STAGES;
+        ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[s], (it / STAGES) & 1, &failed_flag));
+        if (!ok) break;
+        c.tile(p, smem_u32(tiles + s * STAGE_BYTES), k_start + it * BN, k_lo, k_hi);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty_bar[s]);     // this warp is done with the stage
+    }
+    if (!ok && lane == 0) report(&failed_flag, p.status, ERR_CONSUMER_WAIT);
+    c.end();
+    // ---- the four warps' results, through shared memory (the stages are done with; one thread reads for all whether
+    // the CTA gave up, so that all take the same way; rows that are nobody's hold zeros)
+    consumers_sync();
+    c.leave(Om, Mm, Lm, warp, 8 * NT, 8 * NT);
+    if (tid == 0) gave_up = *(volatile int*)&failed_flag;
+    consumers_sync();
+    if (gave_up) return;
+    for (int idx = tid; idx < n_rows * (HD / 4); idx += NCW * 32) {      // four columns of a row per turn
+        const int rr = idx / (HD / 4), d = (idx - rr * (HD / 4)) * 4;
+        float M, den;
+        const float4 num = C::add_up(Om, Mm, Lm, 8 * NT, rr, d, M, den);
+        const size_t row = (size_t)(span.first + rr / ng) * p.n_heads + head0 + rr % ng;
+        if (p.n_splits == 1) {
+            store_row(p.out + row * HD + d, num, den);
+        } else {
+            *reinterpret_cast<float4*>(p.part_o + (row * p.n_splits + split) * HD + d) = num;
+            if (d == 0) {
+                p.part_ml[(row * p.n_splits + split) * 2] = natural(M);
+                p.part_ml[(row * p.n_splits + split) * 2 + 1] = den;
+            }
+        }
+    }
+}
+
+// ---- shares: a CTA takes the pieces of its share one after the other, and the last one adds a request's up.
+// SELFTEST: every third CTA never hands back its first stage, so that its producer's wait for room runs out
+template <int HD, int STAGES, int NT, bool SELFTEST = false>
+__global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_shares_kernel(const __grid_constant__ CUtensorMap map_k,
+                                                                                         const __grid_constant__ CUtensorMap map_v,
+                                                                                         const DecodeParams p) {
+    using C = Consumer<HD, NT>;
+    constexpr unsigned STAGE_BYTES = 2 * C::KV_BYTES;
+    constexpr int NROWS = 8 * NT;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023));
+    // behind the stages, in the same place one after the other: the queries [NROWS][HD + 8], the four warps' results
+    // [NCW][rows][OPITCH] and the weights of the pieces [rows][MERGE_MAX_SPLITS]
+    __nv_bfloat16* Qs = reinterpret_cast<__nv_bfloat16*>(tiles + STAGES * STAGE_BYTES);
+    float* Om = reinterpret_cast<float*>(tiles + STAGES * STAGE_BYTES);
+    __shared__ float Mm[NCW * NROWS], Lm[NCW * NROWS];
+    __shared__ __align__(8) unsigned long long full_bar[STAGES];
+    __shared__ __align__(8) unsigned long long empty_bar[STAGES];
+    __shared__ int failed_flag;
+    __shared__ int arrived, gave_up;
+
+    grid_launch_dependents();
+    // (down to the dependency wait nothing is read that the kernels just before this one write: see above)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned long long limit_ns = SELFTEST ? p.limit_ns : WAIT_NS;
+    Walk w;
+    if (!walk_share<NT>(p, w, lane)) return;            // (the same for all warps)
+    if (tid == NCW * 32) {
+        failed_flag = 0;
+        set_up_barriers<STAGES>(full_bar, empty_bar);
+    }
+    __syncthreads();
+
+    if (warp == NCW) {
+        bool waited = false;
+        int it = 0;
+        bool ok = true;
+        do {
+            const int kvh = w.unit / p.n_gchunks;
+            const int* table = p.block_table + (size_t)w.b * p.table_stride;
+            for (int i = 0; i < w.tiles && ok; ++i, ++it) {
+                const int s = it % STAGES;
+                const int k0 = w.start + i * BN;
+                // tiles go at once, up to one that may hold a key written by the predecessor
+                if (!waited && k0 + BN > w.span.base) {
+                    grid_dependency_wait();
+                    waited = true;
+                }
+                if (it >= STAGES && !warp_wait(&empty_bar[s], ((it / STAGES) - 1) & 1, &failed_flag, p.status, ERR_PRODUCER_WAIT, lane, limit_ns)) {
+                    ok = false;
+                    break;
+                }
+                issue_tile<HD>(p, map_k, map_v, tiles + s * STAGE_BYTES, &full_bar[s], table, kvh, k0, w.hi, lane);
+            }
+        } while (ok && walk_next<NT>(p, w));
+        if (!waited) grid_dependency_wait();
+        // (nothing that is still on its way may land in shared memory that is no longer this CTA's)
+        int never = 0;
+        for (int k = max(0, it - STAGES); k < it; ++k) mbar_wait(&full_bar[k % STAGES], (k / STAGES) & 1, &never, limit_ns);
+        return;
+    }
+
+    // ---- consumers: the same rows, 16 keys of every tile each
+    grid_dependency_wait();
+    C c;
+    c.place(warp, lane);
+    bool ok = true, fresh = true;
+    int it = 0;
+    do {
+        const int kvh = w.unit / p.n_gchunks;
+        const int g0 = (w.unit - kvh * p.n_gchunks) * p.ng;
+        const int ng = min(p.ng, p.group - g0);
+        const int n_rows = w.span.n_tokens * ng, head0 = kvh * p.group + g0;
+        // the next pieces of a request find the queries in registers
+        if (fresh) {
+            fetch_queries<HD, NT>(p, Qs, w.span.first, head0, ng, n_rows);
+            consumers_sync();
+            c.take_queries(Qs, lane);
+        }
+        c.begin(w.span.base, ng, n_rows);
+        for (int i = 0; i < w.tiles; ++i, ++it) {
+            const int s = it % STAGES;
+            if (!ok || !warp_wait(&full_bar[s], (it / STAGES) & 1, &failed_flag, p.status, ERR_CONSUMER_WAIT, lane, limit_ns)) {
+                ok = false;
+                break;
+            }
+            c.tile(p, smem_u32(tiles + s * STAGE_BYTES), w.start + i * BN, w.lo, w.hi);
+            __syncwarp();
+            if (lane == 0 && !(SELFTEST && it == 0 && blockIdx.x % 3 == 1)) mbar_arrive(&empty_bar[s]);     // this warp is done with the stage
+        }
+        c.end();
+
+        // ---- the four warps' results, through shared memory (all have read the queries and the tiles)
+        consumers_sync();
+        c.leave(Om, Mm, Lm, warp, p.rows, n_rows);
         // (the producer may give up at any moment: one thread reads the flag for all, so that all take the same way
         // through the barriers below; what this piece is made of has arrived by now, or a consumer has set the flag)
-        if (tid == 0) gave_up = *failed;
+        if (tid == 0) gave_up = *(volatile int*)&failed_flag;
         consumers_sync();
         const bool sound = gave_up == 0;
-        const int parts = SHARES ? w.span.pieces : p.n_splits;
+        const int parts = w.span.pieces;
         if (sound) {
             for (int idx = tid; idx < n_rows * (HD / 4); idx += NCW * 32) {      // four columns of a row per turn
                 const int rr = idx / (HD / 4), d = (idx - rr * (HD / 4)) * 4;
-                float M = -INFINITY;
-#pragma unroll
-                for (int v = 0; v < NCW; ++v) M = fmaxf(M, Mm[v][rr]);
-                float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
-                float den = 0.f;
-#pragma unroll
-                for (int v = 0; v < NCW; ++v) {
-                    const float mv = Mm[v][rr], lv = Lm[v][rr];
-                    if (mv == -INFINITY) continue;
-                    const float f = exp2f(mv - M);
-                    const float4 o4 = *reinterpret_cast<const float4*>(Om + (v * p.rows + rr) * OPITCH + d);
-                    num.x = fmaf(f, o4.x, num.x); num.y = fmaf(f, o4.y, num.y);
-                    num.z = fmaf(f, o4.z, num.z); num.w = fmaf(f, o4.w, num.w);
-                    den = fmaf(f, lv, den);
-                }
+                float M, den;
+                const float4 num = C::add_up(Om, Mm, Lm, p.rows, rr, d, M, den);
                 if (parts == 1) {
-                    const float inv = den > 0.f ? 1.f / den : 0.f;
-                    uint2 w2;
-                    w2.x = pack_bf16(num.x * inv, num.y * inv);
-                    w2.y = pack_bf16(num.z * inv, num.w * inv);
-                    const int head = kvh * p.group + g0 + rr % ng;
-                    *reinterpret_cast<uint2*>(p.out + ((size_t)(qs + rr / ng) * p.n_heads + head) * HD + d) = w2;
+                    store_row(p.out + ((size_t)(w.span.first + rr / ng) * p.n_heads + head0 + rr % ng) * HD + d, num, den);
                 } else {
-                    const int head = kvh * p.group + g0 + rr % ng;
-                    const size_t place = SHARES ? (((size_t)w.b * p.units + w.unit) * p.n_splits + w.split) * p.rows + rr
-                                                : ((size_t)(qs + rr / ng) * p.n_heads + head) * p.n_splits + w.split;
+                    const size_t place = (((size_t)w.b * p.units + w.unit) * p.n_splits + w.split) * p.rows + rr;
                     __stcg(reinterpret_cast<float4*>(p.part_o + place * HD + d), num);
-                    if (d == 0) __stcg(reinterpret_cast<float2*>(p.part_ml + place * 2), make_float2(M == -INFINITY ? -INFINITY : M * LN2, den));   // natural-log scale
+                    if (d == 0) __stcg(reinterpret_cast<float2*>(p.part_ml + place * 2), make_float2(natural(M), den));
                 }
             }
         }
         // ---- whoever is last with a request's pieces adds them up (in order, as merge_partials_kernel does)
-        const bool last_here = SHARES && (w.split + 1 == parts || w.at + w.span.piece / BN >= w.end);
-        if (SHARES && parts > 1 && last_here) {
+        if (parts > 1 && (w.split + 1 == parts || w.at + worth<NT>(w.span) >= w.end)) {
             consumers_sync();
             const int mine = w.split + 1 - w.first_split;
             int seen = mine;
@@ -630,47 +785,40 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
                     float M = -INFINITY, den = 0.f;
 #pragma unroll
                     for (int i = 0; i < MERGE_MAX_SPLITS / 32; ++i) {
-                        const int c = i * 32 + lane;
+                        const int c1 = i * 32 + lane;
                         ml[i] = make_float2(-INFINITY, 0.f);
-                        if (c < parts) ml[i] = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (place0 + (size_t)c * p.rows + rr) * 2));
+                        if (c1 < parts) ml[i] = __ldcg(reinterpret_cast<const float2*>(p.part_ml + (place0 + (size_t)c1 * p.rows + rr) * 2));
                         M = fmaxf(M, ml[i].x);
                     }
                     M = warp_max(M);
 #pragma unroll
                     for (int i = 0; i < MERGE_MAX_SPLITS / 32; ++i) {
-                        const int c = i * 32 + lane;
+                        const int c1 = i * 32 + lane;
                         const float f = ml[i].x == -INFINITY ? 0.f : __expf(ml[i].x - M);
-                        if (c < parts) weight[rr * MERGE_MAX_SPLITS + c] = f;
+                        if (c1 < parts) weight[rr * MERGE_MAX_SPLITS + c1] = f;
                         den = fmaf(f, ml[i].y, den);
                     }
                     den = warp_sum(den);
-                    if (lane == 0) Lm[0][rr] = den;
+                    if (lane == 0) Lm[rr] = den;
                 }
                 consumers_sync();
                 for (int idx = tid; idx < n_rows * (HD / 4); idx += NCW * 32) {
                     const int rr = idx / (HD / 4), d = (idx - rr * (HD / 4)) * 4;
                     float4 num = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
-                    for (int c = 0; c < parts; ++c) {
-                        const float f = weight[rr * MERGE_MAX_SPLITS + c];
-                        const float4 o4 = __ldcg(reinterpret_cast<const float4*>(p.part_o + (place0 + (size_t)c * p.rows + rr) * HD + d));
+                    for (int c1 = 0; c1 < parts; ++c1) {
+                        const float f = weight[rr * MERGE_MAX_SPLITS + c1];
+                        const float4 o4 = __ldcg(reinterpret_cast<const float4*>(p.part_o + (place0 + (size_t)c1 * p.rows + rr) * HD + d));
                         num.x = fmaf(f, o4.x, num.x); num.y = fmaf(f, o4.y, num.y);
                         num.z = fmaf(f, o4.z, num.z); num.w = fmaf(f, o4.w, num.w);
                     }
-                    const float den = Lm[0][rr];
-                    const float inv = den > 0.f ? 1.f / den : 0.f;
-                    uint2 w2;
-                    w2.x = pack_bf16(num.x * inv, num.y * inv);
-                    w2.y = pack_bf16(num.z * inv, num.w * inv);
-                    const int head = kvh * p.group + g0 + rr % ng;
-                    *reinterpret_cast<uint2*>(p.out + ((size_t)(qs + rr / ng) * p.n_heads + head) * HD + d) = w2;
+                    store_row(p.out + ((size_t)(w.span.first + rr / ng) * p.n_heads + head0 + rr % ng) * HD + d, num, Lm[rr]);
                 }
             }
         }
-        if (!SHARES) return;
         fresh = w.split + 1 == parts;
         consumers_sync();            // the place behind the stages is the next piece's
-    } while (walk_next(p, w));
+    } while (walk_next<NT>(p, w));
 }
 
 // out[row, d] = sum_i e^{m_i - M} o_i[d] / sum_i e^{m_i - M} l_i,  M = max_i m_i: the weights are
@@ -768,7 +916,7 @@ static_assert(NCW * (64 + 4) >= MERGE_MAX_SPLITS, "the pieces' weights lie where
 template <int HD, int NT> int shares_per_sm(int rows) {
     static int known[17] = {};                     // (threads that come here at the same time write the same)
     if (known[rows] == 0) {
-        auto kern = attention_decode_kernel<HD, stages_for<HD>(), NT, true>;
+        auto kern = attention_decode_shares_kernel<HD, stages_for<HD>(), NT>;
         int n = 0;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_shares<HD>(8 * NT)) != cudaSuccess ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, NTHREADS, smem_shares<HD>(rows)) != cudaSuccess || n < 1) {
@@ -831,14 +979,28 @@ Plan make_plan(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int max_q_
             }
         }
     }
-    // More than one wave of CTAs, planned for the longest context there could be: most of them would find few keys, or
-    // none.  (Within one wave shares lose: 24 requests of up to 1,900 tokens, 32 / 8 heads of 64, 576 CTAs: a step of 3,335
-    // us took 3,433.)
+    // Shares pay where a share is made of many pieces, most of them short (planned for the longest context there could be):
+    // then the launch of a CTA to a piece costs more than the pieces.  With few pieces to a share they come out uneven.
+    // Shares to pieces by themselves, contexts all of 320 / of 40 to 600 / of 130 to 1,900 / all of 2,048 tokens, us:
+    //   32 / 8 heads of 128, 40 requests, 2.9 pieces a share:  17.2  17.6  38.0  56.2  to  17.1  18.0  32.6  55.1
+    //                        28           3.5                  14.4  14.4  29.3  41.9      17.1  18.3  28.2  43.3
+    //                        64           6.9                  22.8  22.5  49.7  84.2      28.6  30.0  51.8  86.5
+    //                  64,   96           5.2                  21.1  22.1  44.7  74.5      21.4  23.0  40.9  69.2
+    //                        64           9.2                  18.8  19.3  33.2  49.3      25.1  25.7  37.0  53.4
+    //   128 / 8 heads of 128 (more than 8 rows: more work to a tile), and of 64:
+    //                  64,   48           3.9                  23.3  26.0  41.7  55.5      25.2  27.2  40.4  54.9
+    //                  128,  40           4.3                  32.7  35.0  54.7  82.7      34.0  35.4  54.4  80.4
+    //                        28           5.3                  26.9  34.4  49.4  66.8      33.4  35.1  48.1  64.1
+    //                        64           10.4                 53.1  53.4  89.3  125.6     63.4  65.3  92.8  127.5
+    // With heads of 128 and 5 to 8 rows the warps' results, which shares keep beside the stages, leave room for two CTAs an SM
+    // instead of three (64 requests, 64 / 8 heads, all of 320, of 40 to 600, all of 2,048: 34.0  37.9  100.1 to 33.9  35.3  90.7): they stay pieces.
     pl.shares = 0;
-    if (allow_split == 1 && pl.n_splits > 1 && (long long)n_kv_heads * pl.n_gchunks * n_seqs * pl.n_splits > 148LL * ctas_per_sm(head_dim)) {
+    const long long pieces = (long long)n_kv_heads * pl.n_gchunks * n_seqs * pl.n_splits;
+    if (allow_split == 1 && pl.n_splits > 1 && pieces > 148LL * ctas_per_sm(head_dim)) {
         const int rows = max_q_len * pl.ng;
-        pl.shares = 148 * (head_dim == 128 ? (rows <= 8 ? shares_per_sm<128, 1>(rows) : shares_per_sm<128, 2>(rows))
-                                           : (rows <= 8 ? shares_per_sm<64, 1>(rows) : shares_per_sm<64, 2>(rows)));
+        const int ctas = 148 * (head_dim == 128 ? (rows <= 8 ? shares_per_sm<128, 1>(rows) : shares_per_sm<128, 2>(rows))
+                                                : (rows <= 8 ? shares_per_sm<64, 1>(rows) : shares_per_sm<64, 2>(rows)));
+        if (pieces > (long long)(rows <= 8 ? 6 : 4) * ctas && !(head_dim == 128 && rows > 4 && rows <= 8)) pl.shares = ctas;
     }
     return pl;
 }
@@ -846,7 +1008,7 @@ Plan make_plan(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int max_q_
 // A self-test of the waits: shares of 148 CTAs (a first stage that is not handed back stops each third of them once it
 // has more tiles than stages), heads of 64, up to 8 rows.
 int launch_selftest(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, cudaStream_t s) {
-    auto kern = attention_decode_kernel<64, stages_for<64>(), 1, true, true>;
+    auto kern = attention_decode_shares_kernel<64, stages_for<64>(), 1, true>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_shares<64>(8));
     if (e != cudaSuccess) return (int)e;
     return (int)tl_launch(kern, dim3(148), dim3(NTHREADS), smem_shares<64>(p.rows), s, mk, mv, p);
@@ -855,9 +1017,9 @@ int launch_selftest(const CUtensorMap& mk, const CUtensorMap& mv, const DecodePa
 template <int HD, int NT>
 int launch(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, const Plan& pl, cudaStream_t s) {
     if (pl.shares > 0)          // (shares_per_sm has raised the limit on shared memory)
-        return (int)tl_launch(attention_decode_kernel<HD, stages_for<HD>(), NT, true>, dim3(pl.shares), dim3(NTHREADS), smem_shares<HD>(p.rows), s, mk, mv, p);
+        return (int)tl_launch(attention_decode_shares_kernel<HD, stages_for<HD>(), NT>, dim3(pl.shares), dim3(NTHREADS), smem_shares<HD>(p.rows), s, mk, mv, p);
     constexpr size_t smem = smem_for<HD>();
-    auto kern = attention_decode_kernel<HD, stages_for<HD>(), NT, false>;
+    auto kern = attention_decode_kernel<HD, stages_for<HD>(), NT>;
     static bool raised = false;
     if (!raised) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
