@@ -562,6 +562,42 @@ def test_delta_rule_at_the_edges_of_blocks(backend, d):
 
 
 @pytest.mark.parametrize("backend", BACKENDS)
+@pytest.mark.parametrize("lens,H,dv", [([16], 2, 18), ([17], 2, 18), ([33] * 2, 4, 288), ([33] * 3, 4, 288), ([1, 129], 5, 448), ([1, 1, 256], 5, 448),
+                                       ([1, 1, 255], 5, 448), ([2, 129], 5, 448), ([40], 6, 400), ([1, 300], 6, 400)],
+                         ids=["short", "above", "one-an-sm", "two-an-sm", "beside-one", "beside-two", "beside-too-many", "beside-more", "wide", "wide-beside"])
+def test_delta_rule_on_both_sides_of_the_block_sizes(backend, lens, H, dv):
+    """Blocks of 4 and of 8 tokens, at the lines between them: portions of 16 and 17 tokens, as many CTAs as a GPU has SMs or more, one
+    long portion beside few and many single tokens."""
+    ops, dev = _ops(backend)
+    d, T, n = 80, sum(lens), len(lens)
+    g = torch.Generator().manual_seed(T)
+    dt = _dt(backend)
+    q = torch.nn.functional.normalize(torch.randn(T, 1, d, generator=g), dim=-1) * d ** -0.5
+    k = torch.nn.functional.normalize(torch.randn(T, 1, d, generator=g), dim=-1)
+    v, beta = torch.randn(T, H, dv, generator=g).to(dt), torch.randn(T, H, generator=g).to(dt)
+    z, rate, bias = torch.randn(T, H * d, generator=g).to(dt), torch.rand(H, generator=g) + 0.1, torch.randn(H * d, generator=g) - 2.0
+    decay = torch.exp(-rate.double()[:, None] * torch.nn.functional.softplus(z.double() + bias.double()).view(T, H, d))
+    held = torch.randn(n, H, d, dv, generator=g)
+    state = held.transpose(2, 3).contiguous().to(dev)
+    want, at = [], 0
+    for b, length in enumerate(lens):
+        S = held[b].double()
+        for t in range(at, at + length):
+            S = decay[t][:, :, None] * S
+            u = torch.sigmoid(beta[t].double())[:, None] * (v[t].double() - torch.einsum("hkv,k->hv", S, k[t, 0].double()))
+            S = S + k[t, 0].double()[None, :, None] * u[:, None, :]
+            want.append(torch.einsum("hkv,k->hv", S, q[t, 0].double()).flatten())
+        held[b] = S.float()
+        at += length
+    (q_start, slot_t, fresh_t), how = _steps(lens, list(range(n)), [0] * n, dev)
+    got = ops.linear_recurrence(q.flatten(1).to(dev), k.flatten(1).to(dev), v.flatten(1).to(dev), state, q_start, slot_t, fresh_t, beta_logits=beta.to(dev),
+                                decay_logits=z.to(dev), decay_rate=rate.to(dev), decay_bias=bias.to(dev), **how)
+    want = torch.stack(want)
+    torch.testing.assert_close(got.cpu().double(), want, atol=2e-5 * float(want.abs().max()), rtol=1e-4)      # as above
+    torch.testing.assert_close(state.transpose(2, 3).cpu(), held, atol=2e-5 * float(held.abs().max()), rtol=1e-4)
+
+
+@pytest.mark.parametrize("backend", BACKENDS)
 def test_results_that_are_columns_of_wider_rows(backend):
     """The head norm with a sigmoid gate, and attention with a gate in one key split and in several, writing into a column
     range of wider rows: the same numbers as into a tensor of their own, and nothing beside the range."""

@@ -493,15 +493,36 @@ cudaError_t launch_blocks(const RecurrenceParams& p, int n_seqs, cudaStream_t s)
     return tl_launch(recurrence_blocks_kernel<R, KS, MODE, BLOCK, TV>, dim3((p.dv + L::COLS - 1) / L::COLS, p.H, n_seqs), dim3(NT), smem, s, p);
 }
 
+// Blocks of 8 tokens or of 4, with a decay per channel and keys of 65 to 128.  A walk of 8 takes fewer rounds of sums over the
+// lanes and gives each warp more that does not depend on what came before, but with 203 registers a thread and 162 KB of
+// shared memory there is one CTA to an SM where two with blocks of 4 fit.  So 8 where the CTAs fit one to an SM, and where portions
+// reach into a third block of 4; and beside one long portion where the other requests bring one token each and are
+// few (each of them costs an SM's turn; blocks of 4 take two at a time).  Blocks of 4 and of 8, heads of 128, us:
+//   one request of   9 / 16 / 17 / 33 / 64 / 150 / 601 tokens, 16 heads (128 CTAs):  8.3  9.3 10.8 14.5 20.6 41.4 96.7  to  8.7  9.0  9.7 13.1 15.9 27.4 88.7
+//                                                              8 heads (64 CTAs):    6.4  8.0  9.7 14.2 20.0 41.1 146.  to  8.3  8.3  9.1 12.4 15.0 27.1 86.4
+//                                                              32 heads (256 CTAs):  9.5 10.1 11.8 15.2 21.0 42.8 155.  to 14.3 14.8 16.4 23.0 27.8 52.0 177.
+//   two of 300, 16 heads: 79.0 to 93.3;  one of 300 and 1 / 2 / 4 / 16 of one token, 16 heads: 76.6 79.0 67.8 104. to 53.0 57.6 66.7 118.;
+//   of 900: 221. 223. 228. 249. to 136. 140. 150. 202.;  of 100: 27.0 32.2 30.8 56.5 to 26.5 31.2 40.1 91.2;  of 900, 8 heads, 8 / 12 / 16:
+//   145. 148. 152. to 141. 150. 159.
+// (One column a lane with two CTAs an SM: 131.7 where 88.7 is.  The other decays and sizes keep blocks of 4: theirs is the only form
+// that has been measured.)
+bool blocks_of_eight(long long ctas, int n_seqs, int n_tokens, int max_q_len) {
+    constexpr int SMS = 148;
+    if (max_q_len <= 16) return false;
+    if (ctas * n_seqs <= SMS) return true;
+    return ctas <= SMS && n_tokens - max_q_len == n_seqs - 1 && (n_seqs - 1) * 128 <= max_q_len;
+}
+
 template <int MODE, typename TV>
-cudaError_t launch_block_sizes(const RecurrenceParams& p, int n_seqs, cudaStream_t s) {
-    // A walk of 8 tokens a block takes fewer rounds of sums over the lanes, and gives each warp more that does not depend
-    // on what came before: 601 tokens, 16 heads of 128, a decay per channel: 97.1 us in blocks of 4, 89.0 in blocks
-    // of 8.  (One column a lane with two CTAs an SM: 131.7.)  The other decays and sizes keep blocks of 4: theirs is the
-    // only form that has been measured.
+cudaError_t launch_block_sizes(const RecurrenceParams& p, int n_seqs, int n_tokens, int max_q_len, cudaStream_t s) {
     if (p.dk <= 32) return launch_blocks<8, 4, MODE, 4, TV>(p, n_seqs, s);
     if (p.dk <= 64) return launch_blocks<8, 8, MODE, 4, TV>(p, n_seqs, s);
-    if (p.dk <= 128) return launch_blocks<8, 16, MODE, MODE == CHANNEL ? 8 : 4, TV>(p, n_seqs, s);
+    if (p.dk <= 128) {
+        constexpr int COLS = BlocksLayout<8, 16, MODE, 4>::COLS;
+        if constexpr (MODE == CHANNEL)
+            if (blocks_of_eight((long long)((p.dv + COLS - 1) / COLS) * p.H, n_seqs, n_tokens, max_q_len)) return launch_blocks<8, 16, MODE, 8, TV>(p, n_seqs, s);
+        return launch_blocks<8, 16, MODE, 4, TV>(p, n_seqs, s);
+    }
     return launch_blocks<16, 16, MODE, 4, TV>(p, n_seqs, s);
 }
 
@@ -518,10 +539,11 @@ cudaError_t launch_steps(const RecurrenceParams& p, int n_seqs, cudaStream_t s) 
 }
 
 template <typename TV>
-int launch_mode(const RecurrenceParams& p, int n_seqs, int mode, bool blocks, cudaStream_t s) {
+int launch_mode(const RecurrenceParams& p, int n_seqs, int n_tokens, int mode, int blocks, cudaStream_t s) {
     if (blocks)
-        return (int)(mode == FIXED ? launch_block_sizes<FIXED, TV>(p, n_seqs, s) : mode == HEAD ? launch_block_sizes<HEAD, TV>(p, n_seqs, s)
-                                                                                               : launch_block_sizes<CHANNEL, TV>(p, n_seqs, s));
+        return (int)(mode == FIXED  ? launch_block_sizes<FIXED, TV>(p, n_seqs, n_tokens, blocks, s)
+                     : mode == HEAD ? launch_block_sizes<HEAD, TV>(p, n_seqs, n_tokens, blocks, s)
+                                    : launch_block_sizes<CHANNEL, TV>(p, n_seqs, n_tokens, blocks, s));
     return (int)(mode == FIXED ? launch_steps<FIXED, TV>(p, n_seqs, s) : mode == HEAD ? launch_steps<HEAD, TV>(p, n_seqs, s)
                                                                                      : launch_steps<CHANNEL, TV>(p, n_seqs, s));
 }
@@ -534,7 +556,7 @@ int launch_mode(const RecurrenceParams& p, int n_seqs, int mode, bool blocks, cu
 // logits (of v's dtype), decay is exp(A_log) per head.  mode 1: gate are rows of pitch ldz with `heads` columns and
 // decay_bias [heads] the bias inside the softplus.  mode 2, a decay per channel: gate has heads * dk columns and decay_bias
 // heads * dk numbers, or, with blocks != 0, gate is float32 [n_tokens][heads * dk], the decays themselves.
-// blocks != 0: for steps with long portions, blocks of tokens at a time.
+// blocks != 0: for steps with long portions, blocks of tokens at a time; its value is the longest portion.
 extern "C" int tl_linear_recurrence(const float* q, const float* k, const void* v, int v_dtype, long long ldv, const void* beta,
                                     long long ldg, const void* gate, long long ldz, const float* decay, const float* decay_bias, float* state,
                                     long long state_pitch, const int* q_start, const int* state_slot, const int* fresh,
@@ -551,7 +573,7 @@ extern "C" int tl_linear_recurrence(const float* q, const float* k, const void* 
     p.state = state; p.state_pitch = state_pitch; p.q_start = q_start; p.state_slot = state_slot; p.fresh = fresh; p.out = out;
     p.H = heads; p.G = qk_heads; p.dk = dk; p.dv = dv;
     cudaStream_t s = (cudaStream_t)stream;
-    if (v_dtype == TL_F32) return launch_mode<float>(p, n_seqs, mode, blocks != 0, s);
-    if (v_dtype == TL_BF16) return launch_mode<__nv_bfloat16>(p, n_seqs, mode, blocks != 0, s);
+    if (v_dtype == TL_F32) return launch_mode<float>(p, n_seqs, n_tokens, mode, blocks, s);
+    if (v_dtype == TL_BF16) return launch_mode<__nv_bfloat16>(p, n_seqs, n_tokens, mode, blocks, s);
     return TL_BAD_DTYPE;
 }

@@ -1163,7 +1163,7 @@ class NativeOps:
         rc = self._lib("matrix_recurrence").tl_linear_recurrence(
             _ptr(q), _ptr(k), _ptr(v), _DT[v.dtype], ldv, _ptr(beta_logits), ldg, _ptr(decay_logits), ldz,
             _ptr(decay_rate if delta else decay), _ptr(decay_bias), _ptr(state), pitch, _ptr(q_start), _ptr(state_slot), _ptr(fresh),
-            _ptr(out), T, n_seqs, H, G, dk, dv, mode, 1 if blocks else 0, _stream())
+            _ptr(out), T, n_seqs, H, G, dk, dv, mode, max_q_len if blocks else 0, _stream())
         _check(rc, "linear_recurrence")
         self.launches += 1
         return out
