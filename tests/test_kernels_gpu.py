@@ -81,6 +81,13 @@ def test_swiglu(ops, dtype, n, hidden):
     torch.testing.assert_close(got.float(), want.float(), atol=tol(dtype, 1e-5), rtol=tol(dtype, 1e-5, 1e-2))
 
 
+@pytest.mark.parametrize("n,hidden", [(2500, 64), (131, 8), (33, 2040), (9, 2048), (5, 2056), (1184, 4096), (1185, 4096), (1200, 4104), (300, 8200)])
+def test_swiglu_at_the_edges_of_its_strips(ops, n, hidden):
+    """Rows narrower than a CTA, strips that do not divide a row, one and two runs a thread."""
+    x = rand((n, 2 * hidden), torch.bfloat16, 9, 3.0)
+    torch.testing.assert_close(ops.swiglu(x).float(), TWIN.swiglu(x).float(), atol=1e-5, rtol=1e-2)      # results rounded to bfloat16
+
+
 # ------------------------------------------------------------------------------------ gemm
 
 @pytest.mark.parametrize("M,N,K", [(1, 1, 1), (1, 1000, 96), (7, 65, 17), (64, 64, 16), (65, 129, 100),

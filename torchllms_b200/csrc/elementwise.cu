@@ -275,23 +275,24 @@ extern "C" int tl_rmsnorm(float* h, const void* delta, int delta_dtype, int delt
 // instructions than the kernel has time for at full memory bandwidth
 __device__ __forceinline__ float silu_mul_fast(float g, float u) { return __fdividef(g, 1.f + __expf(-g)) * u; }
 
-// bfloat16 in and out, hidden a multiple of 8, one plane: a CTA takes a strip of a token's columns, eight gates and eight
-// ups at a time (16-byte accesses), all its loads under way together.  Behind the products of a long prompt the chip runs
-// at the power cap's clock, where a pass over memory has instructions to spare for little else: a division of 64-bit
-// numbers and a row's scale for every eight columns made this kernel wait for instruction issue
-// (1,209 tokens x 8,192 in 16 layers of a 1B step: 3,242 us -> 3,213 for the step).
-constexpr int SWIGLU_EACH = 2;        // runs of eight columns of a thread
+// bfloat16 in and out, hidden a multiple of 8, one plane: a CTA takes a strip of runs of eight columns (16-byte accesses).  WIDE:
+// 512 runs of one token, two to a thread, its loads under way together; else blockDim.x runs of blockDim.y tokens.  Behind
+// the products of a long prompt the chip runs at the power cap's clock, where a pass over memory has instructions to spare for
+// little else: with a division of 64-bit numbers and a row's scale for every eight columns this pass waited for instruction issue
+// (2,048 tokens x 8,192 16.4 us, now 14.7; x 14,336 28.6 and 25.7; 1,209 x 8,192 in 16 layers of a 1B step: 3,242 us -> 3,213).
+template <bool WIDE>
 __global__ void __launch_bounds__(256) swiglu_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
                                                             int hidden, int n_tokens, const RowScale rs) {
     grid_launch_dependents();
-    const int f0 = (blockIdx.x * SWIGLU_EACH * 256 + threadIdx.x) << 3;
+    constexpr int EACH = WIDE ? 2 : 1;
+    const int X = WIDE ? 256 : blockDim.x, f0 = (blockIdx.x * EACH * X + threadIdx.x) << 3;
     grid_dependency_wait();
-    for (int t = blockIdx.y; t < n_tokens; t += gridDim.y) {
+    for (int t = WIDE ? blockIdx.y : blockIdx.y * blockDim.y + threadIdx.y; t < n_tokens; t += WIDE ? gridDim.y : gridDim.y * blockDim.y) {
         const __nv_bfloat16* row = in + (long long)t * 2 * hidden;
-        uint4 graw[SWIGLU_EACH], uraw[SWIGLU_EACH];
+        uint4 graw[EACH], uraw[EACH];
 #pragma unroll
-        for (int e = 0; e < SWIGLU_EACH; ++e) {
-            const int f = f0 + e * 2048;
+        for (int e = 0; e < EACH; ++e) {
+            const int f = f0 + e * X * 8;
             if (f < hidden) {
                 graw[e] = *reinterpret_cast<const uint4*>(row + f);
                 uraw[e] = *reinterpret_cast<const uint4*>(row + hidden + f);
@@ -299,8 +300,8 @@ __global__ void __launch_bounds__(256) swiglu_bf16x8_kernel(const __nv_bfloat16*
         }
         const float sc = row_scale(rs, t);
 #pragma unroll
-        for (int e = 0; e < SWIGLU_EACH; ++e) {
-            const int f = f0 + e * 2048;
+        for (int e = 0; e < EACH; ++e) {
+            const int f = f0 + e * X * 8;
             if (f >= hidden) continue;
             const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&graw[e]);
             const __nv_bfloat162* u2 = reinterpret_cast<const __nv_bfloat162*>(&uraw[e]);
@@ -314,6 +315,21 @@ __global__ void __launch_bounds__(256) swiglu_bf16x8_kernel(const __nv_bfloat16*
             *reinterpret_cast<uint4*>(out + (long long)t * hidden + f) = oraw;
         }
     }
+}
+
+// WIDE where all runs fill the GPU's threads more than twice and a token has at least half a strip's worth.  Else a strip is no wider
+// than it need be (a multiple of 8 runs, so that rows stay 128-byte aligned) and takes as many tokens as go with it.  WIDE for all
+// sizes, and as it is, us: 2,048 tokens x 64 2.55 and 1.35, x 512 3.31 2.79, x 1,024 3.62 3.33; 300 x 4,096 3.45 3.03, x 8,192 4.46
+// 3.64, x 14,336 5.36 5.10; 20 x 8,192 1.61 1.40; 1 x 8,192 1.48 1.20; 2,048 x 2,048 (not quite twice the threads) 4.97 5.13.  One
+// run a thread for all sizes: 2,048 x 2,816 6.27 where WIDE takes 5.70, x 8,192 15.6 and 14.7.
+int launch_swiglu_bf16x8(const __nv_bfloat16* in, __nv_bfloat16* out, int n_tokens, int hidden, const RowScale& rs, cudaStream_t s) {
+    const int runs = hidden / 8;
+    const bool wide = runs >= 256 && (long long)n_tokens * runs > 2LL * 148 * 2048;
+    const int strips = (runs + (wide ? 512 : 256) - 1) / (wide ? 512 : 256);
+    const int x = wide ? 256 : ((runs + strips - 1) / strips + 7) / 8 * 8, y = 256 / x, rows = (n_tokens + y - 1) / y;
+    const dim3 grid(strips, rows < 65535 ? rows : 65535), block(x, y);
+    return (int)(wide ? tl_launch(swiglu_bf16x8_kernel<true>, grid, block, 0, s, in, out, hidden, n_tokens, rs)
+                      : tl_launch(swiglu_bf16x8_kernel<false>, grid, block, 0, s, in, out, hidden, n_tokens, rs));
 }
 
 template <typename TI, typename T>
@@ -342,12 +358,8 @@ extern "C" int tl_swiglu(const void* in, int in_dtype, int splits, void* out, in
     const RowScale rs = {in_ssq, in_parts, in_inv_dim, in_eps};
     if (in_dtype == TL_F32 && dtype == TL_F32) return launch_swiglu<float, float>(in, splits, out, n_tokens, hidden, rs, s);
     if (in_dtype == TL_BF16 && dtype == TL_BF16) {
-        if (splits == 1 && hidden % 8 == 0 && aligned16(in) && aligned16(out)) {
-            const int strips = (hidden / 8 + SWIGLU_EACH * 256 - 1) / (SWIGLU_EACH * 256);
-            const dim3 grid(strips, n_tokens < 65535 ? n_tokens : 65535);
-            return (int)tl_launch(swiglu_bf16x8_kernel, grid, dim3(256), 0, s, (const __nv_bfloat16*)in, (__nv_bfloat16*)out, hidden,
-                                  n_tokens, rs);
-        }
+        if (splits == 1 && hidden % 8 == 0 && aligned16(in) && aligned16(out))
+            return launch_swiglu_bf16x8((const __nv_bfloat16*)in, (__nv_bfloat16*)out, n_tokens, hidden, rs, s);
         return launch_swiglu<__nv_bfloat16, __nv_bfloat16>(in, splits, out, n_tokens, hidden, rs, s);
     }
     if (in_dtype == TL_F32 && dtype == TL_BF16) return launch_swiglu<float, __nv_bfloat16>(in, splits, out, n_tokens, hidden, rs, s);
