@@ -60,18 +60,25 @@ struct DecodeParams {
     const int* kv_len;
     float* part_o;   // a CTA to a piece: [T * H, n_splits, head_dim]; shares: [n_seqs * units, n_splits, rows, head_dim]
     float* part_ml;  // the same with 2 in the place of head_dim: maximum (natural-log scale) and sum
-    int* counters;   // shares: [n_seqs * units], zero between launches
     int* status;
     int table_stride;
     int n_heads, n_kv_heads, page_size, page_shift, box_rows;
     int total_rows;             // rows of the page tensor: a copy that starts there reads only the zero fill
-    int group, ng, n_gchunks, units;    // units: kv heads x chunks of a group's heads
-    int n_seqs, max_tokens;     // requests; tokens of a request
-    int rows;                   // rows of a tile in use: max_tokens * ng
+    int group, ng, n_gchunks;
+    int max_tokens;             // tokens of a request
     int n_splits;
     int window;
     int streamed;               // the call reads more keys and values than L2 holds: their copies are marked to leave it first
     float scale_log2;
+};
+// With the two tensor maps a launch's arguments are 384 bytes.  What only the shares need is kept out of them: with 408 the very same
+// kernel took longer (24 requests of 130 to 1,900 tokens, heads of 64, 14.25 us where 384 take 13.6; 20 requests, heads of
+// 128, 19.3 and 18.9; 16 of 600, heads of 64, 7.0 and 7.2 the other way round).
+static_assert(sizeof(DecodeParams) == 128, "the arguments of a launch with the tensor maps: 384 bytes");
+struct ShareParams : DecodeParams {
+    int* counters;              // [n_seqs * units], zero between launches
+    int n_seqs, units;          // requests; kv heads x chunks of a group's heads
+    int rows;                   // rows of a tile in use: max_tokens * ng
     unsigned long long limit_ns;    // self-test only: how long a wait may take
 };
 
@@ -192,7 +199,7 @@ __device__ __forceinline__ void walk_piece(const DecodeParams& p, Walk& w) {
 // 128 / 8 heads 163, 93 and 89.
 template <int NT> __device__ __forceinline__ int worth(const Span& s) { return s.piece / BN + (NT == 1 ? 2 : 3); }
 // On to the next piece of the line; false: it belongs to the next share, or there is none.
-template <int NT> __device__ __forceinline__ bool walk_next(const DecodeParams& p, Walk& w) {
+template <int NT> __device__ __forceinline__ bool walk_next(const ShareParams& p, Walk& w) {
     w.at += worth<NT>(w.span);
     if (++w.split == w.span.pieces) {
         w.split = 0;
@@ -212,7 +219,7 @@ template <int NT> __device__ __forceinline__ bool walk_next(const DecodeParams& 
 // The first piece of this CTA's share.  All pieces of a request's first unit, of its second and so on, then the next
 // request's, lie on one line, a piece as long as it is worth; a share is every piece that starts in an equal
 // part of the line.  false: there is none.
-template <int NT> __device__ __forceinline__ bool walk_share(const DecodeParams& p, Walk& w, int lane) {
+template <int NT> __device__ __forceinline__ bool walk_share(const ShareParams& p, Walk& w, int lane) {
     int total = 0;
     for (int b = lane; b < p.n_seqs; b += 32) {
         const Span s = span_of(p, b);
@@ -645,7 +652,7 @@ __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_ke
 template <int HD, int STAGES, int NT, bool SELFTEST = false>
 __global__ void __launch_bounds__(NTHREADS, NT == 1 ? 3 : 2) attention_decode_shares_kernel(const __grid_constant__ CUtensorMap map_k,
                                                                                          const __grid_constant__ CUtensorMap map_v,
-                                                                                         const DecodeParams p) {
+                                                                                         const ShareParams p) {
     using C = Consumer<HD, NT>;
     constexpr unsigned STAGE_BYTES = 2 * C::KV_BYTES;
     constexpr int NROWS = 8 * NT;
@@ -1007,7 +1014,7 @@ Plan make_plan(int n_seqs, int n_heads, int n_kv_heads, int head_dim, int max_q_
 
 // A self-test of the waits: shares of 148 CTAs (a first stage that is not handed back stops each third of them once it
 // has more tiles than stages), heads of 64, up to 8 rows.
-int launch_selftest(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, cudaStream_t s) {
+int launch_selftest(const CUtensorMap& mk, const CUtensorMap& mv, const ShareParams& p, cudaStream_t s) {
     auto kern = attention_decode_shares_kernel<64, stages_for<64>(), 1, true>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_shares<64>(8));
     if (e != cudaSuccess) return (int)e;
@@ -1015,7 +1022,7 @@ int launch_selftest(const CUtensorMap& mk, const CUtensorMap& mv, const DecodePa
 }
 
 template <int HD, int NT>
-int launch(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, const Plan& pl, cudaStream_t s) {
+int launch(const CUtensorMap& mk, const CUtensorMap& mv, const ShareParams& p, const Plan& pl, cudaStream_t s) {
     if (pl.shares > 0)          // (shares_per_sm has raised the limit on shared memory)
         return (int)tl_launch(attention_decode_shares_kernel<HD, stages_for<HD>(), NT>, dim3(pl.shares), dim3(NTHREADS), smem_shares<HD>(p.rows), s, mk, mv, p);
     constexpr size_t smem = smem_for<HD>();
@@ -1026,7 +1033,7 @@ int launch(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeParams& p, 
         if (e != cudaSuccess) return (int)e;
         raised = true;
     }
-    return (int)tl_launch(kern, dim3(pl.n_splits, p.units, p.n_seqs), dim3(NTHREADS), smem, s, mk, mv, p);
+    return (int)tl_launch(kern, dim3(pl.n_splits, p.units, p.n_seqs), dim3(NTHREADS), smem, s, mk, mv, (const DecodeParams&)p);
 }
 
 }  // namespace
@@ -1078,7 +1085,7 @@ static int attention_decode(const void* q, const void* k_pages, const void* v_pa
     if (pl.shares > 0 && counters == nullptr) return TL_BAD_SIZE;
     if (n_seqs > 65535 || (long long)n_kv_heads * pl.n_gchunks > 65535) return TL_BAD_SIZE;
 
-    DecodeParams p;
+    ShareParams p;
     p.q = (const __nv_bfloat16*)q; p.out = (__nv_bfloat16*)out;
     p.block_table = block_table; p.q_start = q_start; p.kv_len = kv_len; p.table_stride = table_stride;
     p.status = status; p.counters = counters;
