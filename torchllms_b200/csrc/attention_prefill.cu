@@ -670,15 +670,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_prefill_kernel(const __
 //                    registers, and issued a fifth slower); warp 15 brings V.  Pages are looked up a tile ahead.
 // Scores, probabilities and accumulators have tensor memory of their own, so that the scores of a tile's next 128
 // keys are made while the exponentials of these are taken; where they shared it the chain scores, softmax, both
-// products, scores (3,460 cycles for 128 x 128 pairs, of which the softmax is 2,025) set the pace of a tile, and the
-// other tile only filled its gaps (tensor pipe 47 % active).  With head_dim 128 there is room for one score buffer, which the tiles use
+// products, scores set the pace of a tile, and the other tile only filled its gaps (148 CTAs of 49 key tiles, head_dim 128: tensor
+// pipe 47 % active over 219,458 cycles).  With head_dim 128 there is room for one score buffer, which the tiles use
 // in turn; it is free as soon as the scores are in registers.  One warp issues both tiles' products with V, in
 // order: that keeps the tiles half a period apart (a warp to a tile let them fall into step, 222 us where this takes 168,
-// and an explicit turn for the exponentials, 171).  What bounds it now: the way of the score buffer between the tiles (read, free,
-// scores, seen: 1,400 cycles of a period of 3,000) and the exponential unit (2,048).
+// and an explicit turn for the exponentials, 171).  What bounds it now: the way of the score buffer between the tiles (read, seen to be
+// free, scores made, seen to be there), twice a pair of query tiles, and the exponential unit (2,048 cycles a pair).
 //     2,000 tokens behind 5,001, 24 / 8 heads of 128, pages of 16:  200 -> 168 us
 //     a prompt of 2,048, 32 / 8 heads of 128:                      51.8 -> 46.5
 //     two portions of 611, 32 / 8 heads of 64:                     24.4 -> 22.5
+//     a prompt of 96 or 128, one query tile and one key tile:      6.1 -> 6.5 (heads of 64), 7.1 -> 7.4 (of 128)
 // Barriers beside those of the kernel above: s_free (softmax -> scores: the buffer has been read), alpha_ready
 // (softmax -> correction: factors are in shared memory; not before the product of the key tile before is over, when
 // the correction has taken the word of that tile), o_ready (correction -> issuer: the accumulator may take the
