@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_prefill_kernel(const __
 // Scores, probabilities and accumulators have tensor memory of their own, so that the scores of a tile's next 128
 // keys are made while the exponentials of these are taken; where they shared it the chain scores, softmax, both
 // products, scores set the pace of a tile, and the other tile only filled its gaps (148 CTAs of 49 key tiles, head_dim 128: tensor
-// pipe 47 % active over 219,458 cycles).  With head_dim 128 there is room for one score buffer, which the tiles use
+// pipe 47 % of 218,700 cycles; now 55 % of 186,400).  With head_dim 128 there is room for one score buffer, which the tiles use
 // in turn; it is free as soon as the scores are in registers.  One warp issues both tiles' products with V, in
 // order: that keeps the tiles half a period apart (a warp to a tile let them fall into step, 222 us where this takes 168,
 // and an explicit turn for the exponentials, 171).  What bounds it now: the way of the score buffer between the tiles (read, seen to be
